@@ -58,6 +58,26 @@ GKR_HD uint32_t mac_lazy(uint32_t acc, uint32_t a, uint32_t b) {
 // (SumcheckMultiLinearProdHelper::receive_challenge, sumcheck_helper.hpp:115,124-125).
 GKR_HD uint32_t fold(uint32_t a, uint32_t b, uint32_t r) { return add(a, mul(sub(b, a), r)); }
 
+// The fold at challenge r as a weighted sum: lerp(a, b, lerp_at(r)) = a (1 - r) + b r, the same
+// field element as fold(a, b, r).  The weights are kept doubled, 2 (p + 1 - r) and 2 r (2 and 0
+// for r = 0), so that t = a c0 + b c1 <= (p - 1) 2^32 holds twice the sum S: t >> 32 is S >> 31,
+// at most p - 1, and (uint32_t)t >> 1 is S mod 2^31, at most p.  Two wide multiply-adds, one
+// shift-and-add and one conditional subtraction, where fold takes three field operations.
+struct Lerp {
+    uint32_t c0, c1;
+};
+GKR_HD Lerp lerp_at(uint32_t r) {
+    Lerp c;
+    c.c1 = r + r;
+    c.c0 = r ? 0u - c.c1 : 2u;
+    return c;
+}
+GKR_HD uint32_t lerp(uint32_t a, uint32_t b, const Lerp& c) {
+    const uint64_t t = (uint64_t)a * c.c0 + (uint64_t)b * c.c1;
+    const uint32_t s = (uint32_t)(t >> 32) + ((uint32_t)t >> 1);
+    return umin(s, s - P);
+}
+
 // Evaluation at 2 of the degree-2 round polynomial from p0 = h(0), p1 = h(1) and
 // p2raw = sum (f0+f1)(g0+g1) = 4 h(1/2): 6 p1 + 3 p0 - 2 p2raw (sumcheck_helper.hpp:100).
 GKR_HD uint32_t eval_at_two(uint32_t p0, uint32_t p1, uint32_t p2raw) {

@@ -65,16 +65,19 @@ class Transcript {
         has_pre_ = true;
     }
 
-    // Appends three messages of n bytes, each followed by a challenge, exactly as three
-    // append+challenge steps would when nothing else is pending; the three SHA-256 run
-    // interleaved.  Returns false (and does nothing) when bytes are pending.
-    bool append_challenge3(const uint8_t* const msgs[3], uint64_t n, uint32_t out[3]) {
-        if (s_.len != s_.hash_start || has_pre_ || s_.hash != kFsSha256) return false;
-        const uint8_t* at[3];
-        for (int m = 0; m < 3; m++) {
-            at[m] = buf_ + s_.len;
-            append(msgs[m], n);
+    // Appends `count` messages of n bytes, already written one after another at tail(), each
+    // followed by its challenge.  Three with nothing else pending are hashed interleaved (the
+    // SHA-256 rounds of one message depend on each other).
+    void challenge_each(uint64_t n, int count, uint32_t* out) {
+        if (count != 3 || s_.len != s_.hash_start || has_pre_ || s_.hash != kFsSha256) {
+            for (int m = 0; m < count; m++) {
+                appended(n);
+                out[m] = challenge();
+            }
+            return;
         }
+        const uint8_t* at[3] = {buf_ + s_.len, buf_ + s_.len + n, buf_ + s_.len + 2 * n};
+        s_.len += 3 * n;
         uint8_t d[3][32];
         sha256_x3(at, n, d);
         s_.hash_start = s_.len;
@@ -84,7 +87,6 @@ class Transcript {
             memcpy(&x, d[m], 4);
             out[m] = m31::from_u32(x);
         }
-        return true;
     }
 
     uint32_t challenge() {

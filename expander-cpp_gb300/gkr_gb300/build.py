@@ -1,6 +1,6 @@
 """Builds libgkrgpu.so in-tree from csrc/ (nvcc for sm_103a, host C++ with the system compiler).
 
-Three translation units are compiled in parallel and linked with nvcc; the CUDA runtime
+The translation units are compiled in parallel and linked with nvcc; the CUDA runtime
 is linked statically so the library only needs the driver at run time.
 """
 import os
@@ -22,7 +22,7 @@ if platform.machine() in ("aarch64", "arm64"):
     # ARMv8 SHA-2 instructions for the transcript hash (all Neoverse cores have them).
     CXXFLAGS.append("-march=armv8.2-a+crypto")
 
-SOURCES = ["kernels.cu", "prover.cu", "sha256.cpp", "noalloc.cu", "bn254.cu", "circuit2.cpp", "keccak.cpp"]
+SOURCES = ["kernels.cu", "phase.cu", "prover.cu", "sha256.cpp", "noalloc.cu", "bn254.cu", "circuit2.cpp", "keccak.cpp"]
 HEADERS = ["kernels.cuh", "m31.cuh", "sha256.hpp", "transcript.hpp", "bn254.cuh", "bn254_prover.cuh", "fr_host.hpp",
            "verifier.cuh", "keccak.hpp"]
 

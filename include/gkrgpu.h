@@ -257,17 +257,17 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
 int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t nb_vars, uint32_t n_copies,
                                     const uint32_t* r, int n_points, uint32_t* d_out, void* stream);
 
-/* Persistent phase tails.  When the tables of a phase's last rounds are small, those rounds
- * run in one launch (k_tail) that waits on the device for each round's challenges, which
+/* Persistent phases.  When the tables of a phase's last rounds (of all its rounds, for a small
+ * layer) are small, those rounds run in one launch (k_phase) that waits on the device for each round's challenges, which
  * the host writes into host-mapped memory after hashing the round's evaluations, instead of
  * one kernel launch per round.  On by default; gkrgpu_set_round_tail(ctx, 0) runs every
  * round as its own launch (the proof bytes are the same).  A context created under a CUDA
- * injection tool (CUDA_INJECTION64_PATH set, as profilers do) starts with the tails off:
+ * injection tool (CUDA_INJECTION64_PATH set, as profilers do) starts with them off:
  * such tools may run each kernel to completion before the launching thread goes on, and a
- * tail waits for that thread.  No counterpart in the reference, whose sumcheck runs on the
+ * phase waits for that thread.  No counterpart in the reference, whose sumcheck runs on the
  * CPU (sumcheck.hpp:72-97). */
 int gkrgpu_set_round_tail(gkrgpu_ctx* ctx, int enabled);
-/* Checks the bounded device wait of the phase tails: runs a two-round tail whose second
+/* Checks the bounded device wait of the persistent phases: runs a two-round one whose second
  * challenge is never written, with a wait limit of timeout_us, and reports whether the wait
  * expired and the kernel returned (expired = 1) and how many rounds it published (1).  The
  * context stays usable.  A diagnostic with no counterpart in the reference. */

@@ -1,0 +1,42 @@
+"""GPU tests of the persistent sumcheck phases at the edges of their rule and tiles: layers of
+exactly, just over and far over the rows a CTA takes, one-row-pair layers, copy counts that
+leave part of the last CTA idle (516 = 4 * 129 at two quads a CTA), that need wide CTAs (4096)
+and that are beyond the widest (20000, every round launched alone).  The proof bytes equal the
+oracle's and those with the phases off (exact arithmetic: tolerance zero)."""
+import numpy as np
+import pytest
+
+from gkr_gb300 import circuit as gc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("seed,widths,n,p_mul", [
+    (601, [12, 11, 12], 16, 0.6), (602, [13, 12], 16, 0.6), (603, [14, 9], 8, 0.5), (604, [1, 1, 1, 1], 4, 0.5),
+    (605, [2, 1, 3, 0], 20, 0.5), (606, [11, 10], 516, 0.6), (607, [12, 5], 268, 1.0), (608, [9, 10, 7], 1024, 0.0),
+    (609, [6, 7], 4096, 0.5), (610, [5, 4], 20000, 0.5), (611, [3, 9, 3], 28, 1.0),
+])
+def test_phases_give_the_oracle_proof(ctx, oracle, seed, widths, n, p_mul):
+    circ = gc.random_circuit(seed, widths, p_mul=p_mul)
+    w = gc.random_witness(seed, circ.log_input_size, n)
+    dc = ctx.load(circ)
+    cv, proof = ctx.prove(dc, w)
+    try:
+        ctx.set_round_tail(False)
+        assert ctx.prove(dc, w)[1] == proof
+    finally:
+        ctx.set_round_tail(True)
+    ocv, op = oracle.prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
+
+
+def test_many_gates_on_one_row(ctx, oracle):
+    # every mul gate's first input is row 0: one thread sums 2^9 gates of full-range weights
+    st = gc.Stream(612)
+    layer = gc.random_layer(st, 9, 9, p_mul=1.0)
+    layer.mul[:, 1] = 0
+    layer.mul[:, 3] = gc.P - 1
+    circ = gc.Circuit([layer])
+    w = np.full((512, 8), gc.P - 1, np.uint32)
+    dc = ctx.load(circ)
+    assert ctx.prove(dc, w)[1] == oracle.prove(circ, w)[1]
