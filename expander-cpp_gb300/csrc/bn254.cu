@@ -112,73 +112,106 @@ __device__ __forceinline__ Fr sub(const Fr& a, const Fr& b) {
     return o;
 }
 
-// One CIOS step (Koc, Acar, Kaliski 1996): t += a * bi, then t += m * r with
-// m = t0 * (-r^-1) mod 2^32, which clears t0.  t0..t9 are %0..%9, a is %10..%17, bi %18.
-#define GKRGPU_BN_CIOS_STEP                      \
-    "{\n\t.reg .u32 m;\n\t"                      \
-    "mad.lo.cc.u32 %0, %10, %18, %0;\n\t"        \
-    "madc.lo.cc.u32 %1, %11, %18, %1;\n\t"       \
-    "madc.lo.cc.u32 %2, %12, %18, %2;\n\t"       \
-    "madc.lo.cc.u32 %3, %13, %18, %3;\n\t"       \
-    "madc.lo.cc.u32 %4, %14, %18, %4;\n\t"       \
-    "madc.lo.cc.u32 %5, %15, %18, %5;\n\t"       \
-    "madc.lo.cc.u32 %6, %16, %18, %6;\n\t"       \
-    "madc.lo.cc.u32 %7, %17, %18, %7;\n\t"       \
-    "addc.cc.u32 %8, %8, 0;\n\t"                 \
-    "addc.u32 %9, 0, 0;\n\t"                     \
-    "mad.hi.cc.u32 %1, %10, %18, %1;\n\t"        \
-    "madc.hi.cc.u32 %2, %11, %18, %2;\n\t"       \
-    "madc.hi.cc.u32 %3, %12, %18, %3;\n\t"       \
-    "madc.hi.cc.u32 %4, %13, %18, %4;\n\t"       \
-    "madc.hi.cc.u32 %5, %14, %18, %5;\n\t"       \
-    "madc.hi.cc.u32 %6, %15, %18, %6;\n\t"       \
-    "madc.hi.cc.u32 %7, %16, %18, %7;\n\t"       \
-    "madc.hi.cc.u32 %8, %17, %18, %8;\n\t"       \
-    "addc.u32 %9, %9, 0;\n\t"                    \
-    "mul.lo.u32 m, %0, 0xefffffff;\n\t"          \
-    "mad.lo.cc.u32 %0, m, 0xf0000001, %0;\n\t"   \
-    "madc.lo.cc.u32 %1, m, 0x43e1f593, %1;\n\t"  \
-    "madc.lo.cc.u32 %2, m, 0x79b97091, %2;\n\t"  \
-    "madc.lo.cc.u32 %3, m, 0x2833e848, %3;\n\t"  \
-    "madc.lo.cc.u32 %4, m, 0x8181585d, %4;\n\t"  \
-    "madc.lo.cc.u32 %5, m, 0xb85045b6, %5;\n\t"  \
-    "madc.lo.cc.u32 %6, m, 0xe131a029, %6;\n\t"  \
-    "madc.lo.cc.u32 %7, m, 0x30644e72, %7;\n\t"  \
-    "addc.cc.u32 %8, %8, 0;\n\t"                 \
-    "addc.u32 %9, %9, 0;\n\t"                    \
-    "mad.hi.cc.u32 %1, m, 0xf0000001, %1;\n\t"   \
-    "madc.hi.cc.u32 %2, m, 0x43e1f593, %2;\n\t"  \
-    "madc.hi.cc.u32 %3, m, 0x79b97091, %3;\n\t"  \
-    "madc.hi.cc.u32 %4, m, 0x2833e848, %4;\n\t"  \
-    "madc.hi.cc.u32 %5, m, 0x8181585d, %5;\n\t"  \
-    "madc.hi.cc.u32 %6, m, 0xb85045b6, %6;\n\t"  \
-    "madc.hi.cc.u32 %7, m, 0xe131a029, %7;\n\t"  \
-    "madc.hi.cc.u32 %8, m, 0x30644e72, %8;\n\t"  \
-    "addc.u32 %9, %9, 0;\n\t"                    \
-    "}"
-
-// Montgomery product a * b * 2^-256 mod r (inputs < r, output < r).
+// Montgomery product a * b * 2^-256 mod r (inputs < r, output < r): CIOS (Koc, Acar, Kaliski
+// 1996) with the running sum T = x + 2^32 y in two accumulators of eight words, x collecting
+// the products of a's and r's even words and y those of the odd ones.  Every product's low and
+// high word then land on neighbouring words of one accumulator, a 32 x 32 + 64 -> 64-bit
+// multiply-add with carry, where a chain over all low words and another over all high words
+// needs two multiplications a product, the high one at half the rate (30.9 per clock and SM
+// against 61.6; the 64-bit form runs at about the low word's rate).  T < 2^288 as r < 2^254, so
+// x carries out of its top word into y's and y never does.
+// A step: T += a * bi, then T += m * r with m = T * (-r^-1) mod 2^32, which clears x0, then
+// T /= 2^32: y becomes the accumulator at position 0 (its word 0 takes x1, whose carry enters
+// the odd chain of the next step) and x from word 2 on the one at position 1.
 __device__ __forceinline__ Fr mul(const Fr& a, const Fr& b) {
-    uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0, t9 = 0;
+    uint32_t x[8], y[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        asm(GKRGPU_BN_CIOS_STEP
-            : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8), "+r"(t9)
-            : "r"(a.l[0]), "r"(a.l[1]), "r"(a.l[2]), "r"(a.l[3]), "r"(a.l[4]), "r"(a.l[5]), "r"(a.l[6]),
-              "r"(a.l[7]), "r"(b.l[i]));
-        // divide by 2^32: t0 is zero
-        t0 = t1; t1 = t2; t2 = t3; t3 = t4; t4 = t5; t5 = t6; t6 = t7; t7 = t8; t8 = t9; t9 = 0;
+        const uint32_t bi = b.l[i];
+        if (i == 0) {
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                const uint64_t e = (uint64_t)a.l[k] * bi, o = (uint64_t)a.l[k + 1] * bi;
+                x[k] = (uint32_t)e;
+                x[k + 1] = (uint32_t)(e >> 32);
+                y[k] = (uint32_t)o;
+                y[k + 1] = (uint32_t)(o >> 32);
+            }
+        } else {
+            uint32_t z6, z7;
+            // y0 += x1, then the odd products onto x2.. (the next y)
+            asm("add.cc.u32 %0, %0, %9;\n\t"
+                "madc.lo.cc.u32 %1, %10, %14, %1;\n\t"
+                "madc.hi.cc.u32 %2, %10, %14, %2;\n\t"
+                "madc.lo.cc.u32 %3, %11, %14, %3;\n\t"
+                "madc.hi.cc.u32 %4, %11, %14, %4;\n\t"
+                "madc.lo.cc.u32 %5, %12, %14, %5;\n\t"
+                "madc.hi.cc.u32 %6, %12, %14, %6;\n\t"
+                "madc.lo.cc.u32 %7, %13, %14, 0;\n\t"
+                "madc.hi.u32 %8, %13, %14, 0;"
+                : "+r"(y[0]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "=&r"(z6), "=&r"(z7)
+                : "r"(x[1]), "r"(a.l[1]), "r"(a.l[3]), "r"(a.l[5]), "r"(a.l[7]), "r"(bi));
+            const uint32_t z[8] = {x[2], x[3], x[4], x[5], x[6], x[7], z6, z7};
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                x[k] = y[k];
+                y[k] = z[k];
+            }
+            // the even products onto x
+            asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+                "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+                "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+                "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+                "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+                "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+                "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+                "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+                "addc.u32 %8, %8, 0;"
+                : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(y[7])
+                : "r"(a.l[0]), "r"(a.l[2]), "r"(a.l[4]), "r"(a.l[6]), "r"(bi));
+        }
+        const uint32_t m = x[0] * 0xefffffffu;
+        asm("mad.lo.cc.u32 %0, %8, 0x43e1f593, %0;\n\t"
+            "madc.hi.cc.u32 %1, %8, 0x43e1f593, %1;\n\t"
+            "madc.lo.cc.u32 %2, %8, 0x2833e848, %2;\n\t"
+            "madc.hi.cc.u32 %3, %8, 0x2833e848, %3;\n\t"
+            "madc.lo.cc.u32 %4, %8, 0xb85045b6, %4;\n\t"
+            "madc.hi.cc.u32 %5, %8, 0xb85045b6, %5;\n\t"
+            "madc.lo.cc.u32 %6, %8, 0x30644e72, %6;\n\t"
+            "madc.hi.u32 %7, %8, 0x30644e72, %7;"
+            : "+r"(y[0]), "+r"(y[1]), "+r"(y[2]), "+r"(y[3]), "+r"(y[4]), "+r"(y[5]), "+r"(y[6]), "+r"(y[7])
+            : "r"(m));
+        asm("mad.lo.cc.u32 %0, %9, 0xf0000001, %0;\n\t"
+            "madc.hi.cc.u32 %1, %9, 0xf0000001, %1;\n\t"
+            "madc.lo.cc.u32 %2, %9, 0x79b97091, %2;\n\t"
+            "madc.hi.cc.u32 %3, %9, 0x79b97091, %3;\n\t"
+            "madc.lo.cc.u32 %4, %9, 0x8181585d, %4;\n\t"
+            "madc.hi.cc.u32 %5, %9, 0x8181585d, %5;\n\t"
+            "madc.lo.cc.u32 %6, %9, 0xe131a029, %6;\n\t"
+            "madc.hi.cc.u32 %7, %9, 0xe131a029, %7;\n\t"
+            "addc.u32 %8, %8, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(y[7])
+            : "r"(m));
     }
-    // t < 2r < 2^255, so t8 is 0: one conditional subtraction of r
-    const uint32_t t[8] = {t0, t1, t2, t3, t4, t5, t6, t7};
-    uint32_t d[8];
+    // T / 2^32 < 2r < 2^255: one conditional subtraction of r
+    uint32_t t[8], d[8];
+    asm("add.cc.u32 %0, %8, %15;\n\t"
+        "addc.cc.u32 %1, %9, %16;\n\t"
+        "addc.cc.u32 %2, %10, %17;\n\t"
+        "addc.cc.u32 %3, %11, %18;\n\t"
+        "addc.cc.u32 %4, %12, %19;\n\t"
+        "addc.cc.u32 %5, %13, %20;\n\t"
+        "addc.cc.u32 %6, %14, %21;\n\t"
+        "addc.u32 %7, %22, 0;"
+        : "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]), "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]), "=&r"(t[7])
+        : "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(y[0]), "r"(y[1]), "r"(y[2]),
+          "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
     const bool below = minus_r(t, d) != 0u;
     Fr o;
 #pragma unroll
     for (int i = 0; i < 8; i++) o.l[i] = below ? t[i] : d[i];
     return o;
 }
-#undef GKRGPU_BN_CIOS_STEP
 __device__ __forceinline__ Fr from_mont(const Fr& a) {
     Fr u = zero();
     u.l[0] = 1u;
