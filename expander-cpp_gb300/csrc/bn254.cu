@@ -4,6 +4,8 @@
 // 8 x 32-bit limbs (CIOS as PTX multiply-add carry chains).
 #include "bn254.cuh"
 
+#include <atomic>
+
 namespace gkrgpu {
 namespace bn {
 
@@ -827,6 +829,227 @@ __global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals,
     reduce_bn<1>(acc, g, t.active, red, CopyFinBn{out, g.N});
 }
 
+// ---------------------------------------------------------------- persistent phases
+// The rounds of a phase on small tables in one launch (the M31 k_phase of phase.cu, whose
+// notes on the host traffic hold here): a round launched by itself takes 18-27 us on tables
+// of a few hundred rows, mostly the launch, the reduction across CTAs and a chain of dependent
+// 256-bit products in one finishing thread.  One CTA owns one copy and all its rows (a row's
+// element is one 32-byte sector, so narrower is no loss); three threads finish the three
+// evaluations.  All three sums are taken directly: a third product per pair is shorter than
+// the claim's chain of products.
+constexpr uint32_t kPhaseBlock = 256;
+constexpr uint32_t kPhaseWarps = kPhaseBlock / 32;
+constexpr uint32_t kSmemRowsBn = 128;  // rows of a per-copy table kept in shared memory
+constexpr uint32_t kSpinsBn = 256;     // mailbox polls before sleeping between them
+
+__device__ __forceinline__ void st_digits(uint32_t* out, const Fr& v, uint32_t parity) {
+    uint32_t d[12];
+    const uint32_t top = parity << 31;
+    d[0] = (v.l[0] & 0x7fffffffu) | top;
+#pragma unroll
+    for (int k = 1; k < 8; k++) d[k] = (__funnelshift_l(v.l[k - 1], v.l[k], k) & 0x7fffffffu) | top;
+    d[8] = (v.l[7] >> 24) | top;
+    d[9] = d[10] = d[11] = top;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(out + 4 * k), "r"(d[4 * k]),
+                     "r"(d[4 * k + 1]), "r"(d[4 * k + 2]), "r"(d[4 * k + 3])
+                     : "memory");
+}
+// Reads a mailbox slot: 0 not written yet, 1 the challenge is in *r, 2 abort.
+__device__ __forceinline__ int ld_challenge(const uint32_t* box, Fr* r) {
+    uint32_t d[12];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(d[4 * k]), "=r"(d[4 * k + 1]), "=r"(d[4 * k + 2]), "=r"(d[4 * k + 3])
+                     : "l"(box + 4 * k)
+                     : "memory");
+    uint32_t ok = d[0];
+#pragma unroll
+    for (int k = 1; k < 9; k++) ok &= d[k];
+    if (!(ok >> 31)) return d[11] ? 2 : 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) d[k] &= 0x7fffffffu;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r->l[i] = (d[i] >> i) | (d[i + 1] << (31 - i));
+    return 1;
+}
+// Element of a table this kernel also writes (no read-only path); row r at p[r * stride].
+struct RowsBn {
+    Fr* p;
+    size_t stride;
+    __device__ __forceinline__ Fr get(uint32_t r) const {
+        const uint4* q = reinterpret_cast<const uint4*>(p + (size_t)r * stride);
+        const uint4 a = q[0], b = q[1];
+        Fr f;
+        f.l[0] = a.x; f.l[1] = a.y; f.l[2] = a.z; f.l[3] = a.w;
+        f.l[4] = b.x; f.l[5] = b.y; f.l[6] = b.z; f.l[7] = b.w;
+        return f;
+    }
+    __device__ __forceinline__ void set(uint32_t r, const Fr& f) const { sts(p, (size_t)r * stride, f); }
+};
+
+template <bool LANE_HG>
+__global__ void __launch_bounds__(kPhaseBlock, 2) k_phase(PhaseArgsBn a) {
+    extern __shared__ uint4 psm_raw[];
+    __shared__ Fr rch, part[kPhaseWarps][3];
+    __shared__ int stop;
+    const uint32_t tid = threadIdx.x, lane = blockIdx.x, warp = tid >> 5;
+    const size_t gs = a.N;
+    constexpr uint32_t kTabs = LANE_HG ? 2 : 1;
+    const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);  // the first round that folds leaves S1 rows
+    Fr* const psm = reinterpret_cast<Fr*>(psm_raw);              // two buffers of f (and hg)
+    Fr* const sbuf = psm + 2 * kTabs * kSmemRowsBn;              // phase two's scalar tables, S1 and S1 / 2
+    auto mem = [&](uint32_t* b) { return RowsBn{reinterpret_cast<Fr*>(b) + lane, gs}; };
+    // the table round k leaves: which = 0 f, 1 hg
+    auto table = [&](uint32_t k, uint32_t which) -> RowsBn {
+        if ((1u << (a.n - k)) <= kSmemRowsBn) return RowsBn{psm + ((k & 1) * kTabs + which) * kSmemRowsBn, 1};
+        return mem(which == 0 ? ((k & 1) ? a.fA : a.fB) : ((k & 1) ? a.hA : a.hB));
+    };
+    Fr xv = zero();
+    if (!LANE_HG && tid < 3) xv = ldf_cv(a.vx, a.N, lane);
+    if (tid == 0) stop = 0;
+
+    for (uint32_t k = a.k0; k < a.n; k++) {
+        if (tid == 0) {
+            if (k == a.k0) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) rch.l[i] = a.r_first[i];
+            } else {
+                const uint32_t* box = a.mbox + kDigitWords * (k - 1);
+                uint64_t t0 = 0;
+                for (uint32_t it = 0;; it++) {
+                    Fr r;
+                    const int got = ld_challenge(box, &r);
+                    if (got == 1) rch = r;
+                    if (got == 2) stop = 1;
+                    if (got) break;
+                    if (it < kSpinsBn) continue;
+                    uint64_t now;
+                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+                    if (t0 == 0) t0 = now;
+                    if (now - t0 > a.wait_ns) {
+                        *reinterpret_cast<volatile unsigned int*>(a.err) = 1u;
+                        stop = 1;
+                        break;
+                    }
+                    __nanosleep(100);
+                }
+            }
+        }
+        __syncthreads();  // the challenge, and the previous round's tables, are visible
+        if (stop) return;
+        const uint32_t npairs = 1u << (a.n - k - 1);
+        const Fr r = rch;
+        Fr acc[3] = {zero(), zero(), zero()};
+        RowsBn fs = mem(const_cast<uint32_t*>(a.v)), hs = {}, fd = {}, hd = {};
+        const Fr* ssrc = a.s;
+        Fr* sdst = nullptr;
+        if (k > 0) {
+            if (k == a.k0) fs = mem((k & 1) ? a.fB : a.fA);
+            else if (k > 1) fs = table(k - 1, 0);
+            fd = table(k, 0);
+            if (LANE_HG) {
+                hs = k == a.k0 ? mem((k & 1) ? a.hB : a.hA) : k == 1 ? mem(a.h0) : table(k - 1, 1);
+                hd = table(k, 1);
+            } else {
+                const bool odd = (k - kf) & 1;
+                if (k > kf) ssrc = odd ? sbuf : sbuf + S1;
+                sdst = odd ? sbuf + S1 : sbuf;
+            }
+        }
+        for (uint32_t i = tid; i < npairs; i += kPhaseBlock) {
+            Fr f0, f1, h0, h1;
+            if (k == 0) {
+                f0 = ldf(a.v, 2 * i, a.N, lane);
+                f1 = ldf(a.v, 2 * i + 1, a.N, lane);
+                if (LANE_HG) {
+#pragma unroll 1
+                    for (int s = 0; s < 2; s++) {
+                        const uint32_t x = 2 * i + s;
+                        Fr h = lds(a.a, x);
+                        const uint32_t g0 = __ldg(a.mx_off + x), g1 = __ldg(a.mx_off + x + 1);
+                        for (uint32_t g = g0; g < g1; g++)
+                            h = add(h, mul(ldf(a.v, __ldg(&a.mx_g[g].x), a.N, lane), lds(a.w, g)));
+                        mem(a.h0).set(x, h);
+                        if (s == 0) h0 = h;
+                        else h1 = h;
+                    }
+                } else {
+                    h0 = lds(a.s, 2 * i);
+                    h1 = lds(a.s, 2 * i + 1);
+                }
+            } else {
+                // one copy of the fold's product for the two rows: fewer instructions to fetch
+#pragma unroll 1
+                for (int s = 0; s < 2; s++) {
+                    const uint32_t x = 4 * i + 2 * s, o = 2 * i + s;
+                    const Fr f = fold(fs.get(x), fs.get(x + 1), r);
+                    Fr h;
+                    if (LANE_HG) {
+                        h = fold(hs.get(x), hs.get(x + 1), r);
+                        hd.set(o, h);
+                    } else {
+                        const RowsBn sc{const_cast<Fr*>(ssrc), 1};
+                        h = fold(sc.get(x), sc.get(x + 1), r);
+                        sts(sdst, o, h);
+                    }
+                    fd.set(o, f);
+                    if (s == 0) {
+                        f0 = f;
+                        h0 = h;
+                    } else {
+                        f1 = f;
+                        h1 = h;
+                    }
+                }
+            }
+            accum(acc, f0, f1, h0, h1);
+        }
+        // sums over the warps that had pairs
+        const uint32_t nw = npairs >= kPhaseBlock ? kPhaseWarps : (npairs + 31) / 32;
+        if (warp < nw) {
+            uint32_t span = npairs < 32 ? npairs : 32;  // lanes with a pair (a power of two)
+            for (uint32_t off = span / 2; off > 0; off >>= 1)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    Fr o;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) o.l[e] = __shfl_xor_sync(0xffffffffu, acc[c].l[e], off);
+                    acc[c] = add(acc[c], o);
+                }
+            if ((tid & 31) == 0)
+#pragma unroll
+                for (int c = 0; c < 3; c++) part[warp][c] = acc[c];
+        }
+        __syncthreads();
+        const uint32_t par = (a.parity ^ (k - a.k0)) & 1u;
+        if (tid < 3) {
+            Fr v = part[0][tid];
+            for (uint32_t w = 1; w < nw; w++) v = add(v, part[w][tid]);
+            // evaluation 2 from the three sums: 6 p1 + 3 p0 - 2 p2raw
+            Fr p0, p1;
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                p0.l[e] = __shfl_sync(0x7u, v.l[e], 0);
+                p1.l[e] = __shfl_sync(0x7u, v.l[e], 1);
+            }
+            if (tid == 2) {
+                const Fr d = add(p1, p1);
+                v = sub(add(add(add(d, d), d), add(add(p0, p0), p0)), add(v, v));
+            }
+            if (!LANE_HG) v = mul(v, xv);
+            st_digits(a.evals_out + ((size_t)tid * a.N + lane) * kDigitWords, from_mont(v), par);
+        } else if (k + 1 == a.n && tid >= 32 && tid < 34) {
+            // rows 0 and 1 of the last folded f table (the layer input when it has no fold)
+            const uint32_t row = tid - 32;
+            const Fr v = k == 0 ? ldf(a.v, row, a.N, lane) : fd.get(row);
+            st_digits(a.rows_out + ((size_t)row * a.N + lane) * kDigitWords, v, a.rows_parity);
+        }
+    }
+}
+
 uint32_t grid1(uint64_t n) {
     uint64_t b = (n + 255) / 256;
     if (b < 1) b = 1;
@@ -904,6 +1127,29 @@ cudaError_t launch_round(bool lane_hg, bool fold_, const RoundPtrsBn& p, uint64_
     else if (!lane_hg && fold_) k_round<false, true><<<grid, 256, smem, s>>>(p, npairs, vx, g, red, evals_out);
     else if (!lane_hg && !fold_) k_round<false, false><<<grid, 256, smem, s>>>(p, npairs, vx, g, red, evals_out);
     else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s) {
+    if (a.k0 >= a.n || a.n - a.k0 > kMboxRounds || a.N < 1) return cudaErrorInvalidValue;
+    // rows of the first round's source tables; with k0 = 0 the layer input itself
+    if ((1ull << (a.n - (a.k0 ? a.k0 - 1 : 0))) > kPhaseRows) return cudaErrorInvalidValue;
+    if (a.k0 == 0 && (!a.v || (lane_hg && (!a.h0 || !a.mx_off || !a.a || !a.w)))) return cudaErrorInvalidValue;
+    if (!lane_hg && (!a.vx || !a.s)) return cudaErrorInvalidValue;
+    static std::atomic<uint64_t> opted{0};  // one bit per device: shared memory above 48 KiB
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(opted.load(std::memory_order_relaxed) & bit)) {
+        cudaFuncSetAttribute(k_phase<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+        opted.fetch_or(bit);
+    }
+    const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
+    const size_t smem = sizeof(Fr) * (2 * (lane_hg ? 2 : 1) * (size_t)kSmemRowsBn + (lane_hg ? 0 : S1 + S1 / 2));
+    if (lane_hg)
+        k_phase<true><<<a.N, kPhaseBlock, smem, s>>>(a);
+    else
+        k_phase<false><<<a.N, kPhaseBlock, smem, s>>>(a);
     return cudaGetLastError();
 }
 

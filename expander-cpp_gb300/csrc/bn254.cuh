@@ -84,6 +84,34 @@ cudaError_t launch_round(bool lane_hg, bool fold, const RoundPtrsBn& p, uint64_t
                          const GeoBn& g, uint32_t ctas, RedBn red, uint32_t* evals_out, cudaStream_t s);
 cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const Fr* eqc,
                            const Fr* eqrx, Fr* s_out, cudaStream_t s);
+// Persistent sumcheck phase: rounds k0 .. n-1 in one launch, one CTA per copy.  The M31
+// PhaseArgs (kernels.cuh) describes the scheme: round k leaves 2^(n-k) rows in A when k is odd
+// and in B when it is even, or in shared memory; k0 = 0 starts from the layer input v, building
+// hg into h0 in phase one.  A published element is nine 31-bit digits of its 256-bit value in
+// twelve words (nine used), each with the round's parity in bit 31; so is a challenge, in
+// Montgomery form, in the twelve-word mailbox slot of its round (bit 31 set; the last word
+// nonzero: abort).  evals_out: 3 x N elements, canonical; rows_out: 2 x N, Montgomery.
+constexpr uint32_t kDigitWords = 12;
+// Rows of the first round's source tables: a CTA reads all of them.
+constexpr uint32_t kPhaseRows = 2048;
+struct PhaseArgsBn {
+    const uint32_t* v;             // k0 = 0: the layer input
+    uint32_t *fA, *fB, *hA, *hB;   // per-copy tables
+    uint32_t* h0;                  // phase one, k0 = 0: hg of round 0 (2^n rows)
+    const Fr* s;                   // phase two: the scalar table the first round reads
+    const uint32_t* mx_off;        // phase one, k0 = 0
+    const uint4* mx_g;
+    const Fr *a, *w;
+    const uint32_t* vx;            // phase two: N x 8 words, Montgomery form
+    uint32_t r_first[8];           // k0 > 0: challenge of round k0 - 1, Montgomery form
+    uint32_t k0, n, N;
+    uint32_t parity, rows_parity;
+    const uint32_t* mbox;
+    uint32_t *evals_out, *rows_out;
+    unsigned int* err;
+    unsigned long long wait_ns;
+};
+cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s);
 cudaError_t launch_wsum(const uint32_t* vals, uint64_t rows, const Fr* eq, const GeoBn& g, uint32_t ctas, RedBn red,
                         uint32_t* out, cudaStream_t s);
 

@@ -94,6 +94,7 @@ struct BnProver {
         }
     }
     ~BnProver() {
+        c.phase_err = nullptr;
         if (block) cudaFreeAsync(block, c.stream);
     }
 
@@ -108,11 +109,17 @@ struct BnProver {
     // The lane's mapped extra area (words): rows 0..1 of the last table (16N), the claimed
     // values (8N), vx in Montgomery form (8N), the input check flag, and from word 32N + 64
     // the claims of phase one's round 0 (8N).  Small transfers go through it by kernels,
-    // never queueing on the copy engine behind another proof's bulk copies.
+    // never queueing on the copy engine behind another proof's bulk copies.  After the claims:
+    // the persistent phases' challenge mailbox, then what they publish (5N elements of
+    // kDigitWords words: 3N evaluations, 2N rows); their error word is word 32N + 1.
     uint32_t* mapped(bool dev, uint64_t word) const {
         return reinterpret_cast<uint32_t*>(dev ? c.extra_d() : c.extra_h()) + word;
     }
     volatile uint32_t* flag_h() const { return mapped(false, 32ull * N); }
+    volatile uint32_t* err_h() const { return mapped(false, 32ull * N + 1); }
+    uint64_t mbox_word() const { return align_up(40ull * N + 64, 64); }
+    uint64_t phase_word() const { return mbox_word() + bn::kDigitWords * kMboxRounds; }
+    uint64_t mapped_words() const { return phase_word() + 5ull * bn::kDigitWords * N; }
     uint32_t stage(uint32_t* dst, const uint32_t* src, uint64_t words, unsigned int* done) {
         uint32_t incs = 0;
         const uint32_t* srcs[1] = {src};
@@ -131,8 +138,11 @@ struct BnProver {
         block = static_cast<char*>(p);
         ws.plan(block, C, N, sumcheck);
         ck(cudaMemsetAsync(block + ws.zero_off, 0, ws.zero_bytes, c.stream), "cudaMemsetAsync");
-        c.ensure_mapped(3 * rowb(), (40ull * N + 64) * 4);
+        c.ensure_mapped(3 * rowb(), mapped_words() * 4);
         c.resync_done();
+        // no word a persistent phase publishes has its first parity yet
+        memset(mapped(false, phase_word()), 0, 5ull * bn::kDigitWords * N * 4);
+        c.ev_parity = c.rows_parity = 0u;
     }
 
     void layout_values() {
@@ -181,14 +191,87 @@ struct BnProver {
         c.wait_done(groups + more);
     }
 
+    // First round of a phase's persistent part, n if it has none (as the M31 prover's): a CTA a
+    // copy, all of them resident at once.
+    uint32_t phase_start(uint32_t n, uint32_t first) const {
+        if (!X.round_tail || N > 2u * (uint32_t)X.sm_count) return n;
+        uint32_t lg = 0;
+        while ((2u << lg) <= bn::kPhaseRows) lg++;
+        if (n <= lg) return 0;
+        return std::min(n, std::max(first, n + 1 - lg));
+    }
+    // Rounds a.k0 .. a.n-1 of a phase in one launch (the M31 prover's run_phase); false while
+    // other phases hold the device.
+    bool run_phase(Transcript& t, bool lane_hg, bn::PhaseArgsBn a, frh::Fr* rch, bool append_last, uint32_t* last_mont,
+                   uint32_t* last_canon, double bytes) {
+        PhaseSlots slots(X.device, X.sm_count);
+        if (!slots.acquire((int)N)) return false;
+        a.N = N;
+        a.fA = ws.fA;
+        a.fB = ws.fB;
+        a.hA = ws.hgA;
+        a.hB = a.h0 = ws.hg0;  // round 2 writes hB once round 1 has read h0
+        if (a.k0) frh::store(frh::to_mont(rch[a.k0 - 1]), a.r_first);
+        a.parity = c.ev_parity ^ 1u;
+        a.rows_parity = c.rows_parity ^ 1u;
+        a.mbox = mapped(true, mbox_word());
+        a.evals_out = mapped(true, phase_word());
+        a.rows_out = a.evals_out + 3ull * bn::kDigitWords * N;
+        a.err = mapped(true, 32ull * N + 1);
+        a.wait_ns = 10ull * 1000 * 1000 * 1000;
+        volatile uint32_t* mb = mapped(false, mbox_word());
+        for (uint32_t i = 0; i < bn::kDigitWords * kMboxRounds; i++) mb[i] = 0u;
+        *err_h() = 0u;
+        std::atomic_thread_fence(std::memory_order_seq_cst);
+        // a phase left early (an error below) is told to return before its slots are given up
+        struct Abort {
+            volatile uint32_t* mb;
+            ~Abort() {
+                if (!mb) return;
+                for (uint32_t k = 0; k < kMboxRounds; k++) mb[bn::kDigitWords * (k + 1) - 1] = 1u;
+                std::atomic_thread_fence(std::memory_order_seq_cst);
+            }
+        } abort{mb};
+        c.launch(K_BN_PHASE, bytes, [&] { return bn::launch_phase(lane_hg, a, c.stream); });
+        c.phase_err = err_h();
+        const uint32_t* out = mapped(false, phase_word());
+        for (uint32_t k = a.k0; k < a.n; k++) {
+            c.ev_parity = (a.parity ^ (k - a.k0)) & 1u;
+            c.collect_digits(out, 3ull * N, c.ev_parity, t.tail());
+            t.appended(3 * rowb());
+            if (k + 1 < a.n) {
+                rch[k] = t.challenge_bn254();
+                uint32_t w[8], d[9];
+                frh::store(frh::to_mont(rch[k]), w);
+                d[0] = w[0];
+                for (int i = 1; i < 8; i++) d[i] = (w[i - 1] >> (32 - i)) | (w[i] << i);
+                d[8] = w[7] >> 24;
+                for (int i = 0; i < 9; i++) mb[bn::kDigitWords * k + i] = d[i] | 0x80000000u;
+                std::atomic_thread_fence(std::memory_order_release);
+            } else {
+                c.collect_digits(out + 3ull * bn::kDigitWords * N, 2ull * N, a.rows_parity, mapped(false, 0));
+                c.rows_parity = a.rows_parity;
+                last_fold(t, rch, k, append_last, last_mont, last_canon);
+            }
+        }
+        abort.mb = nullptr;
+        c.phase_err = nullptr;
+        return true;
+    }
+
     // One round's transcript step (sumcheck.hpp:74-96 with R = 1): append the 3 rows, take
     // the challenge; in the last round fold rows 0..1 by it into vx / vy (Montgomery copy in
     // `last_mont`, canonical in `last_canon`, appended at once when `append_last`).
     void transcript_round(Transcript& t, frh::Fr* rch, uint32_t k, bool last, bool append_last, uint32_t* last_mont,
                           uint32_t* last_canon) {
         t.append(c.evals_h(), 3 * rowb());
+        if (last)
+            last_fold(t, rch, k, append_last, last_mont, last_canon);
+        else
+            rch[k] = t.challenge_bn254();
+    }
+    void last_fold(Transcript& t, frh::Fr* rch, uint32_t k, bool append_last, uint32_t* last_mont, uint32_t* last_canon) {
         rch[k] = t.challenge_bn254();
-        if (!last) return;
         const frh::Fr rm = frh::to_mont(rch[k]);
         const uint32_t* f0 = mapped(false, 0);
         const uint32_t* f1 = f0 + (size_t)N * 8;
@@ -215,18 +298,15 @@ struct BnProver {
         c.launch(K_BN_EQ, 32.0 * (double)(1ull << nvars), [&] { return bn::launch_eq(out, a, c.stream); });
     }
 
-    void sumcheck_layer(Transcript& t, size_t li, const frh::Fr* rz1, const frh::Fr* rz2, const frh::Fr& alpha,
-                        const frh::Fr& beta, frh::Fr* rx, frh::Fr* ry) {
+    // Phase one's rounds launched one by one, the persistent part from round kt1 (n: none).
+    void phase_one_rounds(Transcript& t, size_t li, uint32_t kt1, const frh::Fr& alpha, const frh::Fr& beta, frh::Fr* rx,
+                          uint32_t* vx_c) {
         const DevLayer& Ly = C.layers[li];
-        const uint32_t n = Ly.nin, m = Ly.nout;
+        const uint32_t n = Ly.nin;
         const uint64_t I = 1ull << n;
         const double rb = (double)rowb();
         uint32_t* v = vals[li];
         uint32_t* vx_m = mapped(false, 24ull * N);
-        std::vector<uint32_t> vx_c((size_t)N * 8), vy_m((size_t)N * 8), vy_c((size_t)N * 8);
-
-        // phase one: eqc = alpha eq(rz1) + beta eq(rz2), gate weights, hg + round 0
-        eq_table(ws.eqc, rz1, rz2, alpha, beta, m);
         // round 0's claims, alpha v(rz1) + beta v(rz2) per copy (sumcheck.hpp:129-132)
         {
             uint32_t* cl = mapped(false, 32ull * N + 64);
@@ -236,21 +316,23 @@ struct BnProver {
                            cl + 8 * i);
             std::atomic_thread_fence(std::memory_order_seq_cst);
         }
-        c.launch(K_BN_WEIGHTS, 80.0 * Ly.nmul + 72.0 * Ly.nadd + 40.0 * I, [&] {
-            return bn::launch_weights(I, Ly.nmul, ws.eqc, Ly.mx_g, Ly.mx_c, Ly.ax_off, Ly.ax_g, Ly.ax_c, ws.a, ws.w,
-                                      c.stream);
-        });
         c.launch(K_BN_HG_ROUND0, rb * (2.0 * I + Ly.nmul) + 52.0 * Ly.nmul + 36.0 * I, [&] {
             return bn::launch_hg_round0(v, I, Ly.mx_off, Ly.mx_g, ws.a, ws.w, ws.hg0, gk[K_BN_HG_ROUND0],
                                         ctas[K_BN_HG_ROUND0], red_mapped(0), mapped(true, 32ull * N + 64),
                                         c.evals_d(), c.stream);
         });
         fetch(groups(K_BN_HG_ROUND0), n == 1 ? v : nullptr);
-        transcript_round(t, rx, 0, n == 1, true, vx_m, vx_c.data());
+        transcript_round(t, rx, 0, n == 1, true, vx_m, vx_c);
 
         const uint32_t* cur_f = v;
         const uint32_t* cur_h = ws.hg0;
         for (uint32_t k = 1; k < n; k++) {
+            if (k == kt1) {
+                bn::PhaseArgsBn ph = {};
+                ph.k0 = k;
+                ph.n = n;
+                if (run_phase(t, true, ph, rx, true, vx_m, vx_c, rb * 6.0 * (double)(I >> k))) break;
+            }
             bn::RoundPtrsBn p;
             memset(&p, 0, sizeof(p));
             p.fsrc = cur_f;
@@ -265,17 +347,19 @@ struct BnProver {
             });
             const bool last = (k == n - 1);
             fetch(groups(K_BN_ROUND_LANE), last ? p.fdst : nullptr);
-            transcript_round(t, rx, k, last, true, vx_m, vx_c.data());
+            transcript_round(t, rx, k, last, true, vx_m, vx_c);
             cur_f = p.fdst;
             cur_h = p.hdst;
         }
+    }
 
-        // phase two: h(y) = vx * s(y)
-        const frh::Fr one = frh::from_u32(1), zero = frh::zero();
-        eq_table(ws.eqrx, rx, nullptr, one, zero, n);
-        c.launch(K_BN_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 32.0 * I + 96.0 * Ly.nmul, [&] {
-            return bn::launch_s_build(I, Ly.my_off, Ly.my_g, Ly.my_c, ws.eqc, ws.eqrx, ws.sb[0], c.stream);
-        });
+    // Phase two's rounds launched one by one, the persistent part from round kt2 (n: none).
+    void phase_two_rounds(Transcript& t, size_t li, uint32_t kt2, frh::Fr* ry, uint32_t* vy_m, uint32_t* vy_c) {
+        const DevLayer& Ly = C.layers[li];
+        const uint32_t n = Ly.nin;
+        const uint64_t I = 1ull << n;
+        const double rb = (double)rowb();
+        uint32_t* v = vals[li];
         stage(ws.vx, mapped(true, 24ull * N), 8ull * N, nullptr);
         {
             bn::RoundPtrsBn p;
@@ -288,10 +372,18 @@ struct BnProver {
                                         red_mapped(0), c.evals_d(), c.stream);
             });
             fetch(groups(K_BN_ROUND_SCALAR), n == 1 ? v : nullptr);
-            transcript_round(t, ry, 0, n == 1, false, vy_m.data(), vy_c.data());
+            transcript_round(t, ry, 0, n == 1, false, vy_m, vy_c);
         }
-        cur_f = v;
+        const uint32_t* cur_f = v;
         for (uint32_t k = 1; k < n; k++) {
+            if (k == kt2) {
+                bn::PhaseArgsBn ph = {};
+                ph.k0 = k;
+                ph.n = n;
+                ph.s = ws.sb[(k - 1) & 1];
+                ph.vx = ws.vx;
+                if (run_phase(t, false, ph, ry, false, vy_m, vy_c, rb * 6.0 * (double)(I >> k))) break;
+            }
             bn::RoundPtrsBn p;
             memset(&p, 0, sizeof(p));
             p.fsrc = cur_f;
@@ -306,9 +398,51 @@ struct BnProver {
             });
             const bool last = (k == n - 1);
             fetch(groups(K_BN_ROUND_SCALAR), last ? p.fdst : nullptr);
-            transcript_round(t, ry, k, last, false, vy_m.data(), vy_c.data());
+            transcript_round(t, ry, k, last, false, vy_m, vy_c);
             cur_f = p.fdst;
         }
+    }
+
+    void sumcheck_layer(Transcript& t, size_t li, const frh::Fr* rz1, const frh::Fr* rz2, const frh::Fr& alpha,
+                        const frh::Fr& beta, frh::Fr* rx, frh::Fr* ry) {
+        const DevLayer& Ly = C.layers[li];
+        const uint32_t n = Ly.nin, m = Ly.nout;
+        const uint64_t I = 1ull << n;
+        const double rb = (double)rowb();
+        uint32_t* v = vals[li];
+        uint32_t* vx_m = mapped(false, 24ull * N);
+        std::vector<uint32_t> vx_c((size_t)N * 8), vy_m((size_t)N * 8), vy_c((size_t)N * 8);
+
+        // phase one: eqc = alpha eq(rz1) + beta eq(rz2), gate weights, hg + round 0
+        eq_table(ws.eqc, rz1, rz2, alpha, beta, m);
+        c.launch(K_BN_WEIGHTS, 80.0 * Ly.nmul + 72.0 * Ly.nadd + 40.0 * I, [&] {
+            return bn::launch_weights(I, Ly.nmul, ws.eqc, Ly.mx_g, Ly.mx_c, Ly.ax_off, Ly.ax_g, Ly.ax_c, ws.a, ws.w,
+                                      c.stream);
+        });
+        const uint32_t kt1 = phase_start(n, 2), kt2 = kt1;
+        bn::PhaseArgsBn a1 = {};
+        a1.n = n;
+        a1.v = v;
+        a1.mx_off = Ly.mx_off;
+        a1.mx_g = Ly.mx_g;
+        a1.a = ws.a;
+        a1.w = ws.w;
+        if (kt1 != 0 || !run_phase(t, true, a1, rx, true, vx_m, vx_c.data(), rb * (6.0 * I + Ly.nmul)))
+            phase_one_rounds(t, li, kt1, alpha, beta, rx, vx_c.data());
+
+        // phase two: h(y) = vx * s(y)
+        const frh::Fr one = frh::from_u32(1), zero = frh::zero();
+        eq_table(ws.eqrx, rx, nullptr, one, zero, n);
+        c.launch(K_BN_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 32.0 * I + 96.0 * Ly.nmul, [&] {
+            return bn::launch_s_build(I, Ly.my_off, Ly.my_g, Ly.my_c, ws.eqc, ws.eqrx, ws.sb[0], c.stream);
+        });
+        bn::PhaseArgsBn a2 = {};
+        a2.n = n;
+        a2.v = v;
+        a2.s = ws.sb[0];
+        a2.vx = mapped(true, 24ull * N);
+        if (kt2 != 0 || !run_phase(t, false, a2, ry, false, vy_m.data(), vy_c.data(), rb * 4.0 * I))
+            phase_two_rounds(t, li, kt2, ry, vy_m.data(), vy_c.data());
         t.append(vy_c.data(), rowb());
         // the next layer's sum is alpha vx + beta vy (gkr.hpp:113-119)
         cv1.swap(vx_c);

@@ -120,6 +120,7 @@ enum KernelId {
     K_BN_S_BUILD,
     K_BN_WSUM,
     K_BN_UNLOAD,
+    K_BN_PHASE,  // rounds of a phase in one persistent launch (bn::k_phase)
     K_NUM_KERNELS
 };
 extern const char* const kKernelNames[K_NUM_KERNELS];

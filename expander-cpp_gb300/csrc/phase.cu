@@ -33,7 +33,6 @@ constexpr uint32_t kSmemRows = 256;            // rows x tpr of a table kept in 
 constexpr uint32_t kSpins = 256;               // mailbox polls before sleeping between them
 
 __device__ __forceinline__ uint32_t comp(const uint4& v, int l) { return l == 0 ? v.x : l == 1 ? v.y : l == 2 ? v.z : v.w; }
-__device__ __forceinline__ uint4 mk4(const uint32_t (&a)[4]) { return make_uint4(a[0], a[1], a[2], a[3]); }
 __device__ __forceinline__ void mad64(uint64_t& acc, uint32_t a, uint32_t b) { acc += (uint64_t)a * b; }
 // x mod p, partly reduced: 2^32 == 2, so lo + 2 hi < 3 2^32; four more products of canonical
 // values keep a 64-bit sum below 2^64 (4 (p - 1)^2 = 2^64 - 2^35 + 16).

@@ -363,6 +363,33 @@ struct Lane {
         pending_bytes = 0;
     }
 
+    // The same for n elements of bn::kDigitWords words holding nine 31-bit digits each: dst
+    // receives their 32 bytes.
+    void collect_digits(const uint32_t* src, uint64_t n, uint32_t parity, void* dst) {
+        const auto t0 = std::chrono::steady_clock::now();
+        const uint32_t want = parity << 31;
+        bool idle = false;
+        uint64_t it = 0;
+        for (uint64_t e = 0; e < n;) {
+            uint32_t d[9], w[8], other = 0;
+            memcpy(d, src + bn::kDigitWords * e, sizeof(d));
+            std::atomic_signal_fence(std::memory_order_seq_cst);  // read again each turn
+            for (int i = 0; i < 9; i++) {
+                other |= d[i] ^ want;
+                d[i] &= 0x7fffffffu;
+            }
+            if (other >> 31) {
+                pause(it++, t0, idle);
+                continue;
+            }
+            for (int i = 0; i < 8; i++) w[i] = (d[i] >> i) | (d[i + 1] << (31 - i));
+            memcpy(static_cast<char*>(dst) + 32 * e, w, 32);
+            e++;
+            idle = false;
+        }
+        pending_bytes = 0;
+    }
+
     ~Lane() {
         if (map_h) cudaFreeHost(map_h);
         for (PinnedBuf* b : {&h_evals, &h_rows, &h_vx, &h_cv, &h_flag}) b->release();

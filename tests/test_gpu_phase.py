@@ -40,3 +40,24 @@ def test_many_gates_on_one_row(ctx, oracle):
     w = np.full((512, 8), gc.P - 1, np.uint32)
     dc = ctx.load(circ)
     assert ctx.prove(dc, w)[1] == oracle.prove(circ, w)[1]
+
+
+@pytest.mark.parametrize("seed,widths,n", [
+    (621, [11, 10], 3), (622, [12, 11], 2), (623, [13, 4], 1), (624, [1, 1, 1], 5), (625, [2, 0], 1), (626, [5, 4], 310),
+    (627, [8, 9, 7], 33),
+])
+def test_bn254_phases_give_the_oracle_proof(ctx, seed, widths, n):
+    # the whole phase in one launch (2^11 rows), its start at a later round, one-pair layers, and
+    # more copies than resident CTAs (310: every round launched alone)
+    from oracle.oracle import OracleBn254
+    circ = gc.random_circuit(seed, widths, p_mul=0.6)
+    w = gc.random_witness_bn254(seed, circ.log_input_size, n)
+    dc = ctx.load(circ, "BN254")
+    cv, proof = ctx.prove(dc, w)
+    try:
+        ctx.set_round_tail(False)
+        assert ctx.prove(dc, w)[1] == proof
+    finally:
+        ctx.set_round_tail(True)
+    ocv, op = OracleBn254().prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
