@@ -3,21 +3,21 @@
 // Data layout in HBM: every per-copy table is row-major rows x N u32 (row r, copy k at
 // r*N + k), the byte layout of a proof vector (VectorizedM31::to_bytes, M31.hpp:420-426),
 // so a warp's 16-byte loads along a row are fully coalesced.  Scalar tables that do not
-// depend on the copy (eq tables, gate weights, the phase-two h(y) factor) are plain
+// depend on the copy (gate weights, the phase-two h(y) factor) are plain
 // arrays of u32 read by broadcast.
 //
 // Reference counterparts:
 //   k_evaluate       CircuitLayer::evaluate                     include/circuit/circuit.hpp:92-105
-//   k_eq             _eq_evals_at                               include/LinearGKR/sumcheck_common.hpp:17-53
+//   eq_build, eq_at  _eq_evals_at                               include/LinearGKR/sumcheck_common.hpp:17-53
 //   k_weights        the scalar factors of _prepare_g_x_vals    include/LinearGKR/sumcheck_helper.hpp:188-229
 //   k_hg_round0      _prepare_g_x_vals + poly_eval_at(0)        sumcheck_helper.hpp:172-231, 68-102
 //   k_hg_round1      hg rebuilt + receive_challenge + poly_eval_at(1)
 //   k_round          receive_challenge + poly_eval_at(k)        sumcheck_helper.hpp:104-133, 68-102
-//   k_s_build(4)     _prepare_h_y_vals (copy-independent part)  sumcheck_helper.hpp:233-261
+//   k_s_build        _prepare_h_y_vals (copy-independent part)  sumcheck_helper.hpp:233-261
 //   k_p2_round01     phase-two poly_eval_at of rounds 0 and 1 from one pass (round 1's sums are
 //                    quadratic in round 0's challenge); k_p2_round1_fin finishes round 1
 //   k_p2_round2      phase-two round 2 refolding the layer input
-//   k_wsum           eval_multilinear via an eq table           include/poly_commit/poly.hpp:88-104
+//   k_wsum           eval_multilinear                           include/poly_commit/poly.hpp:88-104
 //
 // k_round gives each CTA one repetition j = blockIdx.x % R: the R CTAs of a row chunk are
 // adjacent in launch order, run together and share their common source rows through L2,
@@ -31,7 +31,7 @@
 
 namespace gkrgpu {
 
-const char* const kKernelNames[K_NUM_KERNELS] = {"check_canonical", "evaluate", "eq_table", "gate_weights",
+const char* const kKernelNames[K_NUM_KERNELS] = {"check_canonical", "evaluate", "gate_weights",
                                                  "hg_build_round0", "round_fold_lane", "round_fold_scalar",
                                                  "phase2_s_build", "weighted_row_sum", "hg_rebuild_round1",
                                                  "verifier_gate_sums", "canonicalize", "phase2_round0", "stage_words", "round_tail",
@@ -63,6 +63,25 @@ __device__ __forceinline__ uint32_t reduce64(unsigned long long x) {
     x = (x & m31::P) + (x >> 31);
     uint32_t s = (uint32_t)x;
     return m31::umin(s, s - m31::P);
+}
+
+// x == x mod p for any 64-bit x: x = hi 2^32 + lo and 2^32 == 2 (mod 2^31 - 1), so the result
+// lo + 2 hi < 3 * 2^32.  Formed with a shift and an add with carry on the integer ALU (the
+// multiply pipe is what the sum kernels saturate).  After it, four more products
+// <= (p - 1)^2 keep a 64-bit sum below 3 * 2^32 + 2^64 - 2^35 + 16 < 2^64.
+__device__ __forceinline__ uint64_t fold64(uint64_t x) {
+    const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
+    uint32_t nl, nh;
+    asm("{\n\t"
+        ".reg .u32 t;\n\t"
+        "shl.b32 t, %2, 1;\n\t"
+        "add.cc.u32 %0, %3, t;\n\t"
+        "shr.u32 t, %2, 31;\n\t"
+        "addc.u32 %1, t, 0;\n\t"
+        "}"
+        : "=r"(nl), "=r"(nh)
+        : "r"(hi), "r"(lo));
+    return ((uint64_t)nh << 32) | nl;
 }
 
 // Canonical total of component c at `lane`, re-zeroing the accumulator for the next launch.
@@ -202,63 +221,6 @@ __global__ void k_canonicalize(uint32_t* v, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) v[i] = m31::from_u32(v[i]);
 }
 
-// ---------------------------------------------------------------- verifier gate sums
-// eval_sparse_circuit_connect_poly (include/LinearGKR/sumcheck_verifier_utils.hpp:22-56)
-// for R points at once: mul sums c * eqz_j[o] * eqx_j[i0] * eqy_j[i1] over the mul gates
-// (MUL), or add sums c * eqz_j[o] * eqx_j[i0] over the add gates, walked by output o (the
-// evaluate CSR).  Block partials go to 64-bit accumulators; the last block writes the R
-// canonical totals and re-zeroes the scratch.
-template <bool MUL>
-__global__ void __launch_bounds__(256) k_gate_sums(uint64_t O, uint64_t I, const uint32_t* __restrict__ off,
-                                                   const uint32_t* __restrict__ gates, const uint32_t* __restrict__ eqz,
-                                                   const uint32_t* __restrict__ eqx, const uint32_t* __restrict__ eqy,
-                                                   uint32_t reps, unsigned long long* acc, unsigned int* ticket,
-                                                   uint32_t* out) {
-    uint32_t s[3] = {0u, 0u, 0u};
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < O; o += stride) {
-        const uint32_t k0 = __ldg(off + o), k1 = __ldg(off + o + 1);
-        for (uint32_t k = k0; k < k1; k++) {
-            uint32_t i0, i1 = 0, c;
-            if (MUL) {
-                const uint4 g = __ldg(reinterpret_cast<const uint4*>(gates) + k);  // (i0, i1, c, 0)
-                i0 = g.x; i1 = g.y; c = g.z;
-            } else {
-                const uint2 g = __ldg(reinterpret_cast<const uint2*>(gates) + k);  // (i0, c)
-                i0 = g.x; c = g.y;
-            }
-            for (uint32_t j = 0; j < reps; j++) {
-                uint32_t t = mul(mul(c, __ldg(eqz + (uint64_t)j * O + o)), __ldg(eqx + (uint64_t)j * I + i0));
-                if (MUL) t = mul(t, __ldg(eqy + (uint64_t)j * I + i1));
-                s[j] = add(s[j], t);
-            }
-        }
-    }
-    __shared__ unsigned long long part[3];
-    if (threadIdx.x < 3) part[threadIdx.x] = 0ull;
-    __syncthreads();
-    for (uint32_t j = 0; j < reps; j++) {
-        unsigned long long x = s[j];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&part[j], x);
-    }
-    __syncthreads();
-    if (threadIdx.x < reps) atomicAdd(&acc[threadIdx.x], part[threadIdx.x]);
-    __threadfence();
-    __syncthreads();
-    __shared__ unsigned int is_last;
-    if (threadIdx.x == 0) is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    if (threadIdx.x < reps) {
-        out[threadIdx.x] = reduce64(__ldcg(&acc[threadIdx.x]));
-        acc[threadIdx.x] = 0ull;
-    }
-    if (threadIdx.x == 0) *ticket = 0u;
-}
-
 // ---------------------------------------------------------------- layer evaluation
 // out[o] = sum over mul gates (o, i0, i1, c) of in[i0]*in[i1]*c + sum over add gates
 // (o, i0, c) of in[i0]*c, gates grouped by o (CSR), so every output row is written once.
@@ -288,40 +250,69 @@ __global__ void __launch_bounds__(256) k_evaluate(const uint32_t* __restrict__ i
     }
 }
 
-// ---------------------------------------------------------------- eq tables
-// out[j][z] = f1 * eq(r1_j, z) + f2 * eq(r2_j, z), bit t of z paired with r[t]
-// (little-endian, sumcheck_common.hpp:17-53); eq(r, 0) = 1 - r, eq(r, 1) = r.
-__global__ void k_eq(uint32_t* __restrict__ out, EqArgs a) {
-    const uint64_t size = 1ull << a.nvars;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t z = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; z < size; z += stride) {
-        for (uint32_t j = 0; j < a.reps; j++) {
-            uint32_t e1 = a.f1, e2 = a.f2;
-            for (uint32_t t = 0; t < a.nvars; t++) {
-                const bool bit = (z >> t) & 1;
-                e1 = mul(e1, bit ? a.r1[j][t] : sub(1u, a.r1[j][t]));
-                if (a.f2) e2 = mul(e2, bit ? a.r2[j][t] : sub(1u, a.r2[j][t]));
-            }
-            out[(uint64_t)j * size + z] = add(e1, a.f2 ? e2 : 0u);
+// ---------------------------------------------------------------- eq factors
+// eq(r_j, z) = prod over bits t of z of (bit ? r_j[t] : 1 - r_j[t]), bit t paired with r[t]
+// (little-endian, _eq_evals_at, sumcheck_common.hpp:17-53).  No table over z is stored: a CTA
+// builds one table of 32 entries per five bits, repetition and point (at most 36 of them), and
+// a kernel multiplies the entries of z where it needs the factor, three products at 2^20.  The
+// tables over z took a launch of their own per use (7 us at 2^10 entries, 71 us for two points
+// at 2^20, 18 products an entry) and a gather from memory per gate.
+constexpr uint32_t kEqBits = 5, kEqTabs = 6, kEqWords = 3 * kEqTabs * 32;  // words per point
+
+__device__ __forceinline__ uint32_t eq_digits(const EqArgs& a) {
+    return a.nvars > kEqBits ? (a.nvars + kEqBits - 1) / kEqBits : 1u;
+}
+// Fills t (kEqWords words per point); the caller synchronises the CTA.
+__device__ __forceinline__ void eq_build(uint32_t* t, const EqArgs& a) {
+    const uint32_t nd = eq_digits(a), per = nd * a.reps * 32, total = per * (a.f2 ? 2 : 1);
+    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+        const uint32_t p = i / per, k = i - p * per, x = k & 31, jd = k >> 5, j = jd / nd, d = jd - j * nd;
+        uint32_t e = d ? 1u : (p ? a.f2 : a.f1);
+#pragma unroll
+        for (uint32_t b = 0; b < kEqBits; b++) {
+            const uint32_t v = d * kEqBits + b;
+            if (v >= a.nvars) break;
+            const uint32_t r = p ? a.r2[j][v] : a.r1[j][v];
+            e = mul(e, (x >> b) & 1 ? r : sub(1u, r));
         }
+        t[p * kEqWords + (j * kEqTabs + d) * 32 + x] = e;
     }
+}
+// f1 eq(r1_j, z) + f2 eq(r2_j, z)
+__device__ __forceinline__ uint32_t eq_at(const uint32_t* t, uint32_t nd, bool two, uint32_t j, uint32_t z) {
+    const uint32_t* t1 = t + j * kEqTabs * 32;
+    uint32_t e = t1[z & 31];
+    for (uint32_t d = 1; d < nd; d++) e = mul(e, t1[d * 32 + ((z >> (kEqBits * d)) & 31)]);
+    if (!two) return e;
+    const uint32_t* t2 = t1 + kEqWords;
+    uint32_t f = t2[z & 31];
+    for (uint32_t d = 1; d < nd; d++) f = mul(f, t2[d * 32 + ((z >> (kEqBits * d)) & 31)]);
+    return add(e, f);
 }
 
 // ---------------------------------------------------------------- phase-one scalar factors
-// w[k].j = c_k * eqc_j[z_k] for every mul gate k (gates in CSR-by-x order) and
-// a[x].j = sum over add gates (z, x, c) of c * eqc_j[z]: the copy-independent parts of
-// hg(x) = sum_mul v(y) c eqc(z) + sum_add c eqc(z) (sumcheck_helper.hpp:203-229).
-__global__ void k_weights(uint64_t I, uint64_t Gm, uint64_t O, const uint32_t* __restrict__ eqc,
-                          const uint4* __restrict__ mx_g, const uint32_t* __restrict__ ax_off,
-                          const uint2* __restrict__ ax_g, uint4* __restrict__ a_out, uint4* __restrict__ w_out,
-                          uint32_t reps) {
+// w[k].j = c_k * eqc_j(z_k) for every mul gate k (gates in CSR-by-x order) and
+// a[x].j = sum over add gates (z, x, c) of c * eqc_j(z): the copy-independent parts of
+// hg(x) = sum_mul v(y) c eqc(z) + sum_add c eqc(z) (sumcheck_helper.hpp:203-229), with
+// eqc_j = alpha eq(rz1_j) + beta eq(rz2_j).
+__global__ void __launch_bounds__(256) k_weights(uint64_t I, uint64_t Gm, const __grid_constant__ EqArgs eqc,
+                                                 const uint4* __restrict__ mx_g, const uint32_t* __restrict__ ax_off,
+                                                 const uint2* __restrict__ ax_g, uint4* __restrict__ a_out,
+                                                 uint4* __restrict__ w_out) {
+    __shared__ uint32_t t[2 * kEqWords];
+    eq_build(t, eqc);
+    __syncthreads();
+    const uint32_t nd = eq_digits(eqc), reps = eqc.reps;
+    const bool two = eqc.f2 != 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t n = I > Gm ? I : Gm;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         if (i < Gm) {
             const uint4 gt = __ldg(mx_g + i);  // (y, z, c, 0)
             uint32_t w[3] = {0u, 0u, 0u};
-            for (uint32_t j = 0; j < reps; j++) w[j] = mul(gt.z, __ldg(eqc + (uint64_t)j * O + gt.y));
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+                if (j < reps) w[j] = mul(gt.z, eq_at(t, nd, two, j, gt.y));
             w_out[i] = make_uint4(w[0], w[1], w[2], 0u);
         }
         if (i < I) {
@@ -329,11 +320,83 @@ __global__ void k_weights(uint64_t I, uint64_t Gm, uint64_t O, const uint32_t* _
             const uint32_t k0 = __ldg(ax_off + i), k1 = __ldg(ax_off + i + 1);
             for (uint32_t k = k0; k < k1; k++) {
                 const uint2 gt = __ldg(ax_g + k);  // (z, c)
-                for (uint32_t j = 0; j < reps; j++) s[j] = add(s[j], mul(gt.y, __ldg(eqc + (uint64_t)j * O + gt.x)));
+#pragma unroll
+                for (uint32_t j = 0; j < 3; j++)
+                    if (j < reps) s[j] = add(s[j], mul(gt.y, eq_at(t, nd, two, j, gt.x)));
             }
             a_out[i] = make_uint4(s[0], s[1], s[2], 0u);
         }
     }
+}
+
+// ---------------------------------------------------------------- verifier gate sums
+// eval_sparse_circuit_connect_poly (include/LinearGKR/sumcheck_verifier_utils.hpp:22-56)
+// for R points at once: mul sums c * eqz_j(o) * eqx_j(i0) * eqy_j(i1) over the mul gates
+// (MUL), or add sums c * eqz_j(o) * eqx_j(i0) over the add gates, walked by output o (the
+// evaluate CSR).  Block partials go to 64-bit accumulators; the last block writes the R
+// canonical totals and re-zeroes the scratch.
+template <bool MUL>
+__global__ void __launch_bounds__(256) k_gate_sums(uint64_t O, const uint32_t* __restrict__ off,
+                                                   const uint32_t* __restrict__ gates, const __grid_constant__ GateEq eq,
+                                                   unsigned long long* acc, unsigned int* ticket, uint32_t* out) {
+    __shared__ uint32_t tz[2 * kEqWords], tx[kEqWords], ty[MUL ? kEqWords : 1];
+    eq_build(tz, eq.z);
+    eq_build(tx, eq.x);
+    if (MUL) eq_build(ty, eq.y);
+    __syncthreads();
+    const uint32_t ndz = eq_digits(eq.z), ndx = eq_digits(eq.x), reps = eq.z.reps;
+    const bool two = eq.z.f2 != 0;
+    uint32_t s[3] = {0u, 0u, 0u};
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < O; o += stride) {
+        const uint32_t k0 = __ldg(off + o), k1 = __ldg(off + o + 1);
+        if (k0 == k1) continue;
+        uint32_t ez[3] = {0u, 0u, 0u};
+#pragma unroll
+        for (uint32_t j = 0; j < 3; j++)
+            if (j < reps) ez[j] = eq_at(tz, ndz, two, j, (uint32_t)o);
+        for (uint32_t k = k0; k < k1; k++) {
+            uint32_t i0, i1 = 0, c;
+            if (MUL) {
+                const uint4 g = __ldg(reinterpret_cast<const uint4*>(gates) + k);  // (i0, i1, c, 0)
+                i0 = g.x; i1 = g.y; c = g.z;
+            } else {
+                const uint2 g = __ldg(reinterpret_cast<const uint2*>(gates) + k);  // (i0, c)
+                i0 = g.x; c = g.y;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+                if (j < reps) {
+                    uint32_t t = mul(mul(c, ez[j]), eq_at(tx, ndx, false, j, i0));
+                    if (MUL) t = mul(t, eq_at(ty, ndx, false, j, i1));
+                    s[j] = add(s[j], t);
+                }
+        }
+    }
+    __shared__ unsigned long long part[3];
+    if (threadIdx.x < 3) part[threadIdx.x] = 0ull;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < 3; j++) {
+        unsigned long long x = s[j];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&part[j], x);
+    }
+    __syncthreads();
+    if (threadIdx.x < reps) atomicAdd(&acc[threadIdx.x], part[threadIdx.x]);
+    __threadfence();
+    __syncthreads();
+    __shared__ unsigned int is_last;
+    if (threadIdx.x == 0) is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    if (threadIdx.x < reps) {
+        out[threadIdx.x] = reduce64(__ldcg(&acc[threadIdx.x]));
+        acc[threadIdx.x] = 0ull;
+    }
+    if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // w_j[k] (1 - r_j) for the mul gates of even input rows x, w_j[k] r_j for odd x: the weights
@@ -1079,25 +1142,6 @@ __global__ void __launch_bounds__(256) k_p2_round2(RoundPtrs p, uint64_t npairs,
                         ClaimFin{red, evals_out, nullptr, {p.r[0], p.r[1], p.r[2]}, g.N, (uint32_t)R, vx});
 }
 
-// x == x mod p for any 64-bit x: x = hi 2^32 + lo and 2^32 == 2 (mod 2^31 - 1), so the result
-// lo + 2 hi < 3 * 2^32.  Formed with a shift and an add with carry on the integer ALU (the
-// multiply pipe is what the sum kernels saturate).  After it, four more products
-// <= (p - 1)^2 keep a 64-bit sum below 3 * 2^32 + 2^64 - 2^35 + 16 < 2^64.
-__device__ __forceinline__ uint64_t fold64(uint64_t x) {
-    const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
-    uint32_t nl, nh;
-    asm("{\n\t"
-        ".reg .u32 t;\n\t"
-        "shl.b32 t, %2, 1;\n\t"
-        "add.cc.u32 %0, %3, t;\n\t"
-        "shr.u32 t, %2, 31;\n\t"
-        "addc.u32 %1, t, 0;\n\t"
-        "}"
-        : "=r"(nl), "=r"(nh)
-        : "r"(hi), "r"(lo));
-    return ((uint64_t)nh << 32) | nl;
-}
-
 // acc += a * b with one 32 x 32 -> 64-bit multiply-add.
 __device__ __forceinline__ void mad64(uint64_t& acc, uint32_t a, uint32_t b) {
     asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
@@ -1400,79 +1444,120 @@ __global__ void __launch_bounds__(256) k_p2_round1_fin(const uint32_t* __restric
 }
 
 // ---------------------------------------------------------------- phase two: s(y)
-// s_j[y] = sum over mul gates (z, x, y, c) of eqc_j[z] * eq_rx_j[x] * c: the
-// copy-independent factor of h(y) = v(rx) s(y) (sumcheck_helper.hpp:250-259).
-__global__ void k_s_build(uint64_t I, uint64_t O, const uint32_t* __restrict__ my_off, const uint4* __restrict__ my_g,
-                          const uint32_t* __restrict__ eqc, const uint32_t* __restrict__ eqrx, uint32_t* __restrict__ s_out,
-                          uint64_t s_stride, uint32_t reps) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t y = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; y < I; y += stride) {
-        uint32_t s[3] = {0u, 0u, 0u};
-        const uint32_t k0 = __ldg(my_off + y), k1 = __ldg(my_off + y + 1);
-        for (uint32_t k = k0; k < k1; k++) {
-            const uint4 gt = __ldg(my_g + k);  // (x, z, c, 0)
-            for (uint32_t j = 0; j < reps; j++) {
-                const uint32_t e = mul(__ldg(eqc + (uint64_t)j * O + gt.y), __ldg(eqrx + (uint64_t)j * I + gt.x));
-                s[j] = add(s[j], mul(e, gt.z));
-            }
-        }
-        for (uint32_t j = 0; j < reps; j++) s_out[(uint64_t)j * s_stride + y] = s[j];
-    }
-}
-
-// k_s_build over groups of four rows (I a multiple of 4), one thread per group, which also
-// writes t_j(i) = (s_j(4i) + s_j(4i+2), s_j(4i+1) + s_j(4i+3), s_j(4i) + s_j(4i+1),
-// s_j(4i+2) + s_j(4i+3)), the scalar pair sums that k_p2_round01 stages with each group.
-__global__ void k_s_build4(uint64_t I, uint64_t O, const uint32_t* __restrict__ my_off, const uint4* __restrict__ my_g,
-                           const uint32_t* __restrict__ eqc, const uint32_t* __restrict__ eqrx, uint32_t* __restrict__ s_out,
-                           uint32_t* __restrict__ t_out, uint64_t s_stride, uint32_t reps) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, ngroups = I / 4;
-    for (uint64_t gi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < ngroups; gi += stride) {
-        uint32_t s[3][4] = {};
+// s_j[y] = sum over mul gates (z, x, y, c) of eqc_j(z) * eq(rx_j, x) * c: the
+// copy-independent factor of h(y) = v(rx) s(y) (sumcheck_helper.hpp:250-259).  With T4 one
+// thread takes a group of four rows (I a multiple of 4) and also writes t_j(i) =
+// (s_j(4i) + s_j(4i+2), s_j(4i+1) + s_j(4i+3), s_j(4i) + s_j(4i+1), s_j(4i+2) + s_j(4i+3)),
+// the scalar pair sums that k_p2_round01 stages with each group.
+template <bool T4>
+__global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __restrict__ my_off,
+                                                 const uint4* __restrict__ my_g, const __grid_constant__ EqArgs eqc,
+                                                 const __grid_constant__ EqArgs eqx, uint32_t* __restrict__ s_out,
+                                                 uint32_t* __restrict__ t_out, uint64_t s_stride) {
+    __shared__ uint32_t tz[2 * kEqWords], tx[kEqWords];
+    eq_build(tz, eqc);
+    eq_build(tx, eqx);
+    __syncthreads();
+    const uint32_t ndz = eq_digits(eqc), ndx = eq_digits(eqx), reps = eqc.reps;
+    const bool two = eqc.f2 != 0;
+    constexpr int G = T4 ? 4 : 1;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, n = I / G;
+    for (uint64_t gi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < n; gi += stride) {
+        uint32_t s[3][G] = {};
+        uint32_t off[G + 1];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint64_t y = 4 * gi + k;
-            const uint32_t k0 = __ldg(my_off + y), k1 = __ldg(my_off + y + 1);
-            for (uint32_t e = k0; e < k1; e++) {
-                const uint4 gt = __ldg(my_g + e);  // (x, z, c, 0)
-                for (uint32_t j = 0; j < reps; j++) {
-                    const uint32_t w = mul(__ldg(eqc + (uint64_t)j * O + gt.y), __ldg(eqrx + (uint64_t)j * I + gt.x));
-                    s[j][k] = add(s[j][k], mul(w, gt.z));
+        for (int k = 0; k <= G; k++) off[k] = __ldg(my_off + G * gi + k);
+        for (uint32_t e = off[0]; e < off[G]; e++) {
+            const uint4 gt = __ldg(my_g + e);  // (x, z, c, 0)
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+                if (j < reps) {
+                    const uint32_t w = mul(mul(eq_at(tz, ndz, two, j, gt.y), eq_at(tx, ndx, false, j, gt.x)), gt.z);
+#pragma unroll
+                    for (int k = 0; k < G; k++)
+                        if (e >= off[k] && e < off[k + 1]) s[j][k] = add(s[j][k], w);
                 }
-            }
         }
-        for (uint32_t j = 0; j < reps; j++) {
-            reinterpret_cast<uint4*>(s_out + (uint64_t)j * s_stride)[gi] = make_uint4(s[j][0], s[j][1], s[j][2], s[j][3]);
-            reinterpret_cast<uint4*>(t_out + (uint64_t)j * s_stride)[gi] =
-                make_uint4(add(s[j][0], s[j][2]), add(s[j][1], s[j][3]), add(s[j][0], s[j][1]), add(s[j][2], s[j][3]));
+#pragma unroll
+        for (uint32_t j = 0; j < 3; j++) {
+            if (j >= reps) break;
+            if (T4) {
+                reinterpret_cast<uint4*>(s_out + (uint64_t)j * s_stride)[gi] =
+                    make_uint4(s[j][0], s[j][1 % G], s[j][2 % G], s[j][3 % G]);
+                reinterpret_cast<uint4*>(t_out + (uint64_t)j * s_stride)[gi] =
+                    make_uint4(add(s[j][0], s[j][2 % G]), add(s[j][1 % G], s[j][3 % G]), add(s[j][0], s[j][1 % G]),
+                               add(s[j][2 % G], s[j][3 % G]));
+            } else {
+                s_out[(uint64_t)j * s_stride + gi] = s[j][0];
+            }
         }
     }
 }
 
 // ---------------------------------------------------------------- weighted row sums
-// out[j] = sum_z eq_j[z] * vals[z]: eval_multilinear at r_j for each repetition.
+// out[j] = sum_z eq(r_j, z) vals[z]: eval_multilinear at r_j for each point
+// (include/poly_commit/poly.hpp:88-104).  The table is read once, so the bound is HBM: 2^18
+// rows of 1024 copies at three points take 160 us at the copy peak.  Products are summed
+// unreduced in 64 bits and folded every four rows (as separate field operations the sums took
+// 430 us, bound by instruction issue); a thread reads four consecutive rows at once, and their
+// weights, computed per block of rows from the digit tables, come from shared memory.
+constexpr uint32_t kWsumRows = 256;  // rows a CTA takes at a time, at least
+
+__host__ __device__ inline uint32_t wsum_block(const Geo& g, uint64_t rows, uint32_t ctas) {
+    const uint32_t step = 4 * g.rps;
+    uint64_t per = rows / ((uint64_t)step * (ctas ? ctas : 1));  // small tables: one step a CTA
+    const uint32_t most = (kWsumRows + step - 1) / step;
+    if (per > most) per = most;
+    return step * (per > 1 ? (uint32_t)per : 1u);
+}
+
 template <int R>
-__global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows,
-                                              const uint32_t* __restrict__ eq, Geo g, RedScratch red,
-                                              uint32_t* out) {
+__global__ void __launch_bounds__(256, 4) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows, uint32_t rb,
+                                                 const __grid_constant__ EqArgs eq, Geo g, RedScratch red, uint32_t* out) {
+    extern __shared__ uint32_t smem[];  // R x rb weights, then the reduction's scratch
+    __shared__ uint32_t tab[kEqWords];
     const TileIdx t = tile_idx(g);
-    uint32_t acc[R][4];
+    eq_build(tab, eq);
+    const uint32_t nd = eq_digits(eq);
+    uint64_t acc[R][4];
 #pragma unroll
     for (int c = 0; c < R; c++)
 #pragma unroll
-        for (int l = 0; l < 4; l++) acc[c][l] = 0u;
-    if (t.active) {
-        for (uint64_t z = (uint64_t)blockIdx.x * g.rps + t.rs; z < rows; z += (uint64_t)gridDim.x * g.rps) {
-            const uint4 v = ld4(vals, z, g.N, t.lane0);
+        for (int l = 0; l < 4; l++) acc[c][l] = 0ull;
+    for (uint64_t z0 = (uint64_t)blockIdx.x * rb; z0 < rows; z0 += (uint64_t)gridDim.x * rb) {
+        __syncthreads();  // the digit tables, or the last block's weights, are done with
+        for (uint32_t i = threadIdx.x; i < rb; i += blockDim.x)
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                smem[j * rb + i] = z0 + i < rows ? eq_at(tab, nd, false, j, (uint32_t)(z0 + i)) : 0u;
+        __syncthreads();
+        if (!t.active) continue;
+        for (uint32_t i = 4 * t.rs; i < rb && z0 + i < rows; i += 4 * g.rps) {
+            uint4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint64_t z = z0 + i + k;  // a table of fewer than four rows repeats its last (weight 0)
+                v[k] = ld4(vals, z < rows ? z : rows - 1, g.N, t.lane0);
+            }
 #pragma unroll
             for (int j = 0; j < R; j++) {
-                const uint32_t w = __ldg(eq + (uint64_t)j * rows + z);
+                const uint4 w = *reinterpret_cast<const uint4*>(smem + j * rb + i);
 #pragma unroll
-                for (int l = 0; l < 4; l++) acc[j][l] = add(acc[j][l], mul(comp(v, l), w));
+                for (int l = 0; l < 4; l++) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) acc[j][l] += (uint64_t)comp(v[k], l) * comp(w, k);
+                    acc[j][l] = fold64(acc[j][l]);
+                }
             }
         }
     }
-    reduce_group<R>(acc, g, t.active, red, 0, CopyFin{red, out, g.N, (uint32_t)R});
+    uint32_t sum[R][4];
+#pragma unroll
+    for (int c = 0; c < R; c++)
+#pragma unroll
+        for (int l = 0; l < 4; l++) sum[c][l] = reduce64(acc[c][l]);
+    __syncthreads();  // the weights' space is the reduction's scratch
+    reduce_group<R>(sum, g, t.active, red, 0, CopyFin{red, out, g.N, (uint32_t)R});
 }
 
 uint32_t grid_1d(uint64_t n, uint32_t block) {
@@ -1526,19 +1611,14 @@ cudaError_t launch_canonicalize(uint32_t* v, uint64_t n, cudaStream_t s) {
     k_canonicalize<<<grid_1d(n, 256), 256, 0, s>>>(v, n);
     return cudaGetLastError();
 }
-cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, uint64_t I, const uint32_t* off, const uint32_t* gates,
-                             const uint32_t* eqz, const uint32_t* eqx, const uint32_t* eqy, uint32_t reps,
+cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const GateEq& eq,
                              unsigned long long* acc, unsigned int* ticket, uint32_t* out, cudaStream_t s) {
-    if (reps < 1 || reps > 3) return cudaErrorInvalidValue;
+    if (eq.z.reps < 1 || eq.z.reps > 3) return cudaErrorInvalidValue;
     const uint32_t grid = grid_1d(O, 256);
     if (mul_gates)
-        k_gate_sums<true><<<grid, 256, 0, s>>>(O, I, off, gates, eqz, eqx, eqy, reps, acc, ticket, out);
+        k_gate_sums<true><<<grid, 256, 0, s>>>(O, off, gates, eq, acc, ticket, out);
     else
-        k_gate_sums<false><<<grid, 256, 0, s>>>(O, I, off, gates, eqz, eqx, eqy, reps, acc, ticket, out);
-    return cudaGetLastError();
-}
-cudaError_t launch_eq(uint32_t* out, const EqArgs& a, cudaStream_t s) {
-    k_eq<<<grid_1d(1ull << a.nvars, 256), 256, 0, s>>>(out, a);
+        k_gate_sums<false><<<grid, 256, 0, s>>>(O, off, gates, eq, acc, ticket, out);
     return cudaGetLastError();
 }
 
@@ -1550,10 +1630,9 @@ cudaError_t launch_scale_weights(uint64_t I, const uint32_t* mx_off, const uint4
     return cudaGetLastError();
 }
 
-cudaError_t launch_weights(uint64_t I, uint64_t Gm, uint64_t O, const uint32_t* eqc, const uint4* mx_g,
-                           const uint32_t* ax_off, const uint2* ax_g, uint4* a_out, uint4* w_out, uint32_t reps,
-                           cudaStream_t s) {
-    k_weights<<<grid_1d(I > Gm ? I : Gm, 256), 256, 0, s>>>(I, Gm, O, eqc, mx_g, ax_off, ax_g, a_out, w_out, reps);
+cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgs& eqc, const uint4* mx_g, const uint32_t* ax_off,
+                           const uint2* ax_g, uint4* a_out, uint4* w_out, cudaStream_t s) {
+    k_weights<<<grid_1d(I > Gm ? I : Gm, 256), 256, 0, s>>>(I, Gm, eqc, mx_g, ax_off, ax_g, a_out, w_out);
     return cudaGetLastError();
 }
 
@@ -1814,27 +1893,28 @@ cudaError_t launch_p2_round1_fin(int reps, const uint32_t* sums, const uint32_t*
     return cudaGetLastError();
 }
 
-cudaError_t launch_s_build4(uint64_t I, uint64_t O, const uint32_t* my_off, const uint4* my_g, const uint32_t* eqc,
-                            const uint32_t* eqrx, uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, uint32_t reps,
-                            cudaStream_t s) {
-    if (I % 4 || (s_stride % 4)) return cudaErrorInvalidValue;
-    k_s_build4<<<grid_1d(I / 4, 256), 256, 0, s>>>(I, O, my_off, my_g, eqc, eqrx, s_out, t_out, s_stride, reps);
+cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const EqArgs& eqc, const EqArgs& eqx,
+                           uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, cudaStream_t s) {
+    if (t_out && (I % 4 || s_stride % 4)) return cudaErrorInvalidValue;
+    if (t_out)
+        k_s_build<true><<<grid_1d(I / 4, 256), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, t_out, s_stride);
+    else
+        k_s_build<false><<<grid_1d(I, 256), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, nullptr, s_stride);
     return cudaGetLastError();
 }
 
-cudaError_t launch_s_build(uint64_t I, uint64_t O, const uint32_t* my_off, const uint4* my_g, const uint32_t* eqc,
-                           const uint32_t* eqrx, uint32_t* s_out, uint64_t s_stride, uint32_t reps, cudaStream_t s) {
-    k_s_build<<<grid_1d(I, 256), 256, 0, s>>>(I, O, my_off, my_g, eqc, eqrx, s_out, s_stride, reps);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_wsum(int reps, const uint32_t* vals, uint64_t rows, const uint32_t* eq, const Geo& g,
-                        uint32_t block, uint32_t ctas, RedScratch red, uint32_t* out, cudaStream_t s) {
-    LaunchShape sh = row_shape(g, rows, block, ctas, reps);
-    switch (reps) {
-        case 1: k_wsum<1><<<sh.grid, sh.block, sh.smem, s>>>(vals, rows, eq, g, red, out); break;
-        case 2: k_wsum<2><<<sh.grid, sh.block, sh.smem, s>>>(vals, rows, eq, g, red, out); break;
-        case 3: k_wsum<3><<<sh.grid, sh.block, sh.smem, s>>>(vals, rows, eq, g, red, out); break;
+cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,
+                        RedScratch red, uint32_t* out, cudaStream_t s) {
+    const uint64_t rows = 1ull << eq.nvars;
+    const uint32_t groups = g.N / (4 * g.tpr), cap = ctas / groups ? ctas / groups : 1, rb = wsum_block(g, rows, cap);
+    const uint64_t need = (rows + rb - 1) / rb;
+    const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);
+    const size_t weights = 4 * (size_t)eq.reps * rb, scratch = 4 * (size_t)eq.reps * 4 * block;
+    const size_t smem = weights > scratch ? weights : scratch;
+    switch (eq.reps) {
+        case 1: k_wsum<1><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
+        case 2: k_wsum<2><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
+        case 3: k_wsum<3><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

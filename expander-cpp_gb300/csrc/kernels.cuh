@@ -36,6 +36,11 @@ struct EqArgs {
     uint32_t reps;
 };
 
+// eq factors of the verifier's gate sums: outputs, first inputs and (mul gates) second inputs.
+struct GateEq {
+    EqArgs z, x, y;
+};
+
 struct RoundPtrs {
     const uint32_t* fsrc[3];
     uint32_t* fdst[3];
@@ -96,7 +101,6 @@ struct LaunchShape {
 enum KernelId {
     K_CHECK = 0,
     K_EVALUATE,
-    K_EQ,
     K_WEIGHTS,
     K_HG_ROUND0,
     K_ROUND_LANE,
@@ -132,17 +136,15 @@ LaunchShape row_shape(const Geo& g, uint64_t rows, uint32_t block, uint32_t ctas
 cudaError_t launch_check_canonical(const uint32_t* v, uint64_t n, unsigned int* flag, cudaStream_t s);
 // v[i] = v[i] mod p in place (M31::from_bytes of raw proof words).
 cudaError_t launch_canonicalize(uint32_t* v, uint64_t n, cudaStream_t s);
-// Verifier gate sums for `reps` points: over the mul gates (CSR by output: off, (i0, i1, c, 0)
-// gates) sum c eqz_j[o] eqx_j[i0] eqy_j[i1], or over the add gates ((i0, c) gates) sum
-// c eqz_j[o] eqx_j[i0]; eq tables are reps x O / reps x I.  acc (3 x u64) and ticket must be
-// zero and are left zero; out receives reps canonical totals.
-cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, uint64_t I, const uint32_t* off, const uint32_t* gates,
-                             const uint32_t* eqz, const uint32_t* eqx, const uint32_t* eqy, uint32_t reps,
+// Verifier gate sums for eq.z.reps points: over the mul gates (CSR by output: off, (i0, i1, c, 0)
+// gates) sum c eqz_j(o) eqx_j(i0) eqy_j(i1), or over the add gates ((i0, c) gates) sum
+// c eqz_j(o) eqx_j(i0).  acc (3 x u64) and ticket must be zero and are left zero; out receives
+// the canonical totals.
+cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const GateEq& eq,
                              unsigned long long* acc, unsigned int* ticket, uint32_t* out, cudaStream_t s);
 cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint32_t* mo_off, const uint4* mo_g,
                             const uint32_t* ao_off, const uint2* ao_g, const Geo& g, uint32_t block, uint32_t ctas,
                             cudaStream_t s);
-cudaError_t launch_eq(uint32_t* out, const EqArgs& a, cudaStream_t s);
 // dst[k * n + i] = srcs[k][i] (nsrc <= 3 tables of n words) by a small kernel instead of the
 // copy engine, for transfers between device and host-mapped memory; with `done`, every CTA
 // increments it after its writes are visible to the host.  Returns the CTA count (the
@@ -153,9 +155,10 @@ uint32_t launch_stage_words(uint32_t* dst, const uint32_t* const* srcs, uint32_t
 // rows (CSR-by-x offsets mx_off over I rows): the weights of launch_hg_round1.
 cudaError_t launch_scale_weights(uint64_t I, const uint32_t* mx_off, const uint4* w4, uint4* w4r, const uint32_t r[3],
                                  int reps, cudaStream_t s);
-cudaError_t launch_weights(uint64_t I, uint64_t Gm, uint64_t O, const uint32_t* eqc, const uint4* mx_g,
-                           const uint32_t* ax_off, const uint2* ax_g, uint4* a_out, uint4* w_out, uint32_t reps,
-                           cudaStream_t s);
+// Gate weights w_out (mul gates in CSR-by-x order) and add weights a_out (I rows) for
+// eqc_j = f1 eq(r1_j) + f2 eq(r2_j) over the outputs.
+cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgs& eqc, const uint4* mx_g, const uint32_t* ax_off,
+                           const uint2* ax_g, uint4* a_out, uint4* w_out, cudaStream_t s);
 // Phase-one hg (not stored) and the round-0 evaluations over `npairs` pairs of input rows:
 // pair i is (2q, 2q+1) with q = pairs[i], or q = i without a list (pairs = null).  Pairs
 // left out of the list must have no gate whose first input is in them (their hg is zero).
@@ -218,20 +221,19 @@ uint32_t p2_round01_groups(uint32_t N);
 cudaError_t launch_p2_round1_fin(int reps, const uint32_t* sums, const uint32_t* vx, const uint32_t* const* s,
                                  uint32_t* const* sd, const uint32_t* r, uint64_t ngroups, uint32_t N,
                                  uint32_t* evals_out, uint32_t* evals_dev, unsigned int* done, cudaStream_t st);
-// launch_s_build plus the pair sums t_j(i) = (s_j(4i) + s_j(4i+2), s_j(4i+1) + s_j(4i+3),
-// s_j(4i) + s_j(4i+1), s_j(4i+2) + s_j(4i+3)) into t_out (4 I/4 entries, stride s_stride);
-// I and s_stride multiples of 4.
-cudaError_t launch_s_build4(uint64_t I, uint64_t O, const uint32_t* my_off, const uint4* my_g, const uint32_t* eqc,
-                            const uint32_t* eqrx, uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, uint32_t reps,
-                            cudaStream_t s);
-cudaError_t launch_s_build(uint64_t I, uint64_t O, const uint32_t* my_off, const uint4* my_g, const uint32_t* eqc,
-                           const uint32_t* eqrx, uint32_t* s_out, uint64_t s_stride, uint32_t reps, cudaStream_t s);
+// Scalar tables s_j(y) (stride s_stride) for eqc over the outputs and eq(rx_j) over the first
+// inputs; with t_out also the pair sums t_j(i) = (s_j(4i) + s_j(4i+2), s_j(4i+1) + s_j(4i+3),
+// s_j(4i) + s_j(4i+1), s_j(4i+2) + s_j(4i+3)) (I and s_stride multiples of 4).
+cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const EqArgs& eqc, const EqArgs& eqx,
+                           uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, cudaStream_t s);
 // CTAs of a persistent phase for N copies at tpr quads a CTA, the smallest tpr that needs at
 // most max_ctas of them (0: none does), and the launch.
 uint32_t phase_tpr(uint32_t N, uint32_t max_ctas);
 uint32_t phase_ctas(uint32_t N, uint32_t tpr);
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s);
-cudaError_t launch_wsum(int reps, const uint32_t* vals, uint64_t rows, const uint32_t* eq, const Geo& g,
-                        uint32_t block, uint32_t ctas, RedScratch red, uint32_t* out, cudaStream_t s);
+// eval_multilinear of vals (2^eq.nvars rows) at eq.r1_j for eq.reps points (eq.f1 = 1, no second
+// point): out receives reps x N.
+cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,
+                        RedScratch red, uint32_t* out, cudaStream_t s);
 
 }  // namespace gkrgpu

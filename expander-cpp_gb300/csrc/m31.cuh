@@ -38,7 +38,14 @@ GKR_HD uint32_t reduce62(uint64_t x) {
     return umin(s, s - P);
 }
 
-GKR_HD uint32_t mul(uint32_t a, uint32_t b) { return reduce62((uint64_t)a * b); }
+// a * b, formed as a * 2b: the product's high word is then (a b) >> 31 and half its low word
+// (a b) mod 2^31, one shift-and-add apart (reduce62 of the plain product takes a mask, a
+// 64-bit shift and an add).
+GKR_HD uint32_t mul(uint32_t a, uint32_t b) {
+    const uint64_t t = (uint64_t)a * (b + b);
+    const uint32_t s = (uint32_t)(t >> 32) + ((uint32_t)t >> 1);
+    return umin(s, s - P);
+}
 
 // Canonical form of an arbitrary u32 (M31::from_bytes, include/field/M31.hpp:111-116).
 GKR_HD uint32_t from_u32(uint32_t x) {

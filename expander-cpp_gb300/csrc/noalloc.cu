@@ -25,14 +25,13 @@ namespace {
 constexpr uint32_t kMaxVars = 18;       // tables of up to 2^18 rows
 constexpr uint32_t kMaxCopies = 4096;   // up to 4096 copies per row
 constexpr int kMaxPoints = 3;           // up to 3 evaluation points per call
-constexpr size_t kEqBytes = (size_t)kMaxPoints * (1u << kMaxVars) * 4;  // 3 MiB of eq tables
 constexpr size_t kAccBytes = (size_t)kMaxPoints * kMaxCopies * 8;       // 96 KiB of 64-bit sums
 // One arrival ticket per lane group of the reduction: a group covers 4 * tpr copies, so
 // 4096 copies at one thread per row slice (tpr = 1, when n_copies / 4 has no larger
 // divisor up to 32) give the most groups, 1024.
 constexpr uint32_t kMaxLaneGroups = kMaxCopies / 4;
 constexpr size_t kTicketBytes = (size_t)kMaxLaneGroups * 4;
-constexpr size_t kScratchBytes = kEqBytes + kAccBytes + kTicketBytes;
+constexpr size_t kScratchBytes = kAccBytes + kTicketBytes;
 
 // The scratch.  Host code must not use this name as an address (it is a host-side stand-in
 // for the symbol); the device address comes from cudaGetSymbolAddress below.
@@ -93,12 +92,11 @@ extern "C" int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     unsigned char* base = g_scratch_ptr[dev];
-    uint32_t* eq = reinterpret_cast<uint32_t*>(base);
-    gkrgpu::RedScratch red{reinterpret_cast<unsigned long long*>(base + kEqBytes),
-                           reinterpret_cast<unsigned int*>(base + kEqBytes + kAccBytes)};
+    gkrgpu::RedScratch red{reinterpret_cast<unsigned long long*>(base),
+                           reinterpret_cast<unsigned int*>(base + kAccBytes)};
 
     // The scratch keeps the previous call's contents: zero the sums and the ticket.
-    e = cudaMemsetAsync(base + kEqBytes, 0, kAccBytes + kTicketBytes, s);
+    e = cudaMemsetAsync(base, 0, kAccBytes + kTicketBytes, s);
     if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));
 
     gkrgpu::EqArgs a;
@@ -107,8 +105,6 @@ extern "C" int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t
     a.f1 = 1u;
     a.nvars = nb_vars;
     a.reps = (uint32_t)n_points;
-    e = gkrgpu::launch_eq(eq, a, s);
-    if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));
 
     gkrgpu::Geo g;
     g.N = n_copies;
@@ -118,7 +114,7 @@ extern "C" int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t
     g.rps = 256 / g.tpr;
     if (Q % g.tpr || Q / g.tpr > kMaxLaneGroups)
         return fail(GKRGPU_ERR_INVALID, "no row tile with at most 1024 lane groups for this copy count");
-    e = gkrgpu::launch_wsum(n_points, d_evals, 1ull << nb_vars, eq, g, 256, (uint32_t)g_sm_count[dev] * 4, red, d_out, s);
+    e = gkrgpu::launch_wsum(d_evals, a, g, 256, (uint32_t)g_sm_count[dev] * 4, red, d_out, s);
     if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));

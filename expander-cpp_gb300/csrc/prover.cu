@@ -296,6 +296,12 @@ struct Lane {
         memset(map_h, 0, need);
         done_seen = 0;
     }
+    // Reduction scratch of the entry points outside a proof (comps x N sums and the tickets),
+    // kept for the lane's life and left zeroed by every launch: allocating and clearing it per
+    // call cost more than a small call's kernel.
+    void* red_block = nullptr;
+    size_t red_cap = 0;
+    RedScratch scratch(uint64_t comps, uint64_t N);
     // The stream is idle: take the counter as consumed.
     void resync_done() { done_seen = *done_h(); }
     // Waits until `groups` more finishing CTAs have published their results.  A stream that
@@ -395,6 +401,7 @@ struct Lane {
         for (PinnedBuf* b : {&h_evals, &h_rows, &h_vx, &h_cv, &h_flag}) b->release();
         for (auto e : events) cudaEventDestroy(e);
         if (done_ev) cudaEventDestroy(done_ev);
+        if (red_block) cudaFree(red_block);
         if (stream) cudaStreamDestroy(stream);
     }
     size_t next_event() {
@@ -561,6 +568,21 @@ struct gkrgpu_ctx {
         mem_cv.notify_all();
     }
 };
+
+RedScratch Lane::scratch(uint64_t comps, uint64_t N) {
+    constexpr size_t kTickets = 4096;
+    const size_t need = align_up(comps * N * 8, 256) + kTickets;
+    if (need > red_cap) {
+        if (red_block) ck(cudaFree(red_block), "reduction scratch");
+        red_block = nullptr;
+        red_cap = 0;
+        ck(cudaMalloc(&red_block, need), "reduction scratch");
+        red_cap = need;
+        ck(cudaMemsetAsync(red_block, 0, need, stream), "cudaMemsetAsync");
+    }
+    char* b = static_cast<char*>(red_block);
+    return RedScratch{reinterpret_cast<unsigned long long*>(b + kTickets), reinterpret_cast<unsigned int*>(b)};
+}
 
 template <class F>
 void Lane::launch(int kid, double algo_bytes, F&& f) {
@@ -802,7 +824,7 @@ struct Workspace {
     uint32_t *hg0[3] = {}, *hgA[3] = {}, *fA[3] = {}, *fB[3] = {};
     uint32_t* hgF[3] = {};  // hg of round 0 of the phases that run in one launch
     uint32_t* sb[2] = {};
-    uint32_t *eqc = nullptr, *eqrx = nullptr, *evals = nullptr, *vx = nullptr, *cv = nullptr;
+    uint32_t *evals = nullptr, *vx = nullptr, *cv = nullptr;
     uint32_t* p2s = nullptr;  // 9R x N sums of phase-two rounds 0 and 1 (launch_p2_round01)
     uint4 *a4 = nullptr, *w4 = nullptr, *w4r = nullptr;
     unsigned long long* acc = nullptr;
@@ -821,7 +843,7 @@ struct Workspace {
             return p;
         };
         const uint64_t rowb = (uint64_t)N * 4;
-        const uint64_t maxI = 1ull << C.max_in_vars, maxO = 1ull << C.max_out_vars;
+        const uint64_t maxI = 1ull << C.max_in_vars;
         const uint64_t rows = C.value_rows() - (own_input ? 0 : C.in_rows(0));
         vals = (uint32_t*)take(rows * rowb);
         if (sumcheck) {
@@ -835,13 +857,11 @@ struct Workspace {
             sstride = align_up(maxI, 64);
             sb[0] = (uint32_t*)take(R * sstride * 4);
             sb[1] = (uint32_t*)take(R * sstride * 4);
-            eqrx = (uint32_t*)take(R * maxI * 4);
             a4 = (uint4*)take(maxI * 16);
             w4 = (uint4*)take(std::max<uint64_t>(C.max_mul, 1) * 16);
             w4r = (uint4*)take(std::max<uint64_t>(C.max_mul, 1) * 16);
             p2s = (uint32_t*)take(27ull * N * 4);
         }
-        eqc = (uint32_t*)take(R * maxO * 4);
         evals = (uint32_t*)take(9ull * N * 4);
         vx = (uint32_t*)take(3ull * N * 4);
         cv = (uint32_t*)take(3ull * N * 4);
@@ -858,6 +878,21 @@ uint64_t workspace_bytes(const gkrgpu_circuit& C, uint32_t N, int R, bool own_in
     Workspace w;
     w.plan(nullptr, C, N, R, own_input, sumcheck);
     return w.total;
+}
+
+// f1 eq(r1_j, z) + f2 eq(r2_j, z) over nvars bits (r2 null: the first alone).
+EqArgs eq_args(int reps, const uint32_t (*r1)[32], const uint32_t (*r2)[32], uint32_t f1, uint32_t f2, uint32_t nvars) {
+    EqArgs a;
+    memset(&a, 0, sizeof(a));
+    for (int j = 0; j < reps; j++) {
+        memcpy(a.r1[j], r1[j], 4 * nvars);
+        if (r2) memcpy(a.r2[j], r2[j], 4 * nvars);
+    }
+    a.f1 = f1;
+    a.f2 = r2 ? f2 : 0u;
+    a.nvars = nvars;
+    a.reps = (uint32_t)reps;
+    return a;
 }
 
 // ------------------------------------------------------------------ persistent phase slots
@@ -1128,20 +1163,6 @@ struct Prover {
         }
     }
 
-    void eq_table(uint32_t* out, uint32_t (*r1)[32], uint32_t (*r2)[32], uint32_t f1, uint32_t f2, uint32_t nvars) {
-        EqArgs a;
-        memset(&a, 0, sizeof(a));
-        for (int j = 0; j < R; j++) {
-            memcpy(a.r1[j], r1[j], 4 * nvars);
-            if (r2) memcpy(a.r2[j], r2[j], 4 * nvars);
-        }
-        a.f1 = f1;
-        a.f2 = r2 ? f2 : 0u;
-        a.nvars = nvars;
-        a.reps = R;
-        c.launch(K_EQ, 4.0 * R * (double)(1ull << nvars), [&] { return launch_eq(out, a, c.stream); });
-    }
-
     // Phase one's rounds launched one by one, the persistent part from round kt1 (n: none).
     void phase_one_rounds(Transcript& t, size_t li, uint32_t kt1, uint32_t alpha, uint32_t beta, uint32_t (*rx)[32]) {
         const DevLayer& Ly = C.layers[li];
@@ -1374,7 +1395,7 @@ struct Prover {
                         uint32_t beta, uint32_t (*rx)[32], uint32_t (*ry)[32]) {
         const DevLayer& Ly = C.layers[li];
         const uint32_t n = Ly.nin, m = Ly.nout;
-        const uint64_t I = 1ull << n, O = 1ull << m;
+        const uint64_t I = 1ull << n;
         const uint64_t rowb = (uint64_t)N * 4;
         const double rb = 4.0 * N;
         uint32_t* v = vals[li];
@@ -1382,12 +1403,12 @@ struct Prover {
         std::vector<uint32_t> vy((size_t)R * N);
         const uint64_t RN = (uint64_t)R * N;
 
-        // phase one: eqc_j = alpha eq(rz1_j) + beta eq(rz2_j), gate weights, hg + round 0
+        // phase one: gate weights for eqc_j = alpha eq(rz1_j) + beta eq(rz2_j)
         c.tag = ((uint32_t)li << 16) | (1u << 8);
-        eq_table(ws.eqc, rz1, rz2, alpha, beta, m);
-        const double wb = 32.0 * Ly.nmul + 20.0 * I + 8.0 * Ly.nadd + 4.0 * R * (Ly.nmul + Ly.nadd);
+        const EqArgs eqc = eq_args(R, rz1, rz2, alpha, beta, m);
+        const double wb = 32.0 * Ly.nmul + 20.0 * I + 8.0 * Ly.nadd;
         c.launch(K_WEIGHTS, wb, [&] {
-            return launch_weights(I, Ly.nmul, O, ws.eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, R, c.stream);
+            return launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, c.stream);
         });
         // the rounds on small tables run in one persistent launch: every round of a small layer,
         // otherwise from round 4 on (rounds 2 and 3 refold the input and recompute
@@ -1405,17 +1426,14 @@ struct Prover {
 
         // phase two: h(y) = vx * s(y)
         c.tag = ((uint32_t)li << 16) | (2u << 8);
-        eq_table(ws.eqrx, rx, nullptr, 1u, 0u, n);
+        const EqArgs eqx = eq_args(R, rx, nullptr, 1u, 0u, n);
         const size_t sstride = ws.sstride;
         const uint32_t kt2 = phase_start(n, 3);
         const bool fused01 = kt2 != 0 && n >= 3 && p2_round01_groups(N) > 0;
-        c.launch(K_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 4.0 * R * I + 8.0 * R * Ly.nmul + (fused01 ? 4.0 * R * I : 0.0),
-                 [&] {
-                     return fused01 ? launch_s_build4(I, O, Ly.my_off, Ly.my_g, ws.eqc, ws.eqrx, ws.sb[0], ws.sb[1],
-                                                      sstride, R, c.stream)
-                                    : launch_s_build(I, O, Ly.my_off, Ly.my_g, ws.eqc, ws.eqrx, ws.sb[0], sstride,
-                                                     R, c.stream);
-                 });
+        c.launch(K_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 4.0 * R * I * (fused01 ? 2 : 1), [&] {
+            return launch_s_build(I, Ly.my_off, Ly.my_g, eqc, eqx, ws.sb[0], fused01 ? ws.sb[1] : nullptr, sstride,
+                                  c.stream);
+        });
         PhaseArgs a2 = {};
         a2.n = n;
         a2.v = v;
@@ -1457,11 +1475,10 @@ struct Prover {
         uint32_t alpha = 1, beta = 0;
 
         // claimed_v[j] = eval_multilinear(output, rz1[j]) = sum_z eq(rz1_j, z) out[z]
-        eq_table(ws.eqc, rz1, nullptr, 1u, 0u, nz);
         const uint64_t OL = C.out_rows(L - 1);
-        c.launch(K_WSUM, 4.0 * N * OL + 4.0 * R * OL, [&] {
-            return launch_wsum(R, vals[L], OL, ws.eqc, gk[K_WSUM], X.block, ck_ctas[K_WSUM], red(),
-                               mapped(true, 6ull * N), c.stream);
+        c.launch(K_WSUM, 4.0 * N * OL, [&] {
+            return launch_wsum(vals[L], eq_args(R, rz1, nullptr, 1u, 0u, nz), gk[K_WSUM], X.block, ck_ctas[K_WSUM],
+                               red(), mapped(true, 6ull * N), c.stream);
         });
         c.sync();
         require_canonical();
@@ -2109,37 +2126,26 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
         if (g.tpr * ((n_copies / 4) / g.tpr) != n_copies / 4) fail(GKRGPU_ERR_INVALID, "no row tile divides n_copies");
         if ((n_copies / 4) / g.tpr > 1024) fail(GKRGPU_ERR_INVALID, "more than 1024 lane groups");
         on_idle_lane(ctx, [&](Lane& c) {
-            const uint64_t rows = 1ull << nb_vars, rowb = (uint64_t)n_copies * 4;
-            const size_t eq_b = align_up(n_points * rows * 4, 256), acc_b = align_up(9ull * n_copies * 8, 256);
-            const size_t cv_b = align_up(3 * rowb, 256), total = eq_b + acc_b + 4096 + cv_b;
-            void* p = nullptr;
-            ck(cudaMallocFromPoolAsync(&p, total, ctx->pool, c.stream), "workspace allocation");
-            char* base = static_cast<char*>(p);
-            uint32_t* eq = reinterpret_cast<uint32_t*>(base);
-            RedScratch red{reinterpret_cast<unsigned long long*>(base + eq_b),
-                           reinterpret_cast<unsigned int*>(base + eq_b + acc_b)};
-            uint32_t* cv = reinterpret_cast<uint32_t*>(base + eq_b + acc_b + 4096);
-            struct Free {
-                void* p;
-                cudaStream_t s;
-                ~Free() { cudaFreeAsync(p, s); }
-            } guard{p, c.stream};
-            ck(cudaMemsetAsync(base + eq_b, 0, acc_b + 4096, c.stream), "cudaMemsetAsync");
-            c.h_cv.ensure(3 * rowb, "pinned claims");
+            const uint64_t rowb = (uint64_t)n_copies * 4;
             EqArgs a;
             memset(&a, 0, sizeof(a));
             for (int j = 0; j < n_points; j++) memcpy(a.r1[j], r + (size_t)j * nb_vars, 4 * nb_vars);
             a.f1 = 1u;
             a.nvars = nb_vars;
             a.reps = n_points;
-            c.launch(K_EQ, 4.0 * n_points * rows, [&] { return launch_eq(eq, a, c.stream); });
-            c.launch(K_WSUM, 4.0 * n_copies * rows + 4.0 * n_points * rows, [&] {
-                return launch_wsum(n_points, d_evals, rows, eq, g, ctx->block, ctx->cta_budget(K_WSUM), red, cv,
-                                   c.stream);
+            // the result goes straight to the lane's mapped staging
+            RedScratch red = c.scratch(n_points, n_copies);
+            c.ensure_mapped(0, n_points * rowb);
+            c.resync_done();
+            red.done = c.done_d();
+            c.launch(K_WSUM, (double)rowb * (double)(1ull << nb_vars), [&] {
+                return launch_wsum(d_evals, a, g, ctx->block, ctx->cta_budget(K_WSUM), red,
+                                   reinterpret_cast<uint32_t*>(c.extra_d()), c.stream);
             });
-            c.copy(c.h_cv.p, cv, n_points * rowb, cudaMemcpyDeviceToHost, "result readback");
-            c.sync();
-            memcpy(out, c.h_cv.p, n_points * rowb);
+            c.pending_bytes = 0;  // spin: the caller's thread may not sleep to the microsecond
+            c.wait_done((n_copies / 4) / g.tpr);
+            memcpy(out, c.extra_h(), n_points * rowb);
+            if (ctx->timing) c.sync();  // the launch's closing event
             c.resolve_events();
         });
     });
