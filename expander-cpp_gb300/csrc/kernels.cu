@@ -34,7 +34,7 @@ namespace gkrgpu {
 const char* const kKernelNames[K_NUM_KERNELS] = {"check_canonical", "evaluate", "gate_weights",
                                                  "hg_build_round0", "round_fold_lane", "round_fold_scalar",
                                                  "phase2_s_build", "weighted_row_sum", "hg_rebuild_round1",
-                                                 "verifier_gate_sums", "canonicalize", "phase2_round0", "stage_words", "round_tail",
+                                                 "verifier_gate_sums", "canonicalize", "phase2_round0", "stage_words", "round_tail", "hg_build",
                                                  "bn254_load",
                                                  "bn254_evaluate", "bn254_eq_table", "bn254_gate_weights",
                                                  "bn254_hg_build_round0", "bn254_round_fold_lane",
@@ -326,6 +326,61 @@ __global__ void __launch_bounds__(256) k_weights(uint64_t I, uint64_t Gm, const 
             }
             a_out[i] = make_uint4(s[0], s[1], s[2], 0u);
         }
+    }
+}
+
+// hg of a layer whose phase one runs in one launch (phase.cu), with a copy of the layer input,
+// in the CTAs' own tables: hg_j(x) = sum over add gates (z, x, c) of c eqc_j(z) + sum over mul
+// gates (z, x, y, c) of c eqc_j(z) v(y), the weights computed where they are used (a thread per
+// row and four copies; the factors are few products next to a launch that stored them).
+// Building it inside the phase, whose few CTAs have a chain of three gathers a row, took 11 us
+// of a 63 us phase at 2^10 rows and 16 copies.
+__global__ void __launch_bounds__(256) k_hg_build(const uint32_t* __restrict__ v, uint32_t I, uint32_t N, uint32_t tpr,
+                                                  const __grid_constant__ EqArgs eqc, const uint32_t* __restrict__ mx_off,
+                                                  const uint4* __restrict__ mx_g, const uint32_t* __restrict__ ax_off,
+                                                  const uint2* __restrict__ ax_g, uint4* __restrict__ priv,
+                                                  size_t priv_stride) {
+    __shared__ uint32_t t[2 * kEqWords];
+    eq_build(t, eqc);
+    __syncthreads();
+    const uint32_t nd = eq_digits(eqc), reps = eqc.reps, Q = N / 4;
+    const bool two = eqc.f2 != 0;
+    const uint64_t total = (uint64_t)I * Q, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const uint32_t x = (uint32_t)(i / Q), quad = (uint32_t)(i - (uint64_t)x * Q);
+        const uint32_t m0 = __ldg(mx_off + x), m1 = __ldg(mx_off + x + 1);
+        const uint32_t a0 = __ldg(ax_off + x), a1 = __ldg(ax_off + x + 1);
+        uint32_t s[3] = {0u, 0u, 0u};
+        for (uint32_t k = a0; k < a1; k++) {
+            const uint2 gt = __ldg(ax_g + k);  // (z, c)
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+                if (j < reps) s[j] = add(s[j], mul(gt.y, eq_at(t, nd, two, j, gt.x)));
+        }
+        uint64_t h[3][4];
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+#pragma unroll
+            for (int l = 0; l < 4; l++) h[j][l] = s[j];
+        for (uint32_t k = m0; k < m1; k++) {
+            const uint4 gt = __ldg(mx_g + k);  // (y, z, c, 0)
+            const uint4 vy = ld4(v, gt.x, N, 4 * quad);
+#pragma unroll
+            for (uint32_t j = 0; j < 3; j++)
+                if (j < reps) {
+                    const uint32_t w = mul(gt.z, eq_at(t, nd, two, j, gt.y));
+#pragma unroll
+                    for (int l = 0; l < 4; l++) h[j][l] = fold64(h[j][l] + (uint64_t)comp(vy, l) * w);
+                }
+        }
+        const uint32_t at = (I >= 4 ? (x & 3) * (I >> 2) + (x >> 2) : x) * tpr + quad % tpr;  // place() of phase.cu
+        uint4* o = priv + (size_t)(quad / tpr) * priv_stride + at;
+        o[0] = ld4(v, x, N, 4 * quad);
+#pragma unroll
+        for (uint32_t j = 0; j < 3; j++)
+            if (j < reps)
+                o[(size_t)(1 + j) * I * tpr] =
+                    make_uint4(reduce64(h[j][0]), reduce64(h[j][1]), reduce64(h[j][2]), reduce64(h[j][3]));
     }
 }
 
@@ -1633,6 +1688,14 @@ cudaError_t launch_scale_weights(uint64_t I, const uint32_t* mx_off, const uint4
 cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgs& eqc, const uint4* mx_g, const uint32_t* ax_off,
                            const uint2* ax_g, uint4* a_out, uint4* w_out, cudaStream_t s) {
     k_weights<<<grid_1d(I > Gm ? I : Gm, 256), 256, 0, s>>>(I, Gm, eqc, mx_g, ax_off, ax_g, a_out, w_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_hg_build(const uint32_t* v, uint32_t I, uint32_t N, uint32_t tpr, const EqArgs& eqc,
+                            const uint32_t* mx_off, const uint4* mx_g, const uint32_t* ax_off, const uint2* ax_g,
+                            uint4* priv, size_t priv_stride, cudaStream_t s) {
+    k_hg_build<<<grid_1d((uint64_t)I * (N / 4), 256), 256, 0, s>>>(v, I, N, tpr, eqc, mx_off, mx_g, ax_off, ax_g, priv,
+                                                                  priv_stride);
     return cudaGetLastError();
 }
 

@@ -57,30 +57,30 @@ struct RoundPtrs {
 };
 
 // Persistent sumcheck phase (k_phase, phase.cu): rounds k0 .. n-1 in one launch, one CTA per
-// 4 tpr copies.  Round k folds the tables of round k-1 at its challenges (round k leaves
-// 2^(n-k) rows in A when k is odd, in B when k is even, or in shared memory), and publishes
-// the round's evaluations to evals_out, every word with `parity ^ (k - k0)` in bit 31; the
-// last round also publishes rows 0..1 of each repetition's folded f table to rows_out (bit 31:
-// rows_parity).  With k0 = 0 the first round reads the layer input v (2^n rows): phase one
-// builds hg into h0 from the gate weights, phase two takes the scalar tables s, and round 1
-// folds v and h0 / s.  With k0 > 0 the first round folds stored tables (f and hg of round
-// k0 - 1, or f and the scalar tables s) at r_first.
+// 4 tpr copies.  Round k folds the tables of round k-1 at its challenges and publishes its
+// evaluations to evals_out, every word with `parity ^ (k - k0)` in bit 31; the last round also
+// publishes rows 0..1 of each repetition's folded f table to rows_out (bit 31: rows_parity).
+// The tables are the CTAs' own (priv, priv_stride quads of copies each).  With k0 = 0 they hold
+// the layer input (2^n rows) and, in phase one, hg (launch_hg_build); phase two takes the
+// scalar tables s.  With k0 > 0 the first round folds the caller's tables of round k0 - 1
+// (fsrc, hsrc or s; 2^(n-k0+1) rows of N copies) at r_first.
 // The challenges of round k come from the host through the mailbox (host-mapped words
 // [4k .. 4k+2] = r_j(k) with bit 31 set, [4k+3] abort; cleared by the host before the launch).
 // Each wait is bounded by wait_ns: when it expires the kernel sets *err and returns; a
 // nonzero abort word makes it return at once.
 constexpr uint32_t kMboxRounds = 32;
 constexpr uint32_t kMboxWords = 4 * kMboxRounds;
-// Rows x tpr of the first round's source tables: a CTA reads all of its rows alone.
-constexpr uint32_t kPhaseItems = 4096;
+// Rows x tpr of the tables the first round reads: a CTA reads all of its rows alone.  A layer
+// whose input is within kPhaseItems runs its phases whole (2^13 rows of 112 copies: 12 layers
+// in 5.83 ms against 6.40 from round 4 on); a larger layer's last rounds start where their
+// tables are within kPhaseTailItems (1024 copies, two quads a CTA: 2048 rows; at 4096 rows the
+// rounds launched over the whole chip are as fast).
+constexpr uint32_t kPhaseItems = 8192, kPhaseTailItems = 4096;
 struct PhaseArgs {
-    const uint32_t* v;        // k0 = 0: the layer input
-    uint32_t *fA[3], *fB[3];  // per-copy f tables
-    uint32_t *hA[3], *hB[3];  // phase one: per-copy hg tables
-    uint32_t* h0[3];          // phase one, k0 = 0: hg of round 0 (2^n rows)
+    uint4* priv;
+    size_t priv_stride;
+    const uint32_t *fsrc[3], *hsrc[3];  // k0 > 0
     const uint32_t* s[3];     // phase two: scalar tables the first round reads
-    const uint32_t* mx_off;   // phase one, k0 = 0: mul gates by first input, weights (k_weights)
-    const uint4 *mx_g, *a4, *w4;
     const uint32_t* vx;       // phase two: R x N claims the sums are multiplied by
     uint32_t r_first[3];      // k0 > 0: challenges of round k0 - 1
     uint32_t k0, n, reps, N, tpr;
@@ -113,6 +113,7 @@ enum KernelId {
     K_P2_ROUND0,
     K_STAGE,  // small transfers between device and host-mapped memory
     K_TAIL,   // rounds of a phase in one persistent launch (k_phase)
+    K_HG_BUILD,  // hg of such a phase (k_hg_build)
     // BN254 kernels (bn254.cuh)
     K_BN_LOAD,
     K_BN_EVALUATE,
@@ -230,7 +231,13 @@ cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g
 // most max_ctas of them (0: none does), and the launch.
 uint32_t phase_tpr(uint32_t N, uint32_t max_ctas);
 uint32_t phase_ctas(uint32_t N, uint32_t tpr);
+// Quads a CTA's tables take when the first round reads `items` rows x tpr.
+size_t phase_priv_quads(uint64_t items);
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s);
+// The layer input (I rows) and hg in the tables of a phase-one launch with k0 = 0.
+cudaError_t launch_hg_build(const uint32_t* v, uint32_t I, uint32_t N, uint32_t tpr, const EqArgs& eqc,
+                            const uint32_t* mx_off, const uint4* mx_g, const uint32_t* ax_off, const uint2* ax_g,
+                            uint4* priv, size_t priv_stride, cudaStream_t s);
 // eval_multilinear of vals (2^eq.nvars rows) at eq.r1_j for eq.reps points (eq.f1 = 1, no second
 // point): out receives reps x N.
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,

@@ -12,12 +12,21 @@
 // So the copies are split over CTAs and nothing else is: each CTA owns 4 tpr copies and every
 // row of them, its sums stay inside the CTA, and no CTA waits on another.  The repetitions
 // are split over the CTA's warps (4 warps each), which keeps a thread at one repetition's
-// sums.  Small tables sit in shared memory, larger ones go through L1/L2.
+// sums.
+//
+// A CTA's tables are its own, [row][4 tpr copies], with the rows r of equal r mod 4 side by
+// side: a round reads rows 4i .. 4i+3 in four contiguous streams (with the rows of the
+// caller's tables, N copies apart, every lane of a load touches another line, which made the
+// first two rounds of 2^10 rows 18 us of 63).  Tables of up to 1024 words are in shared memory
+// and taken one copy a thread, which leaves a quarter of the instructions on the chain of a
+// late round (3400 clocks with four copies a thread).
 //
 // Host traffic without fences or counters: an M31 value leaves bit 31 free, so every word
 // published to the host carries the round's parity there, and the host takes a word when its
 // parity is the round's; likewise the host's challenges carry bit 31 in a 16-byte mailbox slot
-// per round (r_0, r_1, r_2, abort) that it clears before the launch, read in one load.
+// per round (r_0, r_1, r_2, abort) that it clears before the launch, read in one load.  A
+// word there and one back take 1.47 us, two turns of polling; loads of the slot in flight
+// together do not shorten that (they come back one after another, 1400 clocks apart).
 #include <atomic>
 
 #include "kernels.cuh"
@@ -60,12 +69,10 @@ __device__ __forceinline__ uint4 ld_mailbox(const uint32_t* p) {
     return v;
 }
 
-// A per-copy table as one thread sees it: row r at p[r * stride] (four copies).
-struct Rows {
-    uint4* p;
-    size_t stride;
-    __device__ __forceinline__ uint4& operator[](uint32_t r) const { return p[(size_t)r * stride]; }
-};
+// Place of row r in a table of `rows` rows (a power of two): rows of equal r mod 4 side by side.
+__device__ __forceinline__ uint32_t place(uint32_t rows, uint32_t r) {
+    return rows >= 4 ? (r & 3) * (rows >> 2) + (r >> 2) : r;
+}
 
 // p0 += f0 h0, p1 += f1 h1, p2raw += (f0 + f1)(h0 + h1), unreduced in 64 bits.
 __device__ __forceinline__ void accum(uint64_t (&acc)[3][4], const uint4& f0, const uint4& f1, const uint4& h0,
@@ -78,33 +85,25 @@ __device__ __forceinline__ void accum(uint64_t (&acc)[3][4], const uint4& f0, co
     }
 }
 
-// hg_j of input row x for four copies: a_j[x] + sum over its mul gates (x, y, k) of
-// v[y] w_j[k]; gates in pairs, so that two gathers are in flight.
-__device__ __forceinline__ uint4 build_h(const PhaseArgs& a, uint32_t j, uint32_t x, const uint4* v, size_t stride) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(a.w4) + j;
-    uint32_t k = __ldg(a.mx_off + x);
-    const uint32_t k1 = __ldg(a.mx_off + x + 1);
-    const uint32_t a0 = __ldg(reinterpret_cast<const uint32_t*>(a.a4 + x) + j);
-    if (k == k1) return make_uint4(a0, a0, a0, a0);
-    uint64_t s[4] = {a0, a0, a0, a0};
-    for (; k + 1 < k1; k += 2) {
-        const uint32_t y0 = __ldg(&a.mx_g[k].x), y1 = __ldg(&a.mx_g[k + 1].x);
-        const uint32_t w0 = __ldg(w + 4 * (size_t)k), w1 = __ldg(w + 4 * (size_t)k + 4);
-        const uint4 v0 = __ldg(v + y0 * stride), v1 = __ldg(v + y1 * stride);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            mad64(s[l], comp(v0, l), w0);
-            mad64(s[l], comp(v1, l), w1);
-            s[l] = fold64(s[l]);
+// Waits for the challenges of a round in its mailbox slot: 0 they are in rch, 1 abort, 2 the
+// limit passed.
+__device__ __forceinline__ int wait_challenge(const uint32_t* box, uint32_t R, unsigned long long wait_ns, uint32_t* rch) {
+    uint64_t t0 = 0;
+    for (uint32_t it = 0;; it++) {
+        const uint4 m = ld_mailbox(box);
+        if ((m.x & (R > 1 ? m.y : m.x) & (R > 2 ? m.z : m.x)) >> 31) {
+            rch[0] = m.x & m31::P;
+            rch[1] = m.y & m31::P;
+            rch[2] = m.z & m31::P;
+            return 0;
         }
+        if (m.w) return 1;
+        if (it < kSpins) continue;
+        const uint64_t now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 > wait_ns) return 2;
+        __nanosleep(100);
     }
-    if (k < k1) {
-        const uint32_t y0 = __ldg(&a.mx_g[k].x), w0 = __ldg(w + 4 * (size_t)k);
-        const uint4 v0 = __ldg(v + y0 * stride);
-#pragma unroll
-        for (int l = 0; l < 4; l++) mad64(s[l], comp(v0, l), w0);
-    }
-    return make_uint4(reduce64(s[0]), reduce64(s[1]), reduce64(s[2]), reduce64(s[3]));
 }
 
 template <bool LANE_HG>
@@ -112,133 +111,153 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
     extern __shared__ uint4 psm[];
     __shared__ uint32_t rch[3];
     __shared__ int stop;
-    const uint32_t R = a.reps, tid = threadIdx.x, tpr = a.tpr, N = a.N;
-    const uint32_t warp = tid >> 5, j = warp / kWarps, t = tid - j * kRepThreads;
+    const uint32_t R = a.reps, tid = threadIdx.x, tpr = a.tpr, N = a.N, L = 4 * tpr;
+    const uint32_t warp = tid >> 5, j = warp / kWarps, w = warp - j * kWarps, t = tid - j * kRepThreads;
     const uint32_t q = t & (tpr - 1), slot = t / tpr, nslots = kRepThreads / tpr;
     const uint32_t quad = blockIdx.x * tpr + q;  // this thread's four copies: 4 quad ..
     const bool active = 4 * quad < N;
-    const size_t gs = N / 4;  // row stride of a table in memory
+    // the CTA's tables in memory: the layer input and hg_0 of each repetition (k0 = 0), then
+    // two buffers of up to six tables; the first folding round kf leaves S1 rows
+    const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf), I = 1u << a.n;
+    uint4* const mine = a.priv + (size_t)blockIdx.x * a.priv_stride;
+    uint4* const folded = mine + (a.k0 ? 0u : (1 + 3) * I * tpr);
     // shared memory: two buffers of small tables (f, then hg in phase one), phase two's scalar
-    // tables (two buffers), the warps' partial sums
+    // tables (two buffers), partial sums
     constexpr uint32_t kTabs = LANE_HG ? 6 : 3;
-    const uint32_t kf = a.k0 ? a.k0 : 1;  // the first round that folds
-    const uint32_t S1 = 1u << (a.n - kf);
     uint32_t* const sbuf = reinterpret_cast<uint32_t*>(psm + 2 * kTabs * kSmemRows);
     uint32_t* const part = sbuf + (LANE_HG ? 0 : 3 * (S1 + S1 / 2));
     // the table round k leaves (2^(n-k) rows): which = 0 f, 1 hg of this thread's repetition
-    auto table = [&](uint32_t k, uint32_t which) -> Rows {
-        const uint32_t rows = 1u << (a.n - k);
-        if (rows * tpr <= kSmemRows)
-            return Rows{psm + ((k & 1) * kTabs + which * 3 + j) * kSmemRows + q, tpr};
-        uint32_t* b;
-        if (which == 0) b = (k & 1) ? (j == 0 ? a.fA[0] : j == 1 ? a.fA[1] : a.fA[2]) : (j == 0 ? a.fB[0] : j == 1 ? a.fB[1] : a.fB[2]);
-        else b = (k & 1) ? (j == 0 ? a.hA[0] : j == 1 ? a.hA[1] : a.hA[2]) : (j == 0 ? a.hB[0] : j == 1 ? a.hB[1] : a.hB[2]);
-        return Rows{reinterpret_cast<uint4*>(b) + quad, gs};
+    auto in_smem = [&](uint32_t k) { return (tpr << (a.n - k)) <= kSmemRows; };
+    auto table = [&](uint32_t k, uint32_t which) -> uint4* {
+        if (in_smem(k)) return psm + ((k & 1) * kTabs + which * 3 + j) * kSmemRows;
+        const uint32_t odd = (k - kf) & 1;
+        return folded + ((odd ? 6 * S1 : 0) + (which * 3 + j) * (odd ? S1 / 2 : S1)) * tpr;
     };
-    // the stored tables the first round reads are in memory whatever their size
-    auto stored = [&](uint32_t which) -> Rows {
-        uint32_t* b;
-        if (which == 0) b = (a.k0 & 1) ? (j == 0 ? a.fB[0] : j == 1 ? a.fB[1] : a.fB[2]) : (j == 0 ? a.fA[0] : j == 1 ? a.fA[1] : a.fA[2]);
-        else b = (a.k0 & 1) ? (j == 0 ? a.hB[0] : j == 1 ? a.hB[1] : a.hB[2]) : (j == 0 ? a.hA[0] : j == 1 ? a.hA[1] : a.hA[2]);
-        return Rows{reinterpret_cast<uint4*>(b) + quad, gs};
-    };
-    const uint4* const v = reinterpret_cast<const uint4*>(a.v) + quad;
-    uint4* const h0t = reinterpret_cast<uint4*>(j == 0 ? a.h0[0] : j == 1 ? a.h0[1] : a.h0[2]) + quad;
     const uint32_t* const s0t = j == 0 ? a.s[0] : j == 1 ? a.s[1] : a.s[2];
-    // the finisher's (repetition, copy) of this thread and phase two's factor v(rx) there
-    const uint32_t fj = tid / (4 * tpr), fl = tid - fj * 4 * tpr, flane = blockIdx.x * 4 * tpr + fl;
-    const bool finisher = fj < R && flane < N;
+    // the first 4 tpr threads of a repetition finish its copies; phase two's factor v(rx) there
+    const uint32_t flane = blockIdx.x * L + t;
+    const bool finisher = t < L && flane < N;
     uint32_t xv = 0;
-    if (!LANE_HG && finisher) xv = __ldcv(a.vx + (size_t)fj * N + flane);
+    if (!LANE_HG && finisher) xv = __ldcv(a.vx + (size_t)j * N + flane);
     if (tid == 0) stop = 0;
 
     for (uint32_t k = a.k0; k < a.n; k++) {
         if (k == a.k0) {
             if (tid < 3) rch[tid] = tid == 0 ? a.r_first[0] : tid == 1 ? a.r_first[1] : a.r_first[2];
         } else if (tid == 0) {
-            const uint32_t* box = a.mbox + 4 * (k - 1);
-            uint64_t t0 = 0;
-            for (uint32_t it = 0;; it++) {
-                const uint4 m = ld_mailbox(box);
-                uint32_t ok = m.x;
-                if (R > 1) ok &= m.y;
-                if (R > 2) ok &= m.z;
-                if (ok >> 31) {
-                    rch[0] = m.x & m31::P;
-                    rch[1] = m.y & m31::P;
-                    rch[2] = m.z & m31::P;
-                    break;
-                }
-                if (m.w) {
-                    stop = 1;
-                    break;
-                }
-                if (it < kSpins) continue;
-                const uint64_t now = global_ns();
-                if (t0 == 0) t0 = now;
-                if (now - t0 > a.wait_ns) {
-                    *reinterpret_cast<volatile unsigned int*>(a.err) = 1u;
-                    stop = 1;
-                    break;
-                }
-                __nanosleep(100);
-            }
+            const int got = wait_challenge(a.mbox + 4 * (k - 1), R, a.wait_ns, rch);
+            if (got == 2) *reinterpret_cast<volatile unsigned int*>(a.err) = 1u;
+            if (got) stop = 1;
         }
         __syncthreads();  // the challenges, and the previous round's tables, are visible
         if (stop) return;
-        const uint32_t npairs = 1u << (a.n - k - 1);
+        const uint32_t npairs = 1u << (a.n - k - 1), out_rows = 2 * npairs;
         const m31::Lerp c = m31::lerp_at(rch[j]);
-        uint64_t acc[3][4] = {};
-        uint32_t since = 0;
-        if (active) {
-            if (k == 0) {
+        // phase two's scalar tables: read from memory by the first round that folds them
+        const bool odd = (k - kf) & 1;
+        const uint32_t* ssrc = k <= kf ? s0t : (odd ? sbuf + j * S1 : sbuf + 3 * S1 + j * (S1 / 2));
+        uint32_t* sdst = odd ? sbuf + 3 * S1 + j * (S1 / 2) : sbuf + j * S1;
+        uint32_t ns;  // partial sums per copy and repetition
+        if (k > kf && in_smem(k - 1)) {
+            // one copy a thread: pair idx / L, copy idx % L; at most two pairs a thread
+            const uint32_t* fs = reinterpret_cast<const uint32_t*>(table(k - 1, 0));
+            uint32_t* fd = reinterpret_cast<uint32_t*>(table(k, 0));
+            const uint32_t* hs = LANE_HG ? reinterpret_cast<const uint32_t*>(table(k - 1, 1)) : nullptr;
+            uint32_t* hd = LANE_HG ? reinterpret_cast<uint32_t*>(table(k, 1)) : nullptr;
+            const uint32_t items = npairs * L;
+            uint64_t acc[3] = {0ull, 0ull, 0ull};
+            for (uint32_t idx = t; idx < items; idx += kRepThreads) {
+                const uint32_t i = idx / L, lane = idx & (L - 1);
+                const uint32_t f0 = m31::lerp(fs[idx], fs[items + idx], c);
+                const uint32_t f1 = m31::lerp(fs[2 * items + idx], fs[3 * items + idx], c);
+                const uint32_t o0 = place(out_rows, 2 * i) * L + lane, o1 = place(out_rows, 2 * i + 1) * L + lane;
+                uint32_t h0, h1;
+                if (LANE_HG) {
+                    h0 = m31::lerp(hs[idx], hs[items + idx], c);
+                    h1 = m31::lerp(hs[2 * items + idx], hs[3 * items + idx], c);
+                    hd[o0] = h0;
+                    hd[o1] = h1;
+                } else {
+                    const uint4 s = reinterpret_cast<const uint4*>(ssrc)[i];
+                    h0 = m31::lerp(s.x, s.y, c);
+                    h1 = m31::lerp(s.z, s.w, c);
+                    if (lane == 0) reinterpret_cast<uint2*>(sdst)[i] = make_uint2(h0, h1);
+                }
+                fd[o0] = f0;
+                fd[o1] = f1;
+                mad64(acc[0], f0, h0);
+                mad64(acc[1], f1, h1);
+                mad64(acc[2], m31::add(f0, f1), m31::add(h0, h1));
+            }
+            // threads of one copy: within a warp when a pair's copies fit in one
+            const uint32_t used = items < kRepThreads ? items : kRepThreads;
+            ns = L <= 32 ? (used + 31) / 32 : (used + L - 1) / L;
+            if (32 * w < used) {
+                uint32_t x[3];
+#pragma unroll
+                for (int e = 0; e < 3; e++) x[e] = reduce64(acc[e]);
+                for (uint32_t off = 16; off >= L; off >>= 1)
+#pragma unroll
+                    for (int e = 0; e < 3; e++) x[e] = m31::add(x[e], __shfl_xor_sync(0xffffffffu, x[e], off));
+                const uint32_t sl = L <= 32 ? w : t / L, lane = t & (L - 1);
+                if (L > 32 || (tid & 31) < L)
+#pragma unroll
+                    for (int e = 0; e < 3; e++) part[((j * kWarps + sl) * 3 + e) * L + lane] = x[e];
+            }
+        } else {
+            uint64_t acc[3][4] = {};
+            uint32_t since = 0;
+            auto tidy = [&] {
+                if ((++since & 3) == 0)
+#pragma unroll
+                    for (int l = 0; l < 4; l++)
+#pragma unroll
+                        for (int e = 0; e < 3; e++) acc[e][l] = fold64(acc[e][l]);
+            };
+            if (active && k == 0) {
+                const uint4 *fs = mine + q, *hs = mine + (1 + j) * I * tpr + q;
                 for (uint32_t i = slot; i < npairs; i += nslots) {
-                    const uint4 f0 = __ldg(v + (size_t)(2 * i) * gs), f1 = __ldg(v + (size_t)(2 * i + 1) * gs);
+                    const uint32_t o0 = place(out_rows, 2 * i) * tpr, o1 = place(out_rows, 2 * i + 1) * tpr;
                     uint4 h0, h1;
                     if (LANE_HG) {
-                        h0 = build_h(a, j, 2 * i, v, gs);
-                        h1 = build_h(a, j, 2 * i + 1, v, gs);
-                        h0t[(size_t)(2 * i) * gs] = h0;
-                        h0t[(size_t)(2 * i + 1) * gs] = h1;
+                        h0 = hs[o0];
+                        h1 = hs[o1];
                     } else {
                         const uint2 s = __ldg(reinterpret_cast<const uint2*>(s0t) + i);
                         h0 = make_uint4(s.x, s.x, s.x, s.x);
                         h1 = make_uint4(s.y, s.y, s.y, s.y);
                     }
-                    accum(acc, f0, f1, h0, h1);
-                    if ((++since & 3) == 0)
-#pragma unroll
-                        for (int l = 0; l < 4; l++)
-#pragma unroll
-                            for (int e = 0; e < 3; e++) acc[e][l] = fold64(acc[e][l]);
+                    accum(acc, fs[o0], fs[o1], h0, h1);
+                    tidy();
                 }
-            } else {
-                Rows fs, hs = {};
-                if (k == a.k0) fs = stored(0);
-                else if (k == 1) fs = Rows{const_cast<uint4*>(v), gs};
-                else fs = table(k - 1, 0);
-                const Rows fd = table(k, 0);
-                Rows hd = {};
-                const uint32_t* ssrc = nullptr;
-                uint32_t* sdst = nullptr;
-                if (LANE_HG) {
-                    if (k == a.k0) hs = stored(1);
-                    else if (k == 1) hs = Rows{h0t, gs};
-                    else hs = table(k - 1, 1);
-                    hd = table(k, 1);
+            } else if (active) {
+                // the first round reads the caller's tables (row r at r N + copy) when k0 > 0
+                const bool given = k == a.k0;
+                const uint4 *fs, *hs = nullptr;
+                if (given) {
+                    fs = reinterpret_cast<const uint4*>(j == 0 ? a.fsrc[0] : j == 1 ? a.fsrc[1] : a.fsrc[2]) + quad;
+                    if (LANE_HG) hs = reinterpret_cast<const uint4*>(j == 0 ? a.hsrc[0] : j == 1 ? a.hsrc[1] : a.hsrc[2]) + quad;
                 } else {
-                    ssrc = k == kf ? s0t : sbuf + ((k - kf) & 1 ? 0 : 3 * S1) + j * ((k - kf) & 1 ? S1 : S1 / 2);
-                    sdst = sbuf + ((k - kf) & 1 ? 3 * S1 : 0) + j * ((k - kf) & 1 ? S1 / 2 : S1);
+                    fs = (k == 1 ? mine : table(k - 1, 0)) + q;
+                    if (LANE_HG) hs = (k == 1 ? mine + (1 + j) * I * tpr : table(k - 1, 1)) + q;
                 }
+                // row 4i + e: at 4i + e of the caller's tables, at e rows / 4 + i of the CTA's
+                const size_t step = given ? N / 4 : tpr, ri = given ? 4 * step : step;
+                const size_t re = given ? step : (size_t)npairs * step;
+                uint4* fd = table(k, 0) + q;
+                uint4* hd = LANE_HG ? table(k, 1) + q : nullptr;
                 for (uint32_t i = slot; i < npairs; i += nslots) {
-                    const uint4 x0 = fs[4 * i], x1 = fs[4 * i + 1], x2 = fs[4 * i + 2], x3 = fs[4 * i + 3];
+                    const uint4* x = fs + i * ri;
+                    const uint4 x0 = x[0], x1 = x[re], x2 = x[2 * re], x3 = x[3 * re];
+                    const uint32_t o0 = place(out_rows, 2 * i) * tpr, o1 = place(out_rows, 2 * i + 1) * tpr;
                     uint4 h0, h1;
                     if (LANE_HG) {
-                        const uint4 y0 = hs[4 * i], y1 = hs[4 * i + 1], y2 = hs[4 * i + 2], y3 = hs[4 * i + 3];
+                        const uint4* y = hs + i * ri;
+                        const uint4 y0 = y[0], y1 = y[re], y2 = y[2 * re], y3 = y[3 * re];
                         h0 = lerp4(y0, y1, c);
                         h1 = lerp4(y2, y3, c);
-                        hd[2 * i] = h0;
-                        hd[2 * i + 1] = h1;
+                        hd[o0] = h0;
+                        hd[o1] = h1;
                     } else {
                         const uint4 s = reinterpret_cast<const uint4*>(ssrc)[i];
                         const uint32_t s0 = m31::lerp(s.x, s.y, c), s1 = m31::lerp(s.z, s.w, c);
@@ -247,44 +266,41 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
                         h1 = make_uint4(s1, s1, s1, s1);
                     }
                     const uint4 f0 = lerp4(x0, x1, c), f1 = lerp4(x2, x3, c);
-                    fd[2 * i] = f0;
-                    fd[2 * i + 1] = f1;
+                    fd[o0] = f0;
+                    fd[o1] = f1;
                     accum(acc, f0, f1, h0, h1);
-                    if ((++since & 3) == 0)
-#pragma unroll
-                        for (int l = 0; l < 4; l++)
-#pragma unroll
-                            for (int e = 0; e < 3; e++) acc[e][l] = fold64(acc[e][l]);
+                    tidy();
                 }
             }
-        }
-        // sums over the repetition's threads with the same q: shuffles within a warp, then the
-        // warps that had pairs (all of them when npairs tpr covers the repetition's threads)
-        const uint32_t nw = npairs * tpr >= kRepThreads ? kWarps : (npairs * tpr + 31) / 32;
-        const uint32_t w = warp - j * kWarps;
-        if (w < nw) {
-            uint32_t x[12];
-#pragma unroll
-            for (int e = 0; e < 3; e++)
-#pragma unroll
-                for (int l = 0; l < 4; l++) x[4 * e + l] = reduce64(acc[e][l]);
-            for (uint32_t off = 16; off >= tpr; off >>= 1)
-#pragma unroll
-                for (int e = 0; e < 12; e++) x[e] = m31::add(x[e], __shfl_xor_sync(0xffffffffu, x[e], off));
-            if ((tid & 31) < tpr)
+            // sums over the repetition's threads with the same q: shuffles within a warp, then
+            // the warps that had pairs
+            const uint32_t used = npairs * tpr < kRepThreads ? npairs * tpr : kRepThreads;
+            ns = (used + 31) / 32;
+            if (w < ns) {
+                uint32_t x[12];
 #pragma unroll
                 for (int e = 0; e < 3; e++)
 #pragma unroll
-                    for (int l = 0; l < 4; l++) part[((j * kWarps + w) * 3 + e) * 4 * tpr + 4 * q + l] = x[4 * e + l];
+                    for (int l = 0; l < 4; l++) x[4 * e + l] = reduce64(acc[e][l]);
+                for (uint32_t off = 16; off >= tpr; off >>= 1)
+#pragma unroll
+                    for (int e = 0; e < 12; e++) x[e] = m31::add(x[e], __shfl_xor_sync(0xffffffffu, x[e], off));
+                if ((tid & 31) < tpr)
+#pragma unroll
+                    for (int e = 0; e < 3; e++)
+#pragma unroll
+                        for (int l = 0; l < 4; l++) part[((j * kWarps + w) * 3 + e) * L + 4 * q + l] = x[4 * e + l];
+            }
         }
-        __syncthreads();
+        if (ns > 1) __syncthreads();  // (one warp's own sums and rows need no more than __syncwarp)
+        else __syncwarp();
         if (finisher) {
             uint32_t p0 = 0, p1 = 0, p2 = 0;
-            for (uint32_t i = 0; i < nw; i++) {
-                const uint32_t* s = part + (fj * kWarps + i) * 3 * 4 * tpr + fl;
+            for (uint32_t i = 0; i < ns; i++) {
+                const uint32_t* s = part + (j * kWarps + i) * 3 * L + t;
                 p0 = m31::add(p0, s[0]);
-                p1 = m31::add(p1, s[4 * tpr]);
-                p2 = m31::add(p2, s[8 * tpr]);
+                p1 = m31::add(p1, s[L]);
+                p2 = m31::add(p2, s[2 * L]);
             }
             p2 = m31::eval_at_two(p0, p1, p2);
             if (!LANE_HG) {
@@ -293,24 +309,18 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
                 p2 = m31::mul(p2, xv);
             }
             const uint32_t par = (a.parity ^ (k - a.k0)) << 31;
-            volatile uint32_t* out = a.evals_out + (size_t)(3 * fj) * N + flane;
+            volatile uint32_t* out = a.evals_out + (size_t)(3 * j) * N + flane;
             out[0] = p0 | par;
             out[N] = p1 | par;
             out[2 * (size_t)N] = p2 | par;
             if (k + 1 == a.n) {
-                // rows 0 and 1 of the last folded f table (the layer input when it has no fold)
-                uint32_t r0, r1;
-                if (k == 0) {
-                    r0 = __ldg(a.v + flane);
-                    r1 = __ldg(a.v + N + flane);
-                } else {  // two rows are always in shared memory
-                    const uint32_t* s = reinterpret_cast<const uint32_t*>(psm + ((k & 1) * kTabs + fj) * kSmemRows);
-                    r0 = s[fl];
-                    r1 = s[4 * tpr + fl];
-                }
-                volatile uint32_t* ro = a.rows_out + (size_t)(2 * fj) * N + flane;
-                ro[0] = r0 | (a.rows_parity << 31);
-                ro[N] = r1 | (a.rows_parity << 31);
+                // rows 0 and 1 of the last folded f table (the layer input when it has no fold;
+                // two rows are always in shared memory)
+                const uint32_t* s = k == 0 ? reinterpret_cast<const uint32_t*>(mine)
+                                           : reinterpret_cast<const uint32_t*>(psm + ((k & 1) * kTabs + j) * kSmemRows);
+                volatile uint32_t* ro = a.rows_out + (size_t)(2 * j) * N + flane;
+                ro[0] = s[t] | (a.rows_parity << 31);
+                ro[N] = s[L + t] | (a.rows_parity << 31);
             }
         }
     }
@@ -327,24 +337,26 @@ uint32_t phase_tpr(uint32_t N, uint32_t max_ctas) {
 }
 uint32_t phase_ctas(uint32_t N, uint32_t tpr) { return (N / 4 + tpr - 1) / tpr; }
 
+size_t phase_priv_quads(uint64_t items) { return items * 4 + items / 2 * 6 + items / 4 * 6; }
+
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
     if (a.reps < 1 || a.reps > 3 || a.k0 >= a.n || a.n - a.k0 > kMboxRounds || a.N % 4) return cudaErrorInvalidValue;
     if (a.tpr < 1 || a.tpr > 32 || (a.tpr & (a.tpr - 1))) return cudaErrorInvalidValue;
     // rows of the first round's source tables; with k0 = 0 the layer input itself
     const uint64_t rows = 1ull << (a.n - (a.k0 ? a.k0 - 1 : 0));
-    if (rows * a.tpr > kPhaseItems) return cudaErrorInvalidValue;
-    if (a.k0 == 0 && (!a.v || (lane_hg && (!a.h0[0] || !a.mx_off || !a.a4 || !a.w4)))) return cudaErrorInvalidValue;
+    if (rows * a.tpr > kPhaseItems || !a.priv || a.priv_stride < phase_priv_quads(rows * a.tpr)) return cudaErrorInvalidValue;
+    if (a.k0 && (!a.fsrc[0] || (lane_hg && !a.hsrc[0]))) return cudaErrorInvalidValue;
     if (!lane_hg && (!a.vx || !a.s[0])) return cudaErrorInvalidValue;
     static std::atomic<uint64_t> opted{0};  // one bit per device: shared memory above 48 KiB
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
     if (!(opted.load(std::memory_order_relaxed) & bit)) {
-        cudaFuncSetAttribute(k_phase<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        cudaFuncSetAttribute(k_phase<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+        cudaFuncSetAttribute(k_phase<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+        cudaFuncSetAttribute(k_phase<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
         opted.fetch_or(bit);
     }
-    const uint32_t kf = a.k0 ? a.k0 : 1, S1 = a.n >= kf ? 1u << (a.n - kf) : 1u;
+    const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
     const size_t smem = 2 * (lane_hg ? 6 : 3) * (size_t)kSmemRows * 16 + (lane_hg ? 0 : 4 * 3 * (size_t)(S1 + S1 / 2)) +
                         4 * (size_t)a.reps * kWarps * 3 * 4 * a.tpr;
     const dim3 grid(phase_ctas(a.N, a.tpr)), block(a.reps * kRepThreads);

@@ -822,7 +822,8 @@ void validate_layers(const gkrgpu_layer_desc* layers, int n, int field) {
 struct Workspace {
     uint32_t* vals = nullptr;  // every layer's values (the input's rows excluded when it is on the device)
     uint32_t *hg0[3] = {}, *hgA[3] = {}, *fA[3] = {}, *fB[3] = {};
-    uint32_t* hgF[3] = {};  // hg of round 0 of the phases that run in one launch
+    uint4* priv = nullptr;  // the CTAs' tables of the phases that run in one launch
+    size_t priv_stride = 0;
     uint32_t* sb[2] = {};
     uint32_t *evals = nullptr, *vx = nullptr, *cv = nullptr;
     uint32_t* p2s = nullptr;  // 9R x N sums of phase-two rounds 0 and 1 (launch_p2_round01)
@@ -834,8 +835,8 @@ struct Workspace {
     size_t sstride = 0;
     size_t total = 0;
 
-    // Lays the parts out from `base` (null: only sizes the block).
-    void plan(char* base, const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck) {
+    // Lays the parts out from `base` (null: only sizes the block); tpr as Prover::tpr_phase.
+    void plan(char* base, const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck, uint32_t tpr) {
         size_t o = 0;
         auto take = [&](size_t bytes) -> char* {
             char* p = base ? base + o : nullptr;
@@ -852,7 +853,10 @@ struct Workspace {
                 hgA[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 2, 1) * rowb);
                 fA[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 2, 1) * rowb);
                 fB[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 4, 1) * rowb);
-                hgF[j] = (uint32_t*)take(std::min<uint64_t>(maxI, kPhaseItems) * rowb);
+            }
+            if (tpr) {
+                priv_stride = phase_priv_quads(std::min<uint64_t>(maxI * tpr, kPhaseItems));
+                priv = (uint4*)take(phase_ctas(N, tpr) * priv_stride * 16);
             }
             sstride = align_up(maxI, 64);
             sb[0] = (uint32_t*)take(R * sstride * 4);
@@ -874,10 +878,19 @@ struct Workspace {
     }
 };
 
-uint64_t workspace_bytes(const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck) {
+uint64_t workspace_bytes(const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck, uint32_t tpr) {
     Workspace w;
-    w.plan(nullptr, C, N, R, own_input, sumcheck);
+    w.plan(nullptr, C, N, R, own_input, sumcheck, tpr);
     return w.total;
+}
+
+// Quads of copies per CTA of a proof's persistent phases (0: they are off): as few as the
+// lane's share of the resident CTAs allows, at most 128 CTAs.  (1024 copies: 256 CTAs of one
+// quad, whose 16-byte results are partial lines for the host to gather, took 52.6 ms for the
+// 2^18 / 2^20 proof, 128 of two 51.5.)
+uint32_t tpr_phase(const gkrgpu_ctx& X, uint32_t N) {
+    if (!X.round_tail) return 0;
+    return phase_tpr(N, std::min(128u, std::max(1u, 2u * (uint32_t)X.sm_count / (uint32_t)X.n_lanes)));
 }
 
 // f1 eq(r1_j, z) + f2 eq(r2_j, z) over nvars bits (r2 null: the first alone).
@@ -930,6 +943,7 @@ struct Prover {
     const gkrgpu_circuit& C;
     uint32_t N;
     int R;
+    uint32_t tpr;  // of the persistent phases
     Geo gk[K_NUM_KERNELS];
     uint32_t ck_ctas[K_NUM_KERNELS];
     Workspace ws;
@@ -940,7 +954,7 @@ struct Prover {
     std::vector<uint32_t> cv1, cv2;
 
     Prover(gkrgpu_ctx& ctx, Lane& lane, const gkrgpu_circuit& circ, uint32_t n, int reps)
-        : X(ctx), c(lane), C(circ), N(n), R(reps) {
+        : X(ctx), c(lane), C(circ), N(n), R(reps), tpr(tpr_phase(ctx, n)) {
         for (int k = 0; k < K_NUM_KERNELS; k++) {
             gk[k] = ctx.geo(n, k);
             ck_ctas[k] = ctx.cta_budget(k);
@@ -951,53 +965,45 @@ struct Prover {
         if (block) cudaFreeAsync(block, c.stream);
     }
 
-    // Quads of copies per CTA of this proof's persistent phases (0: they are off): as few as
-    // the lane's share of the resident CTAs allows, at most 128 CTAs.  (1024 copies: 256 CTAs
-    // of one quad, whose 16-byte results are partial lines for the host to gather, took
-    // 52.6 ms for the 2^18 / 2^20 proof, 128 of two 51.5.)
-    uint32_t tpr_phase() const {
-        if (!X.round_tail) return 0;
-        return phase_tpr(N, std::min(128u, std::max(1u, 2u * (uint32_t)X.sm_count / (uint32_t)c.X_lanes)));
-    }
     // First round of a phase's persistent part, n if it has none: 0 when the layer input itself
     // is small, else the first round from `first` on whose source tables are.  Measured with 16
     // copies and 2^10 rows: 9.5-14 us a round launched alone, 4-5 us within a phase.
     uint32_t phase_start(uint32_t n, uint32_t first) const {
-        const uint32_t tpr = tpr_phase();
         if (!tpr) return n;
+        if ((uint64_t)tpr << n <= kPhaseItems) return 0;
         uint32_t lg = 0;
-        while (((2ull << lg) * tpr) <= kPhaseItems) lg++;  // at most 2^lg rows
-        if (n <= lg) return 0;
+        while (((2ull << lg) * tpr) <= kPhaseTailItems) lg++;  // at most 2^lg rows
         return std::min(n, std::max(first, n + 1 - lg));
     }
     // Rounds a.k0 .. a.n-1 of a phase in one k_phase launch: after each round's evaluations the
     // host appends them, derives the challenges and writes them to the mailbox, from which
     // the kernel's next round reads them.  The last round's rows 0..1 come with its
-    // evaluations (vx / vy as in transcript_round).  Returns false (and does nothing) while
-    // other phases hold the device.
+    // evaluations (vx / vy as in transcript_round).  `prepare` launches what the phase reads.
+    // Returns false (and does nothing) while other phases hold the device.
+    template <class Prepare>
     bool run_phase(Transcript& t, bool lane_hg, PhaseArgs a, uint32_t (*rch)[32], bool append_last, uint32_t* last_out,
-                   double bytes) {
-        a.tpr = tpr_phase();
+                   double bytes, Prepare&& prepare) {
         PhaseSlots slots(X.device, X.sm_count);
-        if (!slots.acquire((int)phase_ctas(N, a.tpr))) return false;
+        if (!slots.acquire((int)phase_ctas(N, tpr))) return false;
+        prepare();
+        a.tpr = tpr;
+        a.priv = ws.priv;
+        a.priv_stride = ws.priv_stride;
         for (int j = 0; j < R; j++) {
-            a.fA[j] = ws.fA[j];
-            a.fB[j] = ws.fB[j];
-            a.hA[j] = ws.hgA[j];
-            a.hB[j] = ws.hg0[j];
-            a.h0[j] = ws.hgF[j];
+            a.fsrc[j] = (a.k0 & 1) ? ws.fB[j] : ws.fA[j];
+            a.hsrc[j] = (a.k0 & 1) ? ws.hg0[j] : ws.hgA[j];
             a.r_first[j] = a.k0 ? rch[j][a.k0 - 1] : 0u;
         }
         a.reps = (uint32_t)R;
         a.N = N;
         a.parity = c.ev_parity ^ 1u;
         a.rows_parity = c.rows_parity ^ 1u;
-        a.mbox = mapped(true, 12ull * N + 64);
+        a.mbox = mapped(true, mbox_word());
         a.evals_out = mapped(true, phase_word());
         a.rows_out = mapped(true, phase_word() + 9ull * N);
         a.err = mapped(true, 12ull * N + 1);
         a.wait_ns = 10ull * 1000 * 1000 * 1000;
-        volatile uint32_t* mb = mapped(false, 12ull * N + 64);
+        volatile uint32_t* mb = mapped(false, mbox_word());
         for (uint32_t i = 0; i < kMboxWords; i++) mb[i] = 0u;
         *err_h() = 0u;
         std::atomic_thread_fence(std::memory_order_seq_cst);
@@ -1054,7 +1060,8 @@ struct Prover {
     volatile uint32_t* flag_h() const { return mapped(false, 12ull * N); }
     volatile uint32_t* err_h() const { return mapped(false, 12ull * N + 1); }
     // phase-one round 0's claims (R x N), after the mailbox
-    uint64_t claim_word() const { return align_up(12ull * N + 64 + kMboxWords, 64); }
+    uint64_t mbox_word() const { return align_up(12ull * N + 64, 64); }
+    uint64_t claim_word() const { return mbox_word() + kMboxWords; }
     uint64_t phase_word() const { return align_up(claim_word() + 3ull * N, 64); }
     uint64_t mapped_words() const { return phase_word() + 15ull * N; }
     // Moves nsrc tables of n words into dst with k_stage_words (launch accounting as stage_words);
@@ -1071,11 +1078,11 @@ struct Prover {
     uint32_t groups(int kid) const { return N / (4 * gk[kid].tpr); }
 
     void reserve(bool own_input, bool sumcheck) {
-        ws.plan(nullptr, C, N, R, own_input, sumcheck);
+        ws.plan(nullptr, C, N, R, own_input, sumcheck, tpr);
         void* p = nullptr;
         ck(cudaMallocFromPoolAsync(&p, ws.total, X.pool, c.stream), "workspace allocation");
         block = static_cast<char*>(p);
-        ws.plan(block, C, N, R, own_input, sumcheck);
+        ws.plan(block, C, N, R, own_input, sumcheck, tpr);
         ck(cudaMemsetAsync(block + ws.zero_off, 0, ws.zero_bytes, c.stream), "cudaMemsetAsync");
         c.ensure_mapped(9ull * N * 4, mapped_words() * 4);
         c.resync_done();
@@ -1202,7 +1209,7 @@ struct Prover {
                 PhaseArgs a = {};
                 a.k0 = k;
                 a.n = n;
-                if (run_phase(t, true, a, rx, true, vxh, bytes)) break;
+                if (run_phase(t, true, a, rx, true, vxh, bytes, [] {})) break;
             }
             RoundPtrs p;
             memset(&p, 0, sizeof(p));
@@ -1348,7 +1355,7 @@ struct Prover {
                 a.n = n;
                 a.vx = ws.vx;
                 for (int j = 0; j < R; j++) a.s[j] = ws.sb[(k - 1) & 1] + j * sstride;
-                if (run_phase(t, false, a, ry, false, vy, bytes)) break;
+                if (run_phase(t, false, a, ry, false, vy, bytes, [] {})) break;
             }
             RoundPtrs p;
             memset(&p, 0, sizeof(p));
@@ -1406,29 +1413,31 @@ struct Prover {
         // phase one: gate weights for eqc_j = alpha eq(rz1_j) + beta eq(rz2_j)
         c.tag = ((uint32_t)li << 16) | (1u << 8);
         const EqArgs eqc = eq_args(R, rz1, rz2, alpha, beta, m);
-        const double wb = 32.0 * Ly.nmul + 20.0 * I + 8.0 * Ly.nadd;
-        c.launch(K_WEIGHTS, wb, [&] {
-            return launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, c.stream);
-        });
         // the rounds on small tables run in one persistent launch: every round of a small layer,
         // otherwise from round 4 on (rounds 2 and 3 refold the input and recompute
         // copy-independent hg rows)
         const uint32_t kt1 = phase_start(n, 4);
         PhaseArgs a1 = {};
         a1.n = n;
-        a1.v = v;
-        a1.mx_off = Ly.mx_off;
-        a1.mx_g = Ly.mx_g;
-        a1.a4 = ws.a4;
-        a1.w4 = ws.w4;
-        if (kt1 != 0 || !run_phase(t, true, a1, rx, true, vxh, rb * (I + Ly.nmul + 9.0 * R * I)))
-            phase_one_rounds(t, li, kt1, alpha, beta, rx);
+        const bool whole = kt1 == 0 && run_phase(t, true, a1, rx, true, vxh, rb * 9.0 * R * I, [&] {
+            c.launch(K_HG_BUILD, rb * (I + Ly.nmul + (double)(1 + R) * I) + 16.0 * Ly.nmul + 8.0 * Ly.nadd, [&] {
+                return launch_hg_build(v, (uint32_t)I, N, tpr, eqc, Ly.mx_off, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.priv,
+                                       ws.priv_stride, c.stream);
+            });
+        });
+        if (!whole) {
+            c.launch(K_WEIGHTS, 32.0 * Ly.nmul + 20.0 * I + 8.0 * Ly.nadd, [&] {
+                return launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, c.stream);
+            });
+            phase_one_rounds(t, li, std::max(kt1, std::min(n, 4u)), alpha, beta, rx);
+        }
 
         // phase two: h(y) = vx * s(y)
         c.tag = ((uint32_t)li << 16) | (2u << 8);
         const EqArgs eqx = eq_args(R, rx, nullptr, 1u, 0u, n);
         const size_t sstride = ws.sstride;
-        const uint32_t kt2 = phase_start(n, 3);
+        // phase two whole in one launch reads the layer input where phase one's left it
+        const uint32_t kt2 = whole ? 0 : std::max(phase_start(n, 3), std::min(n, 3u));
         const bool fused01 = kt2 != 0 && n >= 3 && p2_round01_groups(N) > 0;
         c.launch(K_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 4.0 * R * I * (fused01 ? 2 : 1), [&] {
             return launch_s_build(I, Ly.my_off, Ly.my_g, eqc, eqx, ws.sb[0], fused01 ? ws.sb[1] : nullptr, sstride,
@@ -1436,10 +1445,9 @@ struct Prover {
         });
         PhaseArgs a2 = {};
         a2.n = n;
-        a2.v = v;
         a2.vx = mapped(true, 9ull * N);
         for (int j = 0; j < R; j++) a2.s[j] = ws.sb[0] + j * sstride;
-        if (kt2 != 0 || !run_phase(t, false, a2, ry, false, vy.data(), rb * I * (1.0 + 3.0 * R) + 8.0 * R * I))
+        if (kt2 != 0 || !run_phase(t, false, a2, ry, false, vy.data(), rb * I * (1.0 + 3.0 * R) + 8.0 * R * I, [] {}))
             phase_two_rounds(t, li, kt2, fused01, ry, vy.data());
         for (int j = 0; j < R; j++) t.append(vy.data() + (size_t)j * N, rowb);
         // the next layer's sum is alpha vx + beta vy (gkr.hpp:113-119)
@@ -1685,7 +1693,8 @@ void gpu_worker(gkrgpu_ctx* c, Lane* lane) {
         std::string err;
         const bool bn = j->circuit->field == GKRGPU_FIELD_BN254;
         const uint64_t need = bn ? workspace_bytes_bn(*j->circuit, j->N, true)
-                                 : workspace_bytes(*j->circuit, j->N, j->R, j->d_input == nullptr, true);
+                                 : workspace_bytes(*j->circuit, j->N, j->R, j->d_input == nullptr, true,
+                                                 tpr_phase(*c, j->N));
         c->acquire_hbm(need);
         if (j->marker >= 0) {
             // the device stage begins: this lane's stream has finished its previous proof
@@ -1957,7 +1966,12 @@ int gkrgpu_memory_stats(gkrgpu_ctx* ctx, uint64_t* in_use, uint64_t* peak, uint6
 uint64_t gkrgpu_workspace_bytes(const gkrgpu_circuit* circuit, uint32_t n_copies, int grinding_bits, int input_on_device) {
     if (!circuit) return 0;
     if (circuit->field == GKRGPU_FIELD_BN254) return workspace_bytes_bn(*circuit, n_copies, true);
-    return workspace_bytes(*circuit, n_copies, reps_for(grinding_bits), input_on_device == 0, true);
+    // the largest over the row tiles of the persistent phases, which depend on the lanes
+    uint64_t most = 0;
+    for (uint32_t tpr = 0; tpr <= 32; tpr = tpr ? 2 * tpr : 1)
+        if (tpr == 0 || phase_ctas(n_copies, tpr) <= 128)
+            most = std::max(most, workspace_bytes(*circuit, n_copies, reps_for(grinding_bits), input_on_device == 0, true, tpr));
+    return most;
 }
 
 int gkrgpu_circuit_load(gkrgpu_ctx* ctx, const gkrgpu_layer_desc* layers, int n_layers, gkrgpu_circuit** out) {
@@ -2167,9 +2181,9 @@ int gkrgpu_check_device_wait(gkrgpu_ctx* ctx, uint32_t timeout_us, int* expired,
         on_idle_lane(ctx, [&](Lane& c) {
             // a two-round phase over 8 x 4 tables whose second round's challenge is never written
             const uint32_t N = 4, n = 3;
-            const size_t tb = 8 * N * 4;
+            const size_t tb = 8 * N * 4, priv = phase_priv_quads(8);
             void* p = nullptr;
-            ck(cudaMallocFromPoolAsync(&p, 4 * tb, ctx->pool, c.stream), "workspace allocation");
+            ck(cudaMallocFromPoolAsync(&p, 2 * tb + 16 * priv, ctx->pool, c.stream), "workspace allocation");
             struct Free {
                 void* p;
                 cudaStream_t s;
@@ -2178,17 +2192,17 @@ int gkrgpu_check_device_wait(gkrgpu_ctx* ctx, uint32_t timeout_us, int* expired,
                     cudaStreamSynchronize(s);
                 }
             } guard{p, c.stream};
-            ck(cudaMemsetAsync(p, 0, 4 * tb, c.stream), "cudaMemsetAsync");
-            const uint32_t mbox_at = 12 * N + 64, out_at = mbox_at + kMboxWords;
+            ck(cudaMemsetAsync(p, 0, 2 * tb, c.stream), "cudaMemsetAsync");
+            const uint32_t mbox_at = 128, out_at = mbox_at + kMboxWords;
             c.ensure_mapped(9ull * N * 4, (out_at + 15ull * N) * 4);
             uint32_t* base_h = reinterpret_cast<uint32_t*>(c.extra_h());
             uint32_t* base_d = reinterpret_cast<uint32_t*>(c.extra_d());
             PhaseArgs a = {};
             char* b = static_cast<char*>(p);
-            a.fA[0] = reinterpret_cast<uint32_t*>(b);
-            a.fB[0] = reinterpret_cast<uint32_t*>(b + tb);
-            a.hA[0] = reinterpret_cast<uint32_t*>(b + 2 * tb);
-            a.hB[0] = reinterpret_cast<uint32_t*>(b + 3 * tb);
+            a.fsrc[0] = reinterpret_cast<uint32_t*>(b);
+            a.hsrc[0] = reinterpret_cast<uint32_t*>(b + tb);
+            a.priv = reinterpret_cast<uint4*>(b + 2 * tb);
+            a.priv_stride = priv;
             a.k0 = 1;
             a.n = n;
             a.reps = 1;
@@ -2416,7 +2430,10 @@ int gkrgpu_autotune(gkrgpu_ctx* ctx, const gkrgpu_circuit* circuit, uint32_t n_c
         std::vector<uint32_t> cv((size_t)R * n_copies * elem_bytes(circuit->field) / 4);
         // effective threads per row slice of kind k for this circuit's field
         auto tile_tpr = [&](int k) { return k >= K_BN_LOAD ? geo_bn(*ctx, n_copies, k).tpr : ctx->geo(n_copies, k).tpr; };
-        const bool saved_timing = ctx->timing;
+        const bool saved_timing = ctx->timing, saved_tail = ctx->round_tail;
+        // every round as its own launch, so that each kind is timed (a layer whose phases run
+        // whole in one launch has no other)
+        ctx->round_tail = false;
         const auto saved_tiles = std::vector<gkrgpu_ctx::Tile>(std::begin(ctx->tiles), std::end(ctx->tiles));
         ctx->timing = true;
         auto snapshot = [&](double* ms) {
@@ -2482,9 +2499,11 @@ int gkrgpu_autotune(gkrgpu_ctx* ctx, const gkrgpu_circuit* circuit, uint32_t n_c
         } catch (...) {
             for (int k = 0; k < K_NUM_KERNELS; k++) ctx->tiles[k] = saved_tiles[k];
             ctx->timing = saved_timing;
+            ctx->round_tail = saved_tail;
             throw;
         }
         ctx->timing = saved_timing;
+        ctx->round_tail = saved_tail;
     });
 }
 

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("seed,widths,n,p_mul", [
-    (601, [12, 11, 12], 16, 0.6), (602, [13, 12], 16, 0.6), (603, [14, 9], 8, 0.5), (604, [1, 1, 1, 1], 4, 0.5),
+    (601, [12, 13, 12], 16, 0.6), (602, [13, 12], 16, 0.6), (603, [14, 9], 8, 0.5), (604, [1, 1, 1, 1], 4, 0.5),
     (605, [2, 1, 3, 0], 20, 0.5), (606, [11, 10], 516, 0.6), (607, [12, 5], 268, 1.0), (608, [9, 10, 7], 1024, 0.0),
     (609, [6, 7], 4096, 0.5), (610, [5, 4], 20000, 0.5), (611, [3, 9, 3], 28, 1.0),
 ])
