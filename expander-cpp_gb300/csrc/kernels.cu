@@ -84,6 +84,11 @@ __device__ __forceinline__ uint64_t fold64(uint64_t x) {
     return ((uint64_t)nh << 32) | nl;
 }
 
+// acc += a * b with one 32 x 32 -> 64-bit multiply-add.
+__device__ __forceinline__ void mad64(uint64_t& acc, uint32_t a, uint32_t b) {
+    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
+}
+
 // Canonical total of component c at `lane`, re-zeroing the accumulator for the next launch.
 __device__ __forceinline__ uint32_t take(const RedScratch& red, uint32_t c, uint32_t N, uint32_t lane) {
     unsigned long long* p = &red.acc[(size_t)c * N + lane];
@@ -97,7 +102,7 @@ __device__ __forceinline__ uint32_t take(const RedScratch& red, uint32_t c, uint
 // comp_base + c, then the last CTA of this lane group (ticket blockIdx.y) hands every lane
 // of the group to fin(lane), which collects the totals with take().
 template <class Fin>
-__device__ __forceinline__ void finish_group(const RedScratch& red, uint32_t base, uint32_t lanes, Fin& fin);
+__device__ __forceinline__ void finish_group(const RedScratch& red, uint32_t base, uint32_t lanes, uint32_t N, Fin& fin);
 
 template <int C, class Fin>
 __device__ __forceinline__ void reduce_group(const uint32_t (&acc)[C][4], const Geo& g, bool active, RedScratch red,
@@ -117,16 +122,16 @@ __device__ __forceinline__ void reduce_group(const uint32_t (&acc)[C][4], const 
         for (uint32_t r = 0; r < rps; r++) s += col[r * tpr];
         const uint32_t c = cl >> 2, l = cl & 3;
         const uint32_t lane = (blockIdx.y * tpr + q) * 4 + l;
-        atomicAdd(&red.acc[(size_t)(comp_base + c) * g.N + lane], s);
+        if (lane < g.N) atomicAdd(&red.acc[(size_t)(comp_base + c) * g.N + lane], s);
     }
-    finish_group(red, blockIdx.y * 4 * tpr, 4 * tpr, fin);
+    finish_group(red, blockIdx.y * 4 * tpr, 4 * tpr, g.N, fin);
 }
 
 // After a CTA's atomic adds: the last CTA of lane group blockIdx.y (ticket) hands lanes
-// base .. base + lanes - 1 to fin(lane), re-arms the ticket and, with red.done, publishes
+// base .. base + lanes - 1 (below N) to fin(lane), re-arms the ticket and, with red.done, publishes
 // the group's results to the host (system-scope fence, then the completion counter).
 template <class Fin>
-__device__ __forceinline__ void finish_group(const RedScratch& red, uint32_t base, uint32_t lanes, Fin& fin) {
+__device__ __forceinline__ void finish_group(const RedScratch& red, uint32_t base, uint32_t lanes, uint32_t N, Fin& fin) {
     const uint32_t tid = threadIdx.x, B = blockDim.x;
     __threadfence();
     __syncthreads();
@@ -135,7 +140,7 @@ __device__ __forceinline__ void finish_group(const RedScratch& red, uint32_t bas
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    for (uint32_t li = tid; li < lanes; li += B) fin(base + li);
+    for (uint32_t li = tid; li < lanes && base + li < N; li += B) fin(base + li);
     if (tid == 0) red.ticket[blockIdx.y] = 0u;
     if (red.done) {
         __threadfence_system();
@@ -159,9 +164,9 @@ __device__ __forceinline__ void reduce_group1(const uint32_t (&acc)[C], const Ge
         const uint32_t* col = smem + c * B + q;
         unsigned long long s = 0;
         for (uint32_t r = 0; r < rps; r++) s += col[r * L];
-        atomicAdd(&red.acc[(size_t)c * g.N + blockIdx.y * L + q], s);
+        if (blockIdx.y * L + q < g.N) atomicAdd(&red.acc[(size_t)c * g.N + blockIdx.y * L + q], s);
     }
-    finish_group(red, blockIdx.y * L, L, fin);
+    finish_group(red, blockIdx.y * L, L, g.N, fin);
 }
 
 struct TileIdx {
@@ -173,7 +178,7 @@ __device__ __forceinline__ TileIdx tile_idx(const Geo& g) {
     t.q = threadIdx.x % g.tpr;
     t.rs = threadIdx.x / g.tpr;
     t.lane0 = (blockIdx.y * g.tpr + t.q) * 4;
-    t.active = t.rs < g.rps;
+    t.active = t.rs < g.rps && t.lane0 < g.N;
     return t;
 }
 
@@ -335,27 +340,36 @@ __global__ void __launch_bounds__(256) k_weights(uint64_t I, uint64_t Gm, const 
 // row and four copies; the factors are few products next to a launch that stored them).
 // Building it inside the phase, whose few CTAs have a chain of three gathers a row, took 11 us
 // of a 63 us phase at 2^10 rows and 16 copies.
+template <bool STORED>
 __global__ void __launch_bounds__(256) k_hg_build(const uint32_t* __restrict__ v, uint32_t I, uint32_t N, uint32_t tpr,
                                                   const __grid_constant__ EqArgs eqc, const uint32_t* __restrict__ mx_off,
                                                   const uint4* __restrict__ mx_g, const uint32_t* __restrict__ ax_off,
-                                                  const uint2* __restrict__ ax_g, uint4* __restrict__ priv,
+                                                  const uint2* __restrict__ ax_g, const uint4* __restrict__ a4,
+                                                  const uint4* __restrict__ w4, uint4* __restrict__ priv,
                                                   size_t priv_stride) {
-    __shared__ uint32_t t[2 * kEqWords];
-    eq_build(t, eqc);
-    __syncthreads();
+    __shared__ uint32_t t[STORED ? 1 : 2 * kEqWords];
+    if (!STORED) {
+        eq_build(t, eqc);
+        __syncthreads();
+    }
     const uint32_t nd = eq_digits(eqc), reps = eqc.reps, Q = N / 4;
     const bool two = eqc.f2 != 0;
     const uint64_t total = (uint64_t)I * Q, stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const uint32_t x = (uint32_t)(i / Q), quad = (uint32_t)(i - (uint64_t)x * Q);
         const uint32_t m0 = __ldg(mx_off + x), m1 = __ldg(mx_off + x + 1);
-        const uint32_t a0 = __ldg(ax_off + x), a1 = __ldg(ax_off + x + 1);
         uint32_t s[3] = {0u, 0u, 0u};
-        for (uint32_t k = a0; k < a1; k++) {
-            const uint2 gt = __ldg(ax_g + k);  // (z, c)
+        if (STORED) {
+            const uint4 w = __ldg(a4 + x);
+            s[0] = w.x; s[1] = w.y; s[2] = w.z;
+        } else {
+            const uint32_t a0 = __ldg(ax_off + x), a1 = __ldg(ax_off + x + 1);
+            for (uint32_t k = a0; k < a1; k++) {
+                const uint2 gt = __ldg(ax_g + k);  // (z, c)
 #pragma unroll
-            for (uint32_t j = 0; j < 3; j++)
-                if (j < reps) s[j] = add(s[j], mul(gt.y, eq_at(t, nd, two, j, gt.x)));
+                for (uint32_t j = 0; j < 3; j++)
+                    if (j < reps) s[j] = add(s[j], mul(gt.y, eq_at(t, nd, two, j, gt.x)));
+            }
         }
         uint64_t h[3][4];
 #pragma unroll
@@ -365,10 +379,11 @@ __global__ void __launch_bounds__(256) k_hg_build(const uint32_t* __restrict__ v
         for (uint32_t k = m0; k < m1; k++) {
             const uint4 gt = __ldg(mx_g + k);  // (y, z, c, 0)
             const uint4 vy = ld4(v, gt.x, N, 4 * quad);
+            const uint4 ws = STORED ? __ldg(w4 + k) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (uint32_t j = 0; j < 3; j++)
                 if (j < reps) {
-                    const uint32_t w = mul(gt.z, eq_at(t, nd, two, j, gt.y));
+                    const uint32_t w = STORED ? comp(ws, j) : mul(gt.z, eq_at(t, nd, two, j, gt.y));
 #pragma unroll
                     for (int l = 0; l < 4; l++) h[j][l] = fold64(h[j][l] + (uint64_t)comp(vy, l) * w);
                 }
@@ -551,17 +566,6 @@ struct CopyFin {
         for (uint32_t j = 0; j < reps; j++) out[(size_t)j * N + lane] = take(red, j, N, lane);
     }
 };
-
-// p0 += f0 h0 and p2raw += (f0 + f1)(h0 + h1) for four copies (mac_lazy): the two sums of a
-// round whose p1 comes from its claim (ClaimFin).
-__device__ __forceinline__ void accum_pair2(uint32_t (&acc)[2][4], const uint32_t (&f0)[4], const uint32_t (&f1)[4],
-                                            const uint32_t (&h0)[4], const uint32_t (&h1)[4]) {
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        acc[0][l] = m31::mac_lazy(acc[0][l], f0[l], h0[l]);
-        acc[1][l] = m31::mac_lazy(acc[1][l], add(f0[l], f1[l]), add(h0[l], h1[l]));
-    }
-}
 
 // ---------------------------------------------------------------- asynchronous row staging
 // cp.async copies (global -> shared, no registers held while in flight) let a thread keep
@@ -756,7 +760,7 @@ __global__ void __launch_bounds__(256, 2) k_hg_round0(const uint32_t* __restrict
 // the claim, round 0's polynomial at r_j, less p0); after the first row of a pair only its
 // f and h are kept, for p2raw.
 template <int R>
-__global__ void __launch_bounds__(256) k_hg_round1(const uint32_t* __restrict__ v, uint64_t npairs,
+__global__ void __launch_bounds__(256, 2) k_hg_round1(const uint32_t* __restrict__ v, uint64_t npairs,
                                                    const uint32_t* __restrict__ quads,
                                                    const uint32_t* __restrict__ mx_off, const uint4* __restrict__ mx_g,
                                                    const uint4* __restrict__ a4, const uint4* __restrict__ w4r,
@@ -790,7 +794,7 @@ __global__ void __launch_bounds__(256) k_hg_round1(const uint32_t* __restrict__ 
                 uint32_t h[R][4];
 #pragma unroll
                 for (int j = 0; j < R; j++) {
-                    const uint32_t hs = fold(comp(a0, j), comp(a1, j), p.r[j]);
+                    const uint32_t hs = m31::lerp(comp(a0, j), comp(a1, j), p.c[j]);
 #pragma unroll
                     for (int l = 0; l < 4; l++) h[j][l] = hs;
                 }
@@ -805,7 +809,7 @@ __global__ void __launch_bounds__(256) k_hg_round1(const uint32_t* __restrict__ 
                 for (int j = 0; j < R; j++) {
                     uint32_t f[4];
 #pragma unroll
-                    for (int l = 0; l < 4; l++) f[l] = fold(comp(v0, l), comp(v1, l), p.r[j]);
+                    for (int l = 0; l < 4; l++) f[l] = m31::lerp(comp(v0, l), comp(v1, l), p.c[j]);
                     // null: round 2 refolds the layer input instead of reading stored copies
                     if (p.fdst[0]) st4(p.fdst[j], 2 * i + s, g.N, t.lane0, mk4(f));
                     // a copy-independent hg row is recomputed by round 2 (k_round with H1)
@@ -842,7 +846,7 @@ __global__ void __launch_bounds__(256) k_hg_round1(const uint32_t* __restrict__ 
 // not store it, and it is recomputed by folding their add weights a_j at the challenges of
 // rounds 0 .. HR-1.  Round 2 (HR = 1) does not store its own output rows of that kind.
 template <bool SHARED, bool LANE_HG, bool FOLD, int HR = 0>
-__global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, const uint32_t* __restrict__ vx, Geo g,
+__global__ void __launch_bounds__(256, 4) k_round(RoundPtrs p, uint64_t npairs, const uint32_t* __restrict__ vx, Geo g,
                                                uint32_t reps, RedScratch red, uint32_t* evals_out) {
     const TileIdx t = tile_idx(g);
     const uint32_t j = blockIdx.x % reps, cx = blockIdx.x / reps, nx = gridDim.x / reps;
@@ -851,27 +855,34 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, con
     const uint32_t* __restrict__ hs = j == 0 ? p.hsrc[0] : (j == 1 ? p.hsrc[1] : p.hsrc[2]);
     uint32_t* __restrict__ fd = j == 0 ? p.fdst[0] : (j == 1 ? p.fdst[1] : p.fdst[2]);
     uint32_t* __restrict__ hd = j == 0 ? p.hdst[0] : (j == 1 ? p.hdst[1] : p.hdst[2]);
-    const uint32_t r = j == 0 ? p.r[0] : (j == 1 ? p.r[1] : p.r[2]);
-    uint32_t acc[2][4] = {};  // p0, p2raw
+    const m31::Lerp c = j == 0 ? p.c[0] : (j == 1 ? p.c[1] : p.c[2]);
+    uint32_t acc[2][4] = {};  // p0, p2raw, below 2^32 (64-bit sums cost the registers of a fourth CTA)
+    auto accum = [&](const uint32_t (&f0)[4], const uint32_t (&f1)[4], const uint32_t (&h0)[4], const uint32_t (&h1)[4]) {
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            acc[0][l] = m31::mac_lazy(acc[0][l], f0[l], h0[l]);
+            acc[1][l] = m31::mac_lazy(acc[1][l], add(f0[l], f1[l]), add(h0[l], h1[l]));
+        }
+    };
     if (t.active) {
         uint64_t i = (uint64_t)cx * g.rps + t.rs;
         const uint64_t step = (uint64_t)nx * g.rps;
         if (FOLD && !LANE_HG) {
             // scalar-h folds: two pairs per iteration, their eight row loads issued together
             auto fold_pair = [&](const uint4 (&a)[4], const uint4& sv, uint64_t ii) {
-                const uint32_t s0 = fold(sv.x, sv.y, r), s1 = fold(sv.z, sv.w, r);
+                const uint32_t s0 = m31::lerp(sv.x, sv.y, c), s1 = m31::lerp(sv.z, sv.w, c);
                 if (t.q == 0 && blockIdx.y == 0) *reinterpret_cast<uint2*>(hd + 2 * ii) = make_uint2(s0, s1);
                 uint32_t f0[4], f1[4], h0[4], h1[4];
 #pragma unroll
                 for (int l = 0; l < 4; l++) {
-                    f0[l] = fold(comp(a[0], l), comp(a[1], l), r);
-                    f1[l] = fold(comp(a[2], l), comp(a[3], l), r);
+                    f0[l] = m31::lerp(comp(a[0], l), comp(a[1], l), c);
+                    f1[l] = m31::lerp(comp(a[2], l), comp(a[3], l), c);
                     h0[l] = s0;
                     h1[l] = s1;
                 }
                 st4(fd, 2 * ii, g.N, t.lane0, mk4(f0));
                 st4(fd, 2 * ii + 1, g.N, t.lane0, mk4(f1));
-                accum_pair2(acc, f0, f1, h0, h1);
+                accum(f0, f1, h0, h1);
             };
             for (; i + step < npairs; i += 2 * step) {
                 uint4 a[4], b[4];
@@ -902,14 +913,15 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, con
                         const uint32_t* o = p.hoff + 4 * SPAN * i;
 #pragma unroll
                         for (int k = 0; k <= 4; k++) off[k] = __ldg(o + k * SPAN);
-                        const uint32_t r0 = j == 0 ? p.hr[0][0] : (j == 1 ? p.hr[0][1] : p.hr[0][2]);
-                        const uint32_t r1 = j == 0 ? p.hr[1][0] : (j == 1 ? p.hr[1][1] : p.hr[1][2]);
+                        const m31::Lerp c0 = j == 0 ? p.c0[0] : (j == 1 ? p.c0[1] : p.c0[2]);
+                        const m31::Lerp2 c01 = j == 0 ? p.c01[0] : (j == 1 ? p.c01[1] : p.c01[2]);
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
                             if (off[k] == off[k + 1]) {
                                 const uint32_t* a = reinterpret_cast<const uint32_t*>(p.ha + (4 * i + k) * SPAN) + j;
-                                uint32_t hv = fold(__ldg(a), __ldg(a + 4), r0);
-                                if (HR == 2) hv = fold(hv, fold(__ldg(a + 8), __ldg(a + 12), r0), r1);
+                                const uint32_t hv = HR == 2
+                                                        ? m31::lerp2(__ldg(a), __ldg(a + 4), __ldg(a + 8), __ldg(a + 12), c01)
+                                                        : m31::lerp(__ldg(a), __ldg(a + 4), c0);
                                 b[k] = make_uint4(hv, hv, hv, hv);
                             } else {
                                 b[k] = ld4(hs, 4 * i + k, g.N, t.lane0);
@@ -925,22 +937,22 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, con
                     }
 #pragma unroll
                     for (int l = 0; l < 4; l++) {
-                        h0[l] = fold(comp(b[0], l), comp(b[1], l), r);
-                        h1[l] = fold(comp(b[2], l), comp(b[3], l), r);
+                        h0[l] = m31::lerp(comp(b[0], l), comp(b[1], l), c);
+                        h1[l] = m31::lerp(comp(b[2], l), comp(b[3], l), c);
                     }
                     if (keep0) st4(hd, 2 * i, g.N, t.lane0, mk4(h0));
                     if (keep1) st4(hd, 2 * i + 1, g.N, t.lane0, mk4(h1));
                 } else {
                     const uint4 s = __ldg(reinterpret_cast<const uint4*>(hs) + i);
-                    const uint32_t s0 = fold(s.x, s.y, r), s1 = fold(s.z, s.w, r);
+                    const uint32_t s0 = m31::lerp(s.x, s.y, c), s1 = m31::lerp(s.z, s.w, c);
                     if (t.q == 0 && blockIdx.y == 0) *reinterpret_cast<uint2*>(hd + 2 * i) = make_uint2(s0, s1);
 #pragma unroll
                     for (int l = 0; l < 4; l++) { h0[l] = s0; h1[l] = s1; }
                 }
 #pragma unroll
                 for (int l = 0; l < 4; l++) {
-                    f0[l] = fold(comp(a[0], l), comp(a[1], l), r);
-                    f1[l] = fold(comp(a[2], l), comp(a[3], l), r);
+                    f0[l] = m31::lerp(comp(a[0], l), comp(a[1], l), c);
+                    f1[l] = m31::lerp(comp(a[2], l), comp(a[3], l), c);
                 }
                 st4(fd, 2 * i, g.N, t.lane0, mk4(f0));
                 st4(fd, 2 * i + 1, g.N, t.lane0, mk4(f1));
@@ -958,7 +970,7 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, con
                     for (int l = 0; l < 4; l++) { h0[l] = s.x; h1[l] = s.y; }
                 }
             }
-            accum_pair2(acc, f0, f1, h0, h1);
+            accum(f0, f1, h0, h1);
         }
     }
     reduce_group<2>(acc, g, t.active, red, 2 * j,
@@ -976,7 +988,7 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrs p, uint64_t npairs, con
 // input rows have no mul gates are not stored (round 3 recomputes them), as in
 // k_round<.., HR = 1>.
 template <int R>
-__global__ void __launch_bounds__(256) k_p1_round2(RoundPtrs p, uint64_t npairs, Geo g, RedScratch red,
+__global__ void __launch_bounds__(256, 2) k_p1_round2(RoundPtrs p, uint64_t npairs, Geo g, RedScratch red,
                                                    uint32_t* evals_out) {
     const TileIdx t = tile_idx(g);
     const uint32_t* __restrict__ v = p.fsrc[0];
@@ -1001,14 +1013,13 @@ __global__ void __launch_bounds__(256) k_p1_round2(RoundPtrs p, uint64_t npairs,
                 const bool keep = off[2 * s] != off[2 * s + 2];
 #pragma unroll
                 for (int j = 0; j < R; j++) {
-                    const uint32_t r0 = p.hr[0][j], r1 = p.r[j];
                     uint4 b[2];
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         const int k = 2 * s + e;
                         if (off[k] == off[k + 1]) {
                             const uint32_t* a = reinterpret_cast<const uint32_t*>(p.ha + (4 * i + k) * 2) + j;
-                            const uint32_t hv = fold(__ldg(a), __ldg(a + 4), r0);
+                            const uint32_t hv = m31::lerp(__ldg(a), __ldg(a + 4), p.c0[j]);
                             b[e] = make_uint4(hv, hv, hv, hv);
                         } else {
                             b[e] = ld4(p.hsrc[j], 4 * i + k, g.N, t.lane0);
@@ -1017,8 +1028,8 @@ __global__ void __launch_bounds__(256) k_p1_round2(RoundPtrs p, uint64_t npairs,
                     uint32_t f[4], h[4];
 #pragma unroll
                     for (int l = 0; l < 4; l++) {
-                        f[l] = fold(fold(comp(x0, l), comp(x1, l), r0), fold(comp(x2, l), comp(x3, l), r0), r1);
-                        h[l] = fold(comp(b[0], l), comp(b[1], l), r1);
+                        f[l] = m31::lerp2(comp(x0, l), comp(x1, l), comp(x2, l), comp(x3, l), p.c01[j]);
+                        h[l] = m31::lerp(comp(b[0], l), comp(b[1], l), p.c[j]);
                     }
                     st4(p.fdst[j], 2 * i + s, g.N, t.lane0, mk4(f));
                     if (keep) st4(p.hdst[j], 2 * i + s, g.N, t.lane0, mk4(h));
@@ -1062,13 +1073,13 @@ __global__ void __launch_bounds__(256) k_round_shared(RoundPtrs p, uint64_t npai
             }
 #pragma unroll
             for (int j = 0; j < R; j++) {
-                const uint32_t r = p.r[j];
+                const m31::Lerp c = p.c[j];
                 uint32_t f0[4], f1[4], h0[4], h1[4];
                 if (FOLD) {
 #pragma unroll
                     for (int l = 0; l < 4; l++) {
-                        f0[l] = fold(comp(a[0], l), comp(a[1], l), r);
-                        f1[l] = fold(comp(a[2], l), comp(a[3], l), r);
+                        f0[l] = m31::lerp(comp(a[0], l), comp(a[1], l), c);
+                        f1[l] = m31::lerp(comp(a[2], l), comp(a[3], l), c);
                     }
                     if (p.fdst[j]) {  // null: the next round refolds the source instead
                         st4(p.fdst[j], 2 * i, g.N, t.lane0, mk4(f0));
@@ -1084,14 +1095,14 @@ __global__ void __launch_bounds__(256) k_round_shared(RoundPtrs p, uint64_t npai
                     for (int k = 0; k < 4; k++) b[k] = ld4(p.hsrc[j], 4 * i + k, g.N, t.lane0);
 #pragma unroll
                     for (int l = 0; l < 4; l++) {
-                        h0[l] = fold(comp(b[0], l), comp(b[1], l), r);
-                        h1[l] = fold(comp(b[2], l), comp(b[3], l), r);
+                        h0[l] = m31::lerp(comp(b[0], l), comp(b[1], l), c);
+                        h1[l] = m31::lerp(comp(b[2], l), comp(b[3], l), c);
                     }
                     st4(p.hdst[j], 2 * i, g.N, t.lane0, mk4(h0));
                     st4(p.hdst[j], 2 * i + 1, g.N, t.lane0, mk4(h1));
                 } else if (FOLD) {
                     const uint4 s = __ldg(reinterpret_cast<const uint4*>(p.hsrc[j]) + i);
-                    const uint32_t s0 = fold(s.x, s.y, r), s1 = fold(s.z, s.w, r);
+                    const uint32_t s0 = m31::lerp(s.x, s.y, c), s1 = m31::lerp(s.z, s.w, c);
                     if (t.q == 0 && blockIdx.y == 0) *reinterpret_cast<uint2*>(p.hdst[j] + 2 * i) = make_uint2(s0, s1);
 #pragma unroll
                     for (int l = 0; l < 4; l++) { h0[l] = s0; h1[l] = s1; }
@@ -1125,7 +1136,7 @@ constexpr int kRowStages = 3;
 constexpr int kRowRingSmem = kRowStages * 8 * 16 * 256;
 
 template <int R>
-__global__ void __launch_bounds__(256) k_p2_round2(RoundPtrs p, uint64_t npairs, const uint32_t* __restrict__ vx,
+__global__ void __launch_bounds__(256, 2) k_p2_round2(RoundPtrs p, uint64_t npairs, const uint32_t* __restrict__ vx,
                                                    Geo g, RedScratch red, uint32_t* evals_out) {
     extern __shared__ uint4 rows8[];  // kRowStages x 8 x blockDim.x
     const TileIdx t = tile_idx(g);
@@ -1161,17 +1172,14 @@ __global__ void __launch_bounds__(256) k_p2_round2(RoundPtrs p, uint64_t npairs,
             slot = slot + 1 == kRowStages ? 0 : slot + 1;
 #pragma unroll
             for (int j = 0; j < R; j++) {
-                const uint32_t r0 = p.hr[0][j], r1 = p.r[j];
                 const uint4 sv = __ldg(reinterpret_cast<const uint4*>(p.hsrc[j]) + i);
-                const uint32_t s0 = fold(sv.x, sv.y, r1), s1 = fold(sv.z, sv.w, r1);
+                const uint32_t s0 = m31::lerp(sv.x, sv.y, p.c[j]), s1 = m31::lerp(sv.z, sv.w, p.c[j]);
                 if (t.q == 0 && blockIdx.y == 0) *reinterpret_cast<uint2*>(p.hdst[j] + 2 * i) = make_uint2(s0, s1);
                 uint32_t f0[4], f1[4], h0[4], h1[4];
 #pragma unroll
                 for (int l = 0; l < 4; l++) {
-                    const uint32_t g0 = fold(comp(a[0], l), comp(a[1], l), r0), g1 = fold(comp(a[2], l), comp(a[3], l), r0);
-                    const uint32_t g2 = fold(comp(a[4], l), comp(a[5], l), r0), g3 = fold(comp(a[6], l), comp(a[7], l), r0);
-                    f0[l] = fold(g0, g1, r1);
-                    f1[l] = fold(g2, g3, r1);
+                    f0[l] = m31::lerp2(comp(a[0], l), comp(a[1], l), comp(a[2], l), comp(a[3], l), p.c01[j]);
+                    f1[l] = m31::lerp2(comp(a[4], l), comp(a[5], l), comp(a[6], l), comp(a[7], l), p.c01[j]);
                     h0[l] = s0;
                     h1[l] = s1;
                 }
@@ -1195,11 +1203,6 @@ __global__ void __launch_bounds__(256) k_p2_round2(RoundPtrs p, uint64_t npairs,
     __syncthreads();  // the ring is reused as the reduction's scratch
     reduce_group<2 * R>(acc, g, t.active, red, 0,
                         ClaimFin{red, evals_out, nullptr, {p.r[0], p.r[1], p.r[2]}, g.N, (uint32_t)R, vx});
-}
-
-// acc += a * b with one 32 x 32 -> 64-bit multiply-add.
-__device__ __forceinline__ void mad64(uint64_t& acc, uint32_t a, uint32_t b) {
-    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
 }
 
 // Phase-two round 0 (no fold): p0_j = sum f(2i) s_j(2i), p1_j = sum f(2i+1) s_j(2i+1),
@@ -1360,11 +1363,12 @@ __global__ void __launch_bounds__(256, 2) k_p2_round01(P01Src src, uint64_t ngro
     extern __shared__ uint4 ring01[];  // kP01Stages x warps x kP01WarpSlot bytes
     const uint32_t tid = threadIdx.x, wl = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     const uint32_t L = g.tpr, rs = tid / L;  // L: copies per row slice, a multiple of 32
-    const bool active = rs < g.rps;          // uniform over a warp
     const uint64_t N = g.N;
-    // this thread's global copy, and the 16 bytes it stages: row wl / 8 of the group, copies
-    // 4 (wl % 8) .. of the warp's 32
+    // this warp's first copy, and the 16 bytes the thread stages: row wl / 8 of the group,
+    // copies 4 (wl % 8) .. of the warp's 32 (those below N: the sums of the others are dropped)
     const uint64_t warp_lane0 = (uint64_t)blockIdx.y * L + (tid - rs * L - wl);
+    const bool active = rs < g.rps && warp_lane0 < N;  // uniform over a warp
+    const bool stages = warp_lane0 + 4 * (wl & 7) < N;
     const uint32_t* __restrict__ vst = src.v + (wl >> 3) * N + warp_lane0 + 4 * (wl & 7);
     const uint32_t* __restrict__ sst = nullptr;
     if (wl < 2 * R) {
@@ -1384,7 +1388,7 @@ __global__ void __launch_bounds__(256, 2) k_p2_round01(P01Src src, uint64_t ngro
         auto stage = [&](uint64_t i, uint64_t q, int slot) {
             if (i < ngroups) {
                 char* st = ring + ((size_t)slot * nw + w) * kP01WarpSlot;
-                cp_async16(st + 16 * wl, vst + 4 * q * N);
+                if (stages) cp_async16(st + 16 * wl, vst + 4 * q * N);
                 if (sst) cp_async16(st + 512 + 16 * wl, sst + 4 * q);
             }
             cp_async_commit();  // one group per iteration, empty past the end
@@ -1500,8 +1504,8 @@ __global__ void __launch_bounds__(256) k_p2_round1_fin(const uint32_t* __restric
 
 // ---------------------------------------------------------------- phase two: s(y)
 // s_j[y] = sum over mul gates (z, x, y, c) of eqc_j(z) * eq(rx_j, x) * c: the
-// copy-independent factor of h(y) = v(rx) s(y) (sumcheck_helper.hpp:250-259).  With T4 one
-// thread takes a group of four rows (I a multiple of 4) and also writes t_j(i) =
+// copy-independent factor of h(y) = v(rx) s(y) (sumcheck_helper.hpp:250-259).  With T4 (I a
+// multiple of 4) the threads of four neighbouring rows also write t_j(i) =
 // (s_j(4i) + s_j(4i+2), s_j(4i+1) + s_j(4i+3), s_j(4i) + s_j(4i+1), s_j(4i+2) + s_j(4i+3)),
 // the scalar pair sums that k_p2_round01 stages with each group.
 template <bool T4>
@@ -1515,36 +1519,30 @@ __global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __r
     __syncthreads();
     const uint32_t ndz = eq_digits(eqc), ndx = eq_digits(eqx), reps = eqc.reps;
     const bool two = eqc.f2 != 0;
-    constexpr int G = T4 ? 4 : 1;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, n = I / G;
-    for (uint64_t gi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gi < n; gi += stride) {
-        uint32_t s[3][G] = {};
-        uint32_t off[G + 1];
-#pragma unroll
-        for (int k = 0; k <= G; k++) off[k] = __ldg(my_off + G * gi + k);
-        for (uint32_t e = off[0]; e < off[G]; e++) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    // whole warps go round together: four neighbouring lanes hold a group's rows
+    const uint64_t end = (I + 31) & ~31ull;
+    for (uint64_t y = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; y < end; y += stride) {
+        uint32_t s[3] = {0u, 0u, 0u};
+        const uint32_t k0 = y < I ? __ldg(my_off + y) : 0u, k1 = y < I ? __ldg(my_off + y + 1) : 0u;
+        for (uint32_t e = k0; e < k1; e++) {
             const uint4 gt = __ldg(my_g + e);  // (x, z, c, 0)
 #pragma unroll
             for (uint32_t j = 0; j < 3; j++)
-                if (j < reps) {
-                    const uint32_t w = mul(mul(eq_at(tz, ndz, two, j, gt.y), eq_at(tx, ndx, false, j, gt.x)), gt.z);
-#pragma unroll
-                    for (int k = 0; k < G; k++)
-                        if (e >= off[k] && e < off[k + 1]) s[j][k] = add(s[j][k], w);
-                }
+                if (j < reps)
+                    s[j] = add(s[j], mul(mul(eq_at(tz, ndz, two, j, gt.y), eq_at(tx, ndx, false, j, gt.x)), gt.z));
         }
 #pragma unroll
         for (uint32_t j = 0; j < 3; j++) {
             if (j >= reps) break;
             if (T4) {
-                reinterpret_cast<uint4*>(s_out + (uint64_t)j * s_stride)[gi] =
-                    make_uint4(s[j][0], s[j][1 % G], s[j][2 % G], s[j][3 % G]);
-                reinterpret_cast<uint4*>(t_out + (uint64_t)j * s_stride)[gi] =
-                    make_uint4(add(s[j][0], s[j][2 % G]), add(s[j][1 % G], s[j][3 % G]), add(s[j][0], s[j][1 % G]),
-                               add(s[j][2 % G], s[j][3 % G]));
-            } else {
-                s_out[(uint64_t)j * s_stride + gi] = s[j][0];
+                // lane l of a group: t_l = s_0 + s_2, s_1 + s_3, s_0 + s_1, s_2 + s_3
+                const uint32_t l = threadIdx.x & 3;
+                const uint32_t u = __shfl_sync(0xffffffffu, s[j], l < 2 ? l : 2 * (l - 2), 4);
+                const uint32_t w = __shfl_sync(0xffffffffu, s[j], l < 2 ? l + 2 : 2 * (l - 2) + 1, 4);
+                if (y < I) t_out[(uint64_t)j * s_stride + y] = add(u, w);
             }
+            if (y < I) s_out[(uint64_t)j * s_stride + y] = s[j];
         }
     }
 }
@@ -1615,6 +1613,13 @@ __global__ void __launch_bounds__(256, 4) k_wsum(const uint32_t* __restrict__ va
     reduce_group<R>(sum, g, t.active, red, 0, CopyFin{red, out, g.N, (uint32_t)R});
 }
 
+// CTAs of 256 threads for n threads of a kernel that builds digit tables: one wave at most, a
+// CTA more costs another build.
+uint32_t grid_eq(uint64_t n) {
+    const uint64_t b = (n + 255) / 256;
+    return (uint32_t)(b < 1 ? 1 : b < 152 * 8 ? b : 152 * 8);
+}
+
 uint32_t grid_1d(uint64_t n, uint32_t block) {
     uint64_t b = (n + block - 1) / block;
     if (b < 1) b = 1;
@@ -1638,7 +1643,7 @@ constexpr uint32_t kMinRowIters = 4;
 
 LaunchShape row_shape(const Geo& g, uint64_t rows, uint32_t block, uint32_t ctas_cap, uint32_t smem_components) {
     LaunchShape s;
-    const uint32_t groups = g.N / (4 * g.tpr);
+    const uint32_t groups = lane_groups(g);
     uint64_t need = (rows + (uint64_t)g.rps * kMinRowIters - 1) / ((uint64_t)g.rps * kMinRowIters);
     uint64_t cap = ctas_cap / groups;
     if (cap < 1) cap = 1;
@@ -1669,7 +1674,7 @@ cudaError_t launch_canonicalize(uint32_t* v, uint64_t n, cudaStream_t s) {
 cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const GateEq& eq,
                              unsigned long long* acc, unsigned int* ticket, uint32_t* out, cudaStream_t s) {
     if (eq.z.reps < 1 || eq.z.reps > 3) return cudaErrorInvalidValue;
-    const uint32_t grid = grid_1d(O, 256);
+    const uint32_t grid = grid_eq(O);
     if (mul_gates)
         k_gate_sums<true><<<grid, 256, 0, s>>>(O, off, gates, eq, acc, ticket, out);
     else
@@ -1687,16 +1692,32 @@ cudaError_t launch_scale_weights(uint64_t I, const uint32_t* mx_off, const uint4
 
 cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgs& eqc, const uint4* mx_g, const uint32_t* ax_off,
                            const uint2* ax_g, uint4* a_out, uint4* w_out, cudaStream_t s) {
-    k_weights<<<grid_1d(I > Gm ? I : Gm, 256), 256, 0, s>>>(I, Gm, eqc, mx_g, ax_off, ax_g, a_out, w_out);
+    k_weights<<<grid_eq(I > Gm ? I : Gm), 256, 0, s>>>(I, Gm, eqc, mx_g, ax_off, ax_g, a_out, w_out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_hg_build(const uint32_t* v, uint32_t I, uint32_t N, uint32_t tpr, const EqArgs& eqc,
                             const uint32_t* mx_off, const uint4* mx_g, const uint32_t* ax_off, const uint2* ax_g,
-                            uint4* priv, size_t priv_stride, cudaStream_t s) {
-    k_hg_build<<<grid_1d((uint64_t)I * (N / 4), 256), 256, 0, s>>>(v, I, N, tpr, eqc, mx_off, mx_g, ax_off, ax_g, priv,
-                                                                  priv_stride);
+                            const uint4* a4, const uint4* w4, uint4* priv, size_t priv_stride, cudaStream_t s) {
+    const uint32_t grid = grid_eq((uint64_t)I * (N / 4));
+    if (a4)
+        k_hg_build<true><<<grid, 256, 0, s>>>(v, I, N, tpr, eqc, mx_off, mx_g, ax_off, ax_g, a4, w4, priv, priv_stride);
+    else
+        k_hg_build<false><<<grid, 256, 0, s>>>(v, I, N, tpr, eqc, mx_off, mx_g, ax_off, ax_g, a4, w4, priv, priv_stride);
     return cudaGetLastError();
+}
+
+// p with its fold weights; `both` when hr[0] (round 0's challenges), `r1` when hr[1] rather than
+// r follows it.
+static RoundPtrs with_weights(const RoundPtrs& p, int reps, bool both, bool r1 = false) {
+    RoundPtrs q = p;
+    for (int j = 0; j < reps; j++) {
+        q.c[j] = m31::lerp_at(p.r[j]);
+        if (!both) continue;
+        q.c0[j] = m31::lerp_at(p.hr[0][j]);
+        q.c01[j] = m31::lerp2_at(p.hr[0][j], r1 ? p.hr[1][j] : p.r[j]);
+    }
+    return q;
 }
 
 // Dynamic shared memory of the staged kernels: the cp.async ring, or the reduction's
@@ -1777,9 +1798,11 @@ cudaError_t launch_hg_round1(int reps, const uint32_t* v, uint64_t npairs, const
                              uint32_t* evals_out, cudaStream_t s) {
     if (quads && p.fdst[0]) return cudaErrorInvalidValue;  // stored folded copies need every pair
     if (!red.evals_dev) return cudaErrorInvalidValue;       // the claim is round 0's polynomial
+    if (reps < 1 || reps > 3) return cudaErrorInvalidValue;
+    const RoundPtrs q = with_weights(p, reps, false);
     LaunchShape sh = row_shape(g, npairs, block, ctas, 2 * reps);
 #define GKR_HG1(RR) \
-    k_hg_round1<RR><<<sh.grid, sh.block, sh.smem, s>>>(v, npairs, quads, mx_off, mx_g, a4, w4r, p, g, red, evals_out)
+    k_hg_round1<RR><<<sh.grid, sh.block, sh.smem, s>>>(v, npairs, quads, mx_off, mx_g, a4, w4r, q, g, red, evals_out)
     switch (reps) {
         case 1: GKR_HG1(1); break;
         case 2: GKR_HG1(2); break;
@@ -1828,11 +1851,12 @@ cudaError_t launch_round(int reps, bool shared_src, bool lane_hg, bool fold_, co
         }
         return cudaGetLastError();
     }
+    const RoundPtrs pw = with_weights(p, reps, false);
     if (!red.evals_dev) return cudaErrorInvalidValue;  // fold rounds take their claim from it
     if (shared_src) {
         // one read of the shared layer input for all repetitions
         LaunchShape sh = row_shape(g, npairs, block, ctas, 2 * reps);
-#define GKR_SHARED(RR, LH, FO) k_round_shared<RR, LH, FO><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, vx, g, red, evals_out)
+#define GKR_SHARED(RR, LH, FO) k_round_shared<RR, LH, FO><<<sh.grid, sh.block, sh.smem, s>>>(pw, npairs, vx, g, red, evals_out)
 #define GKR_SHARED_R(RR)                                  \
     if (lane_hg) GKR_SHARED(RR, true, true);              \
     else GKR_SHARED(RR, false, true);
@@ -1846,14 +1870,9 @@ cudaError_t launch_round(int reps, bool shared_src, bool lane_hg, bool fold_, co
         return cudaGetLastError();
     }
     LaunchShape sh = rep_shape(g, npairs, block, ctas, reps);
-#define GKR_ROUND(SH, LH, FO) k_round<SH, LH, FO><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, vx, g, reps, red, evals_out)
-    if (lane_hg) {
-        if (shared_src) GKR_ROUND(true, true, true);
-        else GKR_ROUND(false, true, true);
-    } else {
-        if (shared_src) GKR_ROUND(true, false, true);
-        else GKR_ROUND(false, false, true);
-    }
+#define GKR_ROUND(SH, LH, FO) k_round<SH, LH, FO><<<sh.grid, sh.block, sh.smem, s>>>(pw, npairs, vx, g, reps, red, evals_out)
+    if (lane_hg) GKR_ROUND(false, true, true);
+    else GKR_ROUND(false, false, true);
 #undef GKR_ROUND
     return cudaGetLastError();
 }
@@ -1862,22 +1881,25 @@ cudaError_t launch_round_hr(int round, int reps, const RoundPtrs& p, uint64_t np
                             uint32_t ctas, RedScratch red, uint32_t* evals_out, cudaStream_t s) {
     if (reps < 1 || reps > 3 || !p.hoff || !p.ha || (round != 2 && round != 3) || !red.evals_dev)
         return cudaErrorInvalidValue;
+    const RoundPtrs q = with_weights(p, reps, true, true);
     LaunchShape sh = rep_shape(g, npairs, block, ctas, reps);
     if (round == 2)
-        k_round<false, true, true, 1><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, nullptr, g, reps, red, evals_out);
+        k_round<false, true, true, 1><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, nullptr, g, reps, red, evals_out);
     else
-        k_round<false, true, true, 2><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, nullptr, g, reps, red, evals_out);
+        k_round<false, true, true, 2><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, nullptr, g, reps, red, evals_out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_p1_round2(int reps, const RoundPtrs& p, uint64_t npairs, const Geo& g, uint32_t block,
                              uint32_t ctas, RedScratch red, uint32_t* evals_out, cudaStream_t s) {
     if (!p.hoff || !p.ha || !red.evals_dev) return cudaErrorInvalidValue;
+    if (reps < 1 || reps > 3) return cudaErrorInvalidValue;
+    const RoundPtrs q = with_weights(p, reps, true);
     LaunchShape sh = row_shape(g, npairs, block, ctas, 2 * reps);
     switch (reps) {
-        case 1: k_p1_round2<1><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, g, red, evals_out); break;
-        case 2: k_p1_round2<2><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, g, red, evals_out); break;
-        case 3: k_p1_round2<3><<<sh.grid, sh.block, sh.smem, s>>>(p, npairs, g, red, evals_out); break;
+        case 1: k_p1_round2<1><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, g, red, evals_out); break;
+        case 2: k_p1_round2<2><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, g, red, evals_out); break;
+        case 3: k_p1_round2<3><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, g, red, evals_out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -1886,28 +1908,37 @@ cudaError_t launch_p1_round2(int reps, const RoundPtrs& p, uint64_t npairs, cons
 cudaError_t launch_p2_round2(int reps, const RoundPtrs& p, uint64_t npairs, const uint32_t* vx, const Geo& g,
                              uint32_t block, uint32_t ctas, RedScratch red, uint32_t* evals_out, cudaStream_t s) {
     if (!red.evals_dev || block > 256) return cudaErrorInvalidValue;
+    if (reps < 1 || reps > 3) return cudaErrorInvalidValue;
+    const RoundPtrs q = with_weights(p, reps, true);
     LaunchShape sh = row_shape(g, npairs, block, ctas, 2 * reps);
     const size_t ring = (size_t)kRowStages * 8 * sizeof(uint4) * block;
     const size_t smem = ring > sh.smem ? ring : sh.smem;
     switch (reps) {
-        case 1: k_p2_round2<1><<<sh.grid, sh.block, ring_smem<k_p2_round2<1>>(smem), s>>>(p, npairs, vx, g, red, evals_out); break;
-        case 2: k_p2_round2<2><<<sh.grid, sh.block, ring_smem<k_p2_round2<2>>(smem), s>>>(p, npairs, vx, g, red, evals_out); break;
-        case 3: k_p2_round2<3><<<sh.grid, sh.block, ring_smem<k_p2_round2<3>>(smem), s>>>(p, npairs, vx, g, red, evals_out); break;
+        case 1: k_p2_round2<1><<<sh.grid, sh.block, ring_smem<k_p2_round2<1>>(smem), s>>>(q, npairs, vx, g, red, evals_out); break;
+        case 2: k_p2_round2<2><<<sh.grid, sh.block, ring_smem<k_p2_round2<2>>(smem), s>>>(q, npairs, vx, g, red, evals_out); break;
+        case 3: k_p2_round2<3><<<sh.grid, sh.block, ring_smem<k_p2_round2<3>>(smem), s>>>(q, npairs, vx, g, red, evals_out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-// Lanes per row slice of the one-copy-per-thread kernels: the largest divisor of N up to 256.
+// Copies per row slice of the one-copy-per-thread kernel: the multiple of 32 up to 256 that
+// keeps most of the threads at work (the last slice of a row, and the threads of a CTA that
+// make no whole slice, stay idle), the widest of those; 0 where less than half would work.
 static uint32_t one_copy_slice(uint32_t N) {
-    uint32_t L = N < 256 ? N : 256;
-    while (L > 1 && N % L) L--;
-    return L;
+    uint32_t best = 0;
+    uint64_t best_used = 0;  // of 256 x slices threads, N copies are of use
+    for (uint32_t L = 32; L <= 256; L += 32) {
+        const uint32_t slices = (N + L - 1) / L;
+        const uint64_t used = (uint64_t)N * (256 / L) * 65536 / ((uint64_t)slices * 256);
+        if (slices <= 1024 && used >= best_used) best = L, best_used = used;  // a ticket per slice
+    }
+    return best_used * 2 >= 65536 ? best : 0;
 }
 
 uint32_t p2_round01_groups(uint32_t N) {
-    const uint32_t L = N ? one_copy_slice(N) : 1;
-    return L % 32 ? 0 : N / L;
+    const uint32_t L = one_copy_slice(N);
+    return L ? (N + L - 1) / L : 0;
 }
 
 cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const* s, const uint32_t* const* t,
@@ -1919,7 +1950,7 @@ cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const
     g.N = N;
     g.tpr = one_copy_slice(N);
     g.rps = 256 / g.tpr;
-    const uint32_t groups = N / g.tpr;
+    const uint32_t groups = p2_round01_groups(N);
     uint64_t need = (ngroups + (uint64_t)g.rps * kMinRowIters - 1) / ((uint64_t)g.rps * kMinRowIters), cap = ctas / groups;
     if (cap < 1) cap = 1;
     if (need < 1) need = 1;
@@ -1960,16 +1991,16 @@ cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g
                            uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, cudaStream_t s) {
     if (t_out && (I % 4 || s_stride % 4)) return cudaErrorInvalidValue;
     if (t_out)
-        k_s_build<true><<<grid_1d(I / 4, 256), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, t_out, s_stride);
+        k_s_build<true><<<grid_eq(I), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, t_out, s_stride);
     else
-        k_s_build<false><<<grid_1d(I, 256), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, nullptr, s_stride);
+        k_s_build<false><<<grid_eq(I), 256, 0, s>>>(I, my_off, my_g, eqc, eqx, s_out, nullptr, s_stride);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,
                         RedScratch red, uint32_t* out, cudaStream_t s) {
     const uint64_t rows = 1ull << eq.nvars;
-    const uint32_t groups = g.N / (4 * g.tpr), cap = ctas / groups ? ctas / groups : 1, rb = wsum_block(g, rows, cap);
+    const uint32_t groups = lane_groups(g), cap = ctas / groups ? ctas / groups : 1, rb = wsum_block(g, rows, cap);
     const uint64_t need = (rows + rb - 1) / rb;
     const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);
     const size_t weights = 4 * (size_t)eq.reps * rb, scratch = 4 * (size_t)eq.reps * 4 * block;

@@ -3,17 +3,21 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "m31.cuh"
+
 namespace gkrgpu {
 
 // Thread tile for a table of rows x N lanes stored row-major (row r, lane k at r*N + k).
 // Each thread owns 4 consecutive lanes (one 16-byte load); tpr threads cover a slice of
-// 4*tpr lanes of one row, rps such slices (rows) share a CTA, and gridDim.y = N/(4*tpr)
-// lane groups cover the whole row.
+// 4*tpr lanes of one row, rps such slices (rows) share a CTA, and gridDim.y = lane_groups
+// lane groups cover the whole row (the threads of the last one beyond lane N stay idle).
 struct Geo {
     uint32_t N;    // lanes (data-parallel circuit copies), multiple of 4
     uint32_t tpr;  // threads per row slice
     uint32_t rps;  // row slices per CTA (blockDim.x / tpr)
 };
+
+inline uint32_t lane_groups(const Geo& g) { return (g.N / 4 + g.tpr - 1) / g.tpr; }
 
 // Scratch of the reducing kernels: per-(component, lane) 64-bit accumulators and the
 // arrival ticket of the last-CTA finisher.  Both are left zeroed by every launch.
@@ -54,6 +58,11 @@ struct RoundPtrs {
     const uint32_t* hoff;
     const uint4* ha;
     uint32_t hr[2][3];
+    // Fold weights at r, at hr[0], and at hr[0] then r, set by the launch wrappers: as kernel
+    // parameters they are constant operands of the multiply-adds and take no registers (in
+    // registers, k_p1_round2 went from 128 to 130 of them and from two CTAs an SM to one).
+    m31::Lerp c[3], c0[3];
+    m31::Lerp2 c01[3];
 };
 
 // Persistent sumcheck phase (k_phase, phase.cu): rounds k0 .. n-1 in one launch, one CTA per
@@ -208,8 +217,8 @@ cudaError_t launch_round(int reps, bool shared_src, bool lane_hg, bool fold, con
 // 9 * reps canonical sums per copy go to sums_out (9 reps x N) for launch_p2_round1_fin.
 // s[j] are the scalar tables (16-byte aligned), t[j] their pair sums (launch_s_build4);
 // red.acc needs 9 * reps x N accumulators.  Publishes p2_round01_groups(N) lane groups;
-// p2_round01_groups(N) is 0 where the kernel does not apply (its row slices of up to 256
-// copies must be a multiple of 32 copies).
+// p2_round01_groups(N) is 0 where the kernel does not apply (too many of the threads of its
+// 32-copy warps would be idle).
 // Groups i < ngroups are rows 4q .. 4q+3 with q = quads[i] (q = i without a list); a list
 // may leave out only groups with no mul gate whose second input is in them (s_j zero there).
 cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const* s, const uint32_t* const* t,
@@ -234,10 +243,15 @@ uint32_t phase_ctas(uint32_t N, uint32_t tpr);
 // Quads a CTA's tables take when the first round reads `items` rows x tpr.
 size_t phase_priv_quads(uint64_t items);
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s);
-// The layer input (I rows) and hg in the tables of a phase-one launch with k0 = 0.
+// The layer input (I rows) and hg in the tables of a phase-one launch with k0 = 0: with a4 from
+// the stored weights a4, w4 (launch_weights), without it from eqc.
 cudaError_t launch_hg_build(const uint32_t* v, uint32_t I, uint32_t N, uint32_t tpr, const EqArgs& eqc,
                             const uint32_t* mx_off, const uint4* mx_g, const uint32_t* ax_off, const uint2* ax_g,
-                            uint4* priv, size_t priv_stride, cudaStream_t s);
+                            const uint4* a4, const uint4* w4, uint4* priv, size_t priv_stride, cudaStream_t s);
+// Whether to store a layer's weights first: computing them for every four copies is 150
+// instructions a gate, 4 us of the chip at 2^20 (a launch more costs as much); 2^18 gates at
+// 1024 copies took 1.2 ms that way.
+inline bool hg_build_stored(uint64_t gates, uint32_t N) { return gates * (N / 4) > (1u << 20); }
 // eval_multilinear of vals (2^eq.nvars rows) at eq.r1_j for eq.reps points (eq.f1 = 1, no second
 // point): out receives reps x N.
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,

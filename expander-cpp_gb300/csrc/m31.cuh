@@ -85,6 +85,30 @@ GKR_HD uint32_t lerp(uint32_t a, uint32_t b, const Lerp& c) {
     return umin(s, s - P);
 }
 
+// Two folds in one, at challenges r0 and then r1, as a weighted sum of four rows with weights
+// (1 - r0)(1 - r1), r0 (1 - r1), (1 - r0) r1, r0 r1 (canonical).  t = sum x_e c_e <= 4 (p - 1)^2 =
+// 2^64 - 2^35 + 16; with t = 2^32 hi + lo == lo + 2 hi, the low and high parts are brought below
+// 2^31 + 1 and 2^31 - 15 first, so their sum stays below 2p.  Four wide multiply-adds where three
+// lerps take six.
+struct Lerp2 {
+    uint32_t c[4];
+};
+GKR_HD Lerp2 lerp2_at(uint32_t r0, uint32_t r1) {
+    const uint32_t s0 = sub(1u, r0), s1 = sub(1u, r1);
+    Lerp2 w;
+    w.c[0] = mul(s0, s1);
+    w.c[1] = mul(r0, s1);
+    w.c[2] = mul(s0, r1);
+    w.c[3] = mul(r0, r1);
+    return w;
+}
+GKR_HD uint32_t lerp2(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, const Lerp2& w) {
+    const uint64_t t = (uint64_t)x0 * w.c[0] + (uint64_t)x1 * w.c[1] + (uint64_t)x2 * w.c[2] + (uint64_t)x3 * w.c[3];
+    const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
+    const uint32_t s = ((lo & P) + (lo >> 31)) + (((hi << 1) & P) + (hi >> 30));
+    return umin(s, s - P);
+}
+
 // Evaluation at 2 of the degree-2 round polynomial from p0 = h(0), p1 = h(1) and
 // p2raw = sum (f0+f1)(g0+g1) = 4 h(1/2): 6 p1 + 3 p0 - 2 p2raw (sumcheck_helper.hpp:100).
 GKR_HD uint32_t eval_at_two(uint32_t p0, uint32_t p1, uint32_t p2raw) {

@@ -533,20 +533,35 @@ struct gkrgpu_ctx {
         if (pool) cudaMemPoolDestroy(pool);
     }
 
-    // Tile of kernel kind `kid` for N copies: the largest divisor of N/4 not above its tpr.
+    // Row tile of kernel kind `kid` for N copies: of the widths from half the kind's tpr up to
+    // it, the one that leaves the fewest threads idle (those of the last lane group beyond N and
+    // those of a CTA that make no whole slice), the widest of those; a row narrower than the
+    // kind's tpr is one slice.  (The largest divisor of N/4 left one thread a row at 268 = 4 * 67
+    // copies, whose 16-byte accesses ran at 1.5-2 TB/s.)
     Geo geo(uint32_t N, int kid) const {
-        const uint32_t Q = N / 4;
-        uint32_t tpr = Q;
-        const uint32_t want = std::min<uint32_t>(tiles[kid].tpr, block);
-        if (tpr > want) {
-            tpr = want;
-            while (tpr > 1 && Q % tpr) tpr--;
+        const uint32_t Q = N / 4, want = std::min<uint32_t>(tiles[kid].tpr, block);
+        Geo g{N, divisor_tile(Q, want), 1};
+        if (Q > want) {
+            uint64_t best = 0;
+            for (uint32_t t = (want + 1) / 2; t <= want; t++) {
+                const uint32_t groups = (Q + t - 1) / t;
+                const uint64_t used = ((uint64_t)Q * (block / t) << 20) / groups;
+                if (groups <= kMaxLaneGroups && used >= best) best = used, g.tpr = t;
+            }
         }
-        Geo g;
-        g.N = N;
-        g.tpr = tpr;
-        g.rps = block / tpr;
+        g.rps = block / g.tpr;
         return g;
+    }
+    // Copy counts are accepted as far as the largest divisor of N/4 within the kind's tpr tiles
+    // a row in at most kMaxLaneGroups slices (each has an arrival ticket).
+    static constexpr uint32_t kMaxLaneGroups = 1024;
+    static uint32_t divisor_tile(uint32_t Q, uint32_t want) {
+        uint32_t t = std::min(want, Q);
+        while (t > 1 && Q % t) t--;
+        return t;
+    }
+    bool copies_ok(uint32_t N, int kid) const {
+        return N / 4 / divisor_tile(N / 4, std::min<uint32_t>(tiles[kid].tpr, block)) <= kMaxLaneGroups;
     }
     uint32_t cta_budget(int kid) const {
         if (tiles[kid].ctas) return tiles[kid].ctas;
@@ -1075,7 +1090,7 @@ struct Prover {
         });
         return done ? incs : 0;
     }
-    uint32_t groups(int kid) const { return N / (4 * gk[kid].tpr); }
+    uint32_t groups(int kid) const { return lane_groups(gk[kid]); }
 
     void reserve(bool own_input, bool sumcheck) {
         ws.plan(nullptr, C, N, R, own_input, sumcheck, tpr);
@@ -1419,16 +1434,21 @@ struct Prover {
         const uint32_t kt1 = phase_start(n, 4);
         PhaseArgs a1 = {};
         a1.n = n;
-        const bool whole = kt1 == 0 && run_phase(t, true, a1, rx, true, vxh, rb * 9.0 * R * I, [&] {
-            c.launch(K_HG_BUILD, rb * (I + Ly.nmul + (double)(1 + R) * I) + 16.0 * Ly.nmul + 8.0 * Ly.nadd, [&] {
-                return launch_hg_build(v, (uint32_t)I, N, tpr, eqc, Ly.mx_off, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.priv,
-                                       ws.priv_stride, c.stream);
-            });
-        });
-        if (!whole) {
+        auto weights = [&] {
             c.launch(K_WEIGHTS, 32.0 * Ly.nmul + 20.0 * I + 8.0 * Ly.nadd, [&] {
                 return launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, c.stream);
             });
+        };
+        const bool whole = kt1 == 0 && run_phase(t, true, a1, rx, true, vxh, rb * 9.0 * R * I, [&] {
+            const bool stored = hg_build_stored(Ly.nmul + Ly.nadd, N);
+            if (stored) weights();
+            c.launch(K_HG_BUILD, rb * (I + Ly.nmul + (double)(1 + R) * I) + 16.0 * Ly.nmul + 8.0 * Ly.nadd, [&] {
+                return launch_hg_build(v, (uint32_t)I, N, tpr, eqc, Ly.mx_off, Ly.mx_g, Ly.ax_off, Ly.ax_g,
+                                       stored ? ws.a4 : nullptr, ws.w4, ws.priv, ws.priv_stride, c.stream);
+            });
+        });
+        if (!whole) {
+            weights();
             phase_one_rounds(t, li, std::max(kt1, std::min(n, 4u)), alpha, beta, rx);
         }
 
@@ -1550,12 +1570,8 @@ void check_run(gkrgpu_ctx* ctx, const gkrgpu_circuit* circuit, uint32_t n_copies
     }
     if (n_copies < 4 || n_copies % 4 || n_copies > (1u << 16))
         fail(GKRGPU_ERR_INVALID, "n_copies must be a multiple of 4 in [4, 65536], got %u", n_copies);
-    const uint32_t Q = n_copies / 4;
-    for (int k = 0; k < K_BN_LOAD; k++) {
-        const Geo g = ctx->geo(n_copies, k);
-        if (g.tpr * (Q / g.tpr) != Q) fail(GKRGPU_ERR_INVALID, "no row tile divides %u copies", n_copies);
-        if (Q / g.tpr > 1024) fail(GKRGPU_ERR_INVALID, "more than 1024 lane groups; raise threads_per_row");
-    }
+    for (int k = 0; k < K_BN_LOAD; k++)
+        if (!ctx->copies_ok(n_copies, k)) fail(GKRGPU_ERR_INVALID, "more than 1024 lane groups; raise threads_per_row");
 }
 
 // Commitment (the input rows) + grinding + per layer R x (2n rounds x 3 rows + vx + vy).
@@ -2137,8 +2153,7 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
             for (uint32_t t = 0; t < nb_vars; t++)
                 if (r[(size_t)j * nb_vars + t] >= m31::P) fail(GKRGPU_ERR_INVALID, "point coordinate >= p");
         const Geo g = ctx->geo(n_copies, K_WSUM);
-        if (g.tpr * ((n_copies / 4) / g.tpr) != n_copies / 4) fail(GKRGPU_ERR_INVALID, "no row tile divides n_copies");
-        if ((n_copies / 4) / g.tpr > 1024) fail(GKRGPU_ERR_INVALID, "more than 1024 lane groups");
+        if (!ctx->copies_ok(n_copies, K_WSUM)) fail(GKRGPU_ERR_INVALID, "more than 1024 lane groups");
         on_idle_lane(ctx, [&](Lane& c) {
             const uint64_t rowb = (uint64_t)n_copies * 4;
             EqArgs a;
@@ -2157,7 +2172,7 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
                                    reinterpret_cast<uint32_t*>(c.extra_d()), c.stream);
             });
             c.pending_bytes = 0;  // spin: the caller's thread may not sleep to the microsecond
-            c.wait_done((n_copies / 4) / g.tpr);
+            c.wait_done(lane_groups(g));
             memcpy(out, c.extra_h(), n_points * rowb);
             if (ctx->timing) c.sync();  // the launch's closing event
             c.resolve_events();

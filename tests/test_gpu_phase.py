@@ -61,3 +61,25 @@ def test_bn254_phases_give_the_oracle_proof(ctx, seed, widths, n):
         ctx.set_round_tail(True)
     ocv, op = OracleBn254().prove(circ, w)
     assert proof == op and np.array_equal(cv, ocv)
+
+
+@pytest.mark.parametrize("seed,widths,n", [
+    (631, [13, 14], 268), (632, [14, 13], 148), (633, [12, 14], 44), (634, [10, 15], 36), (635, [13, 14, 13], 1036),
+    (636, [5, 4], 4084),
+])
+def test_row_tiles_that_do_not_divide_the_copies(ctx, oracle, seed, widths, n):
+    # n / 4 = 67, 37, 11, 9, 259, 1021: the last lane group of a row is partly idle; every round
+    # as its own launch, so that every row-tiled kernel runs on such tiles
+    circ = gc.random_circuit(seed, widths, p_mul=0.6)
+    w = gc.random_witness(seed, circ.log_input_size, n)
+    dc = ctx.load(circ)
+    try:
+        ctx.set_round_tail(False)
+        cv, proof = ctx.prove(dc, w)
+    finally:
+        ctx.set_round_tail(True)
+    assert ctx.prove(dc, w)[1] == proof
+    ocv, op = oracle.prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
+    assert np.array_equal(ctx.evaluate(dc, w), oracle.evaluate(circ, w)[-1])
+    assert ctx.verify(dc, proof, cv)
