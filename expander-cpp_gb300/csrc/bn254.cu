@@ -4,6 +4,7 @@
 // 8 x 32-bit limbs (CIOS as PTX multiply-add carry chains).
 #include "bn254.cuh"
 
+#include <algorithm>
 #include <atomic>
 
 namespace gkrgpu {
@@ -533,6 +534,156 @@ __global__ void k_load(const uint32_t* __restrict__ canon, uint32_t* __restrict_
     }
 }
 
+// Montgomery -> canonical, in place.
+__global__ void k_unload(uint32_t* v, uint64_t n) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    Fr* t = reinterpret_cast<Fr*>(v);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint4* p = reinterpret_cast<const uint4*>(t + i);
+        const uint4 a = p[0], b = p[1];
+        Fr x;
+        x.l[0] = a.x; x.l[1] = a.y; x.l[2] = a.z; x.l[3] = a.w;
+        x.l[4] = b.x; x.l[5] = b.y; x.l[6] = b.z; x.l[7] = b.w;
+        sts(t, i, from_mont(x));
+    }
+}
+
+__global__ void __launch_bounds__(256) k_evaluate(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t O,
+                                                  const uint32_t* __restrict__ mo_off, const uint4* __restrict__ mo_g,
+                                                  const Fr* __restrict__ mo_c, const uint32_t* __restrict__ ao_off,
+                                                  const uint2* __restrict__ ao_g, const Fr* __restrict__ ao_c, GeoBn g) {
+    const Tile t = tile(g);
+    if (!t.active) return;
+    for (uint64_t o = (uint64_t)blockIdx.x * g.rps + t.rs; o < O; o += (uint64_t)gridDim.x * g.rps) {
+        Fr acc = zero();
+        const uint32_t m0 = __ldg(mo_off + o), m1 = __ldg(mo_off + o + 1);
+        for (uint32_t k = m0; k < m1; k++) {
+            const uint4 gt = __ldg(mo_g + k);
+            acc = add(acc, mul(mul(ldf(in, gt.x, g.N, t.q), ldf(in, gt.y, g.N, t.q)), lds(mo_c, k)));
+        }
+        const uint32_t a0 = __ldg(ao_off + o), a1 = __ldg(ao_off + o + 1);
+        for (uint32_t k = a0; k < a1; k++) {
+            const uint2 gt = __ldg(ao_g + k);
+            acc = add(acc, mul(ldf(in, gt.x, g.N, t.q), lds(ao_c, k)));
+        }
+        stf(out, o, g.N, t.q, acc);
+    }
+}
+
+// ---------------------------------------------------------------- eq factors
+// f1 eq(r1, z) + f2 eq(r2, z), eq(r, z) = prod over bits t of z of (bit ? r_t : 1 - r_t), from
+// tables of 256 entries per eight bits that a CTA builds in shared memory: one product a point
+// where the factor is used (up to 2^16), where a table over z was a launch of its own (15 us at
+// 2^9 entries, 25 at 2^16) in front of every user.  They are built from tables of 16 entries
+// per four bits, a chain of three products.  (Tables of 32 entries straight from the
+// bits, as for M31, took 21 us of a 2^9 layer's weights and 63 of a 2^16 layer's.)
+constexpr uint32_t kEqBits = 8, kEqEntries = 1u << kEqBits;
+
+__host__ __device__ inline uint32_t eq_tables(const EqArgsBn& a) {
+    return a.nvars > kEqBits ? (a.nvars + kEqBits - 1) / kEqBits : 1u;
+}
+__host__ __device__ inline uint32_t eq_points(const EqArgsBn& a) { return a.has_r2 ? 2u : 1u; }
+// Elements of shared memory: the tables, then the building scratch (shared by several args).
+__host__ __device__ inline uint32_t eq_elems(const EqArgsBn& a) { return eq_points(a) * eq_tables(a) * kEqEntries; }
+__host__ __device__ inline uint32_t eq_scratch(const EqArgsBn& a) { return eq_points(a) * eq_tables(a) * 32; }
+
+// Fills t (eq_elems entries) with the help of u (eq_scratch); the whole CTA calls it, and
+// synchronises before it uses either again.
+__device__ __forceinline__ void eq_build(Fr* t, Fr* u, const EqArgsBn& a) {
+    const uint32_t nt = eq_tables(a), pts = eq_points(a);
+    for (uint32_t i = threadIdx.x; i < pts * nt * 32; i += blockDim.x) {
+        const uint32_t p = i / (nt * 32), d = (i - p * nt * 32) >> 4, x = i & 15;
+        const uint32_t(*r)[8] = p ? a.r2 : a.r1;
+        auto factor = [&](uint32_t b) {
+            Fr f;
+            const bool bit = (x >> b) & 1;
+            const uint32_t v = 4 * d + b;
+            if (v == 0) {  // with the point's factor
+#pragma unroll
+                for (int l = 0; l < 8; l++) f.l[l] = p ? a.first2[bit][l] : a.first1[bit][l];
+                return f;
+            }
+#pragma unroll
+            for (int l = 0; l < 8; l++) f.l[l] = r[v][l];
+            return bit ? f : sub(one(), f);
+        };
+        const uint32_t left = a.nvars > 4 * d ? a.nvars - 4 * d : 0;
+        if (left == 0) {
+            if (d == 0) u[i] = factor(0);  // no variables at all: the point's factor
+            continue;
+        }
+        Fr e = factor(0);
+        if (left > 1) e = mul(e, factor(1));
+        if (left > 2) {
+            Fr g = factor(2);
+            if (left > 3) g = mul(g, factor(3));
+            e = mul(e, g);
+        }
+        u[i] = e;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < pts * nt * kEqEntries; i += blockDim.x) {
+        const uint32_t pd = i >> kEqBits, x = i & (kEqEntries - 1);  // pd = p nt + d
+        const uint32_t bits = a.nvars - (pd % nt) * kEqBits;
+        if (x >> (bits < kEqBits ? bits : kEqBits)) continue;
+        const Fr lo = u[pd * 32 + (x & 15)];
+        t[i] = bits > 4 ? mul(lo, u[pd * 32 + 16 + (x >> 4)]) : lo;
+    }
+}
+__device__ __forceinline__ Fr eq_at(const Fr* t, uint32_t nt, bool two, uint32_t z) {
+    Fr e = t[z & (kEqEntries - 1)];
+    Fr f = two ? t[nt * kEqEntries + (z & (kEqEntries - 1))] : zero();
+#pragma unroll 1
+    for (uint32_t d = 1; d < nt; d++) {
+        const uint32_t x = d * kEqEntries + ((z >> (kEqBits * d)) & (kEqEntries - 1));
+        e = mul(e, t[x]);
+        if (two) f = mul(f, t[nt * kEqEntries + x]);
+    }
+    return two ? add(e, f) : e;
+}
+extern __shared__ uint4 eqsm_raw[];
+
+// Lanes that share a row's gates (about one a row, but four in the longest row of a warp, each a
+// chain of three products), and their sums' total in the first of them.
+constexpr uint32_t kRowLanes = 4;
+__device__ __forceinline__ Fr row_sum(Fr s, uint32_t gates) {
+    const uint32_t m = 0xfu << (threadIdx.x & 28);  // the row's lanes
+    if (gates < 2) return s;                        // (in the first lane already)
+#pragma unroll
+    for (uint32_t off = 2; off > 0; off >>= 1) {
+        Fr o;
+#pragma unroll
+        for (int l = 0; l < 8; l++) o.l[l] = __shfl_xor_sync(m, s.l[l], off);
+        s = add(s, o);
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(256) k_weights(uint64_t I, uint64_t Gm, const __grid_constant__ EqArgsBn eqc,
+                                                 const uint4* __restrict__ mx_g, const Fr* __restrict__ mx_c,
+                                                 const uint32_t* __restrict__ ax_off, const uint2* __restrict__ ax_g,
+                                                 const Fr* __restrict__ ax_c, Fr* __restrict__ a_out, Fr* __restrict__ w_out) {
+    Fr* const t = reinterpret_cast<Fr*>(eqsm_raw);
+    eq_build(t, t + eq_elems(eqc), eqc);
+    __syncthreads();
+    const uint32_t nd = eq_tables(eqc);
+    const bool two = eqc.has_r2;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t n = kRowLanes * I > Gm ? kRowLanes * I : Gm;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        if (i < Gm) sts(w_out, i, mul(lds(mx_c, i), eq_at(t, nd, two, __ldg(&mx_g[i].y))));
+        const uint64_t x = i / kRowLanes;
+        if (x < I) {
+            const uint32_t l = (uint32_t)i % kRowLanes, k0 = __ldg(ax_off + x), k1 = __ldg(ax_off + x + 1);
+            Fr s = zero();
+            for (uint32_t k = k0 + l; k < k1; k += kRowLanes)
+                s = add(s, mul(lds(ax_c, k), eq_at(t, nd, two, __ldg(&ax_g[k].x))));
+            s = row_sum(s, k1 - k0);
+            if (l == 0) sts(a_out, x, s);
+        }
+    }
+}
+
 // Verifier gate sums (eval_sparse_circuit_connect_poly, one repetition): over the mul gates
 // sum c eqz[o] eqx[i0] eqy[i1], or over the add gates sum c eqz[o] eqx[i0], walked by output
 // (the evaluate CSR with Montgomery coefficients).  Thread sums -> warp shuffles -> shared
@@ -540,23 +691,33 @@ __global__ void k_load(const uint32_t* __restrict__ canon, uint32_t* __restrict_
 template <bool MUL>
 __global__ void __launch_bounds__(256) k_gate_sums(uint64_t O, const uint32_t* __restrict__ off,
                                                    const uint32_t* __restrict__ gates, const Fr* __restrict__ coef,
-                                                   const Fr* __restrict__ eqz, const Fr* __restrict__ eqx,
-                                                   const Fr* __restrict__ eqy, unsigned long long* acc,
+                                                   const __grid_constant__ GateEqBn eq, unsigned long long* acc,
                                                    unsigned int* ticket, uint32_t* out) {
+    Fr* const tz = reinterpret_cast<Fr*>(eqsm_raw);
+    Fr* const tx = tz + eq_elems(eq.z);
+    Fr* const ty = tx + eq_elems(eq.x);
+    Fr* const u = ty + (MUL ? eq_elems(eq.y) : 0);
+    eq_build(tz, u, eq.z);
+    __syncthreads();
+    eq_build(tx, u, eq.x);
+    __syncthreads();
+    if (MUL) eq_build(ty, u, eq.y);
+    __syncthreads();
+    const uint32_t ndz = eq_tables(eq.z), ndx = eq_tables(eq.x);
     Fr s = zero();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < O; o += stride) {
         const uint32_t k0 = __ldg(off + o), k1 = __ldg(off + o + 1);
         if (k0 == k1) continue;
-        const Fr ez = lds(eqz, o);
+        const Fr ez = eq_at(tz, ndz, eq.z.has_r2, (uint32_t)o);
         for (uint32_t k = k0; k < k1; k++) {
             Fr t;
             if (MUL) {
                 const uint4 g = __ldg(reinterpret_cast<const uint4*>(gates) + k);  // (i0, i1, c, 0)
-                t = mul(mul(lds(eqx, g.x), lds(eqy, g.y)), lds(coef, k));
+                t = mul(mul(eq_at(tx, ndx, false, g.x), eq_at(ty, ndx, false, g.y)), lds(coef, k));
             } else {
                 const uint2 g = __ldg(reinterpret_cast<const uint2*>(gates) + k);  // (i0, c)
-                t = mul(lds(eqx, g.x), lds(coef, k));
+                t = mul(eq_at(tx, ndx, false, g.x), lds(coef, k));
             }
             s = add(s, mul(t, ez));
         }
@@ -595,110 +756,6 @@ __global__ void __launch_bounds__(256) k_gate_sums(uint64_t O, const uint32_t* _
 #pragma unroll
         for (int k = 0; k < 8; k++) out[k] = r.l[k];
         *ticket = 0u;
-    }
-}
-
-// Montgomery -> canonical, in place.
-__global__ void k_unload(uint32_t* v, uint64_t n) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    Fr* t = reinterpret_cast<Fr*>(v);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint4* p = reinterpret_cast<const uint4*>(t + i);
-        const uint4 a = p[0], b = p[1];
-        Fr x;
-        x.l[0] = a.x; x.l[1] = a.y; x.l[2] = a.z; x.l[3] = a.w;
-        x.l[4] = b.x; x.l[5] = b.y; x.l[6] = b.z; x.l[7] = b.w;
-        sts(t, i, from_mont(x));
-    }
-}
-
-__global__ void __launch_bounds__(256) k_evaluate(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t O,
-                                                  const uint32_t* __restrict__ mo_off, const uint4* __restrict__ mo_g,
-                                                  const Fr* __restrict__ mo_c, const uint32_t* __restrict__ ao_off,
-                                                  const uint2* __restrict__ ao_g, const Fr* __restrict__ ao_c, GeoBn g) {
-    const Tile t = tile(g);
-    if (!t.active) return;
-    for (uint64_t o = (uint64_t)blockIdx.x * g.rps + t.rs; o < O; o += (uint64_t)gridDim.x * g.rps) {
-        Fr acc = zero();
-        const uint32_t m0 = __ldg(mo_off + o), m1 = __ldg(mo_off + o + 1);
-        for (uint32_t k = m0; k < m1; k++) {
-            const uint4 gt = __ldg(mo_g + k);
-            acc = add(acc, mul(mul(ldf(in, gt.x, g.N, t.q), ldf(in, gt.y, g.N, t.q)), lds(mo_c, k)));
-        }
-        const uint32_t a0 = __ldg(ao_off + o), a1 = __ldg(ao_off + o + 1);
-        for (uint32_t k = a0; k < a1; k++) {
-            const uint2 gt = __ldg(ao_g + k);
-            acc = add(acc, mul(ldf(in, gt.x, g.N, t.q), lds(ao_c, k)));
-        }
-        stf(out, o, g.N, t.q, acc);
-    }
-}
-
-// eq(r, z) * f = f * prod_t (bit t of z ? r_t : 1 - r_t) for z < 2^nvars (two tables summed
-// when has_r2).  Split at bit h = min(nvars, 8): every CTA builds the 2^h-entry table of the
-// low bits in shared memory by doubling, then each chunk of 2^h consecutive z shares one
-// high-bit product, so an entry costs one multiplication (two with has_r2).
-constexpr uint32_t kEqLowBits = 8;
-
-__device__ __forceinline__ Fr eq_factor(const uint32_t (*r)[8], uint32_t t, bool bit) {
-    Fr x;
-#pragma unroll
-    for (int k = 0; k < 8; k++) x.l[k] = r[t][k];
-    return bit ? x : sub(one(), x);
-}
-
-__global__ void __launch_bounds__(256) k_eq(Fr* __restrict__ out, EqArgsBn a) {
-    __shared__ Fr lo[2][1u << kEqLowBits];
-    __shared__ Fr hi[2];
-    const uint32_t h = a.nvars < kEqLowBits ? a.nvars : kEqLowBits;
-    const uint32_t L = 1u << h;
-    const uint32_t tabs = a.has_r2 ? 2u : 1u;
-    if (threadIdx.x < tabs) lo[threadIdx.x][0] = one();
-    __syncthreads();
-    for (uint32_t t = 0; t < h; t++) {
-        const uint32_t half = 1u << t;
-        for (uint32_t x = threadIdx.x; x < half * tabs; x += blockDim.x) {
-            const uint32_t k = x >> t, y = x & (half - 1);
-            const uint32_t(*r)[8] = k ? a.r2 : a.r1;
-            const Fr v = lo[k][y];
-            lo[k][y + half] = mul(v, eq_factor(r, t, true));
-            lo[k][y] = mul(v, eq_factor(r, t, false));
-        }
-        __syncthreads();
-    }
-    const uint64_t chunks = 1ull << (a.nvars - h);
-    for (uint64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
-        if (threadIdx.x < tabs) {
-            const uint32_t(*r)[8] = threadIdx.x ? a.r2 : a.r1;
-            Fr e;
-#pragma unroll
-            for (int k = 0; k < 8; k++) e.l[k] = threadIdx.x ? a.f2[k] : a.f1[k];
-            for (uint32_t t = h; t < a.nvars; t++) e = mul(e, eq_factor(r, t, (c >> (t - h)) & 1));
-            hi[threadIdx.x] = e;
-        }
-        __syncthreads();
-        for (uint32_t x = threadIdx.x; x < L; x += blockDim.x) {
-            Fr e = mul(lo[0][x], hi[0]);
-            if (a.has_r2) e = add(e, mul(lo[1][x], hi[1]));
-            sts(out, (c << h) + x, e);
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void k_weights(uint64_t I, uint64_t Gm, const Fr* __restrict__ eqc, const uint4* __restrict__ mx_g,
-                          const Fr* __restrict__ mx_c, const uint32_t* __restrict__ ax_off, const uint2* __restrict__ ax_g,
-                          const Fr* __restrict__ ax_c, Fr* __restrict__ a_out, Fr* __restrict__ w_out) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t n = I > Gm ? I : Gm;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        if (i < Gm) sts(w_out, i, mul(lds(mx_c, i), lds(eqc, __ldg(&mx_g[i].y))));
-        if (i < I) {
-            Fr s = zero();
-            const uint32_t k0 = __ldg(ax_off + i), k1 = __ldg(ax_off + i + 1);
-            for (uint32_t k = k0; k < k1; k++) s = add(s, mul(lds(ax_c, k), lds(eqc, __ldg(&ax_g[k].x))));
-            sts(a_out, i, s);
-        }
     }
 }
 
@@ -804,28 +861,52 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrsBn p, uint64_t npairs, c
         reduce_bn<3>(acc, g, t.active, red, RoundFinBn{evals_out, LANE_HG ? nullptr : vx, g.N, red.evals_dev});
 }
 
-__global__ void k_s_build(uint64_t I, const uint32_t* __restrict__ my_off, const uint4* __restrict__ my_g,
-                          const Fr* __restrict__ my_c, const Fr* __restrict__ eqc, const Fr* __restrict__ eqrx,
-                          Fr* __restrict__ s_out) {
+__global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __restrict__ my_off,
+                                                 const uint4* __restrict__ my_g, const Fr* __restrict__ my_c,
+                                                 const __grid_constant__ EqArgsBn eqc, const __grid_constant__ EqArgsBn eqx,
+                                                 Fr* __restrict__ s_out) {
+    Fr* const tz = reinterpret_cast<Fr*>(eqsm_raw);
+    Fr* const tx = tz + eq_elems(eqc);
+    Fr* const u = tx + eq_elems(eqx);
+    eq_build(tz, u, eqc);
+    eq_build(tx, u + eq_scratch(eqc), eqx);
+    __syncthreads();
+    const uint32_t ndz = eq_tables(eqc), ndx = eq_tables(eqx);
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t y = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; y < I; y += stride) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < kRowLanes * I; i += stride) {
+        const uint64_t y = i / kRowLanes;
+        const uint32_t l = (uint32_t)i % kRowLanes, k0 = __ldg(my_off + y), k1 = __ldg(my_off + y + 1);
         Fr s = zero();
-        const uint32_t k0 = __ldg(my_off + y), k1 = __ldg(my_off + y + 1);
-        for (uint32_t k = k0; k < k1; k++) {
+        for (uint32_t k = k0 + l; k < k1; k += kRowLanes) {
             const uint4 gt = __ldg(my_g + k);  // (x, z, c, 0)
-            s = add(s, mul(mul(lds(eqc, gt.y), lds(eqrx, gt.x)), lds(my_c, k)));
+            s = add(s, mul(mul(eq_at(tz, ndz, eqc.has_r2, gt.y), eq_at(tx, ndx, false, gt.x)), lds(my_c, k)));
         }
-        sts(s_out, y, s);
+        s = row_sum(s, k1 - k0);
+        if (l == 0) sts(s_out, y, s);
     }
 }
 
-__global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows, const Fr* __restrict__ eq,
-                                              GeoBn g, RedBn red, uint32_t* out) {
+// sum_z eq(r, z) vals[z] (eval_multilinear); the weights of a block of rows are computed from
+// the digit tables into shared memory.
+constexpr uint32_t kWsumRows = 128;  // rows a CTA takes at a time
+
+__global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows,
+                                              const __grid_constant__ EqArgsBn eq, GeoBn g, RedBn red, uint32_t* out) {
+    __shared__ Fr w[kWsumRows];
+    Fr* const tab = reinterpret_cast<Fr*>(eqsm_raw);  // then the reduction's scratch
     const Tile t = tile(g);
+    eq_build(tab, tab + eq_elems(eq), eq);
+    const uint32_t nd = eq_tables(eq);
     Fr acc[1] = {zero()};
-    if (t.active)
-        for (uint64_t z = (uint64_t)blockIdx.x * g.rps + t.rs; z < rows; z += (uint64_t)gridDim.x * g.rps)
-            acc[0] = add(acc[0], mul(lds(eq, z), ldf(vals, z, g.N, t.q)));
+    for (uint64_t z0 = (uint64_t)blockIdx.x * kWsumRows; z0 < rows; z0 += (uint64_t)gridDim.x * kWsumRows) {
+        __syncthreads();  // the digit tables are built, the last block's weights are done with
+        const uint32_t n = rows - z0 < kWsumRows ? (uint32_t)(rows - z0) : kWsumRows;
+        if (threadIdx.x < n) w[threadIdx.x] = eq_at(tab, nd, false, (uint32_t)(z0 + threadIdx.x));
+        __syncthreads();
+        if (t.active)
+            for (uint32_t i = t.rs; i < n; i += g.rps) acc[0] = add(acc[0], mul(w[i], ldf(vals, z0 + i, g.N, t.q)));
+    }
+    __syncthreads();
     reduce_bn<1>(acc, g, t.active, red, CopyFinBn{out, g.N});
 }
 
@@ -834,9 +915,9 @@ __global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals,
 // notes on the host traffic hold here): a round launched by itself takes 18-27 us on tables
 // of a few hundred rows, mostly the launch, the reduction across CTAs and a chain of dependent
 // 256-bit products in one finishing thread.  One CTA owns one copy and all its rows (a row's
-// element is one 32-byte sector, so narrower is no loss); three threads finish the three
-// evaluations.  All three sums are taken directly: a third product per pair is shorter than
-// the claim's chain of products.
+// element is one 32-byte sector, so narrower is no loss).  Four lanes take a pair: each folds
+// one of f0, f1, h0, h1, then three of them form the products of the three sums, so a round's
+// chain is two products and the finisher's one (with a thread a pair it was seven in a row).
 constexpr uint32_t kPhaseBlock = 256;
 constexpr uint32_t kPhaseWarps = kPhaseBlock / 32;
 constexpr uint32_t kSmemRowsBn = 128;  // rows of a per-copy table kept in shared memory
@@ -907,8 +988,11 @@ __global__ void __launch_bounds__(kPhaseBlock, 2) k_phase(PhaseArgsBn a) {
         if ((1u << (a.n - k)) <= kSmemRowsBn) return RowsBn{psm + ((k & 1) * kTabs + which) * kSmemRowsBn, 1};
         return mem(which == 0 ? ((k & 1) ? a.fA : a.fB) : ((k & 1) ? a.hA : a.hB));
     };
+    // a published sum is a Montgomery form times a canonical value: v(rx) in phase two, else 1
     Fr xv = zero();
+    xv.l[0] = 1u;
     if (!LANE_HG && tid < 3) xv = ldf_cv(a.vx, a.N, lane);
+    const uint32_t e = tid & 3, quad = tid & 28;  // lane's part of its pair, the pair's first lane
     if (tid == 0) stop = 0;
 
     for (uint32_t k = a.k0; k < a.n; k++) {
@@ -942,110 +1026,88 @@ __global__ void __launch_bounds__(kPhaseBlock, 2) k_phase(PhaseArgsBn a) {
         if (stop) return;
         const uint32_t npairs = 1u << (a.n - k - 1);
         const Fr r = rch;
-        Fr acc[3] = {zero(), zero(), zero()};
-        RowsBn fs = mem(const_cast<uint32_t*>(a.v)), hs = {}, fd = {}, hd = {};
-        const Fr* ssrc = a.s;
-        Fr* sdst = nullptr;
+        // this lane's source and destination tables: f for e < 2, else hg or the scalars
+        RowsBn src = mem(const_cast<uint32_t*>(a.v)), dst = {};
         if (k > 0) {
-            if (k == a.k0) fs = mem((k & 1) ? a.fB : a.fA);
-            else if (k > 1) fs = table(k - 1, 0);
-            fd = table(k, 0);
-            if (LANE_HG) {
-                hs = k == a.k0 ? mem((k & 1) ? a.hB : a.hA) : k == 1 ? mem(a.h0) : table(k - 1, 1);
-                hd = table(k, 1);
+            if (e < 2) {
+                if (k == a.k0) src = mem((k & 1) ? a.fB : a.fA);
+                else if (k > 1) src = table(k - 1, 0);
+                dst = table(k, 0);
+            } else if (LANE_HG) {
+                src = k == a.k0 ? mem((k & 1) ? a.hB : a.hA) : k == 1 ? mem(a.h0) : table(k - 1, 1);
+                dst = table(k, 1);
             } else {
                 const bool odd = (k - kf) & 1;
-                if (k > kf) ssrc = odd ? sbuf : sbuf + S1;
-                sdst = odd ? sbuf + S1 : sbuf;
+                src = RowsBn{k > kf ? (odd ? sbuf : sbuf + S1) : const_cast<Fr*>(a.s), 1};
+                dst = RowsBn{odd ? sbuf + S1 : sbuf, 1};
             }
         }
-        for (uint32_t i = tid; i < npairs; i += kPhaseBlock) {
-            Fr f0, f1, h0, h1;
-            if (k == 0) {
-                f0 = ldf(a.v, 2 * i, a.N, lane);
-                f1 = ldf(a.v, 2 * i + 1, a.N, lane);
-                if (LANE_HG) {
+        const uint32_t nw = npairs >= 8 * kPhaseWarps ? kPhaseWarps : (npairs + 7) / 8;  // warps with pairs
+        Fr acc = zero(), mine = zero();
+        if (warp < nw) {
 #pragma unroll 1
-                    for (int s = 0; s < 2; s++) {
-                        const uint32_t x = 2 * i + s;
-                        Fr h = lds(a.a, x);
+            for (uint32_t i0 = 8 * warp; i0 < npairs; i0 += 8 * kPhaseWarps) {
+                const uint32_t i = i0 + ((tid & 31) >> 2);
+                mine = zero();
+                if (i < npairs) {
+                    if (k > 0) {
+                        const uint32_t x = 4 * i + 2 * (e & 1);
+                        mine = fold(src.get(x), src.get(x + 1), r);
+                        dst.set(2 * i + (e & 1), mine);
+                    } else if (e < 2) {
+                        mine = ldf(a.v, 2 * i + e, a.N, lane);
+                    } else if (LANE_HG) {
+                        const uint32_t x = 2 * i + (e & 1);
+                        mine = lds(a.a, x);
                         const uint32_t g0 = __ldg(a.mx_off + x), g1 = __ldg(a.mx_off + x + 1);
                         for (uint32_t g = g0; g < g1; g++)
-                            h = add(h, mul(ldf(a.v, __ldg(&a.mx_g[g].x), a.N, lane), lds(a.w, g)));
-                        mem(a.h0).set(x, h);
-                        if (s == 0) h0 = h;
-                        else h1 = h;
-                    }
-                } else {
-                    h0 = lds(a.s, 2 * i);
-                    h1 = lds(a.s, 2 * i + 1);
-                }
-            } else {
-                // one copy of the fold's product for the two rows: fewer instructions to fetch
-#pragma unroll 1
-                for (int s = 0; s < 2; s++) {
-                    const uint32_t x = 4 * i + 2 * s, o = 2 * i + s;
-                    const Fr f = fold(fs.get(x), fs.get(x + 1), r);
-                    Fr h;
-                    if (LANE_HG) {
-                        h = fold(hs.get(x), hs.get(x + 1), r);
-                        hd.set(o, h);
+                            mine = add(mine, mul(ldf(a.v, __ldg(&a.mx_g[g].x), a.N, lane), lds(a.w, g)));
+                        mem(a.h0).set(x, mine);
                     } else {
-                        const RowsBn sc{const_cast<Fr*>(ssrc), 1};
-                        h = fold(sc.get(x), sc.get(x + 1), r);
-                        sts(sdst, o, h);
-                    }
-                    fd.set(o, f);
-                    if (s == 0) {
-                        f0 = f;
-                        h0 = h;
-                    } else {
-                        f1 = f;
-                        h1 = h;
+                        mine = lds(a.s, 2 * i + (e & 1));
                     }
                 }
+                __syncwarp();
+                // lanes 0, 1: f times h (of lanes 2, 3); lane 2: (f0 + f1)(h0 + h1)
+                Fr p, q, u;
+#pragma unroll
+                for (int l = 0; l < 8; l++) {
+                    p.l[l] = __shfl_sync(0xffffffffu, mine.l[l], quad | (e ^ 2));
+                    q.l[l] = __shfl_sync(0xffffffffu, mine.l[l], quad | 1);
+                    u.l[l] = __shfl_sync(0xffffffffu, mine.l[l], quad | 3);
+                }
+                const Fr x = e < 2 ? mine : add(p, q), y = e < 2 ? p : add(mine, u);
+                acc = add(acc, mul(x, y));
             }
-            accum(acc, f0, f1, h0, h1);
+            // lane e of a warp's first pair collects component e
+            for (uint32_t off = npairs < 8 ? 2 * npairs : 16; off >= 4; off >>= 1) {
+                Fr o;
+#pragma unroll
+                for (int l = 0; l < 8; l++) o.l[l] = __shfl_xor_sync(0xffffffffu, acc.l[l], off);
+                acc = add(acc, o);
+            }
+            if (nw > 1 && (tid & 31) < 3) part[warp][tid & 31] = acc;
         }
-        // sums over the warps that had pairs
-        const uint32_t nw = npairs >= kPhaseBlock ? kPhaseWarps : (npairs + 31) / 32;
-        if (warp < nw) {
-            uint32_t span = npairs < 32 ? npairs : 32;  // lanes with a pair (a power of two)
-            for (uint32_t off = span / 2; off > 0; off >>= 1)
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    Fr o;
-#pragma unroll
-                    for (int e = 0; e < 8; e++) o.l[e] = __shfl_xor_sync(0xffffffffu, acc[c].l[e], off);
-                    acc[c] = add(acc[c], o);
-                }
-            if ((tid & 31) == 0)
-#pragma unroll
-                for (int c = 0; c < 3; c++) part[warp][c] = acc[c];
-        }
-        __syncthreads();
+        if (nw > 1) __syncthreads();
         const uint32_t par = (a.parity ^ (k - a.k0)) & 1u;
         if (tid < 3) {
-            Fr v = part[0][tid];
+            Fr v = acc;
             for (uint32_t w = 1; w < nw; w++) v = add(v, part[w][tid]);
             // evaluation 2 from the three sums: 6 p1 + 3 p0 - 2 p2raw
             Fr p0, p1;
 #pragma unroll
-            for (int e = 0; e < 8; e++) {
-                p0.l[e] = __shfl_sync(0x7u, v.l[e], 0);
-                p1.l[e] = __shfl_sync(0x7u, v.l[e], 1);
+            for (int l = 0; l < 8; l++) {
+                p0.l[l] = __shfl_sync(0x7u, v.l[l], 0);
+                p1.l[l] = __shfl_sync(0x7u, v.l[l], 1);
             }
             if (tid == 2) {
                 const Fr d = add(p1, p1);
                 v = sub(add(add(add(d, d), d), add(add(p0, p0), p0)), add(v, v));
             }
-            if (!LANE_HG) v = mul(v, xv);
-            st_digits(a.evals_out + ((size_t)tid * a.N + lane) * kDigitWords, from_mont(v), par);
-        } else if (k + 1 == a.n && tid >= 32 && tid < 34) {
-            // rows 0 and 1 of the last folded f table (the layer input when it has no fold)
-            const uint32_t row = tid - 32;
-            const Fr v = k == 0 ? ldf(a.v, row, a.N, lane) : fd.get(row);
-            st_digits(a.rows_out + ((size_t)row * a.N + lane) * kDigitWords, v, a.rows_parity);
+            st_digits(a.evals_out + ((size_t)tid * a.N + lane) * kDigitWords, mul(v, xv), par);
+            // rows 0 and 1 of the last f table are what lanes 0 and 1 hold
+            if (k + 1 == a.n && tid < 2)
+                st_digits(a.rows_out + ((size_t)tid * a.N + lane) * kDigitWords, mine, a.rows_parity);
         }
     }
 }
@@ -1056,6 +1118,10 @@ uint32_t grid1(uint64_t n) {
     if (b > 152ull * 16) b = 152ull * 16;
     return (uint32_t)b;
 }
+
+// CTAs of a kernel that builds eq tables: two an SM at most, since each CTA's build is up to six
+// products a thread (1024 CTAs of a 2^16-row layer spent 22 us of 50 on it).
+uint32_t grid_eq(uint64_t n) { return std::min(grid1(n), 2u * 152u); }
 
 dim3 grid_rows(const GeoBn& g, uint64_t rows, uint32_t ctas) {
     const uint32_t groups = g.N / g.tpr;
@@ -1068,19 +1134,38 @@ dim3 grid_rows(const GeoBn& g, uint64_t rows, uint32_t ctas) {
 
 }  // namespace
 
+// Dynamic shared memory of a kernel that builds eq tables; above 48 KiB the opt-in is set once
+// per device and kernel (30 variables at four points: 140 KiB).
+template <auto Kernel>
+static cudaError_t eq_smem(size_t bytes) {
+    static std::atomic<uint64_t> opted{0};  // one bit per device
+    if (bytes <= 40 * 1024) return cudaSuccess;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (opted.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    if (e == cudaSuccess) opted.fetch_or(bit);
+    return e;
+}
+
 cudaError_t launch_load(const uint32_t* canon, uint32_t* mont, uint64_t n_elems, unsigned int* bad, cudaStream_t s) {
     k_load<<<grid1(n_elems), 256, 0, s>>>(canon, mont, n_elems, bad);
     return cudaGetLastError();
 }
 
 cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const Fr* coef,
-                             const Fr* eqz, const Fr* eqx, const Fr* eqy, unsigned long long* acc,
-                             unsigned int* ticket, uint32_t* out, cudaStream_t s) {
-    const uint32_t grid = grid1(O);
+                             const GateEqBn& eq, unsigned long long* acc, unsigned int* ticket, uint32_t* out,
+                             cudaStream_t s) {
+    const uint32_t grid = grid_eq(O);
+    const uint32_t u = std::max(eq_scratch(eq.z), eq_scratch(eq.x));
+    const size_t smem = sizeof(Fr) * (eq_elems(eq.z) + eq_elems(eq.x) + (mul_gates ? eq_elems(eq.y) : 0) + u);
+    const cudaError_t e = mul_gates ? eq_smem<k_gate_sums<true>>(smem) : eq_smem<k_gate_sums<false>>(smem);
+    if (e != cudaSuccess) return e;
     if (mul_gates)
-        k_gate_sums<true><<<grid, kBlock, 0, s>>>(O, off, gates, coef, eqz, eqx, eqy, acc, ticket, out);
+        k_gate_sums<true><<<grid, kBlock, smem, s>>>(O, off, gates, coef, eq, acc, ticket, out);
     else
-        k_gate_sums<false><<<grid, kBlock, 0, s>>>(O, off, gates, coef, eqz, eqx, eqy, acc, ticket, out);
+        k_gate_sums<false><<<grid, kBlock, smem, s>>>(O, off, gates, coef, eq, acc, ticket, out);
     return cudaGetLastError();
 }
 
@@ -1096,16 +1181,12 @@ cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const
     return cudaGetLastError();
 }
 
-cudaError_t launch_eq(Fr* out, const EqArgsBn& a, cudaStream_t s) {
-    const uint64_t chunks = 1ull << (a.nvars > kEqLowBits ? a.nvars - kEqLowBits : 0);
-    k_eq<<<(uint32_t)(chunks < 152ull * 4 ? chunks : 152ull * 4), 256, 0, s>>>(out, a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_weights(uint64_t I, uint64_t Gm, const Fr* eqc, const uint4* mx_g, const Fr* mx_c,
+cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgsBn& eqc, const uint4* mx_g, const Fr* mx_c,
                            const uint32_t* ax_off, const uint2* ax_g, const Fr* ax_c, Fr* a_out, Fr* w_out,
                            cudaStream_t s) {
-    k_weights<<<grid1(I > Gm ? I : Gm), 256, 0, s>>>(I, Gm, eqc, mx_g, mx_c, ax_off, ax_g, ax_c, a_out, w_out);
+    const size_t smem = sizeof(Fr) * (eq_elems(eqc) + eq_scratch(eqc));
+    if (const cudaError_t e = eq_smem<k_weights>(smem)) return e;
+    k_weights<<<grid_eq(kRowLanes * I > Gm ? kRowLanes * I : Gm), 256, smem, s>>>(I, Gm, eqc, mx_g, mx_c, ax_off, ax_g, ax_c, a_out, w_out);
     return cudaGetLastError();
 }
 
@@ -1153,15 +1234,23 @@ cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const Fr* eqc,
-                           const Fr* eqrx, Fr* s_out, cudaStream_t s) {
-    k_s_build<<<grid1(I), 256, 0, s>>>(I, my_off, my_g, my_c, eqc, eqrx, s_out);
+cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const EqArgsBn& eqc,
+                           const EqArgsBn& eqx, Fr* s_out, cudaStream_t s) {
+    const size_t smem = sizeof(Fr) * (eq_elems(eqc) + eq_elems(eqx) + eq_scratch(eqc) + eq_scratch(eqx));
+    if (const cudaError_t e = eq_smem<k_s_build>(smem)) return e;
+    k_s_build<<<grid_eq(kRowLanes * I), 256, smem, s>>>(I, my_off, my_g, my_c, eqc, eqx, s_out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_wsum(const uint32_t* vals, uint64_t rows, const Fr* eq, const GeoBn& g, uint32_t ctas, RedBn red,
+cudaError_t launch_wsum(const uint32_t* vals, const EqArgsBn& eq, const GeoBn& g, uint32_t ctas, RedBn red,
                         uint32_t* out, cudaStream_t s) {
-    k_wsum<<<grid_rows(g, rows, ctas), 256, 8 * 256 * 4, s>>>(vals, rows, eq, g, red, out);
+    const uint64_t rows = 1ull << eq.nvars, need = (rows + kWsumRows - 1) / kWsumRows;
+    const uint32_t groups = g.N / g.tpr, cap = ctas / groups ? ctas / groups : 1;
+    const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);
+    const size_t tabs = sizeof(Fr) * (eq_elems(eq) + eq_scratch(eq)), scratch = 8 * 256 * 4;
+    const size_t smem = tabs > scratch ? tabs : scratch;
+    if (const cudaError_t e = eq_smem<k_wsum>(smem)) return e;
+    k_wsum<<<grid, 256, smem, s>>>(vals, rows, eq, g, red, out);
     return cudaGetLastError();
 }
 

@@ -42,8 +42,13 @@ struct RedBn {
 struct EqArgsBn {
     uint32_t r1[32][8];
     uint32_t r2[32][8];
-    uint32_t f1[8], f2[8];
+    uint32_t first1[2][8], first2[2][8];  // f (1 - r[0]), f r[0] of each point (f, f if no variables)
     uint32_t nvars, has_r2;
+};
+
+// eq factors of the verifier's gate sums: outputs, first inputs and (mul gates) second inputs.
+struct GateEqBn {
+    EqArgsBn z, x, y;
 };
 
 struct RoundPtrsBn {
@@ -61,14 +66,13 @@ cudaError_t launch_load(const uint32_t* canon, uint32_t* mont, uint64_t n_elems,
 // their Montgomery coefficients; acc (8 x u64) and ticket zero before and after; out receives
 // the canonical total (8 words).
 cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const Fr* coef,
-                             const Fr* eqz, const Fr* eqx, const Fr* eqy, unsigned long long* acc,
-                             unsigned int* ticket, uint32_t* out, cudaStream_t s);
+                             const GateEqBn& eq, unsigned long long* acc, unsigned int* ticket, uint32_t* out,
+                             cudaStream_t s);
 cudaError_t launch_unload(uint32_t* v, uint64_t n_elems, cudaStream_t s);
 cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint32_t* mo_off, const uint4* mo_g,
                             const Fr* mo_c, const uint32_t* ao_off, const uint2* ao_g, const Fr* ao_c, const GeoBn& g,
                             uint32_t ctas, cudaStream_t s);
-cudaError_t launch_eq(Fr* out, const EqArgsBn& a, cudaStream_t s);
-cudaError_t launch_weights(uint64_t I, uint64_t Gm, const Fr* eqc, const uint4* mx_g, const Fr* mx_c,
+cudaError_t launch_weights(uint64_t I, uint64_t Gm, const EqArgsBn& eqc, const uint4* mx_g, const Fr* mx_c,
                            const uint32_t* ax_off, const uint2* ax_g, const Fr* ax_c, Fr* a_out, Fr* w_out,
                            cudaStream_t s);
 // Phase-one hg table and round 0: `claim` (N x 8 words, canonical, device-readable,
@@ -82,8 +86,8 @@ cudaError_t launch_hg_round0(const uint32_t* v, uint64_t I, const uint32_t* mx_o
 // 1 are that claim less those at 0; phase two's round 0 (no fold) sums all three.
 cudaError_t launch_round(bool lane_hg, bool fold, const RoundPtrsBn& p, uint64_t npairs, const uint32_t* vx,
                          const GeoBn& g, uint32_t ctas, RedBn red, uint32_t* evals_out, cudaStream_t s);
-cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const Fr* eqc,
-                           const Fr* eqrx, Fr* s_out, cudaStream_t s);
+cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const EqArgsBn& eqc,
+                           const EqArgsBn& eqx, Fr* s_out, cudaStream_t s);
 // Persistent sumcheck phase: rounds k0 .. n-1 in one launch, one CTA per copy.  The M31
 // PhaseArgs (kernels.cuh) describes the scheme: round k leaves 2^(n-k) rows in A when k is odd
 // and in B when it is even, or in shared memory; k0 = 0 starts from the layer input v, building
@@ -102,7 +106,7 @@ struct PhaseArgsBn {
     const uint32_t* mx_off;        // phase one, k0 = 0
     const uint4* mx_g;
     const Fr *a, *w;
-    const uint32_t* vx;            // phase two: N x 8 words, Montgomery form
+    const uint32_t* vx;            // phase two: N x 8 words, canonical
     uint32_t r_first[8];           // k0 > 0: challenge of round k0 - 1, Montgomery form
     uint32_t k0, n, N;
     uint32_t parity, rows_parity;
@@ -112,7 +116,7 @@ struct PhaseArgsBn {
     unsigned long long wait_ns;
 };
 cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s);
-cudaError_t launch_wsum(const uint32_t* vals, uint64_t rows, const Fr* eq, const GeoBn& g, uint32_t ctas, RedBn red,
+cudaError_t launch_wsum(const uint32_t* vals, const EqArgsBn& eq, const GeoBn& g, uint32_t ctas, RedBn red,
                         uint32_t* out, cudaStream_t s);
 
 }  // namespace bn

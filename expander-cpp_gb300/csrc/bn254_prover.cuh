@@ -21,7 +21,7 @@ struct BnWorkspace {
     uint32_t* vals = nullptr;  // every layer's values (Montgomery), layer 0's input first
     uint32_t* stage = nullptr;  // canonical input rows as uploaded (the hg table's space when proving)
     uint32_t *hg0 = nullptr, *hgA = nullptr, *fA = nullptr, *fB = nullptr;
-    bn::Fr *sb[2] = {}, *eqc = nullptr, *eqrx = nullptr, *a = nullptr, *w = nullptr;
+    bn::Fr *sb[2] = {}, *a = nullptr, *w = nullptr;
     uint32_t *vx = nullptr, *cv = nullptr;
     uint32_t* ev_dev[2] = {};  // device copies of the round evaluations (round k writes ev_dev[k & 1])
     unsigned long long* acc = nullptr;
@@ -37,7 +37,7 @@ struct BnWorkspace {
             return p;
         };
         const uint64_t rowb = (uint64_t)N * 32;
-        const uint64_t maxI = 1ull << C.max_in_vars, maxO = 1ull << C.max_out_vars;
+        const uint64_t maxI = 1ull << C.max_in_vars;
         vals = (uint32_t*)take(C.value_rows() * rowb);
         if (sumcheck) {
             hg0 = (uint32_t*)take(maxI * rowb);
@@ -46,14 +46,12 @@ struct BnWorkspace {
             fB = (uint32_t*)take(std::max<uint64_t>(maxI / 4, 1) * rowb);
             sb[0] = (bn::Fr*)take(maxI * 32);
             sb[1] = (bn::Fr*)take(maxI * 32);
-            eqrx = (bn::Fr*)take(maxI * 32);
             a = (bn::Fr*)take(maxI * 32);
             w = (bn::Fr*)take(std::max<uint64_t>(C.max_mul, 1) * 32);
             stage = hg0;
         } else {
             stage = (uint32_t*)take(C.in_rows(0) * rowb);
         }
-        eqc = (bn::Fr*)take(maxO * 32);
         vx = (uint32_t*)take(rowb);
         cv = (uint32_t*)take(rowb);
         ev_dev[0] = (uint32_t*)take(3 * rowb);
@@ -71,6 +69,26 @@ uint64_t workspace_bytes_bn(const gkrgpu_circuit& C, uint32_t N, bool sumcheck) 
     BnWorkspace w;
     w.plan(nullptr, C, N, sumcheck);
     return w.total;
+}
+
+// f1 eq(r1, z) + f2 eq(r2, z) over nvars bits (r2 null: the first alone), canonical arguments.
+bn::EqArgsBn eq_args_bn(const frh::Fr* r1, const frh::Fr* r2, const frh::Fr& f1, const frh::Fr& f2, uint32_t nvars) {
+    bn::EqArgsBn a;
+    memset(&a, 0, sizeof(a));
+    for (uint32_t t = 0; t < nvars; t++) {
+        frh::store(frh::to_mont(r1[t]), a.r1[t]);
+        if (r2) frh::store(frh::to_mont(r2[t]), a.r2[t]);
+    }
+    auto first = [&](const frh::Fr& f, const frh::Fr* r, uint32_t (*out)[8]) {
+        const frh::Fr fr = nvars ? frh::mul(f, r[0]) : frh::zero();
+        frh::store(frh::to_mont(frh::sub(f, fr)), out[0]);
+        frh::store(frh::to_mont(nvars ? fr : f), out[1]);
+    };
+    first(f1, r1, a.first1);
+    if (r2) first(f2, r2, a.first2);
+    a.nvars = nvars;
+    a.has_r2 = r2 ? 1u : 0u;
+    return a;
 }
 
 struct BnProver {
@@ -283,21 +301,6 @@ struct BnProver {
         if (append_last) t.append(last_canon, rowb());
     }
 
-    void eq_table(bn::Fr* out, const frh::Fr* r1, const frh::Fr* r2, const frh::Fr& f1, const frh::Fr& f2,
-                  uint32_t nvars) {
-        bn::EqArgsBn a;
-        memset(&a, 0, sizeof(a));
-        for (uint32_t t = 0; t < nvars; t++) {
-            frh::store(frh::to_mont(r1[t]), a.r1[t]);
-            if (r2) frh::store(frh::to_mont(r2[t]), a.r2[t]);
-        }
-        frh::store(frh::to_mont(f1), a.f1);
-        frh::store(frh::to_mont(f2), a.f2);
-        a.nvars = nvars;
-        a.has_r2 = r2 ? 1u : 0u;
-        c.launch(K_BN_EQ, 32.0 * (double)(1ull << nvars), [&] { return bn::launch_eq(out, a, c.stream); });
-    }
-
     // Phase one's rounds launched one by one, the persistent part from round kt1 (n: none).
     void phase_one_rounds(Transcript& t, size_t li, uint32_t kt1, const frh::Fr& alpha, const frh::Fr& beta, frh::Fr* rx,
                           uint32_t* vx_c) {
@@ -354,7 +357,8 @@ struct BnProver {
     }
 
     // Phase two's rounds launched one by one, the persistent part from round kt2 (n: none).
-    void phase_two_rounds(Transcript& t, size_t li, uint32_t kt2, frh::Fr* ry, uint32_t* vy_m, uint32_t* vy_c) {
+    void phase_two_rounds(Transcript& t, size_t li, uint32_t kt2, frh::Fr* ry, const uint32_t* vx_c, uint32_t* vy_m,
+                          uint32_t* vy_c) {
         const DevLayer& Ly = C.layers[li];
         const uint32_t n = Ly.nin;
         const uint64_t I = 1ull << n;
@@ -381,7 +385,8 @@ struct BnProver {
                 ph.k0 = k;
                 ph.n = n;
                 ph.s = ws.sb[(k - 1) & 1];
-                ph.vx = ws.vx;
+                memcpy(mapped(false, 32ull * N + 64), vx_c, rowb());
+                ph.vx = mapped(true, 32ull * N + 64);
                 if (run_phase(t, false, ph, ry, false, vy_m, vy_c, rb * 6.0 * (double)(I >> k))) break;
             }
             bn::RoundPtrsBn p;
@@ -414,9 +419,9 @@ struct BnProver {
         std::vector<uint32_t> vx_c((size_t)N * 8), vy_m((size_t)N * 8), vy_c((size_t)N * 8);
 
         // phase one: eqc = alpha eq(rz1) + beta eq(rz2), gate weights, hg + round 0
-        eq_table(ws.eqc, rz1, rz2, alpha, beta, m);
+        const bn::EqArgsBn eqc = eq_args_bn(rz1, rz2, alpha, beta, m);
         c.launch(K_BN_WEIGHTS, 80.0 * Ly.nmul + 72.0 * Ly.nadd + 40.0 * I, [&] {
-            return bn::launch_weights(I, Ly.nmul, ws.eqc, Ly.mx_g, Ly.mx_c, Ly.ax_off, Ly.ax_g, Ly.ax_c, ws.a, ws.w,
+            return bn::launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.mx_c, Ly.ax_off, Ly.ax_g, Ly.ax_c, ws.a, ws.w,
                                       c.stream);
         });
         const uint32_t kt1 = phase_start(n, 2), kt2 = kt1;
@@ -432,17 +437,19 @@ struct BnProver {
 
         // phase two: h(y) = vx * s(y)
         const frh::Fr one = frh::from_u32(1), zero = frh::zero();
-        eq_table(ws.eqrx, rx, nullptr, one, zero, n);
+        const bn::EqArgsBn eqx = eq_args_bn(rx, nullptr, one, zero, n);
         c.launch(K_BN_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 32.0 * I + 96.0 * Ly.nmul, [&] {
-            return bn::launch_s_build(I, Ly.my_off, Ly.my_g, Ly.my_c, ws.eqc, ws.eqrx, ws.sb[0], c.stream);
+            return bn::launch_s_build(I, Ly.my_off, Ly.my_g, Ly.my_c, eqc, eqx, ws.sb[0], c.stream);
         });
         bn::PhaseArgsBn a2 = {};
         a2.n = n;
         a2.v = v;
         a2.s = ws.sb[0];
-        a2.vx = mapped(true, 24ull * N);
+        // the phase multiplies by v(rx) itself (canonical; the claims' place, unused by a phase)
+        memcpy(mapped(false, 32ull * N + 64), vx_c.data(), rowb());
+        a2.vx = mapped(true, 32ull * N + 64);
         if (kt2 != 0 || !run_phase(t, false, a2, ry, false, vy_m.data(), vy_c.data(), rb * 4.0 * I))
-            phase_two_rounds(t, li, kt2, ry, vy_m.data(), vy_c.data());
+            phase_two_rounds(t, li, kt2, ry, vx_c.data(), vy_m.data(), vy_c.data());
         t.append(vy_c.data(), rowb());
         // the next layer's sum is alpha vx + beta vy (gkr.hpp:113-119)
         cv1.swap(vx_c);
@@ -466,11 +473,10 @@ struct BnProver {
         frh::Fr alpha = frh::from_u32(1), beta = frh::zero();
         bool have_rz2 = false;
 
-        eq_table(ws.eqc, rz1, nullptr, alpha, beta, nz);
         const uint64_t OL = C.out_rows(L - 1);
-        c.launch(K_BN_WSUM, 32.0 * N * OL + 32.0 * OL, [&] {
-            return bn::launch_wsum(vals[L], OL, ws.eqc, gk[K_BN_WSUM], ctas[K_BN_WSUM], red(), mapped(true, 16ull * N),
-                                   c.stream);
+        c.launch(K_BN_WSUM, 32.0 * N * OL, [&] {
+            return bn::launch_wsum(vals[L], eq_args_bn(rz1, nullptr, alpha, beta, nz), gk[K_BN_WSUM], ctas[K_BN_WSUM],
+                                   red(), mapped(true, 16ull * N), c.stream);
         });
         c.sync();
         require_canonical();

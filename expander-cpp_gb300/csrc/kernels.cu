@@ -36,7 +36,7 @@ const char* const kKernelNames[K_NUM_KERNELS] = {"check_canonical", "evaluate", 
                                                  "phase2_s_build", "weighted_row_sum", "hg_rebuild_round1",
                                                  "verifier_gate_sums", "canonicalize", "phase2_round0", "stage_words", "round_tail", "hg_build",
                                                  "bn254_load",
-                                                 "bn254_evaluate", "bn254_eq_table", "bn254_gate_weights",
+                                                 "bn254_evaluate", "bn254_gate_weights",
                                                  "bn254_hg_build_round0", "bn254_round_fold_lane",
                                                  "bn254_round_fold_scalar", "bn254_phase2_s_build",
                                                  "bn254_weighted_row_sum", "bn254_unload", "bn254_phase"};

@@ -126,7 +126,6 @@ enum KernelId {
     // BN254 kernels (bn254.cuh)
     K_BN_LOAD,
     K_BN_EVALUATE,
-    K_BN_EQ,
     K_BN_WEIGHTS,
     K_BN_HG_ROUND0,
     K_BN_ROUND_LANE,

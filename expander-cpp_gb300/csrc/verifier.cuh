@@ -233,7 +233,6 @@ struct BnVerifier {
     uint32_t N;
     char* block = nullptr;
     uint32_t *raw = nullptr, *com = nullptr, *sums = nullptr, *cv = nullptr;
-    bn::Fr *eqz = nullptr, *eqx = nullptr, *eqy = nullptr;
     unsigned long long *gacc = nullptr, *wacc = nullptr;
     unsigned int *gticket = nullptr, *wticket = nullptr;
 
@@ -243,11 +242,10 @@ struct BnVerifier {
     }
 
     void reserve() {
-        const uint64_t I0 = C.in_rows(0), maxI = 1ull << C.max_in_vars, maxO = 1ull << C.max_out_vars;
+        const uint64_t I0 = C.in_rows(0);
         std::vector<std::pair<void**, size_t>> parts = {
-            {(void**)&raw, I0 * N * 32}, {(void**)&com, I0 * N * 32},  {(void**)&eqz, maxO * 32},
-            {(void**)&eqx, maxI * 32},   {(void**)&eqy, maxI * 32},    {(void**)&sums, 32},
-            {(void**)&cv, (size_t)N * 32}, {(void**)&gacc, 8 * 8},     {(void**)&gticket, 16},
+            {(void**)&raw, I0 * N * 32},   {(void**)&com, I0 * N * 32}, {(void**)&sums, 32},
+            {(void**)&cv, (size_t)N * 32}, {(void**)&gacc, 8 * 8},      {(void**)&gticket, 16},
             {(void**)&wacc, 3ull * N * 8 * 8}, {(void**)&wticket, 4096},
         };
         size_t o = 0, zero_from = 0;
@@ -267,34 +265,21 @@ struct BnVerifier {
         c.h_cv.ensure((size_t)N * 32 + 64, "pinned verifier results");
     }
 
-    void eq_table(bn::Fr* out, const frh::Fr* r1, const frh::Fr* r2, const frh::Fr& f1, const frh::Fr& f2,
-                  uint32_t nvars) {
-        bn::EqArgsBn a;
-        memset(&a, 0, sizeof(a));
-        for (uint32_t t = 0; t < nvars; t++) {
-            frh::store(frh::to_mont(r1[t]), a.r1[t]);
-            if (r2) frh::store(frh::to_mont(r2[t]), a.r2[t]);
-        }
-        frh::store(frh::to_mont(f1), a.f1);
-        frh::store(frh::to_mont(f2), a.f2);
-        a.nvars = nvars;
-        a.has_r2 = r2 ? 1u : 0u;
-        c.launch(K_BN_EQ, 32.0 * (double)(1ull << nvars), [&] { return bn::launch_eq(out, a, c.stream); });
-    }
-
     frh::Fr gate_sums(size_t li, bool mul_part, const frh::Fr* rz1, const frh::Fr* rz2, const frh::Fr& alpha,
                       const frh::Fr& beta, const frh::Fr* rx, const frh::Fr* ry) {
         const DevLayer& Ly = C.layers[li];
         const uint64_t O = 1ull << Ly.nout;
-        eq_table(eqz, rz1, rz2, alpha, beta, Ly.nout);
-        eq_table(eqx, rx, nullptr, frh::from_u32(1), frh::zero(), Ly.nin);
-        if (mul_part) eq_table(eqy, ry, nullptr, frh::from_u32(1), frh::zero(), Ly.nin);
+        const frh::Fr one = frh::from_u32(1), zero = frh::zero();
+        bn::GateEqBn eq;
+        eq.z = eq_args_bn(rz1, rz2, alpha, beta, Ly.nout);
+        eq.x = eq_args_bn(rx, nullptr, one, zero, Ly.nin);
+        eq.y = mul_part ? eq_args_bn(ry, nullptr, one, zero, Ly.nin) : eq.x;
         const double gates = mul_part ? (double)Ly.nmul : (double)Ly.nadd;
         c.launch(K_GATE_SUMS, (mul_part ? 48.0 : 40.0) * gates + 4.0 * (O + 1) + 32.0 * O, [&] {
             return bn::launch_gate_sums(mul_part, O, mul_part ? Ly.mo_off : Ly.ao_off,
                                         mul_part ? reinterpret_cast<const uint32_t*>(Ly.mo_g)
                                                  : reinterpret_cast<const uint32_t*>(Ly.ao_g),
-                                        mul_part ? Ly.mo_c : Ly.ao_c, eqz, eqx, eqy, gacc, gticket, sums, c.stream);
+                                        mul_part ? Ly.mo_c : Ly.ao_c, eq, gacc, gticket, sums, c.stream);
         });
         c.copy(c.h_cv.p, sums, 32, cudaMemcpyDeviceToHost, "gate sums readback");
         c.sync();
@@ -304,10 +289,10 @@ struct BnVerifier {
     bool raw_pc_verify(const frh::Fr* r, const std::vector<uint32_t>& claims) {
         const uint32_t n0 = C.layers[0].nin;
         const uint64_t rows = 1ull << n0;
-        eq_table(eqx, r, nullptr, frh::from_u32(1), frh::zero(), n0);
+        const bn::EqArgsBn eq = eq_args_bn(r, nullptr, frh::from_u32(1), frh::zero(), n0);
         const bn::GeoBn g = geo_bn(X, N, K_BN_WSUM);
-        c.launch(K_BN_WSUM, 32.0 * N * rows + 32.0 * rows, [&] {
-            return bn::launch_wsum(com, rows, eqx, g, X.cta_budget(K_BN_WSUM), bn::RedBn{wacc, wticket}, cv, c.stream);
+        c.launch(K_BN_WSUM, 32.0 * N * rows, [&] {
+            return bn::launch_wsum(com, eq, g, X.cta_budget(K_BN_WSUM), bn::RedBn{wacc, wticket}, cv, c.stream);
         });
         c.copy(c.h_cv.p, cv, (size_t)N * 32, cudaMemcpyDeviceToHost, "multilinear evaluation readback");
         c.sync();
