@@ -223,7 +223,7 @@ struct BnProver {
     bool run_phase(Transcript& t, bool lane_hg, bn::PhaseArgsBn a, frh::Fr* rch, bool append_last, uint32_t* last_mont,
                    uint32_t* last_canon, double bytes) {
         PhaseSlots slots(X.device, X.sm_count);
-        if (!slots.acquire((int)N)) return false;
+        if (!slots.acquire((int)N, true)) return false;
         a.N = N;
         a.fA = ws.fA;
         a.fB = ws.fB;

@@ -385,7 +385,10 @@ __global__ void __launch_bounds__(256) k_hg_build(const uint32_t* __restrict__ v
                 if (j < reps) {
                     const uint32_t w = STORED ? comp(ws, j) : mul(gt.z, eq_at(t, nd, two, j, gt.y));
 #pragma unroll
-                    for (int l = 0; l < 4; l++) h[j][l] = fold64(h[j][l] + (uint64_t)comp(vy, l) * w);
+                    for (int l = 0; l < 4; l++) {
+                        mad64(h[j][l], comp(vy, l), w);
+                        h[j][l] = fold64(h[j][l]);
+                    }
                 }
         }
         const uint32_t at = (I >= 4 ? (x & 3) * (I >> 2) + (x >> 2) : x) * tpr + quad % tpr;  // place() of phase.cu
@@ -1552,9 +1555,12 @@ __global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __r
 // (include/poly_commit/poly.hpp:88-104).  The table is read once, so the bound is HBM: 2^18
 // rows of 1024 copies at three points take 160 us at the copy peak.  Products are summed
 // unreduced in 64 bits and folded every four rows (as separate field operations the sums took
-// 430 us, bound by instruction issue); a thread reads four consecutive rows at once, and their
-// weights, computed per block of rows from the digit tables, come from shared memory.
-constexpr uint32_t kWsumRows = 256;  // rows a CTA takes at a time, at least
+// 430 us, bound by instruction issue); a thread stages its next steps of four consecutive rows
+// with cp.async, and their weights, computed per block of rows from the digit tables, come from
+// shared memory.  What bounds it is the wide multiply-add, 17 products with their folding per
+// clock and SM: 235 us at three CTAs an SM and four stages, 256 at four and two or three.
+constexpr uint32_t kWsumRows = 256;  // rows of a CTA's weights at a time, at least
+constexpr int kWsumStages = 4;       // steps of four rows a thread has in its cp.async ring
 
 __host__ __device__ inline uint32_t wsum_block(const Geo& g, uint64_t rows, uint32_t ctas) {
     const uint32_t step = 4 * g.rps;
@@ -1565,11 +1571,13 @@ __host__ __device__ inline uint32_t wsum_block(const Geo& g, uint64_t rows, uint
 }
 
 template <int R>
-__global__ void __launch_bounds__(256, 4) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows, uint32_t rb,
+__global__ void __launch_bounds__(256, 3) k_wsum(const uint32_t* __restrict__ vals, uint64_t rows, uint32_t rb,
                                                  const __grid_constant__ EqArgs eq, Geo g, RedScratch red, uint32_t* out) {
-    extern __shared__ uint32_t smem[];  // R x rb weights, then the reduction's scratch
+    extern __shared__ uint4 wring[];  // the ring, then R x rb weights; at the end the reduction's scratch
     __shared__ uint32_t tab[kEqWords];
     const TileIdx t = tile_idx(g);
+    const uint32_t B = blockDim.x, tid = threadIdx.x;
+    uint32_t* const wt = reinterpret_cast<uint32_t*>(wring + kWsumStages * 4 * B);
     eq_build(tab, eq);
     const uint32_t nd = eq_digits(eq);
     uint64_t acc[R][4];
@@ -1577,39 +1585,66 @@ __global__ void __launch_bounds__(256, 4) k_wsum(const uint32_t* __restrict__ va
     for (int c = 0; c < R; c++)
 #pragma unroll
         for (int l = 0; l < 4; l++) acc[c][l] = 0ull;
-    for (uint64_t z0 = (uint64_t)blockIdx.x * rb; z0 < rows; z0 += (uint64_t)gridDim.x * rb) {
-        __syncthreads();  // the digit tables, or the last block's weights, are done with
-        for (uint32_t i = threadIdx.x; i < rb; i += blockDim.x)
-#pragma unroll
-            for (int j = 0; j < R; j++)
-                smem[j * rb + i] = z0 + i < rows ? eq_at(tab, nd, false, j, (uint32_t)(z0 + i)) : 0u;
-        __syncthreads();
-        if (!t.active) continue;
-        for (uint32_t i = 4 * t.rs; i < rb && z0 + i < rows; i += 4 * g.rps) {
-            uint4 v[4];
+    // blocks of rb rows, taken in turn by the CTAs; within one, steps of 4 rps rows
+    const uint64_t stride = (uint64_t)gridDim.x * rb, base = (uint64_t)blockIdx.x * rb;
+    const uint32_t step = 4 * g.rps;
+    // the step staged next: block offset sz, row si of the block (a table of fewer than four
+    // rows repeats its last, weight 0)
+    uint64_t sz = base;
+    uint32_t si = 4 * t.rs;
+    auto stage = [&](int slot) {
+        if (t.active && sz < rows) {
+            uint4* st = wring + slot * 4 * B + tid;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const uint64_t z = z0 + i + k;  // a table of fewer than four rows repeats its last (weight 0)
-                v[k] = ld4(vals, z < rows ? z : rows - 1, g.N, t.lane0);
+                const uint64_t z = sz + si + k < rows ? sz + si + k : rows - 1;
+                cp_async16(st + k * B, vals + z * g.N + t.lane0);
             }
-#pragma unroll
-            for (int j = 0; j < R; j++) {
-                const uint4 w = *reinterpret_cast<const uint4*>(smem + j * rb + i);
-#pragma unroll
-                for (int l = 0; l < 4; l++) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) acc[j][l] += (uint64_t)comp(v[k], l) * comp(w, k);
-                    acc[j][l] = fold64(acc[j][l]);
-                }
+            si += step;
+            if (si >= rb) {
+                si = 4 * t.rs;
+                sz += stride;
             }
         }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int q = 0; q < kWsumStages - 1; q++) stage(q);
+    int slot = 0;
+    for (uint64_t z0 = base; z0 < rows; z0 += stride) {
+        __syncthreads();  // the digit tables, or the last block's weights, are done with
+        for (uint32_t i = tid; i < rb; i += B)
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                wt[j * rb + i] = z0 + i < rows ? eq_at(tab, nd, false, j, (uint32_t)(z0 + i)) : 0u;
+        __syncthreads();
+        for (uint32_t i = 4 * t.rs; i < rb; i += step) {
+            stage(slot == 0 ? kWsumStages - 1 : slot - 1);
+            cp_async_wait<kWsumStages - 1>();
+            if (t.active) {
+                const uint4* st = wring + slot * 4 * B + tid;
+                const uint4 v[4] = {st[0], st[B], st[2 * B], st[3 * B]};
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(wt + j * rb + i);
+#pragma unroll
+                    for (int l = 0; l < 4; l++) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++) mad64(acc[j][l], comp(v[k], l), comp(w, k));
+                        acc[j][l] = fold64(acc[j][l]);
+                    }
+                }
+            }
+            slot = slot + 1 == kWsumStages ? 0 : slot + 1;
+        }
     }
+    cp_async_wait<0>();
     uint32_t sum[R][4];
 #pragma unroll
     for (int c = 0; c < R; c++)
 #pragma unroll
         for (int l = 0; l < 4; l++) sum[c][l] = reduce64(acc[c][l]);
-    __syncthreads();  // the weights' space is the reduction's scratch
+    __syncthreads();  // the ring is the reduction's scratch
     reduce_group<R>(sum, g, t.active, red, 0, CopyFin{red, out, g.N, (uint32_t)R});
 }
 
@@ -2003,12 +2038,13 @@ cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, ui
     const uint32_t groups = lane_groups(g), cap = ctas / groups ? ctas / groups : 1, rb = wsum_block(g, rows, cap);
     const uint64_t need = (rows + rb - 1) / rb;
     const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);
-    const size_t weights = 4 * (size_t)eq.reps * rb, scratch = 4 * (size_t)eq.reps * 4 * block;
-    const size_t smem = weights > scratch ? weights : scratch;
+    if (block > 256 || eq.reps < 1 || eq.reps > 3) return cudaErrorInvalidValue;
+    // (the reduction's scratch, 16 reps bytes a thread, is less than the ring)
+    const size_t smem = (size_t)kWsumStages * 4 * 16 * block + 4 * (size_t)eq.reps * rb;
     switch (eq.reps) {
-        case 1: k_wsum<1><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
-        case 2: k_wsum<2><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
-        case 3: k_wsum<3><<<grid, block, smem, s>>>(vals, rows, rb, eq, g, red, out); break;
+        case 1: k_wsum<1><<<grid, block, ring_smem<k_wsum<1>>(smem), s>>>(vals, rows, rb, eq, g, red, out); break;
+        case 2: k_wsum<2><<<grid, block, ring_smem<k_wsum<2>>(smem), s>>>(vals, rows, rb, eq, g, red, out); break;
+        case 3: k_wsum<3><<<grid, block, ring_smem<k_wsum<3>>(smem), s>>>(vals, rows, rb, eq, g, red, out); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -235,9 +235,7 @@ cudaError_t launch_p2_round1_fin(int reps, const uint32_t* sums, const uint32_t*
 // s_j(4i) + s_j(4i+1), s_j(4i+2) + s_j(4i+3)) (I and s_stride multiples of 4).
 cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const EqArgs& eqc, const EqArgs& eqx,
                            uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, cudaStream_t s);
-// CTAs of a persistent phase for N copies at tpr quads a CTA, the smallest tpr that needs at
-// most max_ctas of them (0: none does), and the launch.
-uint32_t phase_tpr(uint32_t N, uint32_t max_ctas);
+// CTAs of a persistent phase for N copies at tpr quads a CTA, and the launch.
 uint32_t phase_ctas(uint32_t N, uint32_t tpr);
 // Quads a CTA's tables take when the first round reads `items` rows x tpr.
 size_t phase_priv_quads(uint64_t items);

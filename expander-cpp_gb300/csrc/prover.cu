@@ -568,7 +568,7 @@ struct gkrgpu_ctx {
         // the BN254 kernels hold two CTAs an SM by their registers, and each CTA ends in a reduction
         // (5 layers of 2^14..2^16 at 64 copies: 6.84 ms with two, 7.08 with four, 7.32 with eight)
         const bool two = kid > K_BN_EVALUATE && kid < K_NUM_KERNELS;
-        return (uint32_t)sm_count * (kid == K_EVALUATE ? 16u : two ? 2u : 4u);
+        return (uint32_t)sm_count * (kid == K_EVALUATE ? 16u : two ? 2u : kid == K_WSUM ? 3u : 4u);
     }
 
     // Blocks until `bytes` fit in the budget (a proof larger than the whole budget runs alone).
@@ -835,13 +835,17 @@ void validate_layers(const gkrgpu_layer_desc* layers, int n, int field) {
     }
 }
 
+// CTAs of a persistent phase at most.  (1024 copies: 256 CTAs of one quad, whose 16-byte results
+// are partial lines for the host to gather, took 52.6 ms for the 2^18 / 2^20 proof, 128 of two
+// 51.5.)
+constexpr uint32_t kPhaseCtas = 128;
+
 // ------------------------------------------------------------------ per-proof device workspace
 // All device tables of one proof, carved from one pool block (256-byte aligned parts).
 struct Workspace {
     uint32_t* vals = nullptr;  // every layer's values (the input's rows excluded when it is on the device)
     uint32_t *hg0[3] = {}, *hgA[3] = {}, *fA[3] = {}, *fB[3] = {};
     uint4* priv = nullptr;  // the CTAs' tables of the phases that run in one launch
-    size_t priv_stride = 0;
     uint32_t* sb[2] = {};
     uint32_t *evals = nullptr, *vx = nullptr, *cv = nullptr;
     uint32_t* p2s = nullptr;  // 9R x N sums of phase-two rounds 0 and 1 (launch_p2_round01)
@@ -853,8 +857,8 @@ struct Workspace {
     size_t sstride = 0;
     size_t total = 0;
 
-    // Lays the parts out from `base` (null: only sizes the block); tpr as Prover::tpr_phase.
-    void plan(char* base, const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck, uint32_t tpr) {
+    // Lays the parts out from `base` (null: only sizes the block).
+    void plan(char* base, const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck) {
         size_t o = 0;
         auto take = [&](size_t bytes) -> char* {
             char* p = base ? base + o : nullptr;
@@ -872,10 +876,12 @@ struct Workspace {
                 fA[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 2, 1) * rowb);
                 fB[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 4, 1) * rowb);
             }
-            if (tpr) {
-                priv_stride = phase_priv_quads(std::min<uint64_t>(maxI * tpr, kPhaseItems));
-                priv = (uint4*)take(phase_ctas(N, tpr) * priv_stride * 16);
-            }
+            // the row tile of a phase is chosen when it starts: room for any
+            size_t quads = 0;
+            for (uint32_t tpr = 1; tpr <= 32; tpr *= 2)
+                if (phase_ctas(N, tpr) <= kPhaseCtas)
+                    quads = std::max(quads, phase_ctas(N, tpr) * phase_priv_quads(std::min<uint64_t>(maxI * tpr, kPhaseItems)));
+            priv = (uint4*)take(quads * 16);
             sstride = align_up(maxI, 64);
             sb[0] = (uint32_t*)take(R * sstride * 4);
             sb[1] = (uint32_t*)take(R * sstride * 4);
@@ -896,19 +902,10 @@ struct Workspace {
     }
 };
 
-uint64_t workspace_bytes(const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck, uint32_t tpr) {
+uint64_t workspace_bytes(const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck) {
     Workspace w;
-    w.plan(nullptr, C, N, R, own_input, sumcheck, tpr);
+    w.plan(nullptr, C, N, R, own_input, sumcheck);
     return w.total;
-}
-
-// Quads of copies per CTA of a proof's persistent phases (0: they are off): as few as the
-// lane's share of the resident CTAs allows, at most 128 CTAs.  (1024 copies: 256 CTAs of one
-// quad, whose 16-byte results are partial lines for the host to gather, took 52.6 ms for the
-// 2^18 / 2^20 proof, 128 of two 51.5.)
-uint32_t tpr_phase(const gkrgpu_ctx& X, uint32_t N) {
-    if (!X.round_tail) return 0;
-    return phase_tpr(N, std::min(128u, std::max(1u, 2u * (uint32_t)X.sm_count / (uint32_t)X.n_lanes)));
 }
 
 // f1 eq(r1_j, z) + f2 eq(r2_j, z) over nvars bits (r2 null: the first alone).
@@ -936,8 +933,9 @@ class PhaseSlots {
    public:
     PhaseSlots(int device, int sm_count) : used_(counter(device)), cap_(2 * sm_count) {}
     ~PhaseSlots() { used_ -= held_; }
-    bool acquire(int n) {
-        if (used_.fetch_add(n) + n > cap_) {
+    // n more CTAs; beyond a lane's own share of the device only while half of it stays free.
+    bool acquire(int n, bool own_share) {
+        if (used_.fetch_add(n) + n > (own_share ? cap_ : cap_ / 2)) {
             used_ -= n;
             return false;
         }
@@ -961,7 +959,6 @@ struct Prover {
     const gkrgpu_circuit& C;
     uint32_t N;
     int R;
-    uint32_t tpr;  // of the persistent phases
     Geo gk[K_NUM_KERNELS];
     uint32_t ck_ctas[K_NUM_KERNELS];
     Workspace ws;
@@ -972,7 +969,7 @@ struct Prover {
     std::vector<uint32_t> cv1, cv2;
 
     Prover(gkrgpu_ctx& ctx, Lane& lane, const gkrgpu_circuit& circ, uint32_t n, int reps)
-        : X(ctx), c(lane), C(circ), N(n), R(reps), tpr(tpr_phase(ctx, n)) {
+        : X(ctx), c(lane), C(circ), N(n), R(reps) {
         for (int k = 0; k < K_NUM_KERNELS; k++) {
             gk[k] = ctx.geo(n, k);
             ck_ctas[k] = ctx.cta_budget(k);
@@ -983,30 +980,38 @@ struct Prover {
         if (block) cudaFreeAsync(block, c.stream);
     }
 
-    // First round of a phase's persistent part, n if it has none: 0 when the layer input itself
-    // is small, else the first round from `first` on whose source tables are.  Measured with 16
-    // copies and 2^10 rows: 9.5-14 us a round launched alone, 4-5 us within a phase.
-    uint32_t phase_start(uint32_t n, uint32_t first) const {
-        if (!tpr) return n;
-        if ((uint64_t)tpr << n <= kPhaseItems) return 0;
-        uint32_t lg = 0;
-        while (((2ull << lg) * tpr) <= kPhaseTailItems) lg++;  // at most 2^lg rows
-        return std::min(n, std::max(first, n + 1 - lg));
+    // Quads of copies per CTA for a phase whose first round reads `rows` rows, its CTAs taken from
+    // `slots`; 0: it does not run in one launch (off, too many rows, or no room on the device
+    // now).  As few as there is room for, since a round has the more SMs then: a proof alone on
+    // the device, or among small ones, takes more than its lane's share.
+    uint32_t claim(PhaseSlots& slots, uint64_t rows, uint64_t items) const {
+        if (!X.round_tail) return 0;
+        const uint32_t share = std::max(1u, 2u * (uint32_t)X.sm_count / (uint32_t)X.n_lanes);
+        for (uint32_t tpr = 1; tpr <= 32 && rows * tpr <= items; tpr *= 2) {
+            const uint32_t ctas = phase_ctas(N, tpr);
+            if (ctas <= kPhaseCtas && slots.acquire((int)ctas, ctas <= share)) return tpr;
+        }
+        return 0;
     }
     // Rounds a.k0 .. a.n-1 of a phase in one k_phase launch: after each round's evaluations the
     // host appends them, derives the challenges and writes them to the mailbox, from which
     // the kernel's next round reads them.  The last round's rows 0..1 come with its
-    // evaluations (vx / vy as in transcript_round).  `prepare` launches what the phase reads.
-    // Returns false (and does nothing) while other phases hold the device.
+    // evaluations (vx / vy as in transcript_round).  `prepare(stride)` launches what the phase
+    // reads.  Returns the row tile, 0 (having done nothing) when it cannot run now; `tile` asks
+    // for that one.
     template <class Prepare>
-    bool run_phase(Transcript& t, bool lane_hg, PhaseArgs a, uint32_t (*rch)[32], bool append_last, uint32_t* last_out,
-                   double bytes, Prepare&& prepare) {
+    uint32_t run_phase(Transcript& t, bool lane_hg, PhaseArgs a, uint32_t (*rch)[32], bool append_last, uint32_t* last_out,
+                       double bytes, uint32_t tile, Prepare&& prepare) {
         PhaseSlots slots(X.device, X.sm_count);
-        if (!slots.acquire((int)phase_ctas(N, tpr))) return false;
-        prepare();
-        a.tpr = tpr;
+        const uint64_t rows = 1ull << (a.n - (a.k0 ? a.k0 - 1 : 0));
+        if (tile)
+            a.tpr = slots.acquire((int)phase_ctas(N, tile), true) ? tile : 0;
+        else
+            a.tpr = claim(slots, rows, a.k0 ? kPhaseTailItems : kPhaseItems);
+        if (!a.tpr) return 0;
         a.priv = ws.priv;
-        a.priv_stride = ws.priv_stride;
+        a.priv_stride = phase_priv_quads(rows * a.tpr);
+        prepare(a.tpr, a.priv_stride);
         for (int j = 0; j < R; j++) {
             a.fsrc[j] = (a.k0 & 1) ? ws.fB[j] : ws.fA[j];
             a.hsrc[j] = (a.k0 & 1) ? ws.hg0[j] : ws.hgA[j];
@@ -1058,7 +1063,7 @@ struct Prover {
         }
         abort.mb = nullptr;
         c.phase_err = nullptr;
-        return true;
+        return a.tpr;
     }
 
     RedScratch red() const { return RedScratch{ws.acc, ws.ticket}; }
@@ -1096,11 +1101,11 @@ struct Prover {
     uint32_t groups(int kid) const { return lane_groups(gk[kid]); }
 
     void reserve(bool own_input, bool sumcheck) {
-        ws.plan(nullptr, C, N, R, own_input, sumcheck, tpr);
+        ws.plan(nullptr, C, N, R, own_input, sumcheck);
         void* p = nullptr;
         ck(cudaMallocFromPoolAsync(&p, ws.total, X.pool, c.stream), "workspace allocation");
         block = static_cast<char*>(p);
-        ws.plan(block, C, N, R, own_input, sumcheck, tpr);
+        ws.plan(block, C, N, R, own_input, sumcheck);
         ck(cudaMemsetAsync(block + ws.zero_off, 0, ws.zero_bytes, c.stream), "cudaMemsetAsync");
         c.ensure_mapped(9ull * N * 4, mapped_words() * 4);
         c.resync_done();
@@ -1188,8 +1193,8 @@ struct Prover {
         }
     }
 
-    // Phase one's rounds launched one by one, the persistent part from round kt1 (n: none).
-    void phase_one_rounds(Transcript& t, size_t li, uint32_t kt1, uint32_t alpha, uint32_t beta, uint32_t (*rx)[32]) {
+    // Phase one's rounds launched one by one, the last ones in one launch when they can be.
+    void phase_one_rounds(Transcript& t, size_t li, uint32_t alpha, uint32_t beta, uint32_t (*rx)[32]) {
         const DevLayer& Ly = C.layers[li];
         const uint32_t n = Ly.nin;
         const uint64_t I = 1ull << n, RN = (uint64_t)R * N;
@@ -1220,14 +1225,16 @@ struct Prover {
         const uint32_t* cur_f[3] = {v, v, v};
         const uint32_t* cur_h[3] = {nullptr, nullptr, nullptr};  // round 1 rebuilds hg
         for (uint32_t k = 1; k < n; k++) {
-            if (k == kt1) {
+            // from round 4 on (rounds 2 and 3 refold the input and recompute copy-independent hg
+            // rows) the rest runs in one launch once its tables are small
+            if (k >= 4 && I >> (k - 1) <= kPhaseTailItems) {
                 double bytes = 0;
-                for (uint32_t kk = kt1; kk < n; kk++) bytes += rb * 3.0 * R * 4.0 * (double)(I >> (kk + 1));
+                for (uint32_t kk = k; kk < n; kk++) bytes += rb * 3.0 * R * 4.0 * (double)(I >> (kk + 1));
                 c.tag = ((uint32_t)li << 16) | (1u << 8) | k;
                 PhaseArgs a = {};
                 a.k0 = k;
                 a.n = n;
-                if (run_phase(t, true, a, rx, true, vxh, bytes, [] {})) break;
+                if (run_phase(t, true, a, rx, true, vxh, bytes, 0, [](uint32_t, size_t) {})) break;
             }
             RoundPtrs p;
             memset(&p, 0, sizeof(p));
@@ -1305,10 +1312,10 @@ struct Prover {
         }
     }
 
-    // Phase two's rounds launched one by one, the persistent part from round kt2 (n: none).
+    // Phase two's rounds launched one by one, the last ones in one launch when they can be.
     // With at least three rounds, rounds 0 and 1 come from one pass over the layer input
     // (fused01: their sums are quadratic in round 0's challenge) and round 2 refolds the input.
-    void phase_two_rounds(Transcript& t, size_t li, uint32_t kt2, bool fused01, uint32_t (*ry)[32], uint32_t* vy) {
+    void phase_two_rounds(Transcript& t, size_t li, bool fused01, uint32_t (*ry)[32], uint32_t* vy) {
         const DevLayer& Ly = C.layers[li];
         const uint32_t n = Ly.nin;
         const uint64_t I = 1ull << n;
@@ -1361,9 +1368,9 @@ struct Prover {
         // round 2 refolds the layer input
         const bool refold = n >= 3;
         for (uint32_t k = k_first; k < n; k++) {
-            if (k == kt2) {
+            if (k >= 3 && I >> (k - 1) <= kPhaseTailItems) {
                 double bytes = 0;
-                for (uint32_t kk = kt2; kk < n; kk++) {
+                for (uint32_t kk = k; kk < n; kk++) {
                     const double S = 4.0 * (double)(I >> (kk + 1));
                     bytes += rb * (R * S + R * S / 2) + 6.0 * R * S;
                 }
@@ -1373,7 +1380,7 @@ struct Prover {
                 a.n = n;
                 a.vx = ws.vx;
                 for (int j = 0; j < R; j++) a.s[j] = ws.sb[(k - 1) & 1] + j * sstride;
-                if (run_phase(t, false, a, ry, false, vy, bytes, [] {})) break;
+                if (run_phase(t, false, a, ry, false, vy, bytes, 0, [](uint32_t, size_t) {})) break;
             }
             RoundPtrs p;
             memset(&p, 0, sizeof(p));
@@ -1431,10 +1438,7 @@ struct Prover {
         // phase one: gate weights for eqc_j = alpha eq(rz1_j) + beta eq(rz2_j)
         c.tag = ((uint32_t)li << 16) | (1u << 8);
         const EqArgs eqc = eq_args(R, rz1, rz2, alpha, beta, m);
-        // the rounds on small tables run in one persistent launch: every round of a small layer,
-        // otherwise from round 4 on (rounds 2 and 3 refold the input and recompute
-        // copy-independent hg rows)
-        const uint32_t kt1 = phase_start(n, 4);
+        // a small layer's phases run whole in one launch each
         PhaseArgs a1 = {};
         a1.n = n;
         auto weights = [&] {
@@ -1442,26 +1446,24 @@ struct Prover {
                 return launch_weights(I, Ly.nmul, eqc, Ly.mx_g, Ly.ax_off, Ly.ax_g, ws.a4, ws.w4, c.stream);
             });
         };
-        const bool whole = kt1 == 0 && run_phase(t, true, a1, rx, true, vxh, rb * 9.0 * R * I, [&] {
+        const uint32_t whole = run_phase(t, true, a1, rx, true, vxh, rb * 9.0 * R * I, 0, [&](uint32_t tpr, size_t stride) {
             const bool stored = hg_build_stored(Ly.nmul + Ly.nadd, N);
             if (stored) weights();
             c.launch(K_HG_BUILD, rb * (I + Ly.nmul + (double)(1 + R) * I) + 16.0 * Ly.nmul + 8.0 * Ly.nadd, [&] {
                 return launch_hg_build(v, (uint32_t)I, N, tpr, eqc, Ly.mx_off, Ly.mx_g, Ly.ax_off, Ly.ax_g,
-                                       stored ? ws.a4 : nullptr, ws.w4, ws.priv, ws.priv_stride, c.stream);
+                                       stored ? ws.a4 : nullptr, ws.w4, ws.priv, stride, c.stream);
             });
         });
         if (!whole) {
             weights();
-            phase_one_rounds(t, li, std::max(kt1, std::min(n, 4u)), alpha, beta, rx);
+            phase_one_rounds(t, li, alpha, beta, rx);
         }
 
         // phase two: h(y) = vx * s(y)
         c.tag = ((uint32_t)li << 16) | (2u << 8);
         const EqArgs eqx = eq_args(R, rx, nullptr, 1u, 0u, n);
         const size_t sstride = ws.sstride;
-        // phase two whole in one launch reads the layer input where phase one's left it
-        const uint32_t kt2 = whole ? 0 : std::max(phase_start(n, 3), std::min(n, 3u));
-        const bool fused01 = kt2 != 0 && n >= 3 && p2_round01_groups(N) > 0;
+        const bool fused01 = !whole && n >= 3 && p2_round01_groups(N) > 0;
         c.launch(K_S_BUILD, 16.0 * Ly.nmul + 4.0 * I + 4.0 * R * I * (fused01 ? 2 : 1), [&] {
             return launch_s_build(I, Ly.my_off, Ly.my_g, eqc, eqx, ws.sb[0], fused01 ? ws.sb[1] : nullptr, sstride,
                                   c.stream);
@@ -1470,8 +1472,10 @@ struct Prover {
         a2.n = n;
         a2.vx = mapped(true, 9ull * N);
         for (int j = 0; j < R; j++) a2.s[j] = ws.sb[0] + j * sstride;
-        if (kt2 != 0 || !run_phase(t, false, a2, ry, false, vy.data(), rb * I * (1.0 + 3.0 * R) + 8.0 * R * I, [] {}))
-            phase_two_rounds(t, li, kt2, fused01, ry, vy.data());
+        // (phase two whole in one launch reads the layer input where phase one's left it)
+        if (!whole || !run_phase(t, false, a2, ry, false, vy.data(), rb * I * (1.0 + 3.0 * R) + 8.0 * R * I, whole,
+                                 [](uint32_t, size_t) {}))
+            phase_two_rounds(t, li, fused01, ry, vy.data());
         for (int j = 0; j < R; j++) t.append(vy.data() + (size_t)j * N, rowb);
         // the next layer's sum is alpha vx + beta vy (gkr.hpp:113-119)
         cv1.assign(vxh, vxh + RN);
@@ -1712,8 +1716,7 @@ void gpu_worker(gkrgpu_ctx* c, Lane* lane) {
         std::string err;
         const bool bn = j->circuit->field == GKRGPU_FIELD_BN254;
         const uint64_t need = bn ? workspace_bytes_bn(*j->circuit, j->N, true)
-                                 : workspace_bytes(*j->circuit, j->N, j->R, j->d_input == nullptr, true,
-                                                 tpr_phase(*c, j->N));
+                                 : workspace_bytes(*j->circuit, j->N, j->R, j->d_input == nullptr, true);
         c->acquire_hbm(need);
         if (j->marker >= 0) {
             // the device stage begins: this lane's stream has finished its previous proof
@@ -1985,12 +1988,7 @@ int gkrgpu_memory_stats(gkrgpu_ctx* ctx, uint64_t* in_use, uint64_t* peak, uint6
 uint64_t gkrgpu_workspace_bytes(const gkrgpu_circuit* circuit, uint32_t n_copies, int grinding_bits, int input_on_device) {
     if (!circuit) return 0;
     if (circuit->field == GKRGPU_FIELD_BN254) return workspace_bytes_bn(*circuit, n_copies, true);
-    // the largest over the row tiles of the persistent phases, which depend on the lanes
-    uint64_t most = 0;
-    for (uint32_t tpr = 0; tpr <= 32; tpr = tpr ? 2 * tpr : 1)
-        if (tpr == 0 || phase_ctas(n_copies, tpr) <= 128)
-            most = std::max(most, workspace_bytes(*circuit, n_copies, reps_for(grinding_bits), input_on_device == 0, true, tpr));
-    return most;
+    return workspace_bytes(*circuit, n_copies, reps_for(grinding_bits), input_on_device == 0, true);
 }
 
 int gkrgpu_circuit_load(gkrgpu_ctx* ctx, const gkrgpu_layer_desc* layers, int n_layers, gkrgpu_circuit** out) {
