@@ -228,28 +228,55 @@ __global__ void k_canonicalize(uint32_t* v, uint64_t n) {
 
 // ---------------------------------------------------------------- layer evaluation
 // out[o] = sum over mul gates (o, i0, i1, c) of in[i0]*in[i1]*c + sum over add gates
-// (o, i0, c) of in[i0]*c, gates grouped by o (CSR), so every output row is written once.
+// (o, i0, c) of in[i0]*c, gates grouped by o, so every output row is written once.  Bound by the
+// chain of dependent loads to an output's rows (L2 for most): an output of one mul gate or two
+// add gates, nearly all, has its gates in one record, loaded an output ahead, and both its rows
+// are in flight together; by the CSR lists alone the chain was offsets, gate, row, next gate.
 __global__ void __launch_bounds__(256) k_evaluate(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t O,
-                                                  const uint32_t* __restrict__ mo_off, const uint4* __restrict__ mo_g,
-                                                  const uint32_t* __restrict__ ao_off, const uint2* __restrict__ ao_g,
-                                                  Geo g) {
+                                                  const uint4* __restrict__ ev, const uint32_t* __restrict__ mo_off,
+                                                  const uint4* __restrict__ mo_g, const uint32_t* __restrict__ ao_off,
+                                                  const uint2* __restrict__ ao_g, Geo g) {
     const TileIdx t = tile_idx(g);
     if (!t.active) return;
-    for (uint64_t o = (uint64_t)blockIdx.x * g.rps + t.rs; o < O; o += (uint64_t)gridDim.x * g.rps) {
+    const uint64_t step = (uint64_t)gridDim.x * g.rps;
+    uint64_t o = (uint64_t)blockIdx.x * g.rps + t.rs;
+    uint4 next = o < O ? __ldg(ev + o) : make_uint4(0u, 0u, 0u, 0u);
+    for (; o < O; o += step) {
+        const uint4 e = next;
+        if (o + step < O) next = __ldg(ev + o + step);
+        const uint32_t kind = e.x >> 30;
         uint32_t acc[4] = {0u, 0u, 0u, 0u};
-        const uint32_t m0 = __ldg(mo_off + o), m1 = __ldg(mo_off + o + 1);
-        for (uint32_t k = m0; k < m1; k++) {
-            const uint4 gt = __ldg(mo_g + k);
-            const uint4 a = ld4(in, gt.x, g.N, t.lane0), b = ld4(in, gt.y, g.N, t.lane0);
+        if (kind == kEvMul || kind == kEvAdd) {
+            const uint4 a = ld4(in, e.x & 0x3fffffffu, g.N, t.lane0), b = ld4(in, e.y, g.N, t.lane0);
+            if (kind == kEvMul) {
 #pragma unroll
-            for (int l = 0; l < 4; l++) acc[l] = add(acc[l], mul(mul(comp(a, l), comp(b, l)), gt.z));
-        }
-        const uint32_t a0 = __ldg(ao_off + o), a1 = __ldg(ao_off + o + 1);
-        for (uint32_t k = a0; k < a1; k++) {
-            const uint2 gt = __ldg(ao_g + k);
-            const uint4 a = ld4(in, gt.x, g.N, t.lane0);
+                for (int l = 0; l < 4; l++) acc[l] = mul(comp(a, l), comp(b, l));
+                if (e.z != 1u)
 #pragma unroll
-            for (int l = 0; l < 4; l++) acc[l] = add(acc[l], mul(comp(a, l), gt.y));
+                    for (int l = 0; l < 4; l++) acc[l] = mul(acc[l], e.z);
+            } else {
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    uint64_t s = (uint64_t)comp(a, l) * e.z;
+                    mad64(s, comp(b, l), e.w);
+                    acc[l] = reduce64(s);
+                }
+            }
+        } else if (kind == kEvList) {
+            const uint32_t m0 = __ldg(mo_off + o), m1 = __ldg(mo_off + o + 1);
+            for (uint32_t k = m0; k < m1; k++) {
+                const uint4 gt = __ldg(mo_g + k);
+                const uint4 a = ld4(in, gt.x, g.N, t.lane0), b = ld4(in, gt.y, g.N, t.lane0);
+#pragma unroll
+                for (int l = 0; l < 4; l++) acc[l] = add(acc[l], mul(mul(comp(a, l), comp(b, l)), gt.z));
+            }
+            const uint32_t a0 = __ldg(ao_off + o), a1 = __ldg(ao_off + o + 1);
+            for (uint32_t k = a0; k < a1; k++) {
+                const uint2 gt = __ldg(ao_g + k);
+                const uint4 a = ld4(in, gt.x, g.N, t.lane0);
+#pragma unroll
+                for (int l = 0; l < 4; l++) acc[l] = add(acc[l], mul(comp(a, l), gt.y));
+            }
         }
         st4(out, o, g.N, t.lane0, mk4(acc));
     }
@@ -1694,11 +1721,11 @@ cudaError_t launch_check_canonical(const uint32_t* v, uint64_t n, unsigned int* 
     return cudaGetLastError();
 }
 
-cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint32_t* mo_off, const uint4* mo_g,
-                            const uint32_t* ao_off, const uint2* ao_g, const Geo& g, uint32_t block, uint32_t ctas,
-                            cudaStream_t s) {
+cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint4* ev, const uint32_t* mo_off,
+                            const uint4* mo_g, const uint32_t* ao_off, const uint2* ao_g, const Geo& g, uint32_t block,
+                            uint32_t ctas, cudaStream_t s) {
     LaunchShape sh = row_shape(g, O, block, ctas, 0);
-    k_evaluate<<<sh.grid, sh.block, 0, s>>>(in, out, O, mo_off, mo_g, ao_off, ao_g, g);
+    k_evaluate<<<sh.grid, sh.block, 0, s>>>(in, out, O, ev, mo_off, mo_g, ao_off, ao_g, g);
     return cudaGetLastError();
 }
 

@@ -151,9 +151,13 @@ cudaError_t launch_canonicalize(uint32_t* v, uint64_t n, cudaStream_t s);
 // the canonical totals.
 cudaError_t launch_gate_sums(bool mul_gates, uint64_t O, const uint32_t* off, const uint32_t* gates, const GateEq& eq,
                              unsigned long long* acc, unsigned int* ticket, uint32_t* out, cudaStream_t s);
-cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint32_t* mo_off, const uint4* mo_g,
-                            const uint32_t* ao_off, const uint2* ao_g, const Geo& g, uint32_t block, uint32_t ctas,
-                            cudaStream_t s);
+// Records of launch_evaluate: an output's gates in 16 bytes, the kind in the top two bits of the
+// first word: none (0), one mul gate (i0, i1, c, 0), one or two add gates (i0, i1, c0, c1; a
+// single one with c1 = 0 and i1 = i0), or more (by the CSR lists).  Ids are below 2^30.
+constexpr uint32_t kEvMul = 1, kEvAdd = 2, kEvList = 3;
+cudaError_t launch_evaluate(const uint32_t* in, uint32_t* out, uint64_t O, const uint4* ev, const uint32_t* mo_off,
+                            const uint4* mo_g, const uint32_t* ao_off, const uint2* ao_g, const Geo& g, uint32_t block,
+                            uint32_t ctas, cudaStream_t s);
 // dst[k * n + i] = srcs[k][i] (nsrc <= 3 tables of n words) by a small kernel instead of the
 // copy engine, for transfers between device and host-mapped memory; with `done`, every CTA
 // increments it after its writes are visible to the host.  Returns the CTA count (the

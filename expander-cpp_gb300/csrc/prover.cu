@@ -160,6 +160,7 @@ struct DevLayer {
     uint4* mo_g = nullptr;       // (i0, i1, c, 0)
     uint32_t* ao_off = nullptr;  // O+1
     uint2* ao_g = nullptr;       // (i0, c)
+    const uint4* ev = nullptr;   // M31: each output's gates in one record (launch_evaluate)
     // phase one: gates grouped by x = i0
     uint32_t* mx_off = nullptr;  // I+1
     uint4* mx_g = nullptr;       // (y, z, c, 0)
@@ -737,6 +738,22 @@ DevLayer upload_layer(const gkrgpu_layer_desc& d, int field) {
         if (bn) ax_c[k] = ca[ord[k]];
     }
 
+    // evaluate's records: one mul gate, or at most two add gates, or none; other outputs go by the
+    // lists
+    std::vector<uint4> ev(bn ? 0 : O);
+    for (uint64_t o = 0; o < ev.size(); o++) {
+        const uint32_t m0 = off_mo[o], a0 = off_ao[o], nm = off_mo[o + 1] - m0, na = off_ao[o + 1] - a0;
+        if (nm == 1 && na == 0) {
+            ev[o] = make_uint4(mo[m0].x | kEvMul << 30, mo[m0].y, mo[m0].z, 0);
+        } else if (nm == 0 && na <= 2) {
+            ev[o] = make_uint4(0, 0, 0, 0);
+            if (na > 0) ev[o] = make_uint4(ao[a0].x | kEvAdd << 30, ao[a0].x, ao[a0].y, 0);
+            if (na > 1) ev[o].y = ao[a0 + 1].x, ev[o].w = ao[a0 + 1].y;
+        } else {
+            ev[o] = make_uint4(kEvList << 30, 0, 0, 0);
+        }
+    }
+
     // groups with gates (see DevLayer); a list is kept only when it leaves out more than a
     // tenth of the groups, since walking it costs a dependent load per group
     std::vector<uint32_t> l_p1_pairs, l_p1_quads, l_p2_quads;
@@ -775,6 +792,7 @@ DevLayer upload_layer(const gkrgpu_layer_desc& d, int field) {
         {off_ax.data(), off_ax.size() * 4, (void**)&L.ax_off}, {ax.data(), Ga * 8, (void**)&L.ax_g},
         {off_my.data(), off_my.size() * 4, (void**)&L.my_off}, {my.data(), Gm * 16, (void**)&L.my_g},
     };
+    if (!bn) parts.push_back({ev.data(), ev.size() * 16, (void**)&L.ev});
     if (!bn && use_p1p) parts.push_back({l_p1_pairs.data(), l_p1_pairs.size() * 4, (void**)&L.p1_pairs});
     if (!bn && use_p1q) parts.push_back({l_p1_quads.data(), l_p1_quads.size() * 4, (void**)&L.p1_quads});
     if (!bn && use_p2q) parts.push_back({l_p2_quads.data(), l_p2_quads.size() * 4, (void**)&L.p2_quads});
@@ -1148,7 +1166,7 @@ struct Prover {
             const double b = 4.0 * N * (2.0 * Ly.nmul + Ly.nadd + O) + 16.0 * Ly.nmul + 8.0 * Ly.nadd + 8.0 * (O + 1);
             c.tag = (uint32_t)l << 16;
             c.launch(K_EVALUATE, b, [&] {
-                return launch_evaluate(vals[l], vals[l + 1], O, Ly.mo_off, Ly.mo_g, Ly.ao_off, Ly.ao_g,
+                return launch_evaluate(vals[l], vals[l + 1], O, Ly.ev, Ly.mo_off, Ly.mo_g, Ly.ao_off, Ly.ao_g,
                                        gk[K_EVALUATE], X.block, ck_ctas[K_EVALUATE], c.stream);
             });
         }
