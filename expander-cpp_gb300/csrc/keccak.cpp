@@ -1,6 +1,6 @@
 // Keccak-f[1600] and the Keccak-256 / SHA3-256 sponges (keccak.hpp), written from the
 // permutation's definition (theta, rho, pi, chi, iota on a 5 x 5 array of 64-bit lanes).
-// The round constants and rotation offsets are derived at start-up from their definitions
+// The round constants and rotation offsets are derived at compile time from their definitions
 // (the degree-8 LFSR x^8 + x^6 + x^5 + x^4 + 1 and the triangular offsets along the pi walk)
 // rather than tabulated.
 #include "keccak.hpp"
@@ -12,56 +12,53 @@ namespace {
 
 struct Tables {
     uint64_t rc[24];
-    unsigned rot[5][5];  // rot[x][y]
-    Tables() {
-        // rc(t): output bit of the LFSR after t steps
-        auto rc_bit = [](unsigned t) -> uint64_t {
-            unsigned r = 1;
-            for (unsigned i = 0; i < t % 255; i++) {
-                r <<= 1;
-                if (r & 0x100) r ^= 0x171;
-            }
-            return r & 1;
-        };
-        for (unsigned i = 0; i < 24; i++) {
-            rc[i] = 0;
-            for (unsigned j = 0; j < 7; j++) rc[i] |= rc_bit(j + 7 * i) << ((1u << j) - 1);
-        }
-        memset(rot, 0, sizeof(rot));
-        unsigned x = 1, y = 0;
-        for (unsigned t = 0; t < 24; t++) {
-            rot[x][y] = ((t + 1) * (t + 2) / 2) % 64;
-            const unsigned nx = y, ny = (2 * x + 3 * y) % 5;
-            x = nx;
-            y = ny;
-        }
-    }
+    unsigned rot[25];  // rot[x + 5 y]
 };
-
-const Tables& tables() {
-    static const Tables t;
+constexpr Tables make_tables() {
+    Tables t{};
+    // bit j + 7 i of the LFSR's output is bit 2^j - 1 of round i's constant
+    unsigned r = 1;
+    for (unsigned i = 0; i < 24; i++)
+        for (unsigned j = 0; j < 7; j++) {
+            t.rc[i] |= (uint64_t)(r & 1) << ((1u << j) - 1);
+            r <<= 1;
+            if (r & 0x100) r ^= 0x171;
+        }
+    unsigned x = 1, y = 0;
+    for (unsigned k = 0; k < 24; k++) {
+        t.rot[x + 5 * y] = ((k + 1) * (k + 2) / 2) % 64;
+        const unsigned nx = y, ny = (2 * x + 3 * y) % 5;
+        x = nx;
+        y = ny;
+    }
     return t;
 }
+constexpr Tables kT = make_tables();
 
 inline uint64_t rotl(uint64_t v, unsigned n) { return n ? (v << n) | (v >> (64 - n)) : v; }
 
-// a[x + 5 y]
+// a[x + 5 y].  Every loop over the lanes is unrolled, so that the rotations have constant
+// amounts and the lanes stay in registers.
 void keccak_f(uint64_t a[25]) {
-    const Tables& T = tables();
+    uint64_t s[25];
+    memcpy(s, a, sizeof(s));
     for (int round = 0; round < 24; round++) {
         uint64_t c[5], b[25];
-        for (int x = 0; x < 5; x++) c[x] = a[x] ^ a[x + 5] ^ a[x + 10] ^ a[x + 15] ^ a[x + 20];
+#pragma GCC unroll 5
+        for (int x = 0; x < 5; x++) c[x] = s[x] ^ s[x + 5] ^ s[x + 10] ^ s[x + 15] ^ s[x + 20];
+#pragma GCC unroll 5
         for (int x = 0; x < 5; x++) {
             const uint64_t d = c[(x + 4) % 5] ^ rotl(c[(x + 1) % 5], 1);
-            for (int y = 0; y < 5; y++) a[x + 5 * y] ^= d;
+#pragma GCC unroll 5
+            for (int y = 0; y < 5; y++) b[y + 5 * ((2 * x + 3 * y) % 5)] = rotl(s[x + 5 * y] ^ d, kT.rot[x + 5 * y]);
         }
-        for (int x = 0; x < 5; x++)
-            for (int y = 0; y < 5; y++) b[y + 5 * ((2 * x + 3 * y) % 5)] = rotl(a[x + 5 * y], T.rot[x][y]);
-        for (int x = 0; x < 5; x++)
-            for (int y = 0; y < 5; y++)
-                a[x + 5 * y] = b[x + 5 * y] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
-        a[0] ^= T.rc[round];
+#pragma GCC unroll 5
+        for (int y = 0; y < 5; y++)
+#pragma GCC unroll 5
+            for (int x = 0; x < 5; x++) s[x + 5 * y] = b[x + 5 * y] ^ (~b[(x + 1) % 5 + 5 * y] & b[(x + 2) % 5 + 5 * y]);
+        s[0] ^= kT.rc[round];
     }
+    memcpy(a, s, sizeof(s));
 }
 
 void sponge256(const uint8_t* in, size_t len, uint8_t domain, uint8_t out[32]) {
@@ -70,8 +67,8 @@ void sponge256(const uint8_t* in, size_t len, uint8_t domain, uint8_t out[32]) {
     memset(a, 0, sizeof(a));
     auto absorb = [&](const uint8_t* blk) {
         for (size_t i = 0; i < rate / 8; i++) {
-            uint64_t w = 0;
-            for (int k = 7; k >= 0; k--) w = (w << 8) | blk[8 * i + k];
+            uint64_t w;
+            memcpy(&w, blk + 8 * i, 8);  // (both hosts are little-endian)
             a[i] ^= w;
         }
         keccak_f(a);
@@ -87,8 +84,7 @@ void sponge256(const uint8_t* in, size_t len, uint8_t domain, uint8_t out[32]) {
     last[len] ^= domain;
     last[rate - 1] ^= 0x80;
     absorb(last);
-    for (int i = 0; i < 4; i++)
-        for (int k = 0; k < 8; k++) out[8 * i + k] = (uint8_t)(a[i] >> (8 * k));
+    memcpy(out, a, 32);
 }
 
 }  // namespace
