@@ -1082,6 +1082,191 @@ __global__ void __launch_bounds__(256, 2) k_p1_round2(RoundPtrs p, uint64_t npai
                         ClaimFin{red, evals_out, nullptr, {p.r[0], p.r[1], p.r[2]}, g.N, (uint32_t)R});
 }
 
+// Rounds k and k + 1 from one pass over the tables: output rows 4i .. 4i+3 (the tables as round
+// k has them) are folded from the source at the D challenges since it was stored, stored
+// themselves, and summed into what both rounds need.  A round's sums are quadratic in the
+// challenge before it: with E over rows 4i, 4i+1 and U over the sums of rows 4i, 4i+2 and
+// 4i+1, 4i+3, round k + 1's p0 and p2raw at r are (1-r)^2 X00 + r (1-r) (XQ - X00 - X11) +
+// r^2 X11 for X = E and U (k_pair_fin), so round k + 1 reads no table.
+// What bounds it: memory, and that is what the pair saves.  From stored tables of T bytes two
+// single rounds move T + T/2 + T/2 + T/4, a pair at D = 1 T + T/2, each pair after it (D = 2)
+// T + T/4 where single rounds move 9/4 T.
+// One repetition a thread as in k_round: 32 sums and an output row's loads in flight; two CTAs
+// an SM is the registers' bound.  2^20 rows of 1024 copies: rounds 3 and 4 in phase one 1430 us
+// (5.5 TB/s; the add weights' rows are computed), 5 and 6 596 us (6.8 TB/s), rounds 3 to 8 of
+// four such layers 2.1 ms less than one by one.
+// HR = 2: round 3 in phase one, source hg rows as in k_round<.., HR = 2>.
+constexpr int kPairSums = 8;  // E00, E11, EQ, F00 (rows 4i+2, 4i+3), FQ, U00, U11, UQ
+
+// Round k's evaluations from the pair's sums, which stay canonical in `sums` for round k + 1.
+struct PairFin {
+    RedScratch red;
+    uint32_t* out;       // R x 3 x N
+    uint32_t* sums;      // kPairSums R x N
+    uint32_t r[3];       // challenges of round k - 1
+    uint32_t N, reps;
+    const uint32_t* vx;  // R x N, or null
+    __device__ void operator()(uint32_t lane) const {
+        uint32_t* dev = red.evals_dev;
+        for (uint32_t j = 0; j < reps; j++) {
+            uint32_t m[kPairSums];
+#pragma unroll
+            for (int e = 0; e < kPairSums; e++) {
+                m[e] = take(red, kPairSums * j + e, N, lane);
+                sums[(size_t)(kPairSums * j + e) * N + lane] = m[e];
+            }
+            const uint32_t rj = j == 0 ? r[0] : (j == 1 ? r[1] : r[2]);
+            uint32_t* d = dev + (size_t)(3 * j) * N + lane;
+            const uint32_t cl = m31::eval_degree2(d[0], d[N], d[2 * (size_t)N], rj);
+            uint32_t p0 = add(m[0], m[3]), p2raw = add(m[2], m[4]);
+            if (vx) {
+                const uint32_t x = vx[(size_t)j * N + lane];
+                p0 = mul(p0, x);
+                p2raw = mul(p2raw, x);
+            }
+            const uint32_t p1 = sub(cl, p0), p2 = m31::eval_at_two(p0, p1, p2raw);
+            uint32_t* o = out + (size_t)(3 * j) * N + lane;
+            o[0] = d[0] = p0;
+            o[N] = d[N] = p1;
+            o[2 * (size_t)N] = d[2 * (size_t)N] = p2;
+        }
+    }
+};
+
+template <bool LANE_HG, int D, int HR>
+__global__ void __launch_bounds__(256, 2) k_round_pair(RoundPtrs p, uint64_t ngroups, const uint32_t* __restrict__ vx,
+                                                       Geo g, uint32_t reps, RedScratch red, uint32_t* evals_out,
+                                                       uint32_t* sums_out) {
+    const TileIdx t = tile_idx(g);
+    const uint32_t j = blockIdx.x % reps, cx = blockIdx.x / reps, nx = gridDim.x / reps;
+    const uint32_t* __restrict__ fs = j == 0 ? p.fsrc[0] : (j == 1 ? p.fsrc[1] : p.fsrc[2]);
+    const uint32_t* __restrict__ hs = j == 0 ? p.hsrc[0] : (j == 1 ? p.hsrc[1] : p.hsrc[2]);
+    uint32_t* __restrict__ fd = j == 0 ? p.fdst[0] : (j == 1 ? p.fdst[1] : p.fdst[2]);
+    uint32_t* __restrict__ hd = j == 0 ? p.hdst[0] : (j == 1 ? p.hdst[1] : p.hdst[2]);
+    const m31::Lerp c = j == 0 ? p.c[0] : (j == 1 ? p.c[1] : p.c[2]);
+    const m31::Lerp2 c01 = j == 0 ? p.c01[0] : (j == 1 ? p.c01[1] : p.c01[2]);
+    constexpr int S = 1 << D;  // source rows of an output row
+    uint32_t acc[kPairSums][4] = {};
+    auto mac = [&](int e, int l, uint32_t f, uint32_t h) { acc[e][l] = m31::mac_lazy(acc[e][l], f, h); };
+    auto folded = [&](const uint4 (&x)[S], uint32_t (&o)[4]) {
+#pragma unroll
+        for (int l = 0; l < 4; l++)
+            o[l] = D == 2 ? m31::lerp2(comp(x[0], l), comp(x[1], l), comp(x[2 % S], l), comp(x[3 % S], l), c01)
+                          : m31::lerp(comp(x[0], l), comp(x[1], l), c);
+    };
+    if (t.active) {
+        for (uint64_t i = (uint64_t)cx * g.rps + t.rs; i < ngroups; i += (uint64_t)nx * g.rps) {
+            uint32_t hsc[4];
+            if (!LANE_HG) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    if (D == 2) {
+                        const uint4 x = __ldg(reinterpret_cast<const uint4*>(hs) + 4 * i + e);
+                        hsc[e] = m31::lerp2(x.x, x.y, x.z, x.w, c01);
+                    } else {
+                        const uint2 x = __ldg(reinterpret_cast<const uint2*>(hs) + 4 * i + e);
+                        hsc[e] = m31::lerp(x.x, x.y, c);
+                    }
+                }
+                if (t.q == 0 && blockIdx.y == 0)
+                    reinterpret_cast<uint4*>(hd)[i] = make_uint4(hsc[0], hsc[1], hsc[2], hsc[3]);
+            }
+            uint32_t f[4][4], h[4][4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint64_t row = 4 * i + e;
+                uint4 x[S];
+#pragma unroll
+                for (int k = 0; k < S; k++) x[k] = ld4(fs, S * row + k, g.N, t.lane0);
+                if (LANE_HG) {
+                    uint4 y[S];
+#pragma unroll
+                    for (int k = 0; k < S; k++) {
+                        const uint64_t src = S * row + k;
+                        bool stored = true;
+                        if (HR == 2) stored = __ldg(p.hoff + 4 * src) != __ldg(p.hoff + 4 * src + 4);
+                        if (stored) {
+                            y[k] = ld4(hs, src, g.N, t.lane0);
+                        } else {
+                            const uint32_t* a = reinterpret_cast<const uint32_t*>(p.ha + 4 * src) + j;
+                            const uint32_t hv = m31::lerp2(__ldg(a), __ldg(a + 4), __ldg(a + 8), __ldg(a + 12), c01);
+                            y[k] = make_uint4(hv, hv, hv, hv);
+                        }
+                    }
+                    folded(y, h[e]);
+                    st4(hd, row, g.N, t.lane0, mk4(h[e]));
+                } else {
+#pragma unroll
+                    for (int l = 0; l < 4; l++) h[e][l] = hsc[e];
+                }
+                folded(x, f[e]);
+                st4(fd, row, g.N, t.lane0, mk4(f[e]));
+#pragma unroll
+                for (int l = 0; l < 4; l++) {
+                    if (e < 3) mac(e == 2 ? 3 : e, l, f[e][l], h[e][l]);
+                    if (e & 1) mac(e == 1 ? 2 : 4, l, add(f[e - 1][l], f[e][l]), add(h[e - 1][l], h[e][l]));
+                }
+            }
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                const uint32_t f0 = add(f[0][l], f[2][l]), f1 = add(f[1][l], f[3][l]);
+                const uint32_t h0 = add(h[0][l], h[2][l]), h1 = add(h[1][l], h[3][l]);
+                mac(5, l, f0, h0);
+                mac(6, l, f1, h1);
+                mac(7, l, add(f0, f1), add(h0, h1));
+            }
+        }
+    }
+    reduce_group<kPairSums>(acc, g, t.active, red, kPairSums * j,
+                            PairFin{red, evals_out, sums_out, {p.r[0], p.r[1], p.r[2]}, g.N, reps,
+                                    LANE_HG ? nullptr : vx});
+}
+
+// Round k + 1 of a pair at round k's challenges p.r from the sums of k_round_pair, a thread a
+// copy and repetition.  With rows (4 or 8, of the tables that the pair stored) it also folds
+// them at p.r, for the last round or for its rows 0..1: there are only these few then.
+template <bool LANE_HG>
+__global__ void __launch_bounds__(256) k_pair_fin(RoundPtrs p, const uint32_t* __restrict__ sums,
+                                                  const uint32_t* __restrict__ vx, uint32_t rows, uint32_t N,
+                                                  uint32_t reps, uint32_t* evals_out, uint32_t* evals_dev,
+                                                  unsigned int* done) {
+    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < reps * N) {
+        const uint32_t j = idx / N, lane = idx - j * N;
+        const uint32_t r = j == 0 ? p.r[0] : (j == 1 ? p.r[1] : p.r[2]), omr = sub(1u, r);
+        const uint32_t c0 = mul(omr, omr), c1 = mul(r, omr), c2 = mul(r, r);
+        uint32_t m[kPairSums];
+#pragma unroll
+        for (int e = 0; e < kPairSums; e++) m[e] = __ldg(sums + (size_t)(kPairSums * j + e) * N + lane);
+        uint32_t p0 = add(add(mul(c0, m[0]), mul(c1, sub(sub(m[2], m[0]), m[1]))), mul(c2, m[1]));
+        uint32_t p2raw = add(add(mul(c0, m[5]), mul(c1, sub(sub(m[7], m[5]), m[6]))), mul(c2, m[6]));
+        if (!LANE_HG) {
+            const uint32_t x = __ldg(vx + idx);
+            p0 = mul(p0, x);
+            p2raw = mul(p2raw, x);
+        }
+        uint32_t *d = evals_dev + (size_t)(3 * j) * N + lane, *o = evals_out + (size_t)(3 * j) * N + lane;
+        const uint32_t p1 = sub(m31::eval_degree2(d[0], d[N], d[2 * (size_t)N], r), p0);
+        o[0] = d[0] = p0;
+        o[N] = d[N] = p1;
+        o[2 * (size_t)N] = d[2 * (size_t)N] = m31::eval_at_two(p0, p1, p2raw);
+        const m31::Lerp c = m31::lerp_at(r);
+        const uint32_t* fs = j == 0 ? p.fsrc[0] : (j == 1 ? p.fsrc[1] : p.fsrc[2]);
+        const uint32_t* hs = j == 0 ? p.hsrc[0] : (j == 1 ? p.hsrc[1] : p.hsrc[2]);
+        uint32_t* fd = j == 0 ? p.fdst[0] : (j == 1 ? p.fdst[1] : p.fdst[2]);
+        uint32_t* hd = j == 0 ? p.hdst[0] : (j == 1 ? p.hdst[1] : p.hdst[2]);
+        for (uint32_t i = 0; i < rows / 2; i++) {
+            const size_t s0 = (size_t)(2 * i) * N + lane, to = (size_t)i * N + lane;
+            fd[to] = m31::lerp(fs[s0], fs[s0 + N], c);
+            if (LANE_HG) hd[to] = m31::lerp(hs[s0], hs[s0 + N], c);
+            else if (lane == 0) hd[i] = m31::lerp(hs[2 * i], hs[2 * i + 1], c);
+        }
+    }
+    __threadfence_system();
+    __syncthreads();
+    if (done && threadIdx.x == 0) atomicAdd_system(done, 1u);
+}
+
 // Shared-source rounds (phase-1 round 1, phase-2 rounds 0 and 1) with every repetition in
 // one thread: the layer input rows are read once for all R repetitions instead of once per
 // repetition-CTA.  Same semantics as k_round<true, LANE_HG, FOLD>.
@@ -1690,8 +1875,9 @@ uint32_t grid_1d(uint64_t n, uint32_t block) {
 }
 
 // Row tile with repetition-split CTAs: gridDim.x = reps x row chunks.
-LaunchShape rep_shape(const Geo& g, uint64_t rows, uint32_t block, uint32_t ctas_cap, uint32_t reps) {
-    LaunchShape s = row_shape(g, rows, block, ctas_cap / reps, 2);
+LaunchShape rep_shape(const Geo& g, uint64_t rows, uint32_t block, uint32_t ctas_cap, uint32_t reps,
+                      uint32_t smem_components = 2) {
+    LaunchShape s = row_shape(g, rows, block, ctas_cap / reps, smem_components);
     s.grid.x *= reps;
     return s;
 }
@@ -1949,6 +2135,39 @@ cudaError_t launch_round_hr(int round, int reps, const RoundPtrs& p, uint64_t np
         k_round<false, true, true, 1><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, nullptr, g, reps, red, evals_out);
     else
         k_round<false, true, true, 2><<<sh.grid, sh.block, sh.smem, s>>>(q, npairs, nullptr, g, reps, red, evals_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_round_pair(int reps, bool lane_hg, int depth, const RoundPtrs& p, uint64_t ngroups,
+                              const uint32_t* vx, const Geo& g, uint32_t block, uint32_t ctas, RedScratch red,
+                              uint32_t* evals_out, uint32_t* sums_out, cudaStream_t s) {
+    if (reps < 1 || reps > 3 || block > 256 || !red.evals_dev || !sums_out || ngroups < 1 || (!lane_hg && !vx) ||
+        (lane_hg && depth == 1 && (!p.hoff || !p.ha)))
+        return cudaErrorInvalidValue;
+    const RoundPtrs q = with_weights(p, reps, lane_hg || depth == 2, depth == 1);
+    const LaunchShape sh = rep_shape(g, ngroups, block, ctas, reps, kPairSums);
+#define GKR_PAIR(LH, D, HR) \
+    k_round_pair<LH, D, HR><<<sh.grid, sh.block, sh.smem, s>>>(q, ngroups, vx, g, reps, red, evals_out, sums_out)
+    if (depth == 1 && lane_hg) GKR_PAIR(true, 1, 2);
+    else if (depth == 1) GKR_PAIR(false, 1, 0);
+    else if (depth == 2 && lane_hg) GKR_PAIR(true, 2, 0);
+    else if (depth == 2) GKR_PAIR(false, 2, 0);
+    else return cudaErrorInvalidValue;
+#undef GKR_PAIR
+    return cudaGetLastError();
+}
+
+uint32_t pair_fin_ctas(int reps, uint32_t N) { return (uint32_t)(((uint64_t)reps * N + 255) / 256); }
+
+cudaError_t launch_pair_fin(int reps, bool lane_hg, const RoundPtrs& p, const uint32_t* sums, const uint32_t* vx,
+                            uint32_t rows, uint32_t N, uint32_t* evals_out, uint32_t* evals_dev, unsigned int* done,
+                            cudaStream_t s) {
+    if (reps < 1 || reps > 3 || !evals_dev || (!lane_hg && !vx)) return cudaErrorInvalidValue;
+    const uint32_t ctas = pair_fin_ctas(reps, N);
+    if (lane_hg)
+        k_pair_fin<true><<<ctas, 256, 0, s>>>(p, sums, vx, rows, N, (uint32_t)reps, evals_out, evals_dev, done);
+    else
+        k_pair_fin<false><<<ctas, 256, 0, s>>>(p, sums, vx, rows, N, (uint32_t)reps, evals_out, evals_dev, done);
     return cudaGetLastError();
 }
 

@@ -72,7 +72,8 @@ struct RoundPtrs {
 // The tables are the CTAs' own (priv, priv_stride quads of copies each).  With k0 = 0 they hold
 // the layer input (2^n rows) and, in phase one, hg (launch_hg_build); phase two takes the
 // scalar tables s.  With k0 > 0 the first round folds the caller's tables of round k0 - 1
-// (fsrc, hsrc or s; 2^(n-k0+1) rows of N copies) at r_first.
+// (fsrc, hsrc or s; 2^(n-k0+1) rows of N copies) at r_first; after a pair of rounds (two) they
+// are those of round k0 - 2, folded at r_before and then r_first.
 // The challenges of round k come from the host through the mailbox (host-mapped words
 // [4k .. 4k+2] = r_j(k) with bit 31 set, [4k+3] abort; cleared by the host before the launch).
 // Each wait is bounded by wait_ns: when it expires the kernel sets *err and returns; a
@@ -92,6 +93,8 @@ struct PhaseArgs {
     const uint32_t* s[3];     // phase two: scalar tables the first round reads
     const uint32_t* vx;       // phase two: R x N claims the sums are multiplied by
     uint32_t r_first[3];      // k0 > 0: challenges of round k0 - 1
+    uint32_t r_before[3];     // two: challenges of round k0 - 2
+    uint32_t two;
     uint32_t k0, n, reps, N, tpr;
     uint32_t parity, rows_parity;
     const uint32_t* mbox;
@@ -212,6 +215,19 @@ cudaError_t launch_p1_round2(int reps, const RoundPtrs& p, uint64_t npairs, cons
 // (round 1 stored only its scalar tables) and at p.r; outputs p.fdst / p.hdst as k_round.
 cudaError_t launch_p2_round2(int reps, const RoundPtrs& p, uint64_t npairs, const uint32_t* vx, const Geo& g,
                              uint32_t block, uint32_t ctas, RedScratch red, uint32_t* evals_out, cudaStream_t s);
+// Rounds k and k + 1 in one pass: 4 ngroups output rows (p.fdst, p.hdst) folded from the source
+// at p.r (depth 1: round 3, in phase one with hg rows as launch_round_hr(3, ..)) or at p.hr[0]
+// and then p.r (depth 2).  Round k's evaluations are published, and 8 reps canonical sums per
+// copy go to sums_out for launch_pair_fin, which publishes round k + 1's at round k's challenges
+// p.r (pair_fin_ctas completion counts) and, with rows > 0, folds those rows of p.fsrc / p.hsrc
+// at p.r into p.fdst / p.hdst.  red.acc needs 8 reps x N accumulators; red.evals_dev as above.
+cudaError_t launch_round_pair(int reps, bool lane_hg, int depth, const RoundPtrs& p, uint64_t ngroups,
+                              const uint32_t* vx, const Geo& g, uint32_t block, uint32_t ctas, RedScratch red,
+                              uint32_t* evals_out, uint32_t* sums_out, cudaStream_t s);
+uint32_t pair_fin_ctas(int reps, uint32_t N);
+cudaError_t launch_pair_fin(int reps, bool lane_hg, const RoundPtrs& p, const uint32_t* sums, const uint32_t* vx,
+                            uint32_t rows, uint32_t N, uint32_t* evals_out, uint32_t* evals_dev, unsigned int* done,
+                            cudaStream_t s);
 cudaError_t launch_round(int reps, bool shared_src, bool lane_hg, bool fold, const RoundPtrs& p, uint64_t npairs,
                          const uint32_t* vx, const Geo& g, uint32_t block, uint32_t ctas, RedScratch red,
                          uint32_t* evals_out, cudaStream_t s);

@@ -59,6 +59,12 @@ __device__ __forceinline__ uint32_t reduce64(uint64_t x) {
 __device__ __forceinline__ uint4 lerp4(const uint4& a, const uint4& b, const m31::Lerp& c) {
     return make_uint4(m31::lerp(a.x, b.x, c), m31::lerp(a.y, b.y, c), m31::lerp(a.z, b.z, c), m31::lerp(a.w, b.w, c));
 }
+// Rows x[0], x[re], x[2 re], x[3 re] folded twice.
+__device__ __forceinline__ uint4 lerp4(const uint4* x, size_t re, const m31::Lerp2& c) {
+    const uint4 a = x[0], b = x[re], d = x[2 * re], e = x[3 * re];
+    return make_uint4(m31::lerp2(a.x, b.x, d.x, e.x, c), m31::lerp2(a.y, b.y, d.y, e.y, c),
+                      m31::lerp2(a.z, b.z, d.z, e.z, c), m31::lerp2(a.w, b.w, d.w, e.w, c));
+}
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -110,7 +116,9 @@ __device__ __forceinline__ int wait_challenge(const uint32_t* box, uint32_t R, u
     }
 }
 
-template <bool LANE_HG>
+// TWO: the first round folds the caller's tables twice (its own instance: the copies of that
+// round's body in one cost the rounds of every phase spilled registers).
+template <bool LANE_HG, bool TWO>
 __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
     extern __shared__ uint4 psm[];
     __shared__ uint32_t rch[3];
@@ -246,11 +254,40 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
                     if (LANE_HG) hs = (k == 1 ? mine + (1 + j) * I * tpr : table(k - 1, 1)) + q;
                 }
                 // row 4i + e: at 4i + e of the caller's tables, at e rows / 4 + i of the CTA's
-                const size_t step = given ? N / 4 : tpr, ri = given ? 4 * step : step;
+                const size_t step = given ? N / 4 : tpr, ri = given ? (TWO ? 8 : 4) * step : step;
                 const size_t re = given ? step : (size_t)npairs * step;
                 uint4* fd = table(k, 0) + q;
                 uint4* hd = LANE_HG ? table(k, 1) + q : nullptr;
-                for (uint32_t i = slot; i < npairs; i += nslots) {
+                if (TWO && given) {
+                    const m31::Lerp2 c01 =
+                        m31::lerp2_at(j == 0 ? a.r_before[0] : j == 1 ? a.r_before[1] : a.r_before[2], rch[j]);
+                    for (uint32_t i = slot; i < npairs; i += nslots) {
+                        const uint4* x = fs + i * ri;
+                        const uint32_t o0 = place(out_rows, 2 * i) * tpr, o1 = place(out_rows, 2 * i + 1) * tpr;
+                        uint4 h0, h1;
+                        if (LANE_HG) {
+                            const uint4* y = hs + i * ri;
+                            h0 = lerp4(y, re, c01);
+                            h1 = lerp4(y + 4 * re, re, c01);
+                            hd[o0] = h0;
+                            hd[o1] = h1;
+                        } else {
+                            const uint4 sa = reinterpret_cast<const uint4*>(ssrc)[2 * i];
+                            const uint4 sb = reinterpret_cast<const uint4*>(ssrc)[2 * i + 1];
+                            const uint32_t s0 = m31::lerp2(sa.x, sa.y, sa.z, sa.w, c01);
+                            const uint32_t s1 = m31::lerp2(sb.x, sb.y, sb.z, sb.w, c01);
+                            if (q == 0) reinterpret_cast<uint2*>(sdst)[i] = make_uint2(s0, s1);
+                            h0 = make_uint4(s0, s0, s0, s0);
+                            h1 = make_uint4(s1, s1, s1, s1);
+                        }
+                        const uint4 f0 = lerp4(x, re, c01), f1 = lerp4(x + 4 * re, re, c01);
+                        fd[o0] = f0;
+                        fd[o1] = f1;
+                        accum(acc, f0, f1, h0, h1);
+                        tidy();
+                    }
+                }
+                for (uint32_t i = TWO && given ? npairs : slot; i < npairs; i += nslots) {
                     const uint4* x = fs + i * ri;
                     const uint4 x0 = x[0], x1 = x[re], x2 = x[2 * re], x3 = x[3 * re];
                     const uint32_t o0 = place(out_rows, 2 * i) * tpr, o1 = place(out_rows, 2 * i + 1) * tpr;
@@ -342,6 +379,7 @@ cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
     // rows of the first round's source tables; with k0 = 0 the layer input itself
     const uint64_t rows = 1ull << (a.n - (a.k0 ? a.k0 - 1 : 0));
     if (rows * a.tpr > kPhaseItems || !a.priv || a.priv_stride < phase_priv_quads(rows * a.tpr)) return cudaErrorInvalidValue;
+    if (a.two && a.k0 < 2) return cudaErrorInvalidValue;
     if (a.k0 && (!a.fsrc[0] || (lane_hg && !a.hsrc[0]))) return cudaErrorInvalidValue;
     if (!lane_hg && (!a.vx || !a.s[0])) return cudaErrorInvalidValue;
     static std::atomic<uint64_t> opted{0};  // one bit per device: shared memory above 48 KiB
@@ -349,18 +387,17 @@ cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
     if (!(opted.load(std::memory_order_relaxed) & bit)) {
-        cudaFuncSetAttribute(k_phase<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-        cudaFuncSetAttribute(k_phase<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+        for (auto* k : {k_phase<true, false>, k_phase<true, true>, k_phase<false, false>, k_phase<false, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
         opted.fetch_or(bit);
     }
     const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
     const size_t smem = 2 * (lane_hg ? 6 : 3) * (size_t)kSmemRows * 16 + (lane_hg ? 0 : 4 * 3 * (size_t)(S1 + S1 / 2)) +
                         4 * (size_t)a.reps * kWarps * 3 * 4 * a.tpr;
     const dim3 grid(phase_ctas(a.N, a.tpr)), block(a.reps * kRepThreads);
-    if (lane_hg)
-        k_phase<true><<<grid, block, smem, s>>>(a);
-    else
-        k_phase<false><<<grid, block, smem, s>>>(a);
+    auto* const kernel = lane_hg ? (a.two ? k_phase<true, true> : k_phase<true, false>)
+                                 : (a.two ? k_phase<false, true> : k_phase<false, false>);
+    kernel<<<grid, block, smem, s>>>(a);
     return cudaGetLastError();
 }
 

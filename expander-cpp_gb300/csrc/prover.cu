@@ -1011,6 +1011,49 @@ struct Prover {
         }
         return 0;
     }
+    // Whether round k and those after it are taken in pairs (k_round_pair), from round 3 on, before
+    // which the layer input is refolded: on tables well beyond the L2 cache, and with rounds enough
+    // ahead of those a phase takes over, since a pair's second launch costs what a single round
+    // does on a small table.  Phase one's rounds from 3 on at 2^16 rows of 1024 copies (2^24 words
+    // a source table) take 473 us one by one and 481 in pairs, at 2^17 rows 698 and 648, at 2^18
+    // rows 1097 and 973, at 2^13 rows of 20000 copies 3240 and 3340.
+    bool pairs_from(uint32_t n, uint32_t k) const {
+        return k == 3 && 1ull << (n - k) > kPhaseTailItems && (uint64_t)N << (n - k + 1) >= 1ull << 25;
+    }
+    // Rounds k and k + 1 of a phase: p has the source and destination tables, `deep` whether the
+    // source is two rounds back.  When at most one round is left, the stored tables are folded at
+    // round k's challenges as well, into f2 and h2.  Returns whether the next round's source is
+    // two rounds back.
+    bool run_pair(Transcript& t, bool lane_hg, int kid, RoundPtrs p, bool deep, uint32_t k, uint32_t n, uint32_t* const* f2,
+                  uint32_t* const* h2, uint32_t (*rch)[32], uint32_t* last_out, double bytes) {
+        const uint32_t left = n - (k + 2);
+        const uint64_t rows = 1ull << (n - k);
+        const uint32_t* vx = lane_hg ? nullptr : ws.vx;
+        c.launch(kid, bytes, [&] {
+            // (half of a fold round's CTAs: two of this kernel's are resident on an SM)
+            return launch_round_pair(R, lane_hg, deep ? 2 : 1, p, rows / 4, vx, gk[kid], X.block, ck_ctas[kid] / 2,
+                                     red_mapped(), c.evals_d(), ws.p2s, c.stream);
+        });
+        fetch(groups(kid), nullptr, false);
+        transcript_round(t, rch, k, false, lane_hg, last_out);
+        c.tag = (c.tag & ~0xffu) | (k + 1);
+        RoundPtrs q;
+        memset(&q, 0, sizeof(q));
+        for (int j = 0; j < R; j++) {
+            q.fsrc[j] = p.fdst[j];
+            q.hsrc[j] = p.hdst[j];
+            q.fdst[j] = f2[j];
+            q.hdst[j] = h2[j];
+            q.r[j] = rch[j][k];
+        }
+        c.launch(kid, 4.0 * 14 * R * N, [&] {
+            return launch_pair_fin(R, lane_hg, q, ws.p2s, vx, left <= 1 ? (uint32_t)rows : 0u, N, c.evals_d(), ws.evals,
+                                   c.done_d(), c.stream);
+        });
+        fetch(pair_fin_ctas(R, N), left == 0 ? q.fdst : nullptr, false);
+        transcript_round(t, rch, k + 1, left == 0, lane_hg, last_out);
+        return left > 1;
+    }
     // Rounds a.k0 .. a.n-1 of a phase in one k_phase launch: after each round's evaluations the
     // host appends them, derives the challenges and writes them to the mailbox, from which
     // the kernel's next round reads them.  The last round's rows 0..1 come with its
@@ -1031,9 +1074,8 @@ struct Prover {
         a.priv_stride = phase_priv_quads(rows * a.tpr);
         prepare(a.tpr, a.priv_stride);
         for (int j = 0; j < R; j++) {
-            a.fsrc[j] = (a.k0 & 1) ? ws.fB[j] : ws.fA[j];
-            a.hsrc[j] = (a.k0 & 1) ? ws.hg0[j] : ws.hgA[j];
             a.r_first[j] = a.k0 ? rch[j][a.k0 - 1] : 0u;
+            a.r_before[j] = a.two ? rch[j][a.k0 - 2] : 0u;
         }
         a.reps = (uint32_t)R;
         a.N = N;
@@ -1242,7 +1284,8 @@ struct Prover {
 
         const uint32_t* cur_f[3] = {v, v, v};
         const uint32_t* cur_h[3] = {nullptr, nullptr, nullptr};  // round 1 rebuilds hg
-        for (uint32_t k = 1; k < n; k++) {
+        bool two = false, to_a = true;  // the tables are two rounds back; the next ones go to fA, hgA
+        for (uint32_t k = 1; k < n; k++, to_a = !to_a) {
             // from round 4 on (rounds 2 and 3 refold the input and recompute copy-independent hg
             // rows) the rest runs in one launch once its tables are small
             if (k >= 4 && I >> (k - 1) <= kPhaseTailItems) {
@@ -1252,6 +1295,11 @@ struct Prover {
                 PhaseArgs a = {};
                 a.k0 = k;
                 a.n = n;
+                a.two = two;
+                for (int j = 0; j < R; j++) {
+                    a.fsrc[j] = cur_f[j];
+                    a.hsrc[j] = cur_h[j];
+                }
                 if (run_phase(t, true, a, rx, true, vxh, bytes, 0, [](uint32_t, size_t) {})) break;
             }
             RoundPtrs p;
@@ -1259,13 +1307,34 @@ struct Prover {
             for (int j = 0; j < R; j++) {
                 p.fsrc[j] = cur_f[j];
                 p.hsrc[j] = cur_h[j];
-                p.fdst[j] = (k & 1) ? ws.fA[j] : ws.fB[j];
-                p.hdst[j] = (k & 1) ? ws.hgA[j] : ws.hg0[j];
+                p.fdst[j] = to_a ? ws.fA[j] : ws.fB[j];
+                p.hdst[j] = to_a ? ws.hgA[j] : ws.hg0[j];
                 p.r[j] = rx[j][k - 1];
             }
             const uint64_t npairs = I >> (k + 1);
             const double S = 4.0 * npairs;
             c.tag = ((uint32_t)li << 16) | (1u << 8) | k;
+            if (two || pairs_from(n, k)) {
+                double b = rb * 2.0 * R * (two ? 2.5 : 1.5) * S;
+                if (!two) {
+                    p.hoff = Ly.mx_off;
+                    p.ha = ws.a4;
+                    b += (double)R * Ly.h2_scalar_rows * (64.0 - rb) + 20.0 * npairs * R;
+                }
+                for (int j = 0; j < R; j++) {
+                    p.hr[0][j] = two ? rx[j][k - 2] : rx[j][0];
+                    p.hr[1][j] = rx[j][1];
+                }
+                uint32_t *const *f2 = to_a ? ws.fB : ws.fA, *const *h2 = to_a ? ws.hg0 : ws.hgA;
+                two = run_pair(t, true, K_ROUND_LANE, p, two, k, n, f2, h2, rx, vxh, b);
+                if (!two) to_a = !to_a;
+                for (int j = 0; j < R; j++) {
+                    cur_f[j] = two ? p.fdst[j] : f2[j];
+                    cur_h[j] = two ? p.hdst[j] : h2[j];
+                }
+                k++;
+                continue;
+            }
             int kid = K_ROUND_LANE;
             // with a round 2, round 1 stores no folded copies of the layer input (they would be
             // written once and read once): round 2 refolds v at the round-0 challenges
@@ -1385,7 +1454,9 @@ struct Prover {
         const uint32_t* cur_f[3] = {v, v, v};
         // round 2 refolds the layer input
         const bool refold = n >= 3;
-        for (uint32_t k = k_first; k < n; k++) {
+        bool two = false;  // the tables are two rounds back
+        int src = (k_first - 1) & 1;  // scalar tables read; copies written to fA where they are 0
+        for (uint32_t k = k_first; k < n; k++, src ^= 1) {
             if (k >= 3 && I >> (k - 1) <= kPhaseTailItems) {
                 double bytes = 0;
                 for (uint32_t kk = k; kk < n; kk++) {
@@ -1397,22 +1468,37 @@ struct Prover {
                 a.k0 = k;
                 a.n = n;
                 a.vx = ws.vx;
-                for (int j = 0; j < R; j++) a.s[j] = ws.sb[(k - 1) & 1] + j * sstride;
+                a.two = two;
+                for (int j = 0; j < R; j++) {
+                    a.fsrc[j] = cur_f[j];
+                    a.s[j] = ws.sb[src] + j * sstride;
+                }
                 if (run_phase(t, false, a, ry, false, vy, bytes, 0, [](uint32_t, size_t) {})) break;
             }
             RoundPtrs p;
             memset(&p, 0, sizeof(p));
-            const int src = (k - 1) & 1, dst = k & 1;
+            uint32_t* h2[3] = {};
             for (int j = 0; j < R; j++) {
                 p.fsrc[j] = cur_f[j];
-                p.fdst[j] = (k & 1) ? ws.fA[j] : ws.fB[j];
+                p.fdst[j] = src == 0 ? ws.fA[j] : ws.fB[j];
                 p.hsrc[j] = ws.sb[src] + j * sstride;
-                p.hdst[j] = ws.sb[dst] + j * sstride;
+                p.hdst[j] = ws.sb[src ^ 1] + j * sstride;
                 p.r[j] = ry[j][k - 1];
+                h2[j] = ws.sb[src] + j * sstride;
             }
             const uint64_t npairs = I >> (k + 1);
             const double S = 4.0 * npairs;
             c.tag = ((uint32_t)li << 16) | (2u << 8) | k;
+            if (two || pairs_from(n, k)) {
+                for (int j = 0; two && j < R; j++) p.hr[0][j] = ry[j][k - 2];
+                uint32_t* const* f2 = src == 0 ? ws.fB : ws.fA;
+                two = run_pair(t, false, K_ROUND_SCALAR, p, two, k, n, f2, h2, ry, vy,
+                               (rb + 4.0) * R * (two ? 2.5 : 1.5) * S);
+                if (!two) src ^= 1;
+                for (int j = 0; j < R; j++) cur_f[j] = two ? p.fdst[j] : f2[j];
+                k++;
+                continue;
+            }
             // with a round 2, round 1 stores no folded copies (they would be written once and
             // read once): round 2 refolds the layer input
             if (k == 1 && refold)

@@ -83,3 +83,22 @@ def test_row_tiles_that_do_not_divide_the_copies(ctx, oracle, seed, widths, n):
     assert proof == op and np.array_equal(cv, ocv)
     assert np.array_equal(ctx.evaluate(dc, w), oracle.evaluate(circ, w)[-1])
     assert ctx.verify(dc, proof, cv)
+
+
+@pytest.mark.parametrize("seed,widths,n,p_mul,tails", [
+    # the smallest tables whose rounds are taken in pairs, with a partly idle last lane group: six
+    # pairs and a round, seven pairs, and a phase that takes over two rounds behind
+    (641, [16, 14], 2052, 0.3, False), (642, [17, 16], 1024, 1.0, False), (643, [16, 16], 2048, 0.6, True),
+    (644, [17, 15], 1028, 0.5, True),
+])
+def test_rounds_in_pairs_give_the_oracle_proof(ctx, oracle, seed, widths, n, p_mul, tails):
+    circ = gc.random_circuit(seed, widths, p_mul=p_mul)
+    w = gc.random_witness(seed, circ.log_input_size, n)
+    dc = ctx.load(circ)
+    try:
+        ctx.set_round_tail(tails)
+        cv, proof = ctx.prove(dc, w)
+    finally:
+        ctx.set_round_tail(True)
+    ocv, op = oracle.prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
