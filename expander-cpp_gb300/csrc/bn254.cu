@@ -228,6 +228,214 @@ __device__ __forceinline__ Fr to_mont(const Fr& a) {
 }
 __device__ __forceinline__ Fr fold(const Fr& a, const Fr& b, const Fr& r) { return add(a, mul(sub(b, a), r)); }
 
+// Sums of products before their Montgomery reduction, below 16 r^2 < 2^512 - 2^510: a product
+// alone is 64 of mul's 136 multiplications, and a sum is reduced once for kWideTerms of them.
+// The round kernels are bound by the multiply pipe: on 2^16 rows of 64 copies phase two's round 0
+// (three sums a pair) went from 122 to 84 us, the first fold rounds (two sums and four or
+// two folds) from 127 to 114 and 111 to 100.
+struct Wide {
+    uint32_t w[16];
+};
+// Products that may be added to zero or to a lifted sum (lift(x) < 2^256 r < 5.3 r^2).
+constexpr uint32_t kWideTerms = 10;
+
+__device__ __forceinline__ Wide lift(const Fr& x) {
+    Wide s;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        s.w[i] = 0u;
+        s.w[8 + i] = x.l[i];
+    }
+    return s;
+}
+
+// s += a b.  As in mul, the product is formed in two accumulators whose 64-bit pairs start at
+// the even words (e) and at the odd ones (o).  Row i adds four products to four neighbouring
+// pairs of each: to e from word i + (i & 1) on, to o from word i + 1 - (i & 1) on.  The rows that
+// end on a pair not used before leave no carry; the others' carry starts the next pair.
+__device__ __forceinline__ void mac(Wide& s, const Fr& a, const Fr& b) {
+    uint32_t e[16], o[18];  // o[k]: word k + 1... kept at its own word, o[0] unused
+#pragma unroll
+    for (int k = 0; k < 16; k++) e[k] = 0u;
+#pragma unroll
+    for (int k = 0; k < 18; k++) o[k] = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t bi = b.l[i];
+        const int odd = i & 1;
+        // products of the words of a with i's parity meet e, the others o
+        const int pe = i + odd, po = i + 1 - odd;
+        if (i == 0) {
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                const uint64_t x = (uint64_t)a.l[k] * bi, y = (uint64_t)a.l[k + 1] * bi;
+                e[k] = (uint32_t)x;
+                e[k + 1] = (uint32_t)(x >> 32);
+                o[k + 1] = (uint32_t)y;
+                o[k + 2] = (uint32_t)(y >> 32);
+            }
+            continue;
+        }
+        const uint32_t e0 = a.l[odd], e1 = a.l[2 + odd], e2 = a.l[4 + odd], e3 = a.l[6 + odd];
+        const uint32_t o0 = a.l[1 - odd], o1 = a.l[3 - odd], o2 = a.l[5 - odd], o3 = a.l[7 - odd];
+        if (odd) {
+            asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
+                "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+                "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+                "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+                "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+                "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+                "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+                "madc.hi.u32 %7, %11, %12, %7;"
+                : "+r"(e[pe]), "+r"(e[pe + 1]), "+r"(e[pe + 2]), "+r"(e[pe + 3]), "+r"(e[pe + 4]), "+r"(e[pe + 5]),
+                  "+r"(e[pe + 6]), "+r"(e[pe + 7])
+                : "r"(e0), "r"(e1), "r"(e2), "r"(e3), "r"(bi));
+            asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+                "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+                "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+                "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+                "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+                "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+                "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+                "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+                "addc.u32 %8, 0, 0;"
+                : "+r"(o[po]), "+r"(o[po + 1]), "+r"(o[po + 2]), "+r"(o[po + 3]), "+r"(o[po + 4]), "+r"(o[po + 5]),
+                  "+r"(o[po + 6]), "+r"(o[po + 7]), "=r"(o[po + 8])
+                : "r"(o0), "r"(o1), "r"(o2), "r"(o3), "r"(bi));
+        } else {
+            asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+                "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+                "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+                "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+                "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+                "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+                "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+                "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+                "addc.u32 %8, 0, 0;"
+                : "+r"(e[pe]), "+r"(e[pe + 1]), "+r"(e[pe + 2]), "+r"(e[pe + 3]), "+r"(e[pe + 4]), "+r"(e[pe + 5]),
+                  "+r"(e[pe + 6]), "+r"(e[pe + 7]), "=r"(e[pe + 8])
+                : "r"(e0), "r"(e1), "r"(e2), "r"(e3), "r"(bi));
+            asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
+                "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+                "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+                "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+                "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+                "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+                "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+                "madc.hi.u32 %7, %11, %12, %7;"
+                : "+r"(o[po]), "+r"(o[po + 1]), "+r"(o[po + 2]), "+r"(o[po + 3]), "+r"(o[po + 4]), "+r"(o[po + 5]),
+                  "+r"(o[po + 6]), "+r"(o[po + 7])
+                : "r"(o0), "r"(o1), "r"(o2), "r"(o3), "r"(bi));
+        }
+    }
+    auto add8 = [](uint32_t* d, const uint32_t* x, uint32_t carry) {  // d[0..7] += x[0..7] + carry
+        uint32_t out;
+        asm("add.cc.u32 %8, %17, 0xffffffff;\n\t"
+            "addc.cc.u32 %0, %0, %9;\n\t"
+            "addc.cc.u32 %1, %1, %10;\n\t"
+            "addc.cc.u32 %2, %2, %11;\n\t"
+            "addc.cc.u32 %3, %3, %12;\n\t"
+            "addc.cc.u32 %4, %4, %13;\n\t"
+            "addc.cc.u32 %5, %5, %14;\n\t"
+            "addc.cc.u32 %6, %6, %15;\n\t"
+            "addc.cc.u32 %7, %7, %16;\n\t"
+            "addc.u32 %8, 0, 0;"
+            : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]), "=&r"(out)
+            : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(carry));
+        return out;
+    };
+    add8(s.w + 8, e + 8, add8(s.w, e, 0u));
+    add8(s.w + 8, o + 8, add8(s.w, o, 0u));
+}
+
+// s 2^-256 mod r: the low half's Montgomery reduction (mul's steps without its products), at
+// most r, plus the high half, below 4 r together.
+__device__ __forceinline__ Fr reduce(const Wide& s) {
+    uint32_t x[8], y[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        x[k] = s.w[k];
+        y[k] = 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        if (i > 0) {
+            uint32_t z6;
+            asm("add.cc.u32 %0, %0, %8;\n\t"
+                "addc.cc.u32 %1, %1, 0;\n\t"
+                "addc.cc.u32 %2, %2, 0;\n\t"
+                "addc.cc.u32 %3, %3, 0;\n\t"
+                "addc.cc.u32 %4, %4, 0;\n\t"
+                "addc.cc.u32 %5, %5, 0;\n\t"
+                "addc.cc.u32 %6, %6, 0;\n\t"
+                "addc.u32 %7, 0, 0;"
+                : "+r"(y[0]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "=r"(z6)
+                : "r"(x[1]));
+            const uint32_t z[8] = {x[2], x[3], x[4], x[5], x[6], x[7], z6, 0u};
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                x[k] = y[k];
+                y[k] = z[k];
+            }
+        }
+        const uint32_t m = x[0] * 0xefffffffu;
+        asm("mad.lo.cc.u32 %0, %8, 0x43e1f593, %0;\n\t"
+            "madc.hi.cc.u32 %1, %8, 0x43e1f593, %1;\n\t"
+            "madc.lo.cc.u32 %2, %8, 0x2833e848, %2;\n\t"
+            "madc.hi.cc.u32 %3, %8, 0x2833e848, %3;\n\t"
+            "madc.lo.cc.u32 %4, %8, 0xb85045b6, %4;\n\t"
+            "madc.hi.cc.u32 %5, %8, 0xb85045b6, %5;\n\t"
+            "madc.lo.cc.u32 %6, %8, 0x30644e72, %6;\n\t"
+            "madc.hi.u32 %7, %8, 0x30644e72, %7;"
+            : "+r"(y[0]), "+r"(y[1]), "+r"(y[2]), "+r"(y[3]), "+r"(y[4]), "+r"(y[5]), "+r"(y[6]), "+r"(y[7])
+            : "r"(m));
+        asm("mad.lo.cc.u32 %0, %9, 0xf0000001, %0;\n\t"
+            "madc.hi.cc.u32 %1, %9, 0xf0000001, %1;\n\t"
+            "madc.lo.cc.u32 %2, %9, 0x79b97091, %2;\n\t"
+            "madc.hi.cc.u32 %3, %9, 0x79b97091, %3;\n\t"
+            "madc.lo.cc.u32 %4, %9, 0x8181585d, %4;\n\t"
+            "madc.hi.cc.u32 %5, %9, 0x8181585d, %5;\n\t"
+            "madc.lo.cc.u32 %6, %9, 0xe131a029, %6;\n\t"
+            "madc.hi.cc.u32 %7, %9, 0xe131a029, %7;\n\t"
+            "addc.u32 %8, %8, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "+r"(y[7])
+            : "r"(m));
+    }
+    // x[1..7] + y + the high half
+    uint32_t t[8], d[8];
+    asm("add.cc.u32 %0, %8, %15;\n\t"
+        "addc.cc.u32 %1, %9, %16;\n\t"
+        "addc.cc.u32 %2, %10, %17;\n\t"
+        "addc.cc.u32 %3, %11, %18;\n\t"
+        "addc.cc.u32 %4, %12, %19;\n\t"
+        "addc.cc.u32 %5, %13, %20;\n\t"
+        "addc.cc.u32 %6, %14, %21;\n\t"
+        "addc.u32 %7, %22, 0;"
+        : "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]), "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]), "=&r"(t[7])
+        : "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(y[0]), "r"(y[1]), "r"(y[2]),
+          "r"(y[3]), "r"(y[4]), "r"(y[5]), "r"(y[6]), "r"(y[7]));
+    asm("add.cc.u32 %0, %0, %8;\n\t"
+        "addc.cc.u32 %1, %1, %9;\n\t"
+        "addc.cc.u32 %2, %2, %10;\n\t"
+        "addc.cc.u32 %3, %3, %11;\n\t"
+        "addc.cc.u32 %4, %4, %12;\n\t"
+        "addc.cc.u32 %5, %5, %13;\n\t"
+        "addc.cc.u32 %6, %6, %14;\n\t"
+        "addc.u32 %7, %7, %15;"
+        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7])
+        : "r"(s.w[8]), "r"(s.w[9]), "r"(s.w[10]), "r"(s.w[11]), "r"(s.w[12]), "r"(s.w[13]), "r"(s.w[14]), "r"(s.w[15]));
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const bool below = minus_r(t, d) != 0u;
+#pragma unroll
+        for (int i = 0; i < 8; i++) t[i] = below ? t[i] : d[i];
+    }
+    Fr o;
+#pragma unroll
+    for (int i = 0; i < 8; i++) o.l[i] = t[i];
+    return o;
+}
+
 // The canonical value of a sum of Montgomery forms given as 64-bit limb sums:
 // T = sum_k s[k] 2^(32k) is the sum of the x_i R (R = 2^256), so REDC(T) = T R^-1 mod r is
 // sum x_i, already canonical after one conditional subtraction (T < 2^266 keeps
@@ -500,15 +708,24 @@ struct CopyFinBn {
     __device__ void operator()(uint32_t, uint32_t lane, const Fr* t, uint32_t) const { stf(out, 0, N, lane, t[0]); }
 };
 
-__device__ __forceinline__ void accum(Fr (&acc)[3], const Fr& f0, const Fr& f1, const Fr& h0, const Fr& h1) {
-    acc[0] = add(acc[0], mul(f0, h0));
-    acc[1] = add(acc[1], mul(f1, h1));
-    acc[2] = add(acc[2], mul(add(f0, f1), add(h0, h1)));
+__device__ __forceinline__ void accum(Wide (&acc)[3], const Fr& f0, const Fr& f1, const Fr& h0, const Fr& h1) {
+    mac(acc[0], f0, h0);
+    mac(acc[1], f1, h1);
+    mac(acc[2], add(f0, f1), add(h0, h1));
 }
 // p0 and p2raw only (the round's p1 comes from its claim: ClaimFinBn)
-__device__ __forceinline__ void accum(Fr (&acc)[2], const Fr& f0, const Fr& f1, const Fr& h0, const Fr& h1) {
-    acc[0] = add(acc[0], mul(f0, h0));
-    acc[1] = add(acc[1], mul(add(f0, f1), add(h0, h1)));
+__device__ __forceinline__ void accum(Wide (&acc)[2], const Fr& f0, const Fr& f1, const Fr& h0, const Fr& h1) {
+    mac(acc[0], f0, h0);
+    mac(acc[1], add(f0, f1), add(h0, h1));
+}
+// Sums of up to kWideTerms accumulations each: the totals so far, which the next ones go on from.
+template <int C>
+__device__ __forceinline__ void settle(Wide (&acc)[C], Fr (&total)[C]) {
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        total[c] = reduce(acc[c]);
+        acc[c] = lift(total[c]);
+    }
 }
 
 // ---------------------------------------------------------------- kernels
@@ -759,14 +976,16 @@ __global__ void __launch_bounds__(256) k_gate_sums(uint64_t O, const uint32_t* _
     }
 }
 
-__global__ void __launch_bounds__(256) k_hg_round0(const uint32_t* __restrict__ v, uint64_t I,
+__global__ void __launch_bounds__(256, 2) k_hg_round0(const uint32_t* __restrict__ v, uint64_t I,
                                                    const uint32_t* __restrict__ mx_off, const uint4* __restrict__ mx_g,
                                                    const Fr* __restrict__ a, const Fr* __restrict__ w, uint32_t* hg,
                                                    GeoBn g, RedBn red, const uint32_t* claim, uint32_t* evals_out) {
     const Tile t = tile(g);
-    Fr acc[2] = {zero(), zero()};  // p0, p2raw
-    if (t.active) {
-        for (uint64_t i = (uint64_t)blockIdx.x * g.rps + t.rs; i < (I >> 1); i += (uint64_t)gridDim.x * g.rps) {
+    Fr total[2] = {zero(), zero()};  // p0, p2raw
+    Wide acc[2] = {lift(zero()), lift(zero())};
+    uint64_t i = (uint64_t)blockIdx.x * g.rps + t.rs;
+    while (t.active && i < (I >> 1)) {
+        for (uint32_t n = 0; n < kWideTerms && i < (I >> 1); n++, i += (uint64_t)gridDim.x * g.rps) {
             Fr h0, h1;
             // not unrolled: each copy of the gate loop inlines a 256-bit product, and two of
             // them left this kernel waiting on instruction fetch (ncu: no_instruction stalls)
@@ -782,12 +1001,13 @@ __global__ void __launch_bounds__(256) k_hg_round0(const uint32_t* __restrict__ 
             }
             accum(acc, ldf(v, 2 * i, g.N, t.q), ldf(v, 2 * i + 1, g.N, t.q), h0, h1);
         }
+        settle(acc, total);
     }
-    reduce_bn<2>(acc, g, t.active, red, ClaimFinBn{evals_out, red.evals_dev, claim, nullptr, nullptr, zero(), g.N});
+    reduce_bn<2>(total, g, t.active, red, ClaimFinBn{evals_out, red.evals_dev, claim, nullptr, nullptr, zero(), g.N});
 }
 
 template <bool LANE_HG, bool FOLD>
-__global__ void __launch_bounds__(256) k_round(RoundPtrsBn p, uint64_t npairs, const uint32_t* __restrict__ vx, GeoBn g,
+__global__ void __launch_bounds__(256, 2) k_round(RoundPtrsBn p, uint64_t npairs, const uint32_t* __restrict__ vx, GeoBn g,
                                                RedBn red, uint32_t* evals_out) {
     const Tile t = tile(g);
     Fr r;
@@ -795,9 +1015,13 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrsBn p, uint64_t npairs, c
     for (int k = 0; k < 8; k++) r.l[k] = p.r[k];
     // fold rounds sum p0 and p2raw (p1 from the claim), phase two's round 0 all three
     constexpr int C = FOLD ? 2 : 3;
-    Fr acc[C];
+    Fr total[C];
+    Wide acc[C];
 #pragma unroll
-    for (int c = 0; c < C; c++) acc[c] = zero();
+    for (int c = 0; c < C; c++) {
+        total[c] = zero();
+        acc[c] = lift(total[c]);
+    }
     const Fr* hs = reinterpret_cast<const Fr*>(p.hsrc);
     Fr* hd = reinterpret_cast<Fr*>(p.hdst);
     // Phase two folds the lane-independent scalar table: with a power-of-two row tile of at
@@ -808,57 +1032,58 @@ __global__ void __launch_bounds__(256) k_round(RoundPtrsBn p, uint64_t npairs, c
     const uint32_t gq = threadIdx.x & (grp - 1);
     const uint32_t q = threadIdx.x % g.tpr;
     const uint64_t stride = (uint64_t)gridDim.x * g.rps;
-    for (uint64_t i = (uint64_t)blockIdx.x * g.rps + t.rs;; i += stride) {
-        const bool valid = t.active && i < npairs;
-        if (share) {
-            if (!__any_sync(0xffffffffu, valid)) break;
-        } else if (!valid) {
-            break;
-        }
-        Fr f0 = zero(), f1 = zero(), h0, h1;
-        if (FOLD) {
-            if (valid) {
-                f0 = fold(ldf(p.fsrc, 4 * i, g.N, t.q), ldf(p.fsrc, 4 * i + 1, g.N, t.q), r);
-                f1 = fold(ldf(p.fsrc, 4 * i + 2, g.N, t.q), ldf(p.fsrc, 4 * i + 3, g.N, t.q), r);
-                stf(p.fdst, 2 * i, g.N, t.q, f0);
-                stf(p.fdst, 2 * i + 1, g.N, t.q, f1);
-            }
-            if (LANE_HG) {
-                h0 = fold(ldf(p.hsrc, 4 * i, g.N, t.q), ldf(p.hsrc, 4 * i + 1, g.N, t.q), r);
-                h1 = fold(ldf(p.hsrc, 4 * i + 2, g.N, t.q), ldf(p.hsrc, 4 * i + 3, g.N, t.q), r);
-                stf(p.hdst, 2 * i, g.N, t.q, h0);
-                stf(p.hdst, 2 * i + 1, g.N, t.q, h1);
-            } else if (share) {
-                Fr mine = zero();
-                if (valid && gq < 2) mine = fold(lds(hs, 4 * i + 2 * gq), lds(hs, 4 * i + 2 * gq + 1), r);
+    uint64_t i = (uint64_t)blockIdx.x * g.rps + t.rs;
+    for (bool more = true; more;) {
+        for (uint32_t n = 0; n < kWideTerms; n++, i += stride) {
+            const bool valid = t.active && i < npairs;
+            more = share ? __any_sync(0xffffffffu, valid) : valid;
+            if (!more) break;
+            Fr f0 = zero(), f1 = zero(), h0, h1;
+            if (FOLD) {
+                if (valid) {
+                    f0 = fold(ldf(p.fsrc, 4 * i, g.N, t.q), ldf(p.fsrc, 4 * i + 1, g.N, t.q), r);
+                    f1 = fold(ldf(p.fsrc, 4 * i + 2, g.N, t.q), ldf(p.fsrc, 4 * i + 3, g.N, t.q), r);
+                    stf(p.fdst, 2 * i, g.N, t.q, f0);
+                    stf(p.fdst, 2 * i + 1, g.N, t.q, f1);
+                }
+                if (LANE_HG) {
+                    h0 = fold(ldf(p.hsrc, 4 * i, g.N, t.q), ldf(p.hsrc, 4 * i + 1, g.N, t.q), r);
+                    h1 = fold(ldf(p.hsrc, 4 * i + 2, g.N, t.q), ldf(p.hsrc, 4 * i + 3, g.N, t.q), r);
+                    stf(p.hdst, 2 * i, g.N, t.q, h0);
+                    stf(p.hdst, 2 * i + 1, g.N, t.q, h1);
+                } else if (share) {
+                    Fr mine = zero();
+                    if (valid && gq < 2) mine = fold(lds(hs, 4 * i + 2 * gq), lds(hs, 4 * i + 2 * gq + 1), r);
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    h0.l[k] = __shfl_sync(0xffffffffu, mine.l[k], 0, grp);
-                    h1.l[k] = __shfl_sync(0xffffffffu, mine.l[k], 1, grp);
+                    for (int k = 0; k < 8; k++) {
+                        h0.l[k] = __shfl_sync(0xffffffffu, mine.l[k], 0, grp);
+                        h1.l[k] = __shfl_sync(0xffffffffu, mine.l[k], 1, grp);
+                    }
+                } else {
+                    h0 = fold(lds(hs, 4 * i), lds(hs, 4 * i + 1), r);
+                    h1 = fold(lds(hs, 4 * i + 2), lds(hs, 4 * i + 3), r);
+                }
+                // the scalar table is shared by all lanes: the first thread of the row slice in
+                // lane group 0 writes it
+                if (!LANE_HG && valid && q == 0 && blockIdx.y == 0) {
+                    sts(hd, 2 * i, h0);
+                    sts(hd, 2 * i + 1, h1);
                 }
             } else {
-                h0 = fold(lds(hs, 4 * i), lds(hs, 4 * i + 1), r);
-                h1 = fold(lds(hs, 4 * i + 2), lds(hs, 4 * i + 3), r);
+                f0 = ldf(p.fsrc, 2 * i, g.N, t.q);
+                f1 = ldf(p.fsrc, 2 * i + 1, g.N, t.q);
+                h0 = lds(hs, 2 * i);
+                h1 = lds(hs, 2 * i + 1);
             }
-            // the scalar table is shared by all lanes: the first thread of the row slice in
-            // lane group 0 writes it
-            if (!LANE_HG && valid && q == 0 && blockIdx.y == 0) {
-                sts(hd, 2 * i, h0);
-                sts(hd, 2 * i + 1, h1);
-            }
-        } else {
-            f0 = ldf(p.fsrc, 2 * i, g.N, t.q);
-            f1 = ldf(p.fsrc, 2 * i + 1, g.N, t.q);
-            h0 = lds(hs, 2 * i);
-            h1 = lds(hs, 2 * i + 1);
+            if (valid) accum(acc, f0, f1, h0, h1);
         }
-        if (valid) accum(acc, f0, f1, h0, h1);
+        settle(acc, total);
     }
     if constexpr (FOLD)
-        reduce_bn<2>(acc, g, t.active, red,
+        reduce_bn<2>(total, g, t.active, red,
                      ClaimFinBn{evals_out, red.evals_dev, nullptr, red.evals_prev, LANE_HG ? nullptr : vx, r, g.N});
     else
-        reduce_bn<3>(acc, g, t.active, red, RoundFinBn{evals_out, LANE_HG ? nullptr : vx, g.N, red.evals_dev});
+        reduce_bn<3>(total, g, t.active, red, RoundFinBn{evals_out, LANE_HG ? nullptr : vx, g.N, red.evals_dev});
 }
 
 __global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __restrict__ my_off,
@@ -897,17 +1122,20 @@ __global__ void __launch_bounds__(256) k_wsum(const uint32_t* __restrict__ vals,
     const Tile t = tile(g);
     eq_build(tab, tab + eq_elems(eq), eq);
     const uint32_t nd = eq_tables(eq);
-    Fr acc[1] = {zero()};
+    Fr total[1] = {zero()};
+    Wide acc[1] = {lift(zero())};
     for (uint64_t z0 = (uint64_t)blockIdx.x * kWsumRows; z0 < rows; z0 += (uint64_t)gridDim.x * kWsumRows) {
         __syncthreads();  // the digit tables are built, the last block's weights are done with
         const uint32_t n = rows - z0 < kWsumRows ? (uint32_t)(rows - z0) : kWsumRows;
         if (threadIdx.x < n) w[threadIdx.x] = eq_at(tab, nd, false, (uint32_t)(z0 + threadIdx.x));
         __syncthreads();
-        if (t.active)
-            for (uint32_t i = t.rs; i < n; i += g.rps) acc[0] = add(acc[0], mul(w[i], ldf(vals, z0 + i, g.N, t.q)));
+        for (uint32_t i = t.rs; t.active && i < n;) {
+            for (uint32_t k = 0; k < kWideTerms && i < n; k++, i += g.rps) mac(acc[0], w[i], ldf(vals, z0 + i, g.N, t.q));
+            settle(acc, total);
+        }
     }
     __syncthreads();
-    reduce_bn<1>(acc, g, t.active, red, CopyFinBn{out, g.N});
+    reduce_bn<1>(total, g, t.active, red, CopyFinBn{out, g.N});
 }
 
 // ---------------------------------------------------------------- persistent phases

@@ -102,3 +102,18 @@ def test_rounds_in_pairs_give_the_oracle_proof(ctx, oracle, seed, widths, n, p_m
         ctx.set_round_tail(True)
     ocv, op = oracle.prove(circ, w)
     assert proof == op and np.array_equal(cv, ocv)
+
+
+@pytest.mark.parametrize("widths,n", [([13, 3], 250), ([14, 4], 128), ([12, 2], 1000)])
+def test_bn254_sums_of_many_products(ctx, widths, n):
+    # more than ten pairs a thread in the first rounds (sums reduced and gone on from), with input
+    # elements whose Montgomery form is r - 1, the largest factor of a product
+    from oracle.oracle import OracleBn254
+    r = gc.BN254_R
+    x = (r - 1) * pow(2, -256, r) % r
+    circ = gc.random_circuit(651, widths, p_mul=0.6)
+    w = gc.random_witness_bn254(651, circ.log_input_size, n)
+    w[...] = np.frombuffer(x.to_bytes(32, "little"), np.uint64)
+    cv, proof = ctx.prove(ctx.load(circ, "BN254"), w)
+    ocv, op = OracleBn254().prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
