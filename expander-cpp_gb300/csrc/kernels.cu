@@ -1769,7 +1769,8 @@ __global__ void __launch_bounds__(256) k_s_build(uint64_t I, const uint32_t* __r
 // unreduced in 64 bits and folded every four rows (as separate field operations the sums took
 // 430 us, bound by instruction issue); a thread stages its next steps of four consecutive rows
 // with cp.async, and their weights, computed per block of rows from the digit tables, come from
-// shared memory.  What bounds it is the wide multiply-add, 17 products with their folding per
+// shared memory.  (One point, and narrow rows; the others in k_wsum_mma.)  At three points what
+// bounds it is the wide multiply-add, 17 products with their folding per
 // clock and SM: 235 us at three CTAs an SM and four stages, 256 at four and two or three.
 constexpr uint32_t kWsumRows = 256;  // rows of a CTA's weights at a time, at least
 constexpr int kWsumStages = 4;       // steps of four rows a thread has in its cp.async ring
@@ -1858,6 +1859,175 @@ __global__ void __launch_bounds__(256, 3) k_wsum(const uint32_t* __restrict__ va
         for (int l = 0; l < 4; l++) sum[c][l] = reduce64(acc[c][l]);
     __syncthreads();  // the ring is the reduction's scratch
     reduce_group<R>(sum, g, t.active, red, 0, CopyFin{red, out, g.N, (uint32_t)R});
+}
+
+// Two or three points on wide rows: the same sums as a contraction on the tensor cores, exact.
+// With v = sum_d 2^(8d) b_d(v) over its four bytes, sum_z v[z] w[z] is the sum over (z, d) of
+// b_d(v[z]) times 2^(8d) w[z] mod p (a rotation of w's 31 bits), whose bytes are again 2^(8e)
+// apart: for every copy, a sum for each point and byte e over k = (row, digit) of products of two
+// bytes.  A byte widened with zeros is the subnormal 16-bit float b 2^-24, the products are
+// multiples of 2^-48 in the 32-bit sums, and a sum of the 256 products of 64 rows is at most
+// 256 * 255^2 < 2^24 of them: no sum is rounded before it goes on to the integers.
+// mma.sync m16n8k16: the k index may be any order of the (row, digit) pairs, so a thread's four
+// k are one row's digits, two byte permutes a value; the four copies of its 16 bytes are rows g
+// and g + 8 of two tiles.  A value costs a thread one MMA instruction and those two permutes,
+// where k_wsum has three wide multiply-adds and their folding: 2^18 rows of 1024 copies at three
+// points 235 -> 192 us (5.6 TB/s; without the MMAs 193, so what is left is memory).
+// (tcgen05 would need the digits in shared memory first; the tensor cores are a third used.)
+constexpr uint32_t kWmmaRows = 128;               // rows of a CTA's weights at a time, at most
+constexpr uint32_t kWmmaExact = 64;               // rows between conversions of the sums
+constexpr int kWmmaStages = 3;                    // steps of four rows a thread has in its cp.async ring
+constexpr uint32_t kWmmaWords = 32;               // words of a row's weights (16 columns x 4 digits)
+
+__device__ __forceinline__ uint32_t rot31(uint32_t x, uint32_t s) {  // 2^s x mod p, 0 <= s < 31
+    return ((x << s) & m31::P) | (x >> (31 - s));
+}
+// Two bytes of x (sel 0x4140: the low ones, 0x4342: the high ones) as 16-bit floats, each b 2^-24:
+// a byte widened with zeros is that subnormal number.
+__device__ __forceinline__ uint32_t half2_bytes(uint32_t x, uint32_t sel) { return __byte_perm(x, 0u, sel); }
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// wc: groups of 32 copies a CTA takes (a divisor of 8), a warp each; 8 / wc warps share a group's
+// rows, 16 at a time.  rb: rows a block, a multiple of 16 * 8 / wc.
+template <int R>
+__global__ void __launch_bounds__(256, 3) k_wsum_mma(const uint32_t* __restrict__ vals, uint64_t rows, uint32_t rb,
+                                                     const __grid_constant__ EqArgs eq, uint32_t N, uint32_t wc,
+                                                     RedScratch red, uint32_t* out) {
+    constexpr int T = (R + 1) / 2;  // tiles of eight columns, two points each
+    extern __shared__ uint4 wmma_sm[];  // rb rows of weights, the ring; at the end partial sums
+    __shared__ uint32_t tab[kEqWords];
+    uint4* const ring = wmma_sm + rb * (kWmmaWords / 4);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, row8 = lane >> 2, c = lane & 3;
+    const uint32_t cg = w % wc, slice = w / wc, step = 16 * (8 / wc);
+    eq_build(tab, eq);
+    const uint32_t nd = eq_digits(eq);
+    float s[2][T][4] = {};      // [copies 2m, 2m+1 of the four][columns 8t ..]
+    uint32_t acc[2][T][4] = {};
+    auto convert = [&](bool reduce) {
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int t = 0; t < T; t++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    acc[m][t][k] += __float2uint_rn(s[m][t][k] * 281474976710656.0f);  // 2^48
+                    if (reduce) acc[m][t][k] = m31::from_u32(acc[m][t][k]);
+                    s[m][t][k] = 0.0f;
+                }
+    };
+    const uint64_t stride = (uint64_t)gridDim.x * rb, base = (uint64_t)blockIdx.x * rb;
+    // The ring's next step: `step` rows from row si of the block at sz on, a row's copies by
+    // neighbouring threads.  (With 128 bytes of four rows a warp, each for itself and without a
+    // barrier, memory gave 3.75 TB/s.)  Row r's quad q is at q ^ 2 (r mod 4), which spreads the
+    // four rows and two quads that eight threads read over all banks.
+    uint64_t sz = base;
+    uint32_t si = 0;
+    const uint32_t rowq = 8 * wc, first = blockIdx.y * rowq;  // quads a row; the CTA's first
+    const uint32_t sr = tid / rowq, sq = tid % rowq, per = 256 / rowq;  // rows sr, sr + per, ..
+    const bool stages = 4 * (first + sq) < N;
+    const uint32_t* from = vals + base * N + 4 * (first + sq);
+    uint32_t off[4];  // words from `from` (a table of less than a step's rows repeats its last, weight 0)
+    uint4* to[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t r = sr + k * per;
+        off[k] = (r < rows ? r : (uint32_t)rows - 1) * N;
+        to[k] = ring + r * rowq + (sq ^ 2 * (r & 3));
+    }
+    auto stage = [&](int slot) {
+        if (sz < rows) {
+            if (stages)
+#pragma unroll
+                for (int k = 0; k < 4; k++) cp_async16(to[k] + slot * 1024, from + off[k]);
+            si += step;
+            from += (uint64_t)step * N;
+            if (si >= rb) {
+                si = 0;
+                sz += stride;
+                from += (stride - rb) * N;
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int q = 0; q < kWmmaStages - 1; q++) stage(q);
+    int slot = 0;
+    uint32_t since = 0, reduced = 0;
+    for (uint64_t z0 = base; z0 < rows; z0 += stride) {
+        __syncthreads();  // the digit tables are built, or the last block's weights are done with
+        for (uint32_t i = tid; i < rb * 4; i += blockDim.x) {
+            const uint32_t z = i >> 2, j = i & 3;  // j >= R: the columns of no point
+            uint32_t wd[4];
+            wd[0] = j < R && z0 + z < rows ? eq_at(tab, nd, false, j, (uint32_t)(z0 + z)) : 0u;
+#pragma unroll
+            for (int d = 1; d < 4; d++) wd[d] = rot31(wd[0], 8 * d);
+            // 16 bytes per place and row, the four rows of a step that a place's threads read side by side
+            uint32_t* to = reinterpret_cast<uint32_t*>(wmma_sm + (z >> 2) * 32 + 16 * (j & 1) + (z & 3)) + 2 * (j >> 1);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {  // column 4j + e: tile j / 2, place 4 (j % 2) + e
+                const uint32_t sel = e | (e + 4) << 4;
+                *reinterpret_cast<uint2*>(to + 16 * e) = make_uint2(half2_bytes(__byte_perm(wd[0], wd[1], sel), 0x4140),
+                                                                   half2_bytes(__byte_perm(wd[2], wd[3], sel), 0x4140));
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = 16 * slice; i < rb; i += step) {
+            cp_async_wait<kWmmaStages - 2>();
+            __syncthreads();  // the step is there, and every warp is done with the one before
+            stage(slot == 0 ? kWmmaStages - 1 : slot - 1);
+            uint4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[k] = ring[slot * 1024 + (16 * slice + 4 * k + c) * rowq + ((8 * cg + row8) ^ 2 * c)];
+            slot = slot + 1 == kWmmaStages ? 0 : slot + 1;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint4 b = wmma_sm[(i / 4 + k) * 32 + lane];
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    const uint32_t x = comp(v[k], 2 * m), y = comp(v[k], 2 * m + 1);
+                    const uint32_t a[4] = {half2_bytes(x, 0x4140), half2_bytes(y, 0x4140), half2_bytes(x, 0x4342),
+                                           half2_bytes(y, 0x4342)};
+                    mma16816(s[m][0], a, b.x, b.y);
+                    if (T > 1) mma16816(s[m][T - 1], a, b.z, b.w);
+                }
+            }
+            since += 16;
+            if (since == kWmmaExact) {
+                since = 0;
+                convert((++reduced & 63) == 0);  // 64 x 2^24 + 2^31 < 2^32
+            }
+        }
+    }
+    cp_async_wait<0>();
+    convert(true);
+    // 2^(8e) shares of a copy and point are in two neighbouring threads
+    uint32_t* const part = reinterpret_cast<uint32_t*>(wmma_sm);
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int t = 0; t < T; t++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t e = 16 * (c & 1), j = 2 * t + (c >> 1);
+                uint32_t x = add(rot31(acc[m][t][2 * h], e), rot31(acc[m][t][2 * h + 1], e + 8));
+                x = add(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                if (!(c & 1) && j < R) part[j * 256 + 32 * w + 4 * row8 + 2 * m + h] = x;
+            }
+    __syncthreads();
+    uint32_t sum[R];
+#pragma unroll
+    for (int j = 0; j < R; j++) sum[j] = part[256 * j + tid];
+    __syncthreads();
+    Geo g;
+    g.N = N;
+    g.tpr = 32 * wc;
+    g.rps = 8 / wc;
+    reduce_group1<R>(sum, g, true, red, CopyFin{red, out, N, (uint32_t)R});
 }
 
 // CTAs of 256 threads for n threads of a kernel that builds digit tables: one wave at most, a
@@ -2278,9 +2448,43 @@ cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g
     return cudaGetLastError();
 }
 
+// Groups of 32 copies a CTA of k_wsum_mma takes; 0: k_wsum.  From two points on, where its
+// copies are a kilobyte or the whole of a row (128 bytes of each of 2^18 rows of 200 copies took
+// 93 us against 72) and at most an eighth of its threads' are past the end.  One point is memory
+// bound either way (2^18 rows of 1024 copies: 189 us both) and smaller tables are faster with the
+// narrow kernel's shorter blocks (2^14 rows 28 against 32 us).
+static uint32_t wmma_groups(uint32_t reps, uint32_t N) {
+    if (reps < 2) return 0;
+    const uint32_t cgs = (N + 31) / 32;
+    for (uint32_t wc = 8; wc > 1; wc /= 2) {
+        const uint32_t ny = (cgs + wc - 1) / wc;
+        if ((wc == 8 || ny == 1) && (uint64_t)N * 8 >= (uint64_t)ny * wc * 32 * 7 && ny <= 1024) return wc;
+    }
+    return 0;
+}
+
+uint32_t wsum_groups(const EqArgs& eq, const Geo& g) {
+    const uint32_t wc = wmma_groups(eq.reps, g.N);
+    return wc ? (g.N + 32 * wc - 1) / (32 * wc) : lane_groups(g);
+}
+
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,
                         RedScratch red, uint32_t* out, cudaStream_t s) {
     const uint64_t rows = 1ull << eq.nvars;
+    if (const uint32_t wc = wmma_groups(eq.reps, g.N)) {
+        const uint32_t ny = (g.N + 32 * wc - 1) / (32 * wc), step = 16 * (8 / wc), cap2 = ctas / ny ? ctas / ny : 1;
+        uint32_t rbm = step;  // a power of two, as the rows are
+        while (2 * rbm <= kWmmaRows && (uint64_t)2 * rbm * cap2 <= rows) rbm *= 2;
+        const uint64_t nb = (rows + rbm - 1) / rbm;
+        // (the partial sums and the reduction's scratch, 3 KB, are less than the ring)
+        const size_t sm = (size_t)rbm * kWmmaWords * 4 + (size_t)kWmmaStages * 4 * 16 * 256;
+        const dim3 gm((uint32_t)(nb < cap2 ? nb : cap2), ny);
+        switch (eq.reps) {
+            case 2: k_wsum_mma<2><<<gm, 256, ring_smem<k_wsum_mma<2>>(sm), s>>>(vals, rows, rbm, eq, g.N, wc, red, out); break;
+            default: k_wsum_mma<3><<<gm, 256, ring_smem<k_wsum_mma<3>>(sm), s>>>(vals, rows, rbm, eq, g.N, wc, red, out); break;
+        }
+        return cudaGetLastError();
+    }
     const uint32_t groups = lane_groups(g), cap = ctas / groups ? ctas / groups : 1, rb = wsum_block(g, rows, cap);
     const uint64_t need = (rows + rb - 1) / rb;
     const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);

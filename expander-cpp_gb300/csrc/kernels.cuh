@@ -270,7 +270,8 @@ cudaError_t launch_hg_build(const uint32_t* v, uint32_t I, uint32_t N, uint32_t 
 // 1024 copies took 1.2 ms that way.
 inline bool hg_build_stored(uint64_t gates, uint32_t N) { return gates * (N / 4) > (1u << 20); }
 // eval_multilinear of vals (2^eq.nvars rows) at eq.r1_j for eq.reps points (eq.f1 = 1, no second
-// point): out receives reps x N.
+// point): out receives reps x N.  Publishes wsum_groups(eq, g) lane groups.
+uint32_t wsum_groups(const EqArgs& eq, const Geo& g);
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgs& eq, const Geo& g, uint32_t block, uint32_t ctas,
                         RedScratch red, uint32_t* out, cudaStream_t s);
 

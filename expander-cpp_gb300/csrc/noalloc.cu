@@ -114,7 +114,7 @@ extern "C" int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t
     g.rps = 256 / g.tpr;
     if (Q % g.tpr || Q / g.tpr > kMaxLaneGroups)
         return fail(GKRGPU_ERR_INVALID, "no row tile with at most 1024 lane groups for this copy count");
-    e = gkrgpu::launch_wsum(d_evals, a, g, 256, (uint32_t)g_sm_count[dev] * 4, red, d_out, s);
+    e = gkrgpu::launch_wsum(d_evals, a, g, 256, (uint32_t)g_sm_count[dev] * 3, red, d_out, s);
     if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(GKRGPU_ERR_CUDA, cudaGetErrorString(e));

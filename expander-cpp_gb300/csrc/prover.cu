@@ -2277,7 +2277,7 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
                                    reinterpret_cast<uint32_t*>(c.extra_d()), c.stream);
             });
             c.pending_bytes = 0;  // spin: the caller's thread may not sleep to the microsecond
-            c.wait_done(lane_groups(g));
+            c.wait_done(wsum_groups(a, g));
             memcpy(out, c.extra_h(), n_points * rowb);
             if (ctx->timing) c.sync();  // the launch's closing event
             c.resolve_events();
