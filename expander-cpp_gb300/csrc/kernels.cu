@@ -2030,6 +2030,186 @@ __global__ void __launch_bounds__(256, 3) k_wsum_mma(const uint32_t* __restrict_
     reduce_group1<R>(sum, g, true, red, CopyFin{red, out, N, (uint32_t)R});
 }
 
+// k_p2_round01 on the tensor cores, exact in the same way.  Row 4q + e of a group meets four
+// coefficients of each repetition: its own s and its neighbour's (s_e, s_(e^1)), which make E or F
+// and their cross sums, and the two pair sums t0 = s0 + s2, t1 = s1 + s3, which make U and its
+// cross sum: [s_e, s_(e^1), t_(e&1), t_(1-(e&1))], each with four bytes.  A warp takes the rows of
+// one e for 32 copies, an MMA step four of its groups (k = group and digit), so a group costs it
+// twelve MMAs for three repetitions where a thread a copy had 27 wide multiply-adds, their folding
+// and the coefficients' loads, 224 instructions a group and warp.
+// The CTA stages the next steps' rows (64 copies) and coefficients with cp.async, and turns the
+// next step's coefficients into bytes while it multiplies this one's.  The integer sums are in
+// shared memory (a conversion every 64 groups), since with the float sums they would not leave
+// two CTAs their registers.  Three repetitions of 2^17 rows of 1024 copies, 14.8 thousand groups
+// with gates: 197 -> 114 us, four layers of 2^20 rows 3.6 -> 2.3 ms; the tensor cores are active
+// 39% of it, the rest is the barrier a step and the conversions.
+constexpr int kP01mStages = 4;
+constexpr uint32_t kP01mGroups = 8;  // groups of a step
+constexpr uint32_t kP01mCopies = 64;
+template <int R>
+constexpr uint32_t p01m_smem() {
+    return 2 * R * 8 * 256 * 4 + 2 * 2 * 6 * R * 16 * 8 + kP01mStages * (512 + 16 * R) * 16;
+}
+
+template <int R>
+__global__ void __launch_bounds__(256, 2) k_p2_round01_mma(P01Src src, uint32_t ngroups, const uint32_t* __restrict__ quads,
+                                                           const uint32_t* __restrict__ vx, uint32_t N, RedScratch red,
+                                                           uint32_t* evals_out, uint32_t* sums_out) {
+    constexpr int U = 4 * R, T = 2 * R;                // units of four columns (coefficient, repetition); tiles of two
+    constexpr uint32_t kSub = 6 * R * 16, kSlot = 512 + 16 * R;
+    extern __shared__ uint4 p01m[];
+    uint32_t* const sums = reinterpret_cast<uint32_t*>(p01m) + threadIdx.x;     // T * 8 words a thread
+    uint2* const bytes = reinterpret_cast<uint2*>(p01m + T * 8 * 64);            // [2][2 steps of four groups][kSub]
+    uint4* const ring = reinterpret_cast<uint4*>(bytes + 4 * kSub);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, row8 = lane >> 2, c = lane & 3;
+    const uint32_t e = w & 3, cg = w >> 2, copy0 = blockIdx.y * kP01mCopies;
+#pragma unroll
+    for (int k = 0; k < T * 8; k++) sums[256 * k] = 0u;
+    float s[2][T][4] = {};
+    uint32_t since = 0, reduced = 0;
+    auto convert = [&](bool reduce) {
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int t = 0; t < T; t++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    uint32_t* p = sums + 256 * ((m * T + t) * 4 + k);
+                    const uint32_t x = *p + __float2uint_rn(s[m][t][k] * 281474976710656.0f);  // 2^48
+                    *p = reduce ? m31::from_u32(x) : x;
+                    s[m][t][k] = 0.0f;
+                }
+    };
+    // what a thread stages of a step: 16 bytes of row (tid / 16) % 4 of two groups, and of one
+    // repetition's s or t of a group
+    const uint32_t vg = tid >> 6, ve = (tid >> 4) & 3, piece = tid & 15, sg = tid / (2 * R), sr = tid % (2 * R);
+    const bool any = ngroups > 0, stages = any && copy0 + 4 * piece < N, scalars = any && tid < 16 * R;
+    const uint32_t* const vfrom = src.v + (uint64_t)ve * N + copy0 + 4 * piece;
+    const uint32_t sj = sr >> 1;
+    const uint32_t* const sfrom = (sr & 1) ? (sj == 0 ? src.t[0] : (sj == 1 ? src.t[1] : src.t[2]))
+                                           : (sj == 0 ? src.s[0] : (sj == 1 ? src.s[1] : src.s[2]));
+    // the first group of the step staged next, and those of its groups in the list (past the
+    // last group the last one's data are staged again, with no coefficients: build)
+    const uint32_t stride = gridDim.x * kP01mGroups, last = ngroups - 1;
+    uint32_t is = blockIdx.x * kP01mGroups, ga = 0, gb = 0, gs = 0;
+    auto look = [&] {
+        if (!any) return;
+        ga = (uint32_t)group_at(quads, min(is + vg, last));
+        gb = (uint32_t)group_at(quads, min(is + vg + 4, last));
+        if (scalars) gs = (uint32_t)group_at(quads, min(is + sg, last));
+        is = is < ngroups ? is + stride : is;
+    };
+    uint4* const vto = ring + (vg * 4 + ve) * 16 + (piece ^ 2 * vg);
+    auto stage = [&](int slot) {
+        if (stages) {
+            cp_async16(vto + slot * kSlot, vfrom + (uint64_t)ga * (4 * N));
+            cp_async16(vto + slot * kSlot + 256, vfrom + (uint64_t)gb * (4 * N));
+        }
+        if (scalars) cp_async16(ring + slot * kSlot + 512 + tid, sfrom + (uint64_t)gs * 4);
+        cp_async_commit();
+        look();
+    };
+    // the bytes of the coefficients of the step at group i (slot) into buffer `buf`; none past the last group
+    const uint32_t bg = tid & 7, bc = tid >> 3;  // group, coefficient x repetition
+    const uint32_t kappa = bc / R;
+    const uint32_t* const bfrom =
+        reinterpret_cast<const uint32_t*>(ring + 512 + bg * 2 * R + 2 * (bc % R) + (kappa >> 2)) + (kappa & 3);
+    uint2* const bto = bytes + (bg >> 2) * kSub + bc * 16 + (bg & 3);
+    auto build = [&](uint32_t i, int slot, uint32_t buf) {
+        if (bc >= 6 * R) return;
+        uint32_t wd[4];
+        wd[0] = i + bg < ngroups ? bfrom[slot * (4 * kSlot)] : 0u;
+#pragma unroll
+        for (int d = 1; d < 4; d++) wd[d] = rot31(wd[0], 8 * d);
+        uint2* const to = bto + buf * 2 * kSub;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint32_t sel = b | (b + 4) << 4;
+            to[4 * b] = make_uint2(half2_bytes(__byte_perm(wd[0], wd[1], sel), 0x4140),
+                                   half2_bytes(__byte_perm(wd[2], wd[3], sel), 0x4140));
+        }
+    };
+    uint32_t ko[T];  // this thread's bytes of each tile
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        const uint32_t u = 2 * t + (row8 >> 2), f = u / R, j = u % R;
+        const uint32_t x = f < 2 ? e ^ f : 4 + ((f ^ e) & 1);
+        ko[t] = ((x * R + j) * 4 + (row8 & 3)) * 4 + c;
+    }
+    look();
+#pragma unroll
+    for (int q = 0; q < kP01mStages - 1; q++) stage(q);
+    cp_async_wait<kP01mStages - 2>();
+    __syncthreads();
+    build(blockIdx.x * kP01mGroups, 0, 0);
+    int slot = 0;
+    uint32_t buf = 0;
+    for (uint32_t i = blockIdx.x * kP01mGroups; i < ngroups; i += stride) {
+        const int after = slot + 1 == kP01mStages ? 0 : slot + 1;
+        cp_async_wait<kP01mStages - 3>();
+        __syncthreads();  // this step's bytes and the next step's data are there, the last one is done with
+        stage(slot == 0 ? kP01mStages - 1 : slot - 1);
+        build(i + stride, after, buf ^ 1);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint4 v = ring[slot * kSlot + ((4 * h + c) * 4 + e) * 16 + ((8 * cg + row8) ^ 2 * c)];
+            uint32_t a[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                const uint32_t x = comp(v, 2 * m), y = comp(v, 2 * m + 1);
+                a[m][0] = half2_bytes(x, 0x4140);
+                a[m][1] = half2_bytes(y, 0x4140);
+                a[m][2] = half2_bytes(x, 0x4342);
+                a[m][3] = half2_bytes(y, 0x4342);
+            }
+#pragma unroll
+            for (int t = 0; t < T; t++) {
+                const uint2 b = bytes[(buf * 2 + h) * kSub + ko[t]];
+                mma16816(s[0][t], a[0], b.x, b.y);
+                mma16816(s[1][t], a[1], b.x, b.y);
+            }
+        }
+        since += kP01mGroups;
+        if (since == 64) {
+            since = 0;
+            convert((++reduced & 63) == 0);
+        }
+        slot = after;
+        buf ^= 1;
+    }
+    cp_async_wait<0>();
+    convert(true);
+    __syncthreads();  // the ring takes every (e, unit, copy)'s total
+    uint32_t* const part = reinterpret_cast<uint32_t*>(ring);
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int t = 0; t < T; t++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t* p = sums + 256 * ((m * T + t) * 4 + 2 * h), sh = 16 * (c & 1);
+                uint32_t x = add(rot31(p[0], sh), rot31(p[256], sh + 8));
+                x = add(x, __shfl_xor_sync(0xffffffffu, x, 1));
+                if (!(c & 1)) part[(e * U + 2 * t + (c >> 1)) * kP01mCopies + 32 * cg + 4 * row8 + 2 * m + h] = x;
+            }
+    __syncthreads();
+    // the nine sums: coefficients (row e, place f) whose totals they add
+    constexpr uint16_t kAdds[kP01Sums] = {0x0001, 0x0010, 0x0033, 0x0100, 0x1000, 0x3300, 0x0404, 0x4040, 0xcccc};
+    for (uint32_t o = tid; o < kP01Sums * R * kP01mCopies; o += 256) {
+        const uint32_t q = o & (kP01mCopies - 1), kj = o / kP01mCopies, k = kj / R, j = kj - k * R;
+        uint32_t adds = 0;
+#pragma unroll
+        for (int i = 0; i < kP01Sums; i++)
+            if (i == (int)k) adds = kAdds[i];
+        unsigned long long total = 0;
+        for (uint32_t i = 0; i < 16; i++)
+            if (adds >> i & 1) total += part[((i >> 2) * U + (i & 3) * R + j) * kP01mCopies + q];
+        if (copy0 + q < N) atomicAdd(&red.acc[(size_t)(kP01Sums * j + k) * N + copy0 + q], total);
+    }
+    P01Fin fin{red, evals_out, vx, sums_out, N, (uint32_t)R};
+    finish_group(red, copy0, kP01mCopies, N, fin);
+}
+
 // CTAs of 256 threads for n threads of a kernel that builds digit tables: one wave at most, a
 // CTA more costs another build.
 uint32_t grid_eq(uint64_t n) {
@@ -2387,7 +2567,14 @@ static uint32_t one_copy_slice(uint32_t N) {
     return best_used * 2 >= 65536 ? best : 0;
 }
 
+// Groups of copies of k_p2_round01_mma; 0 where more than an eighth of a CTA's would be past the end.
+static uint32_t p01m_groups(uint32_t N) {
+    const uint32_t ny = (N + kP01mCopies - 1) / kP01mCopies;
+    return (uint64_t)N * 8 >= (uint64_t)ny * kP01mCopies * 7 && ny <= 1024 ? ny : 0;
+}
+
 uint32_t p2_round01_groups(uint32_t N) {
+    if (const uint32_t ny = p01m_groups(N)) return ny;
     const uint32_t L = one_copy_slice(N);
     return L ? (N + L - 1) / L : 0;
 }
@@ -2397,6 +2584,26 @@ cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const
                               RedScratch red, uint32_t* evals_out, uint32_t* sums_out, cudaStream_t st) {
     if (reps < 1 || reps > 3 || p2_round01_groups(N) == 0) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(v) & 15) != 0) return cudaErrorInvalidValue;  // 16-byte cp.async
+    P01Src src;
+    src.v = v;
+    for (int j = 0; j < 3; j++) {
+        src.s[j] = j < reps ? s[j] : nullptr;
+        src.t[j] = j < reps ? t[j] : nullptr;
+    }
+    if (const uint32_t ny = p01m_groups(N)) {
+        const uint64_t nsteps = (ngroups + kP01mGroups - 1) / kP01mGroups, cap2 = ctas / 2 / ny ? ctas / 2 / ny : 1;
+        const dim3 gm((uint32_t)(nsteps < 1 ? 1 : nsteps < cap2 ? nsteps : cap2), ny);
+#define GKR_P01M(RR) \
+    k_p2_round01_mma<RR><<<gm, 256, ring_smem<k_p2_round01_mma<RR>>(p01m_smem<RR>()), st>>>(src, (uint32_t)ngroups, quads, vx, N, red, \
+                                                                                           evals_out, sums_out)
+        switch (reps) {
+            case 1: GKR_P01M(1); break;
+            case 2: GKR_P01M(2); break;
+            default: GKR_P01M(3); break;
+        }
+#undef GKR_P01M
+        return cudaGetLastError();
+    }
     Geo g;
     g.N = N;
     g.tpr = one_copy_slice(N);
@@ -2408,12 +2615,6 @@ cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const
     const dim3 grid((uint32_t)(need < cap ? need : cap), groups, 1);
     const size_t ring = (size_t)kP01Stages * 8 * kP01WarpSlot, red_b = (size_t)3 * kP01Sums * 4 * 256;
     const size_t smem = ring > red_b ? ring : red_b;
-    P01Src src;
-    src.v = v;
-    for (int j = 0; j < 3; j++) {
-        src.s[j] = j < reps ? s[j] : nullptr;
-        src.t[j] = j < reps ? t[j] : nullptr;
-    }
     switch (reps) {
         case 1: k_p2_round01<1><<<grid, 256, smem, st>>>(src, ngroups, quads, vx, g, red, evals_out, sums_out); break;
         case 2: k_p2_round01<2><<<grid, 256, smem, st>>>(src, ngroups, quads, vx, g, red, evals_out, sums_out); break;

@@ -117,3 +117,24 @@ def test_bn254_sums_of_many_products(ctx, widths, n):
     cv, proof = ctx.prove(ctx.load(circ, "BN254"), w)
     ocv, op = OracleBn254().prove(circ, w)
     assert proof == op and np.array_equal(cv, ocv)
+
+
+@pytest.mark.parametrize("seed,widths,n,p_mul,ctas", [
+    # no mul gates at all; a step and a part of one; a row's copies and the last 64 partly past the end
+    (661, [9, 8], 64, 0.0, 0), (662, [3, 4, 5], 128, 1.0, 0), (663, [13, 12], 60, 0.6, 0), (664, [10, 11], 452, 0.4, 0),
+    # one CTA for all groups: sums that are reduced between conversions, of the largest inputs
+    (665, [15, 16], 64, 1.0, 1),
+])
+def test_first_rounds_of_phase_two(oracle, seed, widths, n, p_mul, ctas):
+    from gkr_gb300.prover import Context
+    ctx = Context(0)
+    circ = gc.random_circuit(seed, widths, p_mul=p_mul)
+    w = gc.random_witness(seed, circ.log_input_size, n)
+    if ctas:
+        w[...] = gc.P - 1
+    ctx.set_round_tail(False)
+    ctx.set_tile(ctas=ctas)
+    cv, proof = ctx.prove(ctx.load(circ), w)
+    ocv, op = oracle.prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
+    ctx.close()
