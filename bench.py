@@ -375,9 +375,9 @@ def kernel_table(stats, n_steps, traffic_ratios):
     return out
 
 
-# Kinds whose event time is not their own work: a phase tail's launch spans the host round
-# trips of its rounds (it waits for each challenge on the device).
-NOT_BANDWIDTH = {"round_tail"}
+# Kinds whose event time is not their own work: a persistent phase's launch spans the host
+# round trips of its rounds (it waits for each challenge on the device).
+NOT_BANDWIDTH = {"round_tail", "bn254_phase"}
 
 
 def roofline_of(stats, traffic_ratios):

@@ -13,11 +13,15 @@
 //   k_hg_round0      _prepare_g_x_vals + poly_eval_at(0)        sumcheck_helper.hpp:172-231, 68-102
 //   k_hg_round1      hg rebuilt + receive_challenge + poly_eval_at(1)
 //   k_round          receive_challenge + poly_eval_at(k)        sumcheck_helper.hpp:104-133, 68-102
+//   k_round_pair     two rounds from one pass over large tables (the second's sums are quadratic
+//                    in the first's challenge); k_pair_fin finishes the second
 //   k_s_build        _prepare_h_y_vals (copy-independent part)  sumcheck_helper.hpp:233-261
 //   k_p2_round01     phase-two poly_eval_at of rounds 0 and 1 from one pass (round 1's sums are
-//                    quadratic in round 0's challenge); k_p2_round1_fin finishes round 1
+//                    quadratic in round 0's challenge), k_p2_round01_mma the same on the tensor
+//                    cores; k_p2_round1_fin finishes round 1
 //   k_p2_round2      phase-two round 2 refolding the layer input
-//   k_wsum           eval_multilinear                           include/poly_commit/poly.hpp:88-104
+//   k_wsum, k_wsum_mma  eval_multilinear                        include/poly_commit/poly.hpp:88-104
+// (Phases on small tables: phase.cu.)
 //
 // k_round gives each CTA one repetition j = blockIdx.x % R: the R CTAs of a row chunk are
 // adjacent in launch order, run together and share their common source rows through L2,
@@ -2318,8 +2322,6 @@ static RoundPtrs with_weights(const RoundPtrs& p, int reps, bool both, bool r1 =
     return q;
 }
 
-// Dynamic shared memory of the staged kernels: the cp.async ring, or the reduction's
-// scratch where that is larger (they share the allocation).
 // Dynamic shared memory of k_hg_round0: the cp.async ring, or the reduction's scratch where
 // that is larger (they share the allocation).  Above 48 KiB less the kernel's static shared
 // memory a launch needs the opt-in, which is set once per device and instantiation to the

@@ -234,10 +234,10 @@ cudaError_t launch_round(int reps, bool shared_src, bool lane_hg, bool fold, con
 // Phase-two rounds 0 and 1 in one pass over the layer input v (4 ngroups rows, ngroups >= 2):
 // round 0's evaluations (times vx) are published to evals_out as by the round kernels, and
 // 9 * reps canonical sums per copy go to sums_out (9 reps x N) for launch_p2_round1_fin.
-// s[j] are the scalar tables (16-byte aligned), t[j] their pair sums (launch_s_build4);
+// s[j] are the scalar tables (16-byte aligned), t[j] their pair sums (launch_s_build);
 // red.acc needs 9 * reps x N accumulators.  Publishes p2_round01_groups(N) lane groups;
-// p2_round01_groups(N) is 0 where the kernel does not apply (too many of the threads of its
-// 32-copy warps would be idle).
+// p2_round01_groups(N) is 0 where neither kernel applies (too many of the threads of 32-copy
+// warps would be idle).
 // Groups i < ngroups are rows 4q .. 4q+3 with q = quads[i] (q = i without a list); a list
 // may leave out only groups with no mul gate whose second input is in them (s_j zero there).
 cudaError_t launch_p2_round01(int reps, const uint32_t* v, const uint32_t* const* s, const uint32_t* const* t,

@@ -173,7 +173,7 @@ void gkrgpu_sha3_256(const uint8_t* in, uint64_t len, uint8_t* out);
 /* Verifier::verify (include/LinearGKR/LinearGKR.hpp:105-149: gkr_verify, gkr.hpp:75-122, and
  * RawPC::verify, raw.hpp:75-78), GPU-assisted, for M31 and BN254 circuits: the host replays the
  * transcript and checks every round; the device computes each layer's
- * eval_sparse_circuit_connect_poly (eq tables and gate sums,
+ * eval_sparse_circuit_connect_poly (gate sums weighted by eq factors,
  * sumcheck_verifier_utils.hpp:22-56) and the multilinear evaluations of the committed input
  * (the proof's first 2^nb_input_vars(0) rows).  claimed_v: R rows of n_copies lanes.
  * *accepted is 1 when the reference verifier would accept, else 0 (the status is
@@ -234,8 +234,7 @@ int gkrgpu_prove_submit_resident(gkrgpu_ctx* ctx, const gkrgpu_circuit* circuit,
  * canonical values, out (host) receives n_points rows of n_copies lanes, row j being
  * sum_z eq(r_j, z) * evals[z].  This is RawPC::verify's check value
  * (include/poly_commit/raw.hpp:75-78) and gkr_prove's output claim
- * (include/LinearGKR/gkr.hpp:52-55).  The eq tables and the reduction scratch live in
- * the context's workspace. */
+ * (include/LinearGKR/gkr.hpp:52-55).  The reduction scratch is a lane's, kept between calls. */
 int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t nb_vars, uint32_t n_copies,
                             const uint32_t* r, int n_points, uint32_t* out);
 
@@ -258,8 +257,8 @@ int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t nb_vars, u
                                     const uint32_t* r, int n_points, uint32_t* d_out, void* stream);
 
 /* Persistent phases.  When the tables of a phase's last rounds (of all its rounds, for a small
- * layer) are small, those rounds run in one launch (k_phase) that waits on the device for each round's challenges, which
- * the host writes into host-mapped memory after hashing the round's evaluations, instead of
+ * layer) are small, those rounds run in one launch (k_phase) that waits on the device for each
+ * round's challenges, which the host writes into host-mapped memory after hashing the round's evaluations, instead of
  * one kernel launch per round.  On by default; gkrgpu_set_round_tail(ctx, 0) runs every
  * round as its own launch (the proof bytes are the same).  A context created under a CUDA
  * injection tool (CUDA_INJECTION64_PATH set, as profilers do) starts with them off:
