@@ -261,7 +261,7 @@ int gkrgpu_eval_multilinear_noalloc(const uint32_t* d_evals, uint32_t nb_vars, u
  * round's challenges, which the host writes into host-mapped memory after hashing the round's evaluations, instead of
  * one kernel launch per round.  On by default; gkrgpu_set_round_tail(ctx, 0) runs every
  * round as its own launch (the proof bytes are the same).  A context created under a CUDA
- * injection tool (CUDA_INJECTION64_PATH set, as profilers do) starts with them off:
+ * injection tool (CUDA_INJECTION64_PATH or Nsight Compute's variables set) starts with them off:
  * such tools may run each kernel to completion before the launching thread goes on, and a
  * phase waits for that thread.  No counterpart in the reference, whose sumcheck runs on the
  * CPU (sumcheck.hpp:72-97). */

@@ -138,3 +138,17 @@ def test_first_rounds_of_phase_two(oracle, seed, widths, n, p_mul, ctas):
     ocv, op = oracle.prove(circ, w)
     assert proof == op and np.array_equal(cv, ocv)
     ctx.close()
+
+
+@pytest.mark.parametrize("name", ["NV_COMPUTE_PROFILER_PERFWORKS_DIR", "NV_NSIGHT_INJECTION_PORT_BASE"])
+def test_no_persistent_phase_under_a_profiler(monkeypatch, ctx, name):
+    # a profiler may block the launching thread until a kernel ends; a phase waits for that thread
+    from gkr_gb300.prover import Context
+    monkeypatch.setenv(name, "1")
+    profiled = Context(0)
+    circ = gc.random_circuit(671, [7, 8])
+    w = gc.random_witness(671, circ.log_input_size, 16)
+    cv, proof = profiled.prove(profiled.load(circ), w)
+    assert profiled.kernel_stats()["round_tail"]["launches"] == 0
+    profiled.close()
+    assert proof == ctx.prove(ctx.load(circ), w)[1]
