@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
         const uint32_t* ssrc = k <= kf ? s0t : (odd ? sbuf + j * S1 : sbuf + 3 * S1 + j * (S1 / 2));
         uint32_t* sdst = odd ? sbuf + 3 * S1 + j * (S1 / 2) : sbuf + j * S1;
         uint32_t ns;  // partial sums per copy and repetition
+        bool across;  // a finisher reads what another warp wrote (the same for the whole CTA)
         if (k > kf && in_smem(k - 1)) {
             // one copy a thread: pair idx / L, copy idx % L; at most two pairs a thread
             const uint32_t* fs = reinterpret_cast<const uint32_t*>(table(k - 1, 0));
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
             // threads of one copy: within a warp when a pair's copies fit in one
             const uint32_t used = items < kRepThreads ? items : kRepThreads;
             ns = L <= 32 ? (used + 31) / 32 : (used + L - 1) / L;
+            across = ns > 1;  // (one sum: the finisher's own, or its warp's)
             if (32 * w < used) {
                 uint32_t x[3];
 #pragma unroll
@@ -317,6 +319,7 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
             // the warps that had pairs
             const uint32_t used = npairs * tpr < kRepThreads ? npairs * tpr : kRepThreads;
             ns = (used + 31) / 32;
+            across = ns > 1 || L > 32;  // warp 0 has the sums and rows of all the CTA's copies
             if (w < ns) {
                 uint32_t x[12];
 #pragma unroll
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
                         for (int l = 0; l < 4; l++) part[((j * kWarps + w) * 3 + e) * L + 4 * q + l] = x[4 * e + l];
             }
         }
-        if (ns > 1) __syncthreads();  // (one warp's own sums and rows need no more than __syncwarp)
+        if (across) __syncthreads();
         else __syncwarp();
         if (finisher) {
             uint32_t p0 = 0, p1 = 0, p2 = 0;

@@ -152,3 +152,25 @@ def test_no_persistent_phase_under_a_profiler(monkeypatch, ctx, name):
     assert profiled.kernel_stats()["round_tail"]["launches"] == 0
     profiled.close()
     assert proof == ctx.prove(ctx.load(circ), w)[1]
+
+
+@pytest.mark.parametrize("seed,widths,n", [
+    # 16 quads a CTA (4100 and 8192 copies) and 32 (8196 and 16384) on tables of 2 to 8 rows, and
+    # on the last rounds of a layer that starts its phase at round 4
+    (681, [1, 2, 3, 3, 2, 1, 0], 4100), (682, [1, 2, 3, 3, 2, 1, 0], 8192), (683, [1, 2, 3, 3, 2, 1, 0], 8196),
+    (684, [1, 2, 3, 3, 2, 1, 0], 16384), (685, [10, 3, 1], 4100), (686, [10, 3, 1], 16384),
+])
+def test_phases_whose_finishers_are_in_several_warps(ctx, oracle, seed, widths, n):
+    # with more than 8 quads a CTA its copies' sums are all warp 0's on small tables, and are read
+    # by two or four warps
+    circ = gc.random_circuit(seed, widths, p_mul=0.6)
+    w = gc.random_witness(seed, circ.log_input_size, n)
+    dc = ctx.load(circ)
+    cv, proof = ctx.prove(dc, w)
+    try:
+        ctx.set_round_tail(False)
+        assert ctx.prove(dc, w)[1] == proof
+    finally:
+        ctx.set_round_tail(True)
+    ocv, op = oracle.prove(circ, w)
+    assert proof == op and np.array_equal(cv, ocv)
