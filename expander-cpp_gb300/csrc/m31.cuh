@@ -86,10 +86,11 @@ GKR_HD uint32_t lerp(uint32_t a, uint32_t b, const Lerp& c) {
 }
 
 // Two folds in one, at challenges r0 and then r1, as a weighted sum of four rows with weights
-// (1 - r0)(1 - r1), r0 (1 - r1), (1 - r0) r1, r0 r1 (canonical).  t = sum x_e c_e <= 4 (p - 1)^2 =
-// 2^64 - 2^35 + 16; with t = 2^32 hi + lo == lo + 2 hi, the low and high parts are brought below
-// 2^31 + 1 and 2^31 - 15 first, so their sum stays below 2p.  Four wide multiply-adds where three
-// lerps take six.
+// (1 - r0)(1 - r1), r0 (1 - r1), (1 - r0) r1, r0 r1 (canonical).  t = sum x_e c_e <= 4 (p - 1)^2 <
+// 2^64; its bits 0..30, 31..61 and 62..63 weigh 1, 2^31 == 1 and 2^62 == 1 (mod p).  The upper two
+// parts are at most p and 3, so one conditional subtraction brings their sum below p, and a
+// second one the total of it and the lowest part, at most 2p - 1.  (The total of all three
+// reaches 2p + 2.)  Four wide multiply-adds where three lerps take six.
 struct Lerp2 {
     uint32_t c[4];
 };
@@ -104,8 +105,8 @@ GKR_HD Lerp2 lerp2_at(uint32_t r0, uint32_t r1) {
 }
 GKR_HD uint32_t lerp2(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, const Lerp2& w) {
     const uint64_t t = (uint64_t)x0 * w.c[0] + (uint64_t)x1 * w.c[1] + (uint64_t)x2 * w.c[2] + (uint64_t)x3 * w.c[3];
-    const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
-    const uint32_t s = ((lo & P) + (lo >> 31)) + (((hi << 1) & P) + (hi >> 30));
+    const uint32_t u = ((uint32_t)(t >> 31) & P) + (uint32_t)(t >> 62);
+    const uint32_t s = ((uint32_t)t & P) + umin(u, u - P);
     return umin(s, s - P);
 }
 
