@@ -109,25 +109,29 @@ struct Verifier {
         c.launch(K_CANONICAL, 8.0 * C.in_rows(0) * N, [&] { return launch_canonicalize(com, C.in_rows(0) * N, c.stream); });
 
         // transcript: the commitment bytes (hashed in place), grinding
-        std::unique_ptr<uint8_t[]> tbuf(new uint8_t[len + 64 + 9 * rowb]);
-        Transcript t(tbuf.get(), len + 64, X.fs_hash);
+        std::unique_ptr<uint8_t[]> tbuf(new uint8_t[len]);  // each row at its own place in the proof
+        Transcript t(tbuf.get(), len, X.fs_hash);
         uint8_t d[32];
         fs_hash(X.fs_hash, proof, com_bytes, d);
         t.appended_prehashed(com_bytes, d);
         grind(t, grinding_bits);
         uint64_t pos = com_bytes + 32;
-        bool bad = false;
-        // Proof::get_next_and_step of one row (N lanes), reduced, to the transcript's tail + at
+        // Proof::get_next_and_step of one row (N lanes), reduced, to the transcript's tail + at;
+        // false, with nothing written, when the proof has run out
         auto next_row = [&](uint64_t at) {
+            if (len - pos < rowb) return false;
             uint32_t* out = reinterpret_cast<uint32_t*>(t.tail() + at);
-            if (pos + rowb > len) {
-                bad = true;
-                memset(out, 0, rowb);
-                return;
-            }
             memcpy(out, proof + pos, rowb);
             for (uint32_t k = 0; k < N; k++) out[k] = m31::from_u32(out[k]);
             pos += rowb;
+            return true;
+        };
+        // The rejection of a proof that has run out, made at once: what was launched is waited for,
+        // since it reads the proof and writes the lane's mapped area.
+        auto ran_out = [&] {
+            c.sync();
+            c.resolve_events();
+            return false;
         };
 
         const size_t L = C.layers.size();
@@ -144,7 +148,7 @@ struct Verifier {
         std::vector<Pending> pending(L);
         bool ok = true;
 
-        for (int li = (int)L - 1; li >= 0 && !bad; li--) {
+        for (int li = (int)L - 1; li >= 0; li--) {
             const uint32_t n = C.layers[li].nin;
             Pending& pd = pending[li];
             pd.first.resize(RN);
@@ -157,14 +161,16 @@ struct Verifier {
                 uint32_t rs[3];
                 const uint8_t* ev0 = t.tail();
                 if (!vx_round) {
-                    for (int q = 0; q < 3 * R; q++) next_row(q * rowb);
+                    for (int q = 0; q < 3 * R; q++)
+                        if (!next_row(q * rowb)) return ran_out();
                     t.challenge_each(3 * rowb, R, rs);
                 } else {
                     for (int j = 0; j < R; j++) {
-                        for (int q = 0; q < 3; q++) next_row(q * rowb);
+                        for (int q = 0; q < 3; q++)
+                            if (!next_row(q * rowb)) return ran_out();
                         t.appended(3 * rowb);
                         rs[j] = t.challenge();
-                        next_row(0);
+                        if (!next_row(0)) return ran_out();
                         memcpy(pd.vx.data() + (size_t)j * N, t.tail(), rowb);
                         t.appended(rowb);
                     }
@@ -186,7 +192,7 @@ struct Verifier {
                 if (vx_round) gate_sums((size_t)li, false, rz1, rz2, alpha, beta, rx, ry);
             }
             for (int j = 0; j < R; j++) {
-                next_row(0);
+                if (!next_row(0)) return ran_out();
                 memcpy(pd.vy.data() + (size_t)j * N, t.tail(), rowb);
                 t.appended(rowb);
             }
@@ -202,13 +208,11 @@ struct Verifier {
             cv2 = pd.vy;
         }
         // RawPC::verify against the commitment, at rz1_j and rz2_j
-        if (!bad) {
-            raw_pc_eval(rz1, 0);
-            raw_pc_eval(rz2, 1);
-        }
+        raw_pc_eval(rz1, 0);
+        raw_pc_eval(rz2, 1);
         c.sync();
         std::atomic_thread_fence(std::memory_order_acquire);
-        for (size_t li = 0; li < L && ok && !bad; li++) {
+        for (size_t li = 0; li < L && ok; li++) {
             const uint32_t *a = mapped(false, sums_word(li, false)), *m = mapped(false, sums_word(li, true));
             const Pending& pd = pending[li];
             for (size_t i = 0; i < RN; i++) {
@@ -218,9 +222,9 @@ struct Verifier {
             }
         }
         const uint32_t* ev = mapped(false, claims_word());
-        if (ok && !bad) ok = memcmp(ev, cv1.data(), RN * 4) == 0 && memcmp(ev + 3ull * N, cv2.data(), RN * 4) == 0;
+        if (ok) ok = memcmp(ev, cv1.data(), RN * 4) == 0 && memcmp(ev + 3ull * N, cv2.data(), RN * 4) == 0;
         c.resolve_events();
-        return ok && !bad;
+        return ok;
     }
 };
 
@@ -308,23 +312,25 @@ struct BnVerifier {
         c.launch(K_BN_LOAD, 64.0 * C.in_rows(0) * N,
                  [&] { return bn::launch_load(raw, com, C.in_rows(0) * N, nullptr, c.stream); });
 
-        std::unique_ptr<uint8_t[]> tbuf(new uint8_t[len + 64]);
-        Transcript t(tbuf.get(), len + 64, X.fs_hash);
+        std::unique_ptr<uint8_t[]> tbuf(new uint8_t[len]);  // each row at its own place in the proof
+        Transcript t(tbuf.get(), len, X.fs_hash);
         uint8_t d[32];
         fs_hash(X.fs_hash, proof, com_bytes, d);
         t.appended_prehashed(com_bytes, d);
         grind_bn254(t, grinding_bits);
         uint64_t pos = com_bytes + 32;
-        bool bad = false;
-        // one row of N canonical elements (from_bytes reduces each 32-byte word)
+        // one row of N canonical elements (from_bytes reduces each 32-byte word); false when the
+        // proof has run out, which is rejected at once, as above
         auto next_row = [&](uint32_t* out) {
-            if (pos + rowb > len) {
-                bad = true;
-                memset(out, 0, rowb);
-                return;
-            }
+            if (len - pos < rowb) return false;
             for (uint32_t k = 0; k < N; k++) frh::store(frh::from_bytes(proof + pos + 32ull * k), out + 8ull * k);
             pos += rowb;
+            return true;
+        };
+        auto ran_out = [&] {
+            c.sync();
+            c.resolve_events();
+            return false;
         };
         auto el = [](const std::vector<uint32_t>& v, uint64_t row, uint32_t N_, uint32_t k) {
             return frh::load(v.data() + (row * N_ + k) * 8);
@@ -351,9 +357,8 @@ struct BnVerifier {
             for (uint32_t k = 0; k < N; k++)
                 sum[k] = frh::add(frh::mul(el(cv1, 0, N, k), alpha), frh::mul(el(cv2, 0, N, k), beta));
             for (uint32_t i_var = 0; i_var < 2 * n; i_var++) {
-                next_row(ev.data());
-                next_row(ev.data() + rowl);
-                next_row(ev.data() + 2 * rowl);
+                for (int q = 0; q < 3; q++)
+                    if (!next_row(ev.data() + q * rowl)) return ran_out();
                 t.append(ev.data(), 3 * rowb);
                 const frh::Fr r = t.challenge_bn254();
                 (i_var < n ? rx[i_var] : ry[i_var - n]) = r;
@@ -366,13 +371,13 @@ struct BnVerifier {
                     sum[k] = frh::add(c0, frh::mul(frh::add(frh::mul(c2, r), c1), r));
                 }
                 if (i_var == n - 1) {
-                    next_row(vx.data());
+                    if (!next_row(vx.data())) return ran_out();
                     t.append(vx.data(), rowb);
                     const frh::Fr a = gate_sums((size_t)li, false, rz1, have_rz2 ? rz2 : nullptr, alpha, beta, rx, ry);
                     for (uint32_t k = 0; k < N; k++) sum[k] = frh::sub(sum[k], frh::mul(el(vx, 0, N, k), a));
                 }
             }
-            next_row(vy.data());
+            if (!next_row(vy.data())) return ran_out();
             t.append(vy.data(), rowb);
             const frh::Fr m = gate_sums((size_t)li, true, rz1, have_rz2 ? rz2 : nullptr, alpha, beta, rx, ry);
             for (uint32_t k = 0; k < N; k++)
@@ -390,6 +395,6 @@ struct BnVerifier {
         if (!raw_pc_verify(rz1, cv1)) ok = false;
         if (!raw_pc_verify(rz2, cv2)) ok = false;
         c.resolve_events();
-        return ok && !bad;
+        return ok;
     }
 };
