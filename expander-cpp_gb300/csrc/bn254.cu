@@ -1439,22 +1439,45 @@ cudaError_t launch_round(bool lane_hg, bool fold_, const RoundPtrsBn& p, uint64_
     return cudaGetLastError();
 }
 
+// Shared memory of a launch whose first folding round leaves S1 rows.
+static size_t phase_smem(bool lane_hg, uint32_t S1) {
+    return sizeof(Fr) * (2 * (lane_hg ? 2 : 1) * (size_t)kSmemRowsBn + (lane_hg ? 0 : S1 + S1 / 2));
+}
+
+int phase_ctas_per_sm() {
+    static std::atomic<int> known[64];  // of each device, plus one
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<int>& k = known[dev & 63];
+    if (const int v = k.load(std::memory_order_relaxed)) return v - 1;
+    int least = 0;
+    for (int lane_hg = 0; lane_hg < 2; lane_hg++) {
+        auto* const kernel = lane_hg ? k_phase<true> : k_phase<false>;
+        const size_t most = phase_smem(lane_hg != 0, kPhaseRows / 2);
+        int n = 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kPhaseBlock, most);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        if (lane_hg == 0 || n < least) least = n;
+    }
+    k.store(least + 1, std::memory_order_relaxed);
+    return least;
+}
+
 cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s) {
     if (a.k0 >= a.n || a.n - a.k0 > kMboxRounds || a.N < 1) return cudaErrorInvalidValue;
     // rows of the first round's source tables; with k0 = 0 the layer input itself
     if ((1ull << (a.n - (a.k0 ? a.k0 - 1 : 0))) > kPhaseRows) return cudaErrorInvalidValue;
     if (a.k0 == 0 && (!a.v || (lane_hg && (!a.h0 || !a.mx_off || !a.a || !a.w)))) return cudaErrorInvalidValue;
     if (!lane_hg && (!a.vx || !a.s)) return cudaErrorInvalidValue;
-    static std::atomic<uint64_t> opted{0};  // one bit per device: shared memory above 48 KiB
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(opted.load(std::memory_order_relaxed) & bit)) {
-        cudaFuncSetAttribute(k_phase<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-        opted.fetch_or(bit);
-    }
+    if (phase_ctas_per_sm() < 1) return cudaErrorInvalidConfiguration;
     const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
-    const size_t smem = sizeof(Fr) * (2 * (lane_hg ? 2 : 1) * (size_t)kSmemRowsBn + (lane_hg ? 0 : S1 + S1 / 2));
+    const size_t smem = phase_smem(lane_hg, S1);
     if (lane_hg)
         k_phase<true><<<a.N, kPhaseBlock, smem, s>>>(a);
     else

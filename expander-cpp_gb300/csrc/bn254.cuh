@@ -116,6 +116,7 @@ struct PhaseArgsBn {
     unsigned long long wait_ns;
 };
 cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s);
+int phase_ctas_per_sm();  // as the M31 kernels' (kernels.cuh)
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgsBn& eq, const GeoBn& g, uint32_t ctas, RedBn red,
                         uint32_t* out, cudaStream_t s);
 

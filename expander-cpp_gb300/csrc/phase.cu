@@ -374,6 +374,43 @@ __global__ void __launch_bounds__(3 * kRepThreads, 2) k_phase(PhaseArgs a) {
 
 uint32_t phase_ctas(uint32_t N, uint32_t tpr) { return (N / 4 + tpr - 1) / tpr; }
 
+// Shared memory of a launch whose first folding round leaves S1 rows.
+static size_t phase_smem(bool lane_hg, uint32_t S1, uint32_t reps, uint32_t tpr) {
+    return 2 * (lane_hg ? 6 : 3) * (size_t)kSmemRows * 16 + (lane_hg ? 0 : 4 * 3 * (size_t)(S1 + S1 / 2)) +
+           4 * (size_t)reps * kWarps * 3 * 4 * tpr;
+}
+
+int phase_ctas_per_sm() {
+    static std::atomic<int> known[64];  // of each device, plus one
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<int>& k = known[dev & 63];
+    if (const int v = k.load(std::memory_order_relaxed)) return v - 1;
+    int least = 0;
+    for (int i = 0; i < 4; i++) {
+        const bool lane_hg = i < 2;
+        auto* const kernel = lane_hg ? (i & 1 ? k_phase<true, true> : k_phase<true, false>)
+                                     : (i & 1 ? k_phase<false, true> : k_phase<false, false>);
+        size_t most = 0;  // over the tiles that launch_phase takes
+        for (uint32_t tpr = 1; tpr <= 32; tpr *= 2) {
+            const size_t b = phase_smem(lane_hg, kPhaseItems / 2 / tpr, 3, tpr);
+            if (b > most) most = b;
+        }
+        int n = 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 3 * kRepThreads, most);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        if (i == 0 || n < least) least = n;
+    }
+    k.store(least + 1, std::memory_order_relaxed);
+    return least;
+}
+
 size_t phase_priv_quads(uint64_t items) { return items * 4 + items / 2 * 6 + items / 4 * 6; }
 
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
@@ -385,18 +422,9 @@ cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
     if (a.two && a.k0 < 2) return cudaErrorInvalidValue;
     if (a.k0 && (!a.fsrc[0] || (lane_hg && !a.hsrc[0]))) return cudaErrorInvalidValue;
     if (!lane_hg && (!a.vx || !a.s[0])) return cudaErrorInvalidValue;
-    static std::atomic<uint64_t> opted{0};  // one bit per device: shared memory above 48 KiB
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(opted.load(std::memory_order_relaxed) & bit)) {
-        for (auto* k : {k_phase<true, false>, k_phase<true, true>, k_phase<false, false>, k_phase<false, true>})
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-        opted.fetch_or(bit);
-    }
+    if (phase_ctas_per_sm() < 1) return cudaErrorInvalidConfiguration;
     const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
-    const size_t smem = 2 * (lane_hg ? 6 : 3) * (size_t)kSmemRows * 16 + (lane_hg ? 0 : 4 * 3 * (size_t)(S1 + S1 / 2)) +
-                        4 * (size_t)a.reps * kWarps * 3 * 4 * a.tpr;
+    const size_t smem = phase_smem(lane_hg, S1, a.reps, a.tpr);
     const dim3 grid(phase_ctas(a.N, a.tpr)), block(a.reps * kRepThreads);
     auto* const kernel = lane_hg ? (a.two ? k_phase<true, true> : k_phase<true, false>)
                                  : (a.two ? k_phase<false, true> : k_phase<false, false>);

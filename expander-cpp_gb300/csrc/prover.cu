@@ -944,13 +944,16 @@ EqArgs eq_args(int reps, const uint32_t (*r1)[32], const uint32_t (*r2)[32], uin
 // ------------------------------------------------------------------ persistent phase slots
 // The CTAs of a persistent phase wait for their host thread, which waits for all of them, so
 // all must be resident at once: a phase runs only while the CTAs of all running ones (every
-// context and lane of the process) stay within what the device holds, two to an SM (their
-// threads, registers and shared memory take at most half of one), and otherwise the rounds
-// are launched one by one.  Other kernels only delay a phase: they end by themselves.
+// context and lane of the process) stay within what the device holds of the largest of them
+// (phase_ctas_per_sm: two to an SM, so that each takes at most half of one), and otherwise the
+// rounds are launched one by one.  Other kernels only delay a phase: they end by themselves.
 class PhaseSlots {
    public:
-    PhaseSlots(int device, int sm_count) : used_(counter(device)), cap_(2 * sm_count) {}
+    // (`device` is the current one)
+    PhaseSlots(int device, int sm_count)
+        : used_(counter(device)), cap_(sm_count * std::min(phase_ctas_per_sm(), bn::phase_ctas_per_sm())) {}
     ~PhaseSlots() { used_ -= held_; }
+    int capacity() const { return cap_; }
     // n more CTAs; beyond a lane's own share of the device only while half of it stays free.
     bool acquire(int n, bool own_share) {
         if (used_.fetch_add(n) + n > (own_share ? cap_ : cap_ / 2)) {
@@ -1004,7 +1007,7 @@ struct Prover {
     // the device, or among small ones, takes more than its lane's share.
     uint32_t claim(PhaseSlots& slots, uint64_t rows, uint64_t items) const {
         if (!X.round_tail) return 0;
-        const uint32_t share = std::max(1u, 2u * (uint32_t)X.sm_count / (uint32_t)X.n_lanes);
+        const uint32_t share = std::max(1u, (uint32_t)slots.capacity() / (uint32_t)X.n_lanes);
         for (uint32_t tpr = 1; tpr <= 32 && rows * tpr <= items; tpr *= 2) {
             const uint32_t ctas = phase_ctas(N, tpr);
             if (ctas <= kPhaseCtas && slots.acquire((int)ctas, ctas <= share)) return tpr;
@@ -2303,6 +2306,9 @@ int gkrgpu_check_device_wait(gkrgpu_ctx* ctx, uint32_t timeout_us, int* expired,
         if (timeout_us < 1 || timeout_us > 10u * 1000 * 1000) fail(GKRGPU_ERR_INVALID, "timeout_us must be in [1, 10^7]");
         on_idle_lane(ctx, [&](Lane& c) {
             // a two-round phase over 8 x 4 tables whose second round's challenge is never written
+            PhaseSlots slots(ctx->device, ctx->sm_count);  // (other contexts' phases end by themselves)
+            if (slots.capacity() < 1) fail(GKRGPU_ERR_CUDA, "no persistent phase fits on the device");
+            while (!slots.acquire(1, true)) std::this_thread::sleep_for(std::chrono::microseconds(100));
             const uint32_t N = 4, n = 3;
             const size_t tb = 8 * N * 4, priv = phase_priv_quads(8);
             void* p = nullptr;

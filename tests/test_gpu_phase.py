@@ -3,6 +3,9 @@ exactly, just over and far over the rows a CTA takes, one-row-pair layers, copy 
 leave part of the last CTA idle (516 = 4 * 129 at two quads a CTA), that need wide CTAs (4096)
 and that are beyond the widest (20000, every round launched alone).  The proof bytes equal the
 oracle's and those with the phases off (exact arithmetic: tolerance zero)."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -174,3 +177,47 @@ def test_phases_whose_finishers_are_in_several_warps(ctx, oracle, seed, widths, 
         ctx.set_round_tail(True)
     ocv, op = oracle.prove(circ, w)
     assert proof == op and np.array_equal(cv, ocv)
+
+
+@pytest.fixture(scope="module")
+def side_by_side(tmp_path_factory):
+    from gkr_gb300 import build as libbuild
+    objs = [os.path.join(libbuild.OBJ, f + ".o") for f in ("phase.cu", "bn254.cu")]
+    libbuild.build(force=not all(os.path.exists(o) for o in objs))
+    exe = str(tmp_path_factory.mktemp("phases") / "phases_side_by_side")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "adapter", "phases_side_by_side.cu")
+    subprocess.check_call([libbuild.NVCC, *libbuild.ARCH, "-std=c++17", "-I", libbuild.CSRC, "-I", libbuild.INCLUDE, src,
+                           *objs, "-o", exe])
+    return exe
+
+
+@pytest.mark.parametrize("first,second", [
+    # M31 phase two with 25 and 99 KB a CTA, M31 phase one with 50, BN254 with 57 (phase two) and 16
+    ((0, 3), (0, 13)), ((0, 13), (0, 3)), ((0, 13), (1, 13)), ((1, 13), (0, 13)), ((0, 13), (0, 13)), ((2, 11), (0, 13)),
+    ((0, 13), (2, 11)), ((3, 11), (0, 13)), ((0, 3), (2, 11)),
+])
+def test_admitted_phases_are_resident_together(side_by_side, first, second):
+    # a phase's CTAs end only once all of them have started: those of two phases of one CTA an SM must
+    # start beside each other whatever memory each takes
+    out = subprocess.run([side_by_side, *[str(x) for x in first + second]], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0, out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("seed,widths,n", [(691, [3, 2, 3, 1, 2, 1], 512), (692, [7, 3, 2, 6], 512)])
+def test_wide_tiles_on_a_full_device(oracle, seed, widths, n):
+    # 64 lanes of phases that would take 128 CTAs each: the device's share of later ones is down to
+    # tiles of 8, 16 and 32 quads
+    from gkr_gb300.prover import Context
+    ctx = Context(0)
+    ctx.set_concurrency(64)
+    circ = gc.random_circuit(seed, widths, p_mul=0.6)
+    dc = ctx.load(circ)
+    witnesses = [gc.random_witness(seed + k, circ.log_input_size, n) for k in range(8)]
+    want = [oracle.prove(circ, w)[1] for w in witnesses]
+    jobs = []
+    for k in range(192):
+        pb, cb = np.empty(dc.proof_size(n), np.uint8), np.empty((3, n), np.uint32)
+        jobs.append((k % 8, ctx.submit(dc, witnesses[k % 8], pb, cb), pb))
+    wrong = [k for k, job, pb in jobs if pb[:ctx.wait(job)].tobytes() != want[k]]
+    ctx.close()
+    assert not wrong
