@@ -111,7 +111,7 @@ bool field_supported(int field) { return field == GKRGPU_FIELD_M31 || field == G
 // Bytes of one field element: M31 4, BN254 32.
 uint32_t elem_bytes(int field) { return field == GKRGPU_FIELD_BN254 ? 32u : 4u; }
 
-size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+constexpr size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Pinned host buffer that grows on demand.
 struct PinnedBuf {
@@ -230,7 +230,10 @@ struct gkrgpu_job {
 
 // ------------------------------------------------------------------ lanes
 // One device worker's state: its stream, pinned staging buffers, launch accounting.
-constexpr size_t kMinMapped = 2u << 20;  // mapped staging per lane: enough for 16384 copies of M31
+// Mapped staging of a lane at first, a quarter of it for the round evaluations: enough for
+// kMappedCopies copies of M31 (checked after Prover).
+constexpr size_t kMinMapped = 3u << 20;
+constexpr uint64_t kMappedCopies = 16384;
 struct Lane {
     gkrgpu_ctx* X = nullptr;
     cudaStream_t stream = nullptr;
@@ -1146,10 +1149,13 @@ struct Prover {
     volatile uint32_t* flag_h() const { return mapped(false, 12ull * N); }
     volatile uint32_t* err_h() const { return mapped(false, 12ull * N + 1); }
     // phase-one round 0's claims (R x N), after the mailbox
-    uint64_t mbox_word() const { return align_up(12ull * N + 64, 64); }
-    uint64_t claim_word() const { return mbox_word() + kMboxWords; }
-    uint64_t phase_word() const { return align_up(claim_word() + 3ull * N, 64); }
-    uint64_t mapped_words() const { return phase_word() + 15ull * N; }
+    static constexpr uint64_t mbox_at(uint64_t n) { return align_up(12 * n + 64, 64); }
+    static constexpr uint64_t claim_at(uint64_t n) { return mbox_at(n) + kMboxWords; }
+    static constexpr uint64_t phase_at(uint64_t n) { return align_up(claim_at(n) + 3 * n, 64); }
+    static constexpr uint64_t mapped_words(uint64_t n) { return phase_at(n) + 15 * n; }
+    uint64_t mbox_word() const { return mbox_at(N); }
+    uint64_t claim_word() const { return claim_at(N); }
+    uint64_t phase_word() const { return phase_at(N); }
     // Moves nsrc tables of n words into dst with k_stage_words (launch accounting as stage_words);
     // returns the number of completion increments when `done` is given.
     uint32_t stage(uint32_t* dst, const uint32_t* const* srcs, uint32_t nsrc, uint64_t n, unsigned int* done) {
@@ -1170,7 +1176,7 @@ struct Prover {
         block = static_cast<char*>(p);
         ws.plan(block, C, N, R, own_input, sumcheck);
         ck(cudaMemsetAsync(block + ws.zero_off, 0, ws.zero_bytes, c.stream), "cudaMemsetAsync");
-        c.ensure_mapped(9ull * N * 4, mapped_words() * 4);
+        c.ensure_mapped(9ull * N * 4, mapped_words(N) * 4);
         c.resync_done();
         // no word a persistent phase publishes has its first parity yet
         memset(mapped(false, phase_word()), 0, 15ull * N * 4);
@@ -1662,6 +1668,10 @@ struct Prover {
         c.resolve_events();
     }
 };
+
+static_assert(4 * 9 * kMappedCopies <= kMinMapped / 4 &&
+                  4 * Prover::mapped_words(kMappedCopies) <= kMinMapped - kMinMapped / 4,
+              "a lane's first staging block is too small for kMappedCopies copies");
 
 #include "bn254_prover.cuh"
 #include "verifier.cuh"
