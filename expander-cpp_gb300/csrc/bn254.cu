@@ -1456,8 +1456,6 @@ int phase_ctas_per_sm() {
         const size_t most = phase_smem(lane_hg != 0, kPhaseRows / 2);
         int n = 0;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kPhaseBlock, most);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -1469,7 +1467,7 @@ int phase_ctas_per_sm() {
     return least;
 }
 
-cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s) {
+cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, bool dense, cudaStream_t s) {
     if (a.k0 >= a.n || a.n - a.k0 > kMboxRounds || a.N < 1) return cudaErrorInvalidValue;
     // rows of the first round's source tables; with k0 = 0 the layer input itself
     if ((1ull << (a.n - (a.k0 ? a.k0 - 1 : 0))) > kPhaseRows) return cudaErrorInvalidValue;
@@ -1478,11 +1476,22 @@ cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s) {
     if (phase_ctas_per_sm() < 1) return cudaErrorInvalidConfiguration;
     const uint32_t kf = a.k0 ? a.k0 : 1, S1 = 1u << (a.n - kf);
     const size_t smem = phase_smem(lane_hg, S1);
-    if (lane_hg)
-        k_phase<true><<<a.N, kPhaseBlock, smem, s>>>(a);
-    else
-        k_phase<false><<<a.N, kPhaseBlock, smem, s>>>(a);
-    return cudaGetLastError();
+    auto* const kernel = lane_hg ? k_phase<true> : k_phase<false>;
+    if (!dense) {
+        kernel<<<a.N, kPhaseBlock, smem, s>>>(a);
+        return cudaGetLastError();
+    }
+    cudaLaunchAttribute split;
+    split.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    split.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.N);
+    cfg.blockDim = dim3(kPhaseBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &split;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
 cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g, const Fr* my_c, const EqArgsBn& eqc,

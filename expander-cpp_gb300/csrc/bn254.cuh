@@ -115,7 +115,8 @@ struct PhaseArgsBn {
     unsigned int* err;
     unsigned long long wait_ns;
 };
-cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, cudaStream_t s);
+// dense: more CTAs than SMs, for which the launch asks for the largest shared-memory part of an SM.
+cudaError_t launch_phase(bool lane_hg, const PhaseArgsBn& a, bool dense, cudaStream_t s);
 int phase_ctas_per_sm();  // as the M31 kernels' (kernels.cuh)
 cudaError_t launch_wsum(const uint32_t* vals, const EqArgsBn& eq, const GeoBn& g, uint32_t ctas, RedBn red,
                         uint32_t* out, cudaStream_t s);

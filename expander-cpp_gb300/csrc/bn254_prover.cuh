@@ -222,8 +222,8 @@ struct BnProver {
     // other phases hold the device.
     bool run_phase(Transcript& t, bool lane_hg, bn::PhaseArgsBn a, frh::Fr* rch, bool append_last, uint32_t* last_mont,
                    uint32_t* last_canon, double bytes) {
-        PhaseSlots slots(X.device, X.sm_count);
-        if (!slots.acquire((int)N, true)) return false;
+        DevicePhaseSlots slots(X.device, X.sm_count);
+        if (!slots.acquire(N, true)) return false;
         a.N = N;
         a.fA = ws.fA;
         a.fB = ws.fB;
@@ -250,12 +250,13 @@ struct BnProver {
                 std::atomic_thread_fence(std::memory_order_seq_cst);
             }
         } abort{mb};
-        c.launch(K_BN_PHASE, bytes, [&] { return bn::launch_phase(lane_hg, a, c.stream); });
+        c.launch(K_BN_PHASE, bytes, [&] { return bn::launch_phase(lane_hg, a, N > (uint32_t)X.sm_count, c.stream); });
         c.phase_err = err_h();
         const uint32_t* out = mapped(false, phase_word());
         for (uint32_t k = a.k0; k < a.n; k++) {
             c.ev_parity = (a.parity ^ (k - a.k0)) & 1u;
             c.collect_digits(out, 3ull * N, c.ev_parity, t.tail());
+            if (k == a.k0) slots.placed();
             t.appended(3 * rowb());
             if (k + 1 < a.n) {
                 rch[k] = t.challenge_bn254();

@@ -257,10 +257,8 @@ cudaError_t launch_s_build(uint64_t I, const uint32_t* my_off, const uint4* my_g
                            uint32_t* s_out, uint32_t* t_out, uint64_t s_stride, cudaStream_t s);
 // CTAs of a persistent phase for N copies at tpr quads a CTA, and the launch.
 uint32_t phase_ctas(uint32_t N, uint32_t tpr);
-// CTAs of persistent phases an SM of the current device holds at once, whichever launches they are
-// of (0: none).  The kernels ask for the largest shared-memory part of an SM: with the split that
-// suits a launch alone, CTAs of 97 KB did not start on SMs that held one of 26 KB, nor ones of 50 KB
-// beside 97, until those had ended, and a phase's CTAs end only once all of them have started.
+// CTAs that an SM of the current device holds of the largest of the persistent phases' kernels (0:
+// none); see phase_slots.hpp.
 int phase_ctas_per_sm();
 // Quads a CTA's tables take when the first round reads `items` rows x tpr.
 size_t phase_priv_quads(uint64_t items);

@@ -46,6 +46,7 @@
 #include "fr_host.hpp"
 #include "kernels.cuh"
 #include "m31.cuh"
+#include "phase_slots.hpp"
 #include "sha256.hpp"
 #include "transcript.hpp"
 
@@ -945,35 +946,16 @@ EqArgs eq_args(int reps, const uint32_t (*r1)[32], const uint32_t (*r2)[32], uin
 }
 
 // ------------------------------------------------------------------ persistent phase slots
-// The CTAs of a persistent phase wait for their host thread, which waits for all of them, so
-// all must be resident at once: a phase runs only while the CTAs of all running ones (every
-// context and lane of the process) stay within what the device holds of the largest of them
-// (phase_ctas_per_sm: two to an SM, so that each takes at most half of one), and otherwise the
-// rounds are launched one by one.  Other kernels only delay a phase: they end by themselves.
-class PhaseSlots {
-   public:
-    // (`device` is the current one)
-    PhaseSlots(int device, int sm_count)
-        : used_(counter(device)), cap_(sm_count * std::min(phase_ctas_per_sm(), bn::phase_ctas_per_sm())) {}
-    ~PhaseSlots() { used_ -= held_; }
-    int capacity() const { return cap_; }
-    // n more CTAs; beyond a lane's own share of the device only while half of it stays free.
-    bool acquire(int n, bool own_share) {
-        if (used_.fetch_add(n) + n > (own_share ? cap_ : cap_ / 2)) {
-            used_ -= n;
-            return false;
-        }
-        held_ += n;
-        return true;
-    }
+// The slots of a phase on the current device `dev` of `sms` SMs.
+struct DevicePhaseSlots : PhaseSlots {
+    DevicePhaseSlots(int dev, int sms)
+        : PhaseSlots(state(dev), sms, std::min(phase_ctas_per_sm(), bn::phase_ctas_per_sm())) {}
 
    private:
-    static std::atomic<int>& counter(int device) {
-        static std::atomic<int> used[64];
-        return used[device & 63];
+    static std::atomic<uint64_t>& state(int dev) {
+        static std::atomic<uint64_t> states[64];
+        return states[dev & 63];
     }
-    std::atomic<int>& used_;
-    int cap_, held_ = 0;
 };
 
 // ------------------------------------------------------------------ prover
@@ -1010,10 +992,10 @@ struct Prover {
     // the device, or among small ones, takes more than its lane's share.
     uint32_t claim(PhaseSlots& slots, uint64_t rows, uint64_t items) const {
         if (!X.round_tail) return 0;
-        const uint32_t share = std::max(1u, (uint32_t)slots.capacity() / (uint32_t)X.n_lanes);
+        const uint32_t share = std::max(1u, slots.capacity() / (uint32_t)X.n_lanes);
         for (uint32_t tpr = 1; tpr <= 32 && rows * tpr <= items; tpr *= 2) {
             const uint32_t ctas = phase_ctas(N, tpr);
-            if (ctas <= kPhaseCtas && slots.acquire((int)ctas, ctas <= share)) return tpr;
+            if (ctas <= kPhaseCtas && slots.acquire(ctas, ctas <= share)) return tpr;
         }
         return 0;
     }
@@ -1069,10 +1051,10 @@ struct Prover {
     template <class Prepare>
     uint32_t run_phase(Transcript& t, bool lane_hg, PhaseArgs a, uint32_t (*rch)[32], bool append_last, uint32_t* last_out,
                        double bytes, uint32_t tile, Prepare&& prepare) {
-        PhaseSlots slots(X.device, X.sm_count);
+        DevicePhaseSlots slots(X.device, X.sm_count);
         const uint64_t rows = 1ull << (a.n - (a.k0 ? a.k0 - 1 : 0));
         if (tile)
-            a.tpr = slots.acquire((int)phase_ctas(N, tile), true) ? tile : 0;
+            a.tpr = slots.acquire(phase_ctas(N, tile), true) ? tile : 0;
         else
             a.tpr = claim(slots, rows, a.k0 ? kPhaseTailItems : kPhaseItems);
         if (!a.tpr) return 0;
@@ -1113,6 +1095,7 @@ struct Prover {
             c.ev_parity = par;
             if (k + 1 < a.n) {
                 c.collect(src, 3ull * R * N, par, t.tail());
+                if (k == a.k0) slots.placed();
                 uint32_t r[3];
                 t.challenge_each(12ull * N, R, r);
                 for (int j = 0; j < R; j++) {
@@ -2316,7 +2299,7 @@ int gkrgpu_check_device_wait(gkrgpu_ctx* ctx, uint32_t timeout_us, int* expired,
         if (timeout_us < 1 || timeout_us > 10u * 1000 * 1000) fail(GKRGPU_ERR_INVALID, "timeout_us must be in [1, 10^7]");
         on_idle_lane(ctx, [&](Lane& c) {
             // a two-round phase over 8 x 4 tables whose second round's challenge is never written
-            PhaseSlots slots(ctx->device, ctx->sm_count);  // (other contexts' phases end by themselves)
+            DevicePhaseSlots slots(ctx->device, ctx->sm_count);  // (other contexts' phases end by themselves)
             if (slots.capacity() < 1) fail(GKRGPU_ERR_CUDA, "no persistent phase fits on the device");
             while (!slots.acquire(1, true)) std::this_thread::sleep_for(std::chrono::microseconds(100));
             const uint32_t N = 4, n = 3;

@@ -24,7 +24,7 @@ if platform.machine() in ("aarch64", "arm64"):
 
 SOURCES = ["kernels.cu", "phase.cu", "prover.cu", "sha256.cpp", "noalloc.cu", "bn254.cu", "circuit2.cpp", "keccak.cpp"]
 HEADERS = ["kernels.cuh", "m31.cuh", "sha256.hpp", "transcript.hpp", "bn254.cuh", "bn254_prover.cuh", "fr_host.hpp",
-           "verifier.cuh", "keccak.hpp"]
+           "verifier.cuh", "keccak.hpp", "phase_slots.hpp"]
 
 
 def _deps():

@@ -3,9 +3,6 @@ exactly, just over and far over the rows a CTA takes, one-row-pair layers, copy 
 leave part of the last CTA idle (516 = 4 * 129 at two quads a CTA), that need wide CTAs (4096)
 and that are beyond the widest (20000, every round launched alone).  The proof bytes equal the
 oracle's and those with the phases off (exact arithmetic: tolerance zero)."""
-import os
-import subprocess
-
 import numpy as np
 import pytest
 
@@ -179,28 +176,39 @@ def test_phases_whose_finishers_are_in_several_warps(ctx, oracle, seed, widths, 
     assert proof == op and np.array_equal(cv, ocv)
 
 
-@pytest.fixture(scope="module")
-def side_by_side(tmp_path_factory):
-    from gkr_gb300 import build as libbuild
-    objs = [os.path.join(libbuild.OBJ, f + ".o") for f in ("phase.cu", "bn254.cu")]
-    libbuild.build(force=not all(os.path.exists(o) for o in objs))
-    exe = str(tmp_path_factory.mktemp("phases") / "phases_side_by_side")
-    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "adapter", "phases_side_by_side.cu")
-    subprocess.check_call([libbuild.NVCC, *libbuild.ARCH, "-std=c++17", "-I", libbuild.CSRC, "-I", libbuild.INCLUDE, src,
-                           *objs, "-o", exe])
-    return exe
+@pytest.mark.parametrize("copies", [1, 152, 153, 304])
+def test_bn254_phases_of_up_to_two_ctas_an_sm(copies):
+    # a CTA a copy: from 153 on more of them than SMs (with a split of an SM's memory that holds two)
+    from gkr_gb300.prover import Context
+    from oracle.oracle import OracleBn254
+    ctx = Context(0)
+    circ = gc.random_circuit(695, [11, 3, 2], p_mul=0.6)
+    w = gc.random_witness_bn254(695, circ.log_input_size, copies)
+    proof = ctx.prove(ctx.load(circ, "BN254"), w)[1]
+    assert ctx.kernel_stats()["bn254_phase"]["launches"] == 4
+    ctx.close()
+    assert proof == OracleBn254().prove(circ, w)[1]
 
 
-@pytest.mark.parametrize("first,second", [
-    # M31 phase two with 25 and 99 KB a CTA, M31 phase one with 50, BN254 with 57 (phase two) and 16
-    ((0, 3), (0, 13)), ((0, 13), (0, 3)), ((0, 13), (1, 13)), ((1, 13), (0, 13)), ((0, 13), (0, 13)), ((2, 11), (0, 13)),
-    ((0, 13), (2, 11)), ((3, 11), (0, 13)), ((0, 3), (2, 11)),
-])
-def test_admitted_phases_are_resident_together(side_by_side, first, second):
-    # a phase's CTAs end only once all of them have started: those of two phases of one CTA an SM must
-    # start beside each other whatever memory each takes
-    out = subprocess.run([side_by_side, *[str(x) for x in first + second]], capture_output=True, text=True, timeout=60)
-    assert out.returncode == 0, out.stdout + out.stderr
+def test_phases_of_both_fields_together(oracle):
+    # two contexts whose phases would take several times the device: CTAs of 16 to 98 KB
+    from gkr_gb300.prover import Context
+    from oracle.oracle import OracleBn254
+    jobs = []
+    for field, lanes, widths, n, count in (("M31", 16, [13, 12, 9], 64, 48), ("BN254", 6, [11, 9, 10], 96, 24)):
+        ctx = Context(0)
+        ctx.set_concurrency(lanes)
+        circ = gc.random_circuit(696, widths, p_mul=0.6)
+        make = gc.random_witness if field == "M31" else gc.random_witness_bn254
+        w = make(696, circ.log_input_size, n)
+        want = (oracle if field == "M31" else OracleBn254()).prove(circ, w)[1]
+        dc = ctx.load(circ, field)
+        for _ in range(count):
+            pb = np.empty(dc.proof_size(n), np.uint8)
+            cb = np.empty((3, n), np.uint32) if field == "M31" else np.empty((1, n, 4), np.uint64)
+            jobs.append((ctx, ctx.submit(dc, w, pb, cb), pb, want))
+    for ctx, job, pb, want in jobs:
+        assert pb[:ctx.wait(job)].tobytes() == want
 
 
 @pytest.mark.parametrize("seed,widths,n", [(691, [3, 2, 3, 1, 2, 1], 512), (692, [7, 3, 2, 6], 512)])
