@@ -260,8 +260,8 @@ uint32_t phase_ctas(uint32_t N, uint32_t tpr);
 // CTAs that an SM of the current device holds of the largest of the persistent phases' kernels (0:
 // none); see phase_slots.hpp.
 int phase_ctas_per_sm();
-// Quads a CTA's tables take when the first round reads `items` rows x tpr.
-size_t phase_priv_quads(uint64_t items);
+// Quads a CTA's tables take when the first round reads `items` rows x tpr; whole: with k0 = 0.
+size_t phase_priv_quads(uint64_t items, bool whole);
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s);
 // The layer input (I rows) and hg in the tables of a phase-one launch with k0 = 0: with a4 from
 // the stored weights a4, w4 (launch_weights), without it from eqc.

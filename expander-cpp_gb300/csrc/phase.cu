@@ -409,14 +409,14 @@ int phase_ctas_per_sm() {
     return least;
 }
 
-size_t phase_priv_quads(uint64_t items) { return items * 4 + items / 2 * 6 + items / 4 * 6; }
+size_t phase_priv_quads(uint64_t items, bool whole) { return (whole ? items * 4 : 0) + items / 2 * 6 + items / 4 * 6; }
 
 cudaError_t launch_phase(bool lane_hg, const PhaseArgs& a, cudaStream_t s) {
     if (a.reps < 1 || a.reps > 3 || a.k0 >= a.n || a.n - a.k0 > kMboxRounds || a.N % 4) return cudaErrorInvalidValue;
     if (a.tpr < 1 || a.tpr > 32 || (a.tpr & (a.tpr - 1))) return cudaErrorInvalidValue;
     // rows of the first round's source tables; with k0 = 0 the layer input itself
     const uint64_t rows = 1ull << (a.n - (a.k0 ? a.k0 - 1 : 0));
-    if (rows * a.tpr > kPhaseItems || !a.priv || a.priv_stride < phase_priv_quads(rows * a.tpr)) return cudaErrorInvalidValue;
+    if (rows * a.tpr > kPhaseItems || !a.priv || a.priv_stride < phase_priv_quads(rows * a.tpr, a.k0 == 0)) return cudaErrorInvalidValue;
     if (a.two && a.k0 < 2) return cudaErrorInvalidValue;
     if (a.k0 && (!a.fsrc[0] || (lane_hg && !a.hsrc[0]))) return cudaErrorInvalidValue;
     if (!lane_hg && (!a.vx || !a.s[0])) return cudaErrorInvalidValue;

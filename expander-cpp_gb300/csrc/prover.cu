@@ -879,6 +879,22 @@ struct Workspace {
     size_t sstride = 0;
     size_t total = 0;
 
+    // Quads of the phases' own tables.  The row tile of a phase, and whether a small layer's run
+    // whole, is settled when it starts: room for any.  (A phase that starts late reads a quarter of
+    // a layer's rows at most.)
+    static size_t phase_quads(const gkrgpu_circuit& C, uint32_t N) {
+        size_t quads = 0;
+        for (uint32_t tpr = 1; tpr <= 32; tpr *= 2) {
+            const size_t ctas = phase_ctas(N, tpr);
+            if (ctas > kPhaseCtas) continue;
+            for (size_t l = 0; l < C.layers.size(); l++) {
+                const uint64_t items = C.in_rows(l) * tpr;
+                if (items <= kPhaseItems) quads = std::max(quads, ctas * phase_priv_quads(items, true));
+                quads = std::max(quads, ctas * phase_priv_quads(std::min<uint64_t>(items / 4, kPhaseTailItems), false));
+            }
+        }
+        return quads;
+    }
     // Lays the parts out from `base` (null: only sizes the block).
     void plan(char* base, const gkrgpu_circuit& C, uint32_t N, int R, bool own_input, bool sumcheck) {
         size_t o = 0;
@@ -898,12 +914,7 @@ struct Workspace {
                 fA[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 2, 1) * rowb);
                 fB[j] = (uint32_t*)take(std::max<uint64_t>(maxI / 4, 1) * rowb);
             }
-            // the row tile of a phase is chosen when it starts: room for any
-            size_t quads = 0;
-            for (uint32_t tpr = 1; tpr <= 32; tpr *= 2)
-                if (phase_ctas(N, tpr) <= kPhaseCtas)
-                    quads = std::max(quads, phase_ctas(N, tpr) * phase_priv_quads(std::min<uint64_t>(maxI * tpr, kPhaseItems)));
-            priv = (uint4*)take(quads * 16);
+            priv = (uint4*)take(phase_quads(C, N) * 16);
             sstride = align_up(maxI, 64);
             sb[0] = (uint32_t*)take(R * sstride * 4);
             sb[1] = (uint32_t*)take(R * sstride * 4);
@@ -1059,7 +1070,7 @@ struct Prover {
             a.tpr = claim(slots, rows, a.k0 ? kPhaseTailItems : kPhaseItems);
         if (!a.tpr) return 0;
         a.priv = ws.priv;
-        a.priv_stride = phase_priv_quads(rows * a.tpr);
+        a.priv_stride = phase_priv_quads(rows * a.tpr, a.k0 == 0);
         prepare(a.tpr, a.priv_stride);
         for (int j = 0; j < R; j++) {
             a.r_first[j] = a.k0 ? rch[j][a.k0 - 1] : 0u;
@@ -2303,7 +2314,7 @@ int gkrgpu_check_device_wait(gkrgpu_ctx* ctx, uint32_t timeout_us, int* expired,
             if (slots.capacity() < 1) fail(GKRGPU_ERR_CUDA, "no persistent phase fits on the device");
             while (!slots.acquire(1, true)) std::this_thread::sleep_for(std::chrono::microseconds(100));
             const uint32_t N = 4, n = 3;
-            const size_t tb = 8 * N * 4, priv = phase_priv_quads(8);
+            const size_t tb = 8 * N * 4, priv = phase_priv_quads(8, false);
             void* p = nullptr;
             ck(cudaMallocFromPoolAsync(&p, 2 * tb + 16 * priv, ctx->pool, c.stream), "workspace allocation");
             struct Free {

@@ -89,3 +89,34 @@ def test_autotune_picks_tiles_and_keeps_bytes(fresh_ctx):
         assert choice[k]["ms"] > 0
     after = fresh_ctx.prove(dc, w)[1]
     assert before == after
+
+
+
+def _phase_bytes(widths, n):
+    """Tables of the persistent phases: the most, over the row tiles, that its CTAs hold of a layer:
+    8.5 elements an item (rows x quads a CTA) of a phase that runs whole, up to 8192 items, and 4.5 of
+    one that starts at a quarter of the rows or later, up to 4096."""
+    most = 0
+    for tile in (1, 2, 4, 8, 16, 32):
+        ctas = -(-(n // 4) // tile)
+        for rows in (1 << w for w in widths[:-1]):
+            late = 4.5 * min(rows // 4 * tile, 4096)
+            items = max(late, 8.5 * rows * tile if rows * tile <= 8192 else 0)
+            most = max(most, ctas * items if ctas <= 128 else 0)
+    return int(16 * most)
+
+
+@pytest.mark.parametrize("widths,n", [
+    # layers too large for whole phases, at one, two and 32 quads a CTA; the largest that are not; both
+    ([16, 16], 64), ([15, 14], 1024), ([14, 3], 16384), ([13, 13], 64), ([15, 5, 15], 512), ([2, 1], 16384),
+])
+def test_phases_reserve_what_they_can_use(fresh_ctx, widths, n):
+    from gkr_gb300 import _lib
+    circ = gc.random_circuit(711, widths, p_mul=0.6)
+    dc = fresh_ctx.load(circ)
+    big, row = 1 << max(widths[:-1]), 4 * n
+    rest = row * (sum(1 << w for w in widths) + 3 * (2 * max(big // 4, 1) + 2 * (big // 2)))  # values; hg, f
+    rest += 24 * max(big, 64) + 16 * big + 32 * max(max(len(l.mul) for l in circ.layers), 1)  # scalars; weights
+    rest += row * (27 + 9 + 3 + 3 + 54)  # sums, evaluations, claims
+    got = _lib.load().gkrgpu_workspace_bytes(dc.handle, n, 10, 0)
+    assert rest <= got <= rest + _phase_bytes(widths, n) + (1 << 14)
