@@ -207,6 +207,7 @@ struct BnProver {
     void fetch(uint32_t groups, const uint32_t* rows_from) {
         const uint32_t more = rows_from ? stage(mapped(true, 0), rows_from, 16ull * N, c.done_d()) : 0u;
         c.wait_done(groups + more);
+        c.came_back((rows_from ? 5 : 3) * rowb());
     }
 
     // First round of a phase's persistent part, n if it has none (as the M31 prover's): a CTA a
@@ -258,6 +259,7 @@ struct BnProver {
             c.collect_digits(out, 3ull * N, c.ev_parity, t.tail());
             if (k == a.k0) slots.placed();
             t.appended(3 * rowb());
+            c.came_back((k + 1 < a.n ? 3 : 5) * rowb());
             if (k + 1 < a.n) {
                 rch[k] = t.challenge_bn254();
                 uint32_t w[8], d[9];
@@ -482,6 +484,7 @@ struct BnProver {
         c.sync();
         require_canonical();
         memcpy(claimed_v, mapped(false, 16ull * N), rowb());
+        c.came_back(rowb());
         cv1.assign(claimed_v, claimed_v + (size_t)N * 8);
         cv2.assign((size_t)N * 8, 0u);
 

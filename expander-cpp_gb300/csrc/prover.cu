@@ -440,6 +440,8 @@ struct Lane {
         }
     }
     void copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind, const char* what);
+    // n bytes of results that kernels have written into mapped host memory
+    void came_back(uint64_t n);
 };
 
 // ------------------------------------------------------------------ context
@@ -666,6 +668,8 @@ void Lane::copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind, const
     if (kind == cudaMemcpyHostToDevice) X->h2d_bytes += n;
     if (kind == cudaMemcpyDeviceToHost) X->d2h_bytes += n;
 }
+
+void Lane::came_back(uint64_t n) { X->d2h_bytes += n; }
 
 namespace {
 
@@ -1104,6 +1108,7 @@ struct Prover {
         for (uint32_t k = a.k0; k < a.n; k++) {
             const uint32_t *src = mapped(false, phase_word()), par = (a.parity ^ (k - a.k0)) & 1u;
             c.ev_parity = par;
+            c.came_back(4ull * (k + 1 < a.n ? 3 : 5) * R * N);
             if (k + 1 < a.n) {
                 c.collect(src, 3ull * R * N, par, t.tail());
                 if (k == a.k0) slots.placed();
@@ -1228,6 +1233,7 @@ struct Prover {
             more = stage(mapped(true, 0), srcs, (uint32_t)R, 2ull * N, c.done_d());
         }
         c.wait_done(groups + more);
+        c.came_back(4ull * (rows_from ? 5 : 3) * R * N);
     }
 
     // Transcript step of one round for every repetition (sumcheck.hpp:74-96).  With
@@ -1625,6 +1631,7 @@ struct Prover {
         c.sync();
         require_canonical();
         memcpy(claimed_v, cv_h(), R * rowb);
+        c.came_back(R * rowb);
         cv1.assign(claimed_v, claimed_v + (size_t)R * N);
         cv2.assign((size_t)R * N, 0u);
 
@@ -2289,6 +2296,7 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
             c.pending_bytes = 0;  // spin: the caller's thread may not sleep to the microsecond
             c.wait_done(wsum_groups(a, g));
             memcpy(out, c.extra_h(), n_points * rowb);
+            c.came_back(n_points * rowb);
             if (ctx->timing) c.sync();  // the launch's closing event
             c.resolve_events();
         });

@@ -212,6 +212,7 @@ struct Verifier {
         raw_pc_eval(rz2, 1);
         c.sync();
         std::atomic_thread_fence(std::memory_order_acquire);
+        c.came_back(4ull * R * (2 * L + 2ull * N));
         for (size_t li = 0; li < L && ok; li++) {
             const uint32_t *a = mapped(false, sums_word(li, false)), *m = mapped(false, sums_word(li, true));
             const Pending& pd = pending[li];

@@ -323,7 +323,8 @@ int gkrgpu_autotune(gkrgpu_ctx* ctx, const gkrgpu_circuit* circuit, uint32_t n_c
 int gkrgpu_mark(gkrgpu_ctx* ctx, int slot);
 int gkrgpu_elapsed_ms(gkrgpu_ctx* ctx, int from_slot, int to_slot, double* ms);
 
-/* Bytes the library copied host->device and device->host since the last reset. */
+/* Bytes the library copied host->device since the last reset, and device->host, the results that
+ * kernels write into mapped host memory among them. */
 int gkrgpu_transfer_stats(gkrgpu_ctx* ctx, uint64_t* h2d_bytes, uint64_t* d2h_bytes);
 
 /* Proof files in the reference's format, Proof::write_and_compress / read_proof

@@ -108,6 +108,7 @@ struct Lane {
     void copy(void*, const void*, size_t, cudaMemcpyKind, const char*) { in_flight++; }
     void sync() { in_flight = 0; }
     void resolve_events() {}
+    void came_back(uint64_t) {}
 };
 EqArgs eq_args(int, const uint32_t (*)[32], const uint32_t (*)[32], uint32_t, uint32_t, uint32_t) { return EqArgs{}; }
 bn::EqArgsBn eq_args_bn(const frh::Fr*, const frh::Fr*, const frh::Fr&, const frh::Fr&, uint32_t) { return bn::EqArgsBn{}; }
