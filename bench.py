@@ -78,7 +78,7 @@ def parse():
     ap.add_argument("--no-keccak", action="store_true", help="plain: skip the Keccak-256 transcript rate")
     ap.add_argument("--no-parity", action="store_true", help="plain: skip the golden and verifier checks")
     ap.add_argument("--no-round-tail", action="store_true",
-                    help="plain: every sumcheck round as its own launch (no persistent phase tails)")
+                    help="plain: every sumcheck round as its own launch (no persistent phases)")
     ap.add_argument("--rates", default="200,500,1000,2000", help="serve: arrival rates (requests/s)")
     ap.add_argument("--duration", type=float, default=4.0, help="serve: seconds of arrivals per rate")
     ap.add_argument("--serve-size", choices=["mixed", "config2"], default="mixed",
@@ -670,7 +670,7 @@ def measure_mixed(device, n_proofs, lanes, budget, seed=3, host_threads=0):
             done.append((time.perf_counter() - sub[i]) * 1000.0)
         return time.perf_counter() - t0, done
 
-    # the same batch with every round as its own launch (no persistent phase tails)
+    # the same batch with every round as its own launch (no persistent phases)
     ctx.set_round_tail(False)
     notail_s, _ = one_batch()
     same_notail = ms.digests(idx) == ref
@@ -691,7 +691,7 @@ def measure_mixed(device, n_proofs, lanes, budget, seed=3, host_threads=0):
                      "latency_ms": {"p50": statistics.median(lat_plain), "p99": float(np.percentile(lat_plain, 99))}},
            "batched_over_plain": plain_s / batch_s, "byte_identical_to_plain": same,
            "batched_per_round_launches": {"proofs_per_s": n / notail_s, "seconds": notail_s,
-                                          "note": "the same batch with the persistent phase tails off: every "
+                                          "note": "the same batch with the persistent phases off: every "
                                                   "sumcheck round its own kernel launch"},
            "host_threads": host_threads or "default",
            "hbm": {"workspace_peak_bytes": mem["peak"], "budget": mem["budget"]}, "clocks": clk}

@@ -254,7 +254,7 @@ __device__ __forceinline__ Wide lift(const Fr& x) {
 // pairs of each: to e from word i + (i & 1) on, to o from word i + 1 - (i & 1) on.  The rows that
 // end on a pair not used before leave no carry; the others' carry starts the next pair.
 __device__ __forceinline__ void mac(Wide& s, const Fr& a, const Fr& b) {
-    uint32_t e[16], o[18];  // o[k]: word k + 1... kept at its own word, o[0] unused
+    uint32_t e[16], o[18];  // a word at its own index (o[0] unused, o[16] and o[17] zero)
 #pragma unroll
     for (int k = 0; k < 16; k++) e[k] = 0u;
 #pragma unroll
@@ -349,7 +349,7 @@ __device__ __forceinline__ void mac(Wide& s, const Fr& a, const Fr& b) {
 }
 
 // s 2^-256 mod r: the low half's Montgomery reduction (mul's steps without its products), at
-// most r, plus the high half, below 4 r together.
+// most r, plus the high half, below 2.9 r (s < 15.3 r^2, and r < 0.19 2^256): below 4 r together.
 __device__ __forceinline__ Fr reduce(const Wide& s) {
     uint32_t x[8], y[8];
 #pragma unroll

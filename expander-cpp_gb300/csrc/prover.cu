@@ -192,7 +192,7 @@ struct gkrgpu_circuit {
     int device = 0;
     int field = GKRGPU_FIELD_M31;
     std::vector<DevLayer> layers;
-    uint32_t max_in_vars = 0, max_out_vars = 0;
+    uint32_t max_in_vars = 0;
     uint64_t max_mul = 0;
     ~gkrgpu_circuit() {
         for (auto& l : layers)
@@ -2133,7 +2133,6 @@ int gkrgpu_circuit_load_field(gkrgpu_ctx* ctx, const gkrgpu_layer_desc* layers, 
             for (int l = 0; l < n_layers; l++) {
                 c->layers.push_back(upload_layer(layers[l], field));
                 c->max_in_vars = std::max(c->max_in_vars, layers[l].nb_input_vars);
-                c->max_out_vars = std::max(c->max_out_vars, layers[l].nb_output_vars);
                 c->max_mul = std::max<uint64_t>(c->max_mul, layers[l].n_mul);
             }
         } catch (...) {

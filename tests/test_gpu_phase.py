@@ -1,7 +1,8 @@
 """GPU tests of the persistent sumcheck phases at the edges of their rule and tiles: layers of
 exactly, just over and far over the rows a CTA takes, one-row-pair layers, copy counts that
-leave part of the last CTA idle (516 = 4 * 129 at two quads a CTA), that need wide CTAs (4096)
-and that are beyond the widest (20000, every round launched alone).  The proof bytes equal the
+leave part of the last CTA idle (516 = 4 * 129 at two quads a CTA), that need CTAs of 8 quads
+(4096), 16 (4100 to 8192) and 32 (to 16384), and that are beyond the widest (20000, every round
+launched alone).  The proof bytes equal the
 oracle's and those with the phases off (exact arithmetic: tolerance zero)."""
 import numpy as np
 import pytest
