@@ -6,7 +6,7 @@
 //   device : input -> Circuit::evaluate of every layer, kept resident for the sumcheck
 //   device : claimed_v = eval_multilinear(output, rz1_j) for every repetition j
 //   per layer, top down, per sumcheck_prove_gkr_layer (include/LinearGKR/sumcheck.hpp:52-111):
-//     device : eq tables, gate weights, hg build fused with round 0
+//     device : gate weights (with their eq factors), hg build fused with round 0
 //     rounds : device fold+reduce for all repetitions -> 3R rows to the host -> the host
 //              appends them and derives the R challenges in the reference's order
 //     phase 2: s(y) table, rounds over the layer input with h = v(rx) * s
@@ -1271,7 +1271,7 @@ struct Prover {
         uint32_t* v = vals[li];
         uint32_t* vxh = vx_h();
         // round 0's claims, alpha v(rz1) + beta v(rz2) per repetition and copy
-        // (sumcheck.hpp:129-132), while the eq table and the weights are computed
+        // (sumcheck.hpp:129-132), while the weights are computed
         {
             uint32_t* cl = mapped(false, claim_word());
             for (uint64_t i = 0; i < RN; i++) cl[i] = m31::add(m31::mul(alpha, cv1[i]), m31::mul(beta, cv2[i]));

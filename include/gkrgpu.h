@@ -245,7 +245,7 @@ int gkrgpu_eval_multilinear(gkrgpu_ctx* ctx, const uint32_t* d_evals, uint32_t n
  * Same result as gkrgpu_eval_multilinear, but the output d_out is a caller-owned device
  * buffer of n_points x n_copies u32 and no context is needed: the work runs on `stream`
  * (a cudaStream_t; NULL = the legacy default stream) of the current device and the call
- * returns when it has finished.  Its scratch is a fixed 3.1 MiB region inside the library
+ * returns when it has finished.  Its scratch is a fixed 100 KiB region inside the library
  * (held by every GPU that loads the library until the process exits), so the limits are
  * nb_vars <= 18, n_copies <= 4096 (a multiple of 4) and n_points <= 3; larger sizes are
  * rejected with GKRGPU_ERR_INVALID.  The first call on a device looks up the scratch
